@@ -3,13 +3,15 @@
 // 4 x 64-bit representation (crates/field/src/lib.rs:30-36, 321), so a
 // caller's `&[Fr]` crosses the C ABI with no conversion.
 //
-// The multiply is CIOS on the integer multiply pipe: per limb of b, one row of
-// 32x32->64 products (mul.wide) accumulates a*b_i and one accumulates m*p,
-// 136 wide products a multiply, then one conditional subtraction. With
-// a, b < m < 2^254 the accumulator stays below 2m < 2^255 between limbs and
-// below 2^288 inside one, so nine 32-bit words always hold it. (Measured on
-// GB300: 47 G products/s against 38 G/s for the same CIOS written as
-// mad.lo/mad.hi carry chains, which issue two multiplies per partial product.)
+// The multiply is bound by the integer multiply pipe: 136 partial products of
+// 32x32->64 bits, each one wide multiply-add with carry, which the pipe takes
+// at half the rate of a 32-bit one (measured on a GB300: 31 of 64 lanes a
+// clock and SM; a wide multiply-add into a 64-bit sum without carries, the
+// form limbs of 29 bits allow, 20, and 81 + 81 of those in nine limbs 48 G
+// products/s). So a row's products are laid out as two carry chains of four
+// (fe_mul below): 72 G products/s against 50 for rows of 64-bit sums with the
+// carry added by separate instructions, 0.98 of what the pipe's rate allows,
+// and 847 against 1187 clocks for one product alone.
 #pragma once
 #include <cstdint>
 
@@ -169,101 +171,347 @@ __device__ __forceinline__ Fe<C> fe_dbl(const Fe<C>& a) {
   return fe_add(a, a);
 }
 
-// One CIOS row per limb of b with 32x32->64 products (mul.wide): t += a*b_i,
-// m = t0 * inv, t = (t + m*p) >> 32. Each 64-bit step adds one product, one
-// word of t and the previous carry, which cannot overflow:
-// (2^32-1)^2 + 2(2^32-1) = 2^64 - 1.
+// ---- products ------------------------------------------------------------------
+//
+// A value T is held as two arrays of eight words, T = E + 2^32 O: every
+// partial product of limb j and a multiplier lands in words (j, j + 1), so
+// the products of the even limbs fill E in one chain of four wide
+// multiply-adds with carry, those of the odd limbs fill O, and neither chain
+// needs a carry beyond its own words (T stays below 2^288 within a row). The
+// low and the high half of a product are consecutive instructions on
+// consecutive words, which is what lets them run as one wide instruction.
+//
+// A Montgomery row adds a b_i, then m p with m = -E_0 p^-1 mod 2^32, which
+// clears E_0; dividing by 2^32 then makes O the next row's E (its words now
+// stand at 0..7), moves E_2.. down to be the next O, and adds E_1 into the
+// new E_0, the carry of which is the next row's carry into its odd chain.
+
+// (E, O) <- T / 2^32 (word E_0 is zero or retired), returned with the roles
+// as the asm blocks below leave them: the new E in o[], the new O in e[2..7]
+// and two new top words.
+__device__ __forceinline__ void eo_swap(uint32_t e[8], uint32_t o[8], uint32_t n6, uint32_t n7) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t t = o[k];
+    o[k] = k < 6 ? e[k + 2 < 8 ? k + 2 : 7] : k == 6 ? n6 : n7;
+    e[k] = t;
+  }
+}
+
+// E = even limbs of a times b, O = odd limbs (the first row).
+__device__ __forceinline__ void eo_first(uint32_t e[8], uint32_t o[8], const uint32_t a[8], uint32_t b) {
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    const uint64_t x = (uint64_t)a[k] * b, y = (uint64_t)a[k + 1] * b;
+    e[k] = (uint32_t)x;
+    e[k + 1] = (uint32_t)(x >> 32);
+    o[k] = (uint32_t)y;
+    o[k + 1] = (uint32_t)(y >> 32);
+  }
+}
+
+// T <- T / 2^32 + a b.
+__device__ __forceinline__ void eo_mul_row(uint32_t e[8], uint32_t o[8], const uint32_t a[8], uint32_t b) {
+  uint32_t n6, n7;
+  asm("add.cc.u32     %0, %0, %8;\n\t"
+      "madc.lo.cc.u32 %9, %18, %24, %9;\n\t"
+      "madc.hi.cc.u32 %10, %18, %24, %10;\n\t"
+      "madc.lo.cc.u32 %11, %20, %24, %11;\n\t"
+      "madc.hi.cc.u32 %12, %20, %24, %12;\n\t"
+      "madc.lo.cc.u32 %13, %22, %24, %13;\n\t"
+      "madc.hi.cc.u32 %14, %22, %24, %14;\n\t"
+      "madc.lo.cc.u32 %15, %25, %24, 0;\n\t"
+      "madc.hi.u32    %16, %25, %24, 0;\n\t"
+      "mad.lo.cc.u32  %0, %17, %24, %0;\n\t"
+      "madc.hi.cc.u32 %1, %17, %24, %1;\n\t"
+      "madc.lo.cc.u32 %2, %19, %24, %2;\n\t"
+      "madc.hi.cc.u32 %3, %19, %24, %3;\n\t"
+      "madc.lo.cc.u32 %4, %21, %24, %4;\n\t"
+      "madc.hi.cc.u32 %5, %21, %24, %5;\n\t"
+      "madc.lo.cc.u32 %6, %23, %24, %6;\n\t"
+      "madc.hi.cc.u32 %7, %23, %24, %7;\n\t"
+      "addc.u32       %16, %16, 0;"
+      : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7]),
+        "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "=&r"(n6), "=&r"(n7)
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(b), "r"(a[7]));
+  eo_swap(e, o, n6, n7);
+}
+
+// T <- T + m p, m chosen to clear the low word.
+template <class C>
+__device__ __forceinline__ void eo_reduce_row(uint32_t e[8], uint32_t o[8]) {
+  const uint32_t m = e[0] * C::INV;
+  asm("mad.lo.cc.u32  %8, %16, %18, %8;\n\t"
+      "madc.hi.cc.u32 %9, %16, %18, %9;\n\t"
+      "madc.lo.cc.u32 %10, %16, %20, %10;\n\t"
+      "madc.hi.cc.u32 %11, %16, %20, %11;\n\t"
+      "madc.lo.cc.u32 %12, %16, %22, %12;\n\t"
+      "madc.hi.cc.u32 %13, %16, %22, %13;\n\t"
+      "madc.lo.cc.u32 %14, %16, %24, %14;\n\t"
+      "madc.hi.u32    %15, %16, %24, %15;\n\t"
+      "mad.lo.cc.u32  %0, %16, %17, %0;\n\t"
+      "madc.hi.cc.u32 %1, %16, %17, %1;\n\t"
+      "madc.lo.cc.u32 %2, %16, %19, %2;\n\t"
+      "madc.hi.cc.u32 %3, %16, %19, %3;\n\t"
+      "madc.lo.cc.u32 %4, %16, %21, %4;\n\t"
+      "madc.hi.cc.u32 %5, %16, %21, %5;\n\t"
+      "madc.lo.cc.u32 %6, %16, %23, %6;\n\t"
+      "madc.hi.cc.u32 %7, %16, %23, %7;\n\t"
+      "addc.u32       %15, %15, 0;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]),
+        "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7])
+      : "r"(m), "n"(C::P0), "n"(C::P1), "n"(C::P2), "n"(C::P3), "n"(C::P4), "n"(C::P5), "n"(C::P6), "n"(C::P7));
+}
+
+// T <- T / 2^32 + m p, m chosen to clear the low word (a row with no product).
+template <class C>
+__device__ __forceinline__ void eo_shift_reduce_row(uint32_t e[8], uint32_t o[8]) {
+  const uint32_t m = (o[0] + e[1]) * C::INV;
+  uint32_t n6, n7;
+  asm("add.cc.u32     %0, %0, %8;\n\t"
+      "madc.lo.cc.u32 %9, %17, %19, %9;\n\t"
+      "madc.hi.cc.u32 %10, %17, %19, %10;\n\t"
+      "madc.lo.cc.u32 %11, %17, %21, %11;\n\t"
+      "madc.hi.cc.u32 %12, %17, %21, %12;\n\t"
+      "madc.lo.cc.u32 %13, %17, %23, %13;\n\t"
+      "madc.hi.cc.u32 %14, %17, %23, %14;\n\t"
+      "madc.lo.cc.u32 %15, %17, %25, 0;\n\t"
+      "madc.hi.u32    %16, %17, %25, 0;\n\t"
+      "mad.lo.cc.u32  %0, %17, %18, %0;\n\t"
+      "madc.hi.cc.u32 %1, %17, %18, %1;\n\t"
+      "madc.lo.cc.u32 %2, %17, %20, %2;\n\t"
+      "madc.hi.cc.u32 %3, %17, %20, %3;\n\t"
+      "madc.lo.cc.u32 %4, %17, %22, %4;\n\t"
+      "madc.hi.cc.u32 %5, %17, %22, %5;\n\t"
+      "madc.lo.cc.u32 %6, %17, %24, %6;\n\t"
+      "madc.hi.cc.u32 %7, %17, %24, %7;\n\t"
+      "addc.u32       %16, %16, 0;"
+      : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7]),
+        "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "=&r"(n6), "=&r"(n7)
+      : "r"(m), "n"(C::P0), "n"(C::P1), "n"(C::P2), "n"(C::P3), "n"(C::P4), "n"(C::P5), "n"(C::P6), "n"(C::P7));
+  eo_swap(e, o, n6, n7);
+}
+
+// r = T / 2^32 (the low word zero or retired): O plus E's words 1..7.
+__device__ __forceinline__ void eo_merge(uint32_t r[8], const uint32_t e[8], const uint32_t o[8]) {
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, 0;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(e[1]), "r"(e[2]),
+        "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]));
+}
+
+// a b / 2^256 mod p: eight product rows, each followed by its reduction row.
+// With a, b < m < 2^254 T stays below 2m between rows, so the result needs
+// one conditional subtraction.
 template <class C>
 __device__ __forceinline__ Fe<C> fe_mul(const Fe<C>& a, const Fe<C>& b) {
-  const uint32_t p[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
-  uint32_t t[9];
+  uint32_t e[8], o[8];
+  eo_first(e, o, a.v, b.v[0]);
+  eo_reduce_row<C>(e, o);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) t[k] = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uint64_t c = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint64_t uv = (uint64_t)a.v[j] * b.v[i] + t[j] + c;
-      t[j] = (uint32_t)uv;
-      c = uv >> 32;
-    }
-    t[8] += (uint32_t)c;  // t < 2^287 here: no carry out of word 8
-    const uint32_t m = t[0] * C::INV;
-    uint64_t uv = (uint64_t)m * p[0] + t[0];  // low word cancels
-    c = uv >> 32;
-#pragma unroll
-    for (int j = 1; j < 8; ++j) {
-      uv = (uint64_t)m * p[j] + t[j] + c;
-      t[j - 1] = (uint32_t)uv;
-      c = uv >> 32;
-    }
-    uv = (uint64_t)t[8] + c;  // t < 2^288 before the shift, < 2^256 after
-    t[7] = (uint32_t)uv;
-    t[8] = 0;
+  for (int i = 1; i < 8; ++i) {
+    eo_mul_row(e, o, a.v, b.v[i]);
+    eo_reduce_row<C>(e, o);
   }
   Fe<C> r;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) r.v[k] = t[k];
+  eo_merge(r.v, e, o);
   fe_reduce_once<C>(r.v);
   return r;
 }
 
-// a^2 with the cross products computed once: rows of a_i * a_j (i < j) with
-// 64-bit carries into a 512-bit T, T doubled, the squares a_i^2 added, then
-// the eight Montgomery reduction rows. 36 wide products for the square
-// against 64 in a multiply (measured on GB300: 61 G squares/s against 49 G
-// products/s). T < a^2 < 2^508, so the doubling and the additions never
-// carry out of 16 words, and the reduced value is below 2m.
+// (t + M m) / 2^256 for the M below 2^256 that clears the low 256 bits of t
+// (eight words): the reduction rows alone. At most m.
+template <class C>
+__device__ __forceinline__ void eo_redc(uint32_t r[8], const uint32_t t[8]) {
+  const uint32_t p[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
+  uint32_t e[8], o[8];
+  const uint32_t m = t[0] * C::INV;
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    e[k] = t[k];
+    e[k + 1] = t[k + 1];
+    const uint64_t y = (uint64_t)p[k + 1] * m;
+    o[k] = (uint32_t)y;
+    o[k + 1] = (uint32_t)(y >> 32);
+  }
+  asm("mad.lo.cc.u32  %0, %9, %10, %0;\n\t"
+      "madc.hi.cc.u32 %1, %9, %10, %1;\n\t"
+      "madc.lo.cc.u32 %2, %9, %11, %2;\n\t"
+      "madc.hi.cc.u32 %3, %9, %11, %3;\n\t"
+      "madc.lo.cc.u32 %4, %9, %12, %4;\n\t"
+      "madc.hi.cc.u32 %5, %9, %12, %5;\n\t"
+      "madc.lo.cc.u32 %6, %9, %13, %6;\n\t"
+      "madc.hi.cc.u32 %7, %9, %13, %7;\n\t"
+      "addc.u32       %8, %8, 0;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(o[7])
+      : "r"(m), "n"(C::P0), "n"(C::P2), "n"(C::P4), "n"(C::P6));
+#pragma unroll
+  for (int i = 1; i < 8; ++i) eo_shift_reduce_row<C>(e, o);
+  eo_merge(r, e, o);
+}
+
+// The cross products a_i a_j (i < j) of a square, each once, into words 1..14
+// of two arrays by the parity of their position i + j. A row's chain ends
+// either on words no earlier row of its parity has touched (a_7's product) or
+// one short of them (a_6's), where its carry starts the next word.
+__device__ __forceinline__ void eo_cross(uint32_t E[16], uint32_t O[16], const uint32_t a[8]) {
+#pragma unroll
+  for (int j = 1; j < 8; ++j) {
+    const uint64_t x = (uint64_t)a[0] * a[j];
+    uint32_t* w = (j & 1) ? O : E;
+    w[j] = (uint32_t)x;
+    w[j + 1] = (uint32_t)(x >> 32);
+  }
+  asm("mad.lo.cc.u32  %0, %7, %8, %0;\n\t"  // a_1: a_2, a_4, a_6
+      "madc.hi.cc.u32 %1, %7, %8, %1;\n\t"
+      "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
+      "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+      "madc.lo.cc.u32 %4, %7, %10, %4;\n\t"
+      "madc.hi.cc.u32 %5, %7, %10, %5;\n\t"
+      "addc.u32       %6, 0, 0;"
+      : "+r"(O[3]), "+r"(O[4]), "+r"(O[5]), "+r"(O[6]), "+r"(O[7]), "+r"(O[8]), "=r"(O[9])
+      : "r"(a[1]), "r"(a[2]), "r"(a[4]), "r"(a[6]));
+  asm("mad.lo.cc.u32  %0, %6, %7, %0;\n\t"  // a_1: a_3, a_5, a_7
+      "madc.hi.cc.u32 %1, %6, %7, %1;\n\t"
+      "madc.lo.cc.u32 %2, %6, %8, %2;\n\t"
+      "madc.hi.cc.u32 %3, %6, %8, %3;\n\t"
+      "madc.lo.cc.u32 %4, %6, %9, 0;\n\t"
+      "madc.hi.u32    %5, %6, %9, 0;"
+      : "+r"(E[4]), "+r"(E[5]), "+r"(E[6]), "+r"(E[7]), "=&r"(E[8]), "=&r"(E[9])
+      : "r"(a[1]), "r"(a[3]), "r"(a[5]), "r"(a[7]));
+  asm("mad.lo.cc.u32  %0, %6, %7, %0;\n\t"  // a_2: a_3, a_5, a_7
+      "madc.hi.cc.u32 %1, %6, %7, %1;\n\t"
+      "madc.lo.cc.u32 %2, %6, %8, %2;\n\t"
+      "madc.hi.cc.u32 %3, %6, %8, %3;\n\t"
+      "madc.lo.cc.u32 %4, %6, %9, %4;\n\t"
+      "madc.hi.u32    %5, %6, %9, 0;"
+      : "+r"(O[5]), "+r"(O[6]), "+r"(O[7]), "+r"(O[8]), "+r"(O[9]), "=&r"(O[10])
+      : "r"(a[2]), "r"(a[3]), "r"(a[5]), "r"(a[7]));
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"  // a_2: a_4, a_6
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;"
+      : "+r"(E[6]), "+r"(E[7]), "+r"(E[8]), "+r"(E[9]), "=r"(E[10])
+      : "r"(a[2]), "r"(a[4]), "r"(a[6]));
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"  // a_3: a_4, a_6
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;"
+      : "+r"(O[7]), "+r"(O[8]), "+r"(O[9]), "+r"(O[10]), "=r"(O[11])
+      : "r"(a[3]), "r"(a[4]), "r"(a[6]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"  // a_3: a_5, a_7
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;"
+      : "+r"(E[8]), "+r"(E[9]), "+r"(E[10]), "=&r"(E[11])
+      : "r"(a[3]), "r"(a[5]), "r"(a[7]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"  // a_4: a_5, a_7
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;"
+      : "+r"(O[9]), "+r"(O[10]), "+r"(O[11]), "=&r"(O[12])
+      : "r"(a[4]), "r"(a[5]), "r"(a[7]));
+  asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"  // a_4: a_6
+      "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+      "addc.u32       %2, 0, 0;"
+      : "+r"(E[10]), "+r"(E[11]), "=r"(E[12])
+      : "r"(a[4]), "r"(a[6]));
+  asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"  // a_5: a_6
+      "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+      "addc.u32       %2, 0, 0;"
+      : "+r"(O[11]), "+r"(O[12]), "=r"(O[13])
+      : "r"(a[5]), "r"(a[6]));
+  asm("mad.lo.cc.u32  %0, %2, %3, %0;\n\t"  // a_5: a_7
+      "madc.hi.u32    %1, %2, %3, 0;"
+      : "+r"(E[12]), "=&r"(E[13])
+      : "r"(a[5]), "r"(a[7]));
+  asm("mad.lo.cc.u32  %0, %2, %3, %0;\n\t"  // a_6: a_7
+      "madc.hi.u32    %1, %2, %3, 0;"
+      : "+r"(O[13]), "=&r"(O[14])
+      : "r"(a[6]), "r"(a[7]));
+}
+
+// a^2 / 2^256 mod p: the 28 cross products once, doubled, the eight squares
+// added, then the reduction rows: 100 wide products against 128 in a multiply
+// (measured on GB300: 85 G squares/s against 72 G products/s, 728 clocks
+// alone against 847). a^2 < 2^508, so the doubling never carries out of 16
+// words, and the reduced low half (at most m) plus the high half is below 2m.
 template <class C>
 __device__ __forceinline__ Fe<C> fe_sqr(const Fe<C>& a) {
-  const uint32_t p[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
-  uint32_t T[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) T[k] = 0;
-#pragma unroll
-  for (int i = 0; i < 7; ++i) {
-    uint64_t c = 0;
-#pragma unroll
-    for (int j = i + 1; j < 8; ++j) {
-      const uint64_t uv = (uint64_t)a.v[i] * a.v[j] + T[i + j] + c;
-      T[i + j] = (uint32_t)uv;
-      c = uv >> 32;
-    }
-    T[i + 8] = (uint32_t)c;
-  }
+  uint32_t E[16], O[16], T[16], cy;
+  eo_cross(E, O, a.v);
+  T[0] = 0;
+  T[1] = O[1];
+  asm("add.cc.u32  %0, %7, %13;\n\t"
+      "addc.cc.u32 %1, %8, %14;\n\t"
+      "addc.cc.u32 %2, %9, %15;\n\t"
+      "addc.cc.u32 %3, %10, %16;\n\t"
+      "addc.cc.u32 %4, %11, %17;\n\t"
+      "addc.cc.u32 %5, %12, %18;\n\t"
+      "addc.u32    %6, 0, 0;"
+      : "=&r"(T[2]), "=&r"(T[3]), "=&r"(T[4]), "=&r"(T[5]), "=&r"(T[6]), "=&r"(T[7]), "=&r"(cy)
+      : "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(O[2]), "r"(O[3]), "r"(O[4]), "r"(O[5]),
+        "r"(O[6]), "r"(O[7]));
+  asm("{\n\t"
+      ".reg .u32 t;\n\t"
+      "add.cc.u32  t, %20, 0xffffffff;\n\t"  // the carry back into the flag
+      "addc.cc.u32 %0, %7, %13;\n\t"
+      "addc.cc.u32 %1, %8, %14;\n\t"
+      "addc.cc.u32 %2, %9, %15;\n\t"
+      "addc.cc.u32 %3, %10, %16;\n\t"
+      "addc.cc.u32 %4, %11, %17;\n\t"
+      "addc.cc.u32 %5, %12, %18;\n\t"
+      "addc.u32    %6, %19, 0;\n\t"
+      "}"
+      : "=&r"(T[8]), "=&r"(T[9]), "=&r"(T[10]), "=&r"(T[11]), "=&r"(T[12]), "=&r"(T[13]), "=&r"(T[14])
+      : "r"(E[8]), "r"(E[9]), "r"(E[10]), "r"(E[11]), "r"(E[12]), "r"(E[13]), "r"(O[8]), "r"(O[9]), "r"(O[10]),
+        "r"(O[11]), "r"(O[12]), "r"(O[13]), "r"(O[14]), "r"(cy));
   T[15] = T[14] >> 31;
 #pragma unroll
-  for (int k = 14; k > 0; --k) T[k] = (T[k] << 1) | (T[k - 1] >> 31);
-  T[0] <<= 1;
-  uint64_t c = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint64_t sq = (uint64_t)a.v[i] * a.v[i];
-    const uint64_t lo = (uint64_t)T[2 * i] + (uint32_t)sq + c;
-    T[2 * i] = (uint32_t)lo;
-    const uint64_t hi = (uint64_t)T[2 * i + 1] + (uint32_t)(sq >> 32) + (lo >> 32);
-    T[2 * i + 1] = (uint32_t)hi;
-    c = hi >> 32;
-  }
-  uint32_t carry_hi = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t m = T[i] * C::INV;
-    uint64_t cc = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint64_t uv = (uint64_t)m * p[j] + T[i + j] + cc;
-      T[i + j] = (uint32_t)uv;
-      cc = uv >> 32;
-    }
-    const uint64_t s = (uint64_t)T[i + 8] + cc + carry_hi;
-    T[i + 8] = (uint32_t)s;
-    carry_hi = (uint32_t)(s >> 32);
-  }
+  for (int k = 14; k > 1; --k) T[k] = __funnelshift_l(T[k - 1], T[k], 1);
+  T[1] <<= 1;
+  asm("mad.lo.cc.u32  %0, %16, %16, 0;\n\t"
+      "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
+      "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
+      "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
+      "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
+      "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
+      "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
+      "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
+      "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
+      "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
+      "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
+      "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
+      "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
+      "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
+      "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
+      "madc.hi.u32    %15, %23, %23, %15;"
+      : "+r"(T[0]), "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]), "+r"(T[7]), "+r"(T[8]),
+        "+r"(T[9]), "+r"(T[10]), "+r"(T[11]), "+r"(T[12]), "+r"(T[13]), "+r"(T[14]), "+r"(T[15])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]));
+  uint32_t lo[8];
+  eo_redc<C>(lo, T);
   Fe<C> r;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) r.v[k] = T[8 + k];
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+      : "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]), "r"(T[8]),
+        "r"(T[9]), "r"(T[10]), "r"(T[11]), "r"(T[12]), "r"(T[13]), "r"(T[14]), "r"(T[15]));
   fe_reduce_once<C>(r.v);
   return r;
 }
@@ -271,28 +519,8 @@ __device__ __forceinline__ Fe<C> fe_sqr(const Fe<C>& a) {
 // Montgomery form -> canonical limbs (multiply by 1), and back (multiply by R^2).
 template <class C>
 __device__ __forceinline__ Fe<C> fe_from_mont(const Fe<C>& a) {
-  // a * R^-1: the reduction rows of the multiply alone (a * 1 has no product
-  // rows), eight m*p rows of 64-bit steps.
-  const uint32_t p[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
-  uint32_t t[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) t[k] = a.v[k];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t m = t[0] * C::INV;
-    uint64_t uv = (uint64_t)m * p[0] + t[0];
-    uint64_t c = uv >> 32;
-#pragma unroll
-    for (int j = 1; j < 8; ++j) {
-      uv = (uint64_t)m * p[j] + t[j] + c;
-      t[j - 1] = (uint32_t)uv;
-      c = uv >> 32;
-    }
-    t[7] = (uint32_t)c;  // (t + m*p) / 2^32 < 2^256
-  }
   Fe<C> r;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) r.v[k] = t[k];
+  eo_redc<C>(r.v, a.v);
   fe_reduce_once<C>(r.v);
   return r;
 }
