@@ -14,21 +14,22 @@
 //                   threads, each folding an equal slice of the sorted list
 //                   run by run into XYZZ accumulators with mixed adds; runs cut
 //                   by a slice edge are stitched by k_fold_edges.
-//  5. k_level/k_sum bucket reduction sum_k k*B_k as a tree of running sums,
-//                   every column's bucket range at once.
-//  6. k_finish_cols per column, combine windows (Horner) or, with a
+//  5. k_reduce      bucket reduction sum_k k*B_k, every column's bucket range
+//                   at once, four lanes a point.
+//  6. k_finish      per column, combine windows (Horner) or, with a
 //                   precomputed SRS window table, nothing: there every window
 //                   shares one bucket set because the table already holds
 //                   2^(c*w) * P_i; then the canonical affine encoding.
 // The allocation-free variant at the end of this file keeps the first
+// single-MSM form of the sort and the accumulation (k_recode, k_scatter,
+// k_accumulate).
 // single-MSM form of the pipeline (k_recode, k_scatter, k_accumulate, k_finish).
 #include "common.cuh"
+#include "curve_quad.cuh"
 
 namespace apg {
 
 namespace {
-
-constexpr int kLevelFan = 8;  // buckets folded per thread in one reduction level
 
 __device__ __forceinline__ void raise_flag(uint32_t* flags, uint32_t f) { atomicOr(flags, f); }
 
@@ -339,134 +340,222 @@ __global__ void __launch_bounds__(128) k_accumulate(const uint64_t* sorted, cons
   if (!head_written) put_item(okeys, opts, opres, 2 * s, first, nullptr);
 }
 
-// One level of the edge-run folding over items (see k_accumulate).
-__global__ void __launch_bounds__(128) k_fold_edges(const uint32_t* keys, const Xyzz* pts, const uint8_t* pres,
-                                                    size_t len, int seg_len, size_t nseg, Xyzz* buckets,
-                                                    uint32_t* okeys, Xyzz* opts, uint8_t* opres) {
-  size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  const size_t lo = s * (size_t)seg_len;
-  if (lo >= len) {
-    put_item(okeys, opts, opres, 2 * s, kNoKey, nullptr);
-    put_item(okeys, opts, opres, 2 * s + 1, kNoKey, nullptr);
-    return;
-  }
-  const size_t hi = min(lo + (size_t)seg_len, len);
-  const uint32_t first = keys[lo];
-  uint32_t cur = first;
-  const bool starts_before = lo > 0 && keys[lo - 1] == cur;
-  const bool continues = hi < len && keys[hi] == keys[hi - 1];
-  bool first_run = true, head_written = false, any = false;
-  Xyzz acc = xyzz_inf();
-  for (size_t i = lo; i < hi; ++i) {
-    uint32_t b = keys[i];
-    if (b != cur) {
-      if (first_run && starts_before) {
-        put_item(okeys, opts, opres, 2 * s, cur, any ? &acc : nullptr);
-        head_written = true;
+// One level of the edge-run folding over items (see k_accumulate), a quad of
+// lanes a point (curve_quad.cuh). A block takes 63 quads' worth of
+// consecutive items: each quad folds `per` of them in turn, then quad i holds
+// what crosses its left edge (the tail of quad i - 1 plus its own head; quad
+// 63 only closes the block's right edge), and a segmented scan by doubling
+// distances adds up the runs. So a level's chain is per + log2(run) additions
+// and leaves two items a block, where one thread folding eight items in turn
+// leaves a quarter of them. 64 quads are two warps a scheduler, as many as a
+// scheduler's multiply pipe feeds without slowing a chain (128 quads: 4.0 us an
+// addition against 2.3). Measured on a GB300, all levels together: 251 -> 90 us
+// for a 2^16-point commit (155,000 items), 153 -> 38 for a 2^8-point one.
+constexpr int kFoldQuads = 64;
+constexpr int kFoldLastPer = 4;  // items a quad at most in a level of one block
+
+__global__ void __launch_bounds__(4 * kFoldQuads) k_fold_edges(const uint32_t* keys, const Xyzz* pts,
+                                                               const uint8_t* pres, size_t len, int per,
+                                                               Xyzz* buckets, uint32_t* okeys, Xyzz* opts,
+                                                               uint8_t* opres) {
+  __shared__ Fq sv[4 * kFoldQuads];
+  __shared__ uint32_t skey[kFoldQuads];
+  __shared__ uint8_t slive[kFoldQuads], spres[kFoldQuads];
+  const int l = threadIdx.x & 3, i = threadIdx.x >> 2;
+  const size_t base = blockIdx.x * (size_t)(kFoldQuads - 1) * per;
+  const size_t end = min(base + (size_t)(kFoldQuads - 1) * per, len);
+  const size_t lo = min(base + (size_t)i * per, end), hi = min(lo + per, end);
+  // The boundary at lo: live when the run of item lo - 1 goes on past it. Of
+  // the quads that start at the block's end only the first one's counts.
+  const bool mine = i == 0 || lo < end || base + (size_t)(i - 1) * per < end;
+  const bool live = mine && lo > 0 && lo < len && keys[lo - 1] == keys[lo];
+  const bool cont = hi > lo && hi < len && keys[hi - 1] == keys[hi];
+  Fq acc = fe_zero<FqConsts>(), head = acc;
+  bool any = false, head_any = false, first = true;
+  uint32_t cur = lo < hi ? keys[lo] : kNoKey;
+  for (int t = 0; t < per; ++t) {
+    const size_t at = lo + t;
+    const bool in = at < hi;
+    const uint32_t k = in ? keys[at] : cur;
+    const bool pr = in && pres[at];
+    const Fq pt = pr ? quad_ld(&pts[at], l) : fe_zero<FqConsts>();
+    if (k != cur) {
+      if (first && live) {
+        head = acc;
+        head_any = any;
       } else if (any && cur != kNoKey) {
-        st_xyzz(&buckets[cur], acc);
+        quad_st(&buckets[cur], l, acc);
       }
-      first_run = false;
-      cur = b;
-      acc = xyzz_inf();
+      first = false;
+      cur = k;
       any = false;
     }
-    if (pres[i]) {
-      acc = any ? xyzz_add(acc, ld_xyzz(&pts[i])) : ld_xyzz(&pts[i]);
-      any = true;
+    const bool both = pr && any;
+    if (__any_sync(0xffffffffu, both)) {
+      const Fq sum = quad_add(acc, pt);
+      if (both) acc = sum;
+    }
+    if (pr && !any) acc = pt;
+    any |= pr;
+  }
+  bool tail = false;
+  if (lo < hi) {
+    if (first && live) {
+      head = acc;
+      head_any = any;
+    } else if (cont) {
+      tail = any;
+    } else if (any && cur != kNoKey) {
+      quad_st(&buckets[cur], l, acc);
     }
   }
-  if (first_run && starts_before) {
-    put_item(okeys, opts, opres, 2 * s, cur, any ? &acc : nullptr);
-    head_written = true;
-    put_item(okeys, opts, opres, 2 * s + 1, cur, nullptr);
-  } else {
-    if (continues) put_item(okeys, opts, opres, 2 * s + 1, cur, any ? &acc : nullptr);
-    else {
-      if (any && cur != kNoKey) st_xyzz(&buckets[cur], acc);
-      put_item(okeys, opts, opres, 2 * s + 1, cur, nullptr);
+  st_fe(&sv[threadIdx.x], acc);
+  if (l == 0) {
+    spres[i] = tail;
+    slive[i] = live;
+    skey[i] = live ? keys[lo] : kNoKey;
+  }
+  __syncthreads();
+  // What crosses the boundary at lo: the previous quad's tail, this one's head.
+  const bool tp = live && i > 0 && spres[i - 1], hp = live && head_any;
+  Fq v = tp ? ld_fe(&sv[threadIdx.x - 4]) : head;
+  bool have = tp || hp;
+  if (__any_sync(0xffffffffu, tp && hp)) {
+    const Fq sum = quad_add(v, head);
+    if (tp && hp) v = sum;
+  }
+  const uint32_t key = skey[i];
+  __syncthreads();
+  for (int off = 1; off < kFoldQuads; off <<= 1) {
+    st_fe(&sv[threadIdx.x], v);
+    if (l == 0) spres[i] = have;
+    const int j = i + off;
+    const bool match = live && j < kFoldQuads && slive[j] && skey[j] == key;
+    if (!__syncthreads_or(match)) break;  // no run reaches this far
+    const bool take = match && spres[j];
+    const Fq o = take ? ld_fe(&sv[threadIdx.x + 4 * off]) : fe_zero<FqConsts>();
+    if (__any_sync(0xffffffffu, take && have)) {
+      const Fq sum = quad_add(v, o);
+      if (take && have) v = sum;
+    }
+    if (take && !have) v = o;
+    have |= take;
+    __syncthreads();
+  }
+  // The runs' first boundaries hold their sums.
+  const int ne = (int)((end - base + per - 1) / per);  // the boundary at the block's end
+  const bool end_live = slive[ne] != 0, through = end_live && slive[0] && skey[0] == skey[ne];
+  const bool lead = live && (i == 0 || !slive[i - 1] || skey[i - 1] != key);
+  const size_t out = 2 * (size_t)blockIdx.x;
+  if (lead) {
+    const bool left = i == 0, right = !left && end_live && skey[ne] == key;
+    if (left || right) {
+      const size_t slot = out + (left ? 0 : 1);
+      if (have) quad_st(&opts[slot], l, v);
+      if (l == 0) {
+        okeys[slot] = key;
+        opres[slot] = have;
+      }
+    } else if (have && key != kNoKey) {
+      quad_st(&buckets[key], l, v);
     }
   }
-  if (!head_written) put_item(okeys, opts, opres, 2 * s, first, nullptr);
+  if (threadIdx.x == 0) {
+    if (!slive[0]) {
+      okeys[out] = keys[base];
+      opres[out] = 0;
+    }
+    if (!end_live || through) {
+      okeys[out + 1] = keys[end - 1];
+      opres[out + 1] = 0;
+    }
+  }
 }
 
 // ---- bucket reduction -------------------------------------------------------
+//
+// sum_k (k + 1) B_k over a space's K buckets, a quad of lanes a point. A block
+// of Q quads takes Q * 2^lf consecutive entries, each (R_k, T_k) with weight
+// 2^scale k + 1 within the block: quad q folds its 2^lf entries into their sum
+// and their weighted sum W_q = sum_j j R_j, a suffix scan over the quads gives
+// S_q = sum_{q' >= q} R_q', and
+//   R' = S_0,   T' = sum_q (T_q + 2^scale (W_q + [q > 0] 2^lf S_q))
+// is the block's own entry for the next level, whose scale grows by the
+// block's length. The first level reads buckets (T_k = 0, scale 0); the last
+// (`last`) is one block a space and adds R' in, the + 1 of every weight. A
+// block's chain is 2^(lf+1) + 2 log2 Q additions and scale + lf doublings.
+// Measured on a GB300 against eight buckets a thread and level with block sums
+// of each level: 2^15 buckets 697 -> 135 us, 128 buckets 101 -> 48, four sets
+// of 2^19 (bound by the products) 1.9 -> 1.65 ms.
+constexpr int kReduceQuads = 64;  // a block at most: two warps a scheduler (see kFoldQuads)
 
-// in[space*M + k] has weight k+1. Group g of `fan` buckets yields
-// T_g = sum_j (j+1) in[g*fan + j] and R_g = sum_j in[g*fan + j]; the next
-// level takes R_1..R_{G-1} (weights 1..G-1) and an identity pad at weight G:
-//   sum_k k B_k = sum_g T_g + fan * sum_g g R_g.
-__global__ void k_level(const Xyzz* in, int M, int spaces, int fan, Xyzz* outT, Xyzz* outR) {
-  int G = (M + fan - 1) / fan;
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= spaces * G) return;
-  int sp = idx / G, g = idx % G;
-  int lo = g * fan, hi = min(lo + fan, M);
-  Xyzz run = xyzz_inf(), tot = xyzz_inf();
-  for (int k = hi - 1; k >= lo; --k) {
-    run = xyzz_add(run, ld_xyzz(&in[(size_t)sp * M + k]));
-    tot = xyzz_add(tot, run);
-  }
-  st_xyzz(&outT[(size_t)sp * G + g], tot);
-  if (g > 0) st_xyzz(&outR[(size_t)sp * G + g - 1], run);
-  else st_xyzz(&outR[(size_t)sp * G + G - 1], xyzz_inf());
-}
-
-// out[space] = sum of in[space*M .. space*M + M).
-__global__ void k_sum(const Xyzz* in, int M, Xyzz* out) {
-  __shared__ Xyzz sh[128];
-  int sp = blockIdx.x;
-  Xyzz acc = xyzz_inf();
-  for (int k = threadIdx.x; k < M; k += blockDim.x) acc = xyzz_add(acc, ld_xyzz(&in[(size_t)sp * M + k]));
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < (unsigned)off) sh[threadIdx.x] = xyzz_add(sh[threadIdx.x], sh[threadIdx.x + off]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) st_xyzz(&out[sp], sh[0]);
-}
-
-// First stage of a wide sum: block b of space sp folds in[sp*M + b*256 ..
-// +256) into part[sp*gridDim.x + b], two points a thread then a tree.
-__global__ void k_sum_blocks(const Xyzz* in, int M, Xyzz* part) {
-  __shared__ Xyzz sh[128];
-  const int sp = blockIdx.y, b = blockIdx.x;
-  const int k0 = b * 256 + threadIdx.x, k1 = k0 + 128;
-  Xyzz acc = k0 < M ? ld_xyzz(&in[(size_t)sp * M + k0]) : xyzz_inf();
-  if (k1 < M) acc = xyzz_add(acc, ld_xyzz(&in[(size_t)sp * M + k1]));
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int off = 64; off > 0; off >>= 1) {
-    if (threadIdx.x < (unsigned)off) sh[threadIdx.x] = xyzz_add(sh[threadIdx.x], sh[threadIdx.x + off]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) st_xyzz(&part[(size_t)sp * gridDim.x + b], sh[0]);
-}
-
-// tsum[level*spaces + sp] holds level sums; combine by Horner in `fan`, then
-// combine spaces (windows) by Horner in 2^c, normalise and write 64 bytes.
-__global__ void k_finish(const Xyzz* tsum, int levels, int spaces, int fan_log, int c, uint32_t* out64,
-                         uint32_t* flags) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  Xyzz total = xyzz_inf();
-  for (int sp = spaces - 1; sp >= 0; --sp) {
-    for (int j = 0; j < c && sp != spaces - 1; ++j) total = xyzz_dbl(total);
-    Xyzz s = xyzz_inf();
-    for (int l = levels - 1; l >= 0; --l) {
-      for (int j = 0; j < fan_log && l != levels - 1; ++j) s = xyzz_dbl(s);
-      s = xyzz_add(s, ld_xyzz(&tsum[(size_t)l * spaces + sp]));
+__global__ void __launch_bounds__(4 * kReduceQuads) k_reduce(const Xyzz* R, const Xyzz* T, int M, int lf, int scale,
+                                                             int last, Xyzz* outT, Xyzz* outR) {
+  extern __shared__ uint4 sm_points[];
+  Fq* sh = reinterpret_cast<Fq*>(sm_points);
+  const int l = threadIdx.x & 3, q = threadIdx.x >> 2, Q = blockDim.x >> 2, sp = blockIdx.y;
+  const size_t base = (size_t)sp * M;
+  const int f = 1 << lf, k0 = (blockIdx.x * Q + q) << lf;
+  Fq run = fe_zero<FqConsts>(), W = run, Ts = run;
+  for (int j = f - 1; j >= 0; --j) {
+    const int k = k0 + j;
+    const Fq r = k < M ? quad_ld(&R[base + k], l) : fe_zero<FqConsts>();
+    run = j == f - 1 ? r : quad_add(run, r);
+    if (j > 0) W = j == f - 1 ? run : quad_add(W, run);
+    if (T) {
+      const Fq t = k < M ? quad_ld(&T[base + k], l) : fe_zero<FqConsts>();
+      Ts = j == f - 1 ? t : quad_add(Ts, t);
     }
-    total = xyzz_add(total, s);
   }
-  Affine a = xyzz_to_affine(total, flags);
-  Fq x = fe_from_mont(a.x), y = fe_from_mont(a.y);
+  for (int off = 1; off < Q; off <<= 1) {
+    st_fe(&sh[threadIdx.x], run);
+    __syncthreads();
+    const bool has = q + off < Q;
+    const Fq o = has ? ld_fe(&sh[threadIdx.x + 4 * off]) : fe_zero<FqConsts>();
+    if (__any_sync(0xffffffffu, has)) run = quad_add(run, o);
+    __syncthreads();
+  }
+  Fq V = q > 0 ? run : fe_zero<FqConsts>();
+  for (int d = 0; d < lf; ++d) V = quad_dbl(V);
+  if (lf > 0) V = quad_add(V, W);
+  for (int d = 0; d < scale; ++d) V = quad_dbl(V);
+  if (T) V = quad_add(V, Ts);
+  for (int off = Q >> 1; off > 0; off >>= 1) {
+    st_fe(&sh[threadIdx.x], V);
+    __syncthreads();
+    const bool has = q < off;
+    const Fq o = has ? ld_fe(&sh[threadIdx.x + 4 * off]) : fe_zero<FqConsts>();
+    if (__any_sync(0xffffffffu, has)) V = quad_add(V, o);
+    __syncthreads();
+  }
+  if (threadIdx.x >= 32) return;
+  if (last) V = quad_add(V, run);
+  if (q != 0) return;
+  const size_t o = (size_t)sp * gridDim.x + blockIdx.x;
+  quad_st(&outT[o], l, V);
+  if (!last) quad_st(&outR[o], l, run);
+}
+
+// One warp per result: Horner over the result's spaces (windows, in 2^c),
+// then the canonical affine bytes. Every quad runs the same chain. With one
+// space a result (an SRS window table) there is no Horner; a generic-base
+// MSM's 29 windows of 9 bits are 252 doublings after one another, 2.0 us each
+// over a quad (2,484 points: 1243 -> 522 us).
+__global__ void __launch_bounds__(32) k_finish(const Xyzz* tsum, int spaces, int c, uint32_t* out64,
+                                               uint32_t* flags) {
+  const int lane = threadIdx.x & 31, l = lane & 3;
+  const Xyzz* in = tsum + (size_t)blockIdx.x * spaces;
+  Fq total = quad_ld(&in[spaces - 1], l);
+  for (int w = spaces - 2; w >= 0; --w) {
+    for (int j = 0; j < c; ++j) total = quad_dbl(total);
+    total = quad_add(total, quad_ld(&in[w], l));
+  }
+  const Affine a = xyzz_to_affine(quad_gather(total, lane), flags);
+  if (lane >= 2) return;
+  const Fq r = fe_from_mont(lane ? a.y : a.x);
+  uint32_t* o = out64 + 16 * (size_t)blockIdx.x + 8 * lane;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    out64[k] = x.v[k];
-    out64[8 + k] = y.v[k];
-  }
+  for (int k = 0; k < 8; ++k) o[k] = r.v[k];
 }
 
 // ---- the grouped pipeline -----------------------------------------------------
@@ -791,12 +880,6 @@ __device__ __forceinline__ Fq shfl_down_fq(const Fq& a, int off) {
   Fq r;
 #pragma unroll
   for (int w = 0; w < 8; ++w) r.v[w] = __shfl_down_sync(0xffffffffu, a.v[w], off);
-  return r;
-}
-__device__ __forceinline__ Fq shfl_fq(const Fq& a, int lane) {
-  Fq r;
-#pragma unroll
-  for (int w = 0; w < 8; ++w) r.v[w] = __shfl_sync(0xffffffffu, a.v[w], lane);
   return r;
 }
 
@@ -1233,62 +1316,6 @@ __global__ void __launch_bounds__(kPairThreads, APG_PAIR_PF_MIN_BLOCKS)
   }
 }
 
-// Bucket reduction of a small bucket set (K <= kSmallK), one block per space:
-// thread t holds B_t (weight t + 1); a suffix scan turns it into
-// S_t = sum_{k >= t} B_k, and sum_k (k + 1) B_k = sum_t S_t is a tree sum, so
-// the dependent chain is 2 log2 K additions instead of the running-sum levels.
-constexpr int kSmallK = 256;
-
-__global__ void __launch_bounds__(kSmallK) k_reduce_small(const Xyzz* buckets, int K, Xyzz* out) {
-  __shared__ Xyzz shx[kSmallK];
-  const int sp = blockIdx.x, t = threadIdx.x;
-  Xyzz v = ld_xyzz(&buckets[(size_t)sp * K + t]);
-  shx[t] = v;
-  __syncthreads();
-  for (int off = 1; off < K; off <<= 1) {
-    const bool has = t + off < K;
-    Xyzz nb = has ? shx[t + off] : xyzz_inf();
-    __syncthreads();
-    if (has) v = xyzz_add(v, nb);
-    shx[t] = v;
-    __syncthreads();
-  }
-  for (int off = K / 2; off > 0; off >>= 1) {
-    if (t < off) shx[t] = xyzz_add(shx[t], shx[t + off]);
-    __syncthreads();
-  }
-  if (t == 0) st_xyzz(&out[sp], shx[0]);
-}
-
-// One thread per column: Horner over the reduction levels (in `fan`) and the
-// column's spaces (windows, in 2^c), then the canonical affine bytes.
-__global__ void k_finish_cols(const Xyzz* tsum, int levels, int spaces_total, int spaces_per_col, int ncols,
-                              int fan_log, int c, uint32_t* out64, uint32_t* flags) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncols) return;
-  Xyzz total = xyzz_inf();
-  for (int w = spaces_per_col - 1; w >= 0; --w) {
-    if (w != spaces_per_col - 1)
-      for (int j = 0; j < c; ++j) total = xyzz_dbl(total);
-    const int sp = col * spaces_per_col + w;
-    Xyzz s = xyzz_inf();
-    for (int l = levels - 1; l >= 0; --l) {
-      if (l != levels - 1)
-        for (int j = 0; j < fan_log; ++j) s = xyzz_dbl(s);
-      s = xyzz_add(s, ld_xyzz(&tsum[(size_t)l * spaces_total + sp]));
-    }
-    total = xyzz_add(total, s);
-  }
-  const Affine a = xyzz_to_affine(total, flags);
-  const Fq x = fe_from_mont(a.x), y = fe_from_mont(a.y);
-  uint32_t* o = out64 + 16 * (size_t)col;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    o[k] = x.v[k];
-    o[8 + k] = y.v[k];
-  }
-}
-
 // out64 = the sum of m canonical affine points in64[0..m) (a stack whose
 // columns took more than one group).
 __global__ void k_add_points(const uint32_t* in64, int m, uint32_t* out64, uint32_t* flags) {
@@ -1314,6 +1341,48 @@ __global__ void k_add_points(const uint32_t* in64, int m, uint32_t* out64, uint3
     out64[8 + k] = y.v[k];
   }
 }
+
+struct FoldLevel {
+  unsigned blocks;
+  int per;
+};
+// A level of k_fold_edges over len items: one block while its quads take at
+// most kFoldLastPer each, else two items a quad, or four where that saves a
+// level.
+inline FoldLevel fold_level(size_t len) {
+  const size_t q = kFoldQuads - 1;
+  if (len <= q * kFoldLastPer) return {1u, (int)((len + q - 1) / q)};
+  const size_t per = len <= q * q * kFoldLastPer ? 2 : 4;  // (two items leave 2 len / 126 <= 252)
+  return {(unsigned)((len + q * per - 1) / (q * per)), (int)per};
+}
+
+// k_reduce's levels over S spaces of K buckets (a power of two): one block a
+// space for up to 256 buckets; above that a first level of blocks of 64 quads,
+// four buckets a quad while that fits the device (more as the spaces grow past
+// four blocks an SM: the scan's additions are then work, not latency) and then
+// one block a space over the blocks' results.
+constexpr uint32_t kReduceOneBlock = 256;
+struct ReducePlan {
+  unsigned blocks = 1;  // a space, in the first level (last_scale 0: no such level)
+  int lf = 0;
+  int last_quads, last_m, last_lf = 0, last_scale = 0;
+};
+inline ReducePlan reduce_plan(uint32_t K, int S, int sm_count) {
+  ReducePlan p;
+  p.last_m = (int)K;
+  if (K > kReduceOneBlock) {
+    p.lf = 2;
+    auto blocks = [&](int lf) { return K / ((uint32_t)kReduceQuads << lf); };
+    while (blocks(p.lf) > 1 && ((size_t)S * blocks(p.lf) > (size_t)sm_count * 4 || blocks(p.lf) > 1024u)) ++p.lf;
+    p.blocks = blocks(p.lf);
+    p.last_m = (int)p.blocks;
+    for (uint32_t len = (uint32_t)kReduceQuads << p.lf; len > 1; len >>= 1) ++p.last_scale;
+  }
+  while ((p.last_m >> p.last_lf) > kReduceQuads) ++p.last_lf;
+  p.last_quads = std::max(8, p.last_m >> p.last_lf);  // whole warps
+  return p;
+}
+inline size_t reduce_smem(int quads) { return (size_t)quads * sizeof(Xyzz); }
 
 template <class T>
 inline unsigned blocks_for(size_t n, int threads) {
@@ -1545,23 +1614,14 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
 
   const size_t nseg =
       std::max<size_t>(1, std::min(acc_resident_threads(c), (emax + kAccSegMin - 1) / kAccSegMin));
-  constexpr int kFoldLen = 8;
   uint32_t* ikeys[2] = {c.scratch[S_HEAD].as<uint32_t>(2 * nseg), c.scratch[S_TAIL].as<uint32_t>(2 * nseg)};
   Xyzz* ipts[2] = {c.scratch[S_TMP0].as<Xyzz>(2 * nseg), c.scratch[S_TMP1].as<Xyzz>(2 * nseg)};
   uint8_t* ipres[2] = {c.scratch[S_FLAGS].as<uint8_t>(2 * nseg), c.scratch[S_TMP2].as<uint8_t>(2 * nseg)};
 
-  int fan_log = 0;
-  while ((1 << fan_log) < kLevelFan) ++fan_log;
-  int levels = 0;
-  for (int M = (int)K;; M = (M + kLevelFan - 1) / kLevelFan) {
-    ++levels;
-    if (M <= kLevelFan) break;
-  }
-  Xyzz* tsum = c.scratch[S_TSUM].as<Xyzz>((size_t)levels * S);
-  const int G0 = ((int)K + kLevelFan - 1) / kLevelFan;
-  Xyzz* outT = c.scratch[S_LEVEL_T].as<Xyzz>((size_t)S * G0);
-  Xyzz* lvlA = c.scratch[S_LEVEL_A].as<Xyzz>((size_t)S * G0);
-  Xyzz* lvlB = c.scratch[S_LEVEL_B].as<Xyzz>((size_t)S * G0);
+  const ReducePlan rp = reduce_plan(K, S, c.sm_count);
+  Xyzz* tsum = c.scratch[S_TSUM].as<Xyzz>(S);
+  Xyzz* lvlT = c.scratch[S_LEVEL_T].as<Xyzz>((size_t)S * rp.blocks);
+  Xyzz* lvlR = c.scratch[S_LEVEL_A].as<Xyzz>((size_t)S * rp.blocks);
 
   cudaEvent_t t_total = c.timer_begin();
   APG_CUDA(cudaMemsetAsync(counts, 0, (nbins + 1) * sizeof(uint32_t), c.stream));
@@ -1647,42 +1707,20 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
          (uint32_t)nbins, (const uint32_t*)total, nseg, src, buckets, ikeys[0], ipts[0], ipres[0], pair_mode,
          pair_ends, pair_pts);
   c.timer_end(APG_TIMER_MSM_ACCUMULATE, t_acc);
-  {
-    size_t len = 2 * nseg;
-    int cur = 0;
-    for (size_t fseg = nseg; fseg > 1;) {
-      fseg = (len + kFoldLen - 1) / kFoldLen;
-      launch(c, k_fold_edges, blocks_for<int>(fseg, 128), 128, 0, (const uint32_t*)ikeys[cur],
-             (const Xyzz*)ipts[cur], (const uint8_t*)ipres[cur], len, kFoldLen, fseg, buckets, ikeys[cur ^ 1],
-             ipts[cur ^ 1], ipres[cur ^ 1]);
-      cur ^= 1;
-      len = 2 * fseg;
-    }
+  for (size_t len = 2 * nseg, cur = 0; len > 2; cur ^= 1) {
+    const FoldLevel f = fold_level(len);
+    launch(c, k_fold_edges, f.blocks, 4 * kFoldQuads, 0, (const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
+           (const uint8_t*)ipres[cur], len, f.per, buckets, ikeys[cur ^ 1], ipts[cur ^ 1], ipres[cur ^ 1]);
+    len = 2 * (size_t)f.blocks;
   }
-  if ((int)K <= kSmallK) {
-    launch(c, k_reduce_small, (unsigned)S, (unsigned)K, 0, (const Xyzz*)buckets, (int)K, tsum);
-    levels = 1;
-  }
-  const Xyzz* lvl_in = buckets;
-  int M = (int)K;
-  for (int l = 0; l < levels && (int)K > kSmallK; ++l) {
-    const int G = (M + kLevelFan - 1) / kLevelFan;
-    Xyzz* outR = (l & 1) ? lvlB : lvlA;
-    launch(c, k_level, blocks_for<int>((size_t)S * G, 64), 64, 0, lvl_in, M, S, kLevelFan, outT, outR);
-    if (G > 256) {
-      // Wide levels: a two-stage tree keeps the serial chain short.
-      const int nblk = (G + 255) / 256;
-      Xyzz* part = c.scratch[S_TMP3].as<Xyzz>((size_t)S * nblk);
-      launch(c, k_sum_blocks, dim3(nblk, S), 128, 0, (const Xyzz*)outT, G, part);
-      launch(c, k_sum, S, 128, 0, (const Xyzz*)part, nblk, tsum + (size_t)l * S);
-    } else {
-      launch(c, k_sum, S, 128, 0, (const Xyzz*)outT, G, tsum + (size_t)l * S);
-    }
-    lvl_in = outR;
-    M = G;
-  }
-  launch(c, k_finish_cols, blocks_for<int>(nout, 32), 32, 0, (const Xyzz*)tsum, levels, S, spaces_per_col, nout,
-         fan_log, p.c, (uint32_t*)d_out, c.d_flags);
+  const bool two_levels = rp.last_scale > 0;
+  if (two_levels)
+    launch(c, k_reduce, dim3(rp.blocks, S), 4 * kReduceQuads, reduce_smem(kReduceQuads), (const Xyzz*)buckets,
+           (const Xyzz*)nullptr, (int)K, rp.lf, 0, 0, lvlT, lvlR);
+  launch(c, k_reduce, dim3(1, S), 4 * rp.last_quads, reduce_smem(rp.last_quads),
+         (const Xyzz*)(two_levels ? lvlR : buckets), (const Xyzz*)(two_levels ? lvlT : nullptr), rp.last_m, rp.last_lf,
+         rp.last_scale, 1, tsum, (Xyzz*)nullptr);
+  launch(c, k_finish, (unsigned)nout, 32, 0, (const Xyzz*)tsum, spaces_per_col, p.c, (uint32_t*)d_out, c.d_flags);
   c.timer_end(APG_TIMER_MSM_TOTAL, t_total);
 }
 
@@ -1781,9 +1819,6 @@ constexpr size_t kNoAllocBins = (size_t)kNoAllocWindows * kNoAllocK;
 constexpr size_t kNoAllocEntries = (size_t)kNoAllocWindows * kNoAllocMaxPoints;
 constexpr int kNoAllocSeg = 16;
 constexpr size_t kNoAllocSegs = (kNoAllocEntries + kNoAllocSeg - 1) / kNoAllocSeg;
-constexpr int kNoAllocG0 = kNoAllocK / kLevelFan;  // 32 groups in the first reduction level
-constexpr int kNoAllocLevels = 3;                  // 256 -> 32 -> 4 -> one group
-
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Byte offsets of every buffer inside the array.
@@ -1802,11 +1837,8 @@ constexpr size_t kOffPts0 = kOffKeys1 + align256(2 * kNoAllocSegs * 4);
 constexpr size_t kOffPts1 = kOffPts0 + align256(2 * kNoAllocSegs * sizeof(Xyzz));
 constexpr size_t kOffPres0 = kOffPts1 + align256(2 * kNoAllocSegs * sizeof(Xyzz));
 constexpr size_t kOffPres1 = kOffPres0 + align256(2 * kNoAllocSegs);
-constexpr size_t kOffLvlT = kOffPres1 + align256(2 * kNoAllocSegs);
-constexpr size_t kOffLvlA = kOffLvlT + align256((size_t)kNoAllocWindows * kNoAllocG0 * sizeof(Xyzz));
-constexpr size_t kOffLvlB = kOffLvlA + align256((size_t)kNoAllocWindows * kNoAllocG0 * sizeof(Xyzz));
-constexpr size_t kOffTsum = kOffLvlB + align256((size_t)kNoAllocWindows * kNoAllocG0 * sizeof(Xyzz));
-constexpr size_t kNoAllocBytes = kOffTsum + align256((size_t)kNoAllocLevels * kNoAllocWindows * sizeof(Xyzz));
+constexpr size_t kOffTsum = kOffPres1 + align256(2 * kNoAllocSegs);
+constexpr size_t kNoAllocBytes = kOffTsum + align256((size_t)kNoAllocWindows * sizeof(Xyzz));
 
 }  // namespace
 
@@ -1872,9 +1904,6 @@ int msm_noalloc(const void* d_bases, const void* d_scalars, size_t n, void* d_ou
   uint32_t* ikeys[2] = {(uint32_t*)(s + kOffKeys0), (uint32_t*)(s + kOffKeys1)};
   Xyzz* ipts[2] = {(Xyzz*)(s + kOffPts0), (Xyzz*)(s + kOffPts1)};
   uint8_t* ipres[2] = {s + kOffPres0, s + kOffPres1};
-  Xyzz* outT = (Xyzz*)(s + kOffLvlT);
-  Xyzz* lvlA = (Xyzz*)(s + kOffLvlA);
-  Xyzz* lvlB = (Xyzz*)(s + kOffLvlB);
   Xyzz* tsum = (Xyzz*)(s + kOffTsum);
 
   const int K = kNoAllocK, W = kNoAllocWindows, spaces = W;
@@ -1901,34 +1930,18 @@ int msm_noalloc(const void* d_bases, const void* d_scalars, size_t n, void* d_ou
                                                             kNoAllocSeg, nseg, (const Affine*)bases, buckets,
                                                             ikeys[0], ipts[0], ipres[0]);
   APG_NA_LAUNCH();
-  {
-    constexpr int kFold = 8;
-    size_t len = 2 * nseg;
-    int cur = 0;
-    for (size_t fseg = nseg; fseg > 1;) {
-      fseg = (len + kFold - 1) / kFold;
-      k_fold_edges<<<blocks_for<int>(fseg, 128), 128, 0, st>>>((const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
-                                                               (const uint8_t*)ipres[cur], len, kFold, fseg, buckets,
-                                                               ikeys[cur ^ 1], ipts[cur ^ 1], ipres[cur ^ 1]);
-      APG_NA_LAUNCH();
-      cur ^= 1;
-      len = 2 * fseg;
-    }
-  }
-  const Xyzz* lvl_in = buckets;
-  int M = K;
-  for (int l = 0; l < kNoAllocLevels; ++l) {
-    int G = (M + kLevelFan - 1) / kLevelFan;
-    Xyzz* outR = (l & 1) ? lvlB : lvlA;
-    k_level<<<blocks_for<int>((size_t)spaces * G, 64), 64, 0, st>>>(lvl_in, M, spaces, kLevelFan, outT, outR);
-    k_sum<<<spaces, 128, 0, st>>>((const Xyzz*)outT, G, tsum + (size_t)l * spaces);
+  for (size_t len = 2 * nseg, cur = 0; len > 2; cur ^= 1) {
+    const FoldLevel f = fold_level(len);
+    k_fold_edges<<<f.blocks, 4 * kFoldQuads, 0, st>>>((const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
+                                                      (const uint8_t*)ipres[cur], len, f.per, buckets, ikeys[cur ^ 1],
+                                                      ipts[cur ^ 1], ipres[cur ^ 1]);
     APG_NA_LAUNCH();
-    lvl_in = outR;
-    M = G;
+    len = 2 * (size_t)f.blocks;
   }
-  int fan_log = 0;
-  while ((1 << fan_log) < kLevelFan) ++fan_log;
-  k_finish<<<1, 32, 0, st>>>((const Xyzz*)tsum, kNoAllocLevels, spaces, fan_log, kNoAllocC, (uint32_t*)d_out, flags);
+  k_reduce<<<dim3(1, spaces), 4 * kReduceQuads, reduce_smem(kReduceQuads), st>>>(
+      (const Xyzz*)buckets, (const Xyzz*)nullptr, K, 2, 0, 1, tsum, (Xyzz*)nullptr);
+  APG_NA_LAUNCH();
+  k_finish<<<1, 32, 0, st>>>((const Xyzz*)tsum, spaces, kNoAllocC, (uint32_t*)d_out, flags);
   APG_NA_LAUNCH();
   uint32_t f = 0;
   APG_NA(cudaMemcpyAsync(&f, flags, 4, cudaMemcpyDeviceToHost, st));
@@ -1939,8 +1952,7 @@ int msm_noalloc(const void* d_bases, const void* d_scalars, size_t n, void* d_ou
   return APG_OK;
 }
 
-static_assert(kNoAllocLevels == 3 && kNoAllocK / kLevelFan / kLevelFan <= kLevelFan,
-              "the reduction plan above assumes 256 buckets folded 8 at a time");
+static_assert(kNoAllocK == 4 * kReduceQuads, "the reduction above is one block a window");
 
 }  // namespace
 
