@@ -52,8 +52,6 @@ int guarded(apg_ctx* ctx, F&& f) {
 // Mercury's instance rule (crates/pcs-verify/src/lib.rs:97-102).
 bool mercury_num_vars_ok(size_t nv) { return nv >= 2 && nv <= 54 && nv % 2 == 0; }
 
-const SrsTable* commit_table(Ctx& c, size_t n) { return srs_table_for(c, n); }
-
 int commit_common(Ctx& c, const void* evals, bool on_device, bool small, size_t num_vars, uint8_t* out) {
   if (!out || (!evals && num_vars > 0)) return APG_ERR_INVALID_ARGUMENT;
   if (!mercury_num_vars_ok(num_vars)) {
@@ -73,7 +71,7 @@ int commit_common(Ctx& c, const void* evals, bool on_device, bool small, size_t 
     APG_CUDA(cudaMemcpyAsync(buf, evals, n * elem, cudaMemcpyHostToDevice, c.stream));
     d = buf;
   }
-  const SrsTable* t = commit_table(c, n);
+  const SrsTable* t = srs_table_for(c, n, 1);
   if (!t) throw Error(APG_ERR_INTERNAL, "no SRS window table");
   msm_device(c, nullptr, t, d, small, false, n, nullptr, out);
   return APG_OK;
@@ -142,6 +140,7 @@ void apg_ctx_destroy(apg_ctx* ctx) {
     for (auto& b : c.scratch) b.release();
     for (auto& t : c.tables)
       if (t.owned) cudaFree(t.tab);
+    for (auto& t : c.retired) cudaFree(t.tab);
     if (c.srs && c.srs_owned) cudaFree(c.srs);
     if (c.d_flags) cudaFree(c.d_flags);
     if (c.pinned) cudaFreeHost(c.pinned);
@@ -167,6 +166,8 @@ static void drop_srs(Ctx& c) {
   for (auto& t : c.tables)
     if (t.owned) cudaFree(t.tab);
   c.tables.clear();
+  for (auto& t : c.retired) cudaFree(t.tab);
+  c.retired.clear();
   if (c.srs && c.srs_owned) cudaFree(c.srs);
   c.srs = nullptr;
   c.srs_n = 0;
@@ -269,9 +270,10 @@ int apg_srs_prepare(apg_ctx* ctx, int cbits) {
   return guarded(ctx, [&](Ctx& c) {
     if (!c.srs) return (int)APG_ERR_NO_SRS;
     if (cbits == 0) {
-      srs_table(c, 8, std::min(c.srs_n, (size_t)1 << 14));
-      if (c.srs_n > ((size_t)1 << 14)) srs_table(c, 16, c.srs_n);
-      if (c.srs_n >= kWideTableMin) srs_table(c, 20, c.srs_n);
+      srs_table(c, 8, std::min(c.srs_n, kNarrowTableMax));
+      if (c.srs_n > kNarrowTableMax)
+        for (int w : {13, 15}) srs_table(c, w, std::min(c.srs_n, kWideTableMin));
+      if (c.srs_n >= kWideTableMin) srs_table(c, 17, c.srs_n);
     } else {
       if (cbits < 2 || cbits > 20) return (int)APG_ERR_INVALID_ARGUMENT;
       srs_table(c, cbits, c.srs_n);
@@ -344,7 +346,7 @@ static int commit_stack_common(Ctx& c, const void* const* cols, const size_t* nu
     }
     if (!cols[j]) return APG_ERR_INVALID_ARGUMENT;
   }
-  const SrsTable* t = srs_table_for(c, n * k);
+  const SrsTable* t = srs_table_for(c, n * k, 1);
   if (!t) throw Error(APG_ERR_INTERNAL, "no SRS window table");
   std::vector<const void*> ptrs(cols, cols + k);
   if (!on_device) {
@@ -393,7 +395,7 @@ int apg_commit_narrow(apg_ctx* ctx, const void* vals, int bits, size_t num_vars,
     const size_t bytes = bits == 1 ? 8 * ((n + 63) / 64) : n * (size_t)bits / 8;
     void* buf = c.scratch[S_SCALARS].get(bytes);
     APG_CUDA(cudaMemcpyAsync(buf, vals, bytes, cudaMemcpyHostToDevice, c.stream));
-    const SrsTable* t = commit_table(c, n);
+    const SrsTable* t = srs_table_for(c, n, 1);
     if (!t) throw Error(APG_ERR_INTERNAL, "no SRS window table");
     const void* ptr = buf;
     MsmBatchOpts o;
@@ -447,10 +449,21 @@ static void release_lane(Ctx& c) {
   c.lane.reset();
 }
 
-// Groups a batch commit is split into (build knob for measurement).
-#ifndef APG_BATCH_GROUPS
-#define APG_BATCH_GROUPS 4
+// Columns a group of a batch commit takes. Groups alternate between two lanes
+// so that one's latency-bound tail (and the next group's copies) overlaps
+// another's accumulation, which pays once an accumulation is much longer than a
+// tail: a batch is split into as many groups of 2^26 possible digits as it has,
+// four at most. Measured on a GB300 against four groups always: four 2^8-point
+// columns 436 -> 219 us, sixteen of 2^12 894 -> 395, eight of 2^18 3.4 -> 2.5
+// ms (2^23 digits a group) -> 2.5; groups of 2^27 overflow the pair rounds'
+// lists on uniform columns (2 x 2^22: 18.1 -> 24.4 ms).
+#ifndef APG_GROUP_MIN_ENTRIES
+#define APG_GROUP_MIN_ENTRIES ((size_t)1 << 26)
 #endif
+static size_t commit_group(size_t k, size_t n) {
+  const size_t groups = std::min<size_t>(4, std::max<size_t>(1, k * n * 16 / APG_GROUP_MIN_ENTRIES));
+  return std::max<size_t>(1, (k + groups - 1) / groups);
+}
 
 // k commits of one size over the resident SRS. Columns go in groups (one
 // sort, accumulation and bucket reduction per group) that alternate between
@@ -465,7 +478,7 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   const size_t n = (size_t)1 << num_vars;
   if (c.srs_n < n) return APG_ERR_SRS_TOO_SMALL;
   if (k == 0) return APG_OK;
-  if (!commit_table(c, n)) throw Error(APG_ERR_INTERNAL, "no SRS window table");
+  if (!srs_table_for(c, n, k)) throw Error(APG_ERR_INTERNAL, "no SRS window table");
   Ctx& L = lane_of(c);
   Ctx* lanes[2] = {&c, &L};
   uint8_t* d_out = c.scratch[S_TMP5].as<uint8_t>(64 * k);
@@ -474,7 +487,7 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   APG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   APG_CUDA(cudaEventRecord(ev, c.stream));
   APG_CUDA(cudaStreamWaitEvent(L.stream, ev, 0));
-  const size_t group = std::max<size_t>(1, (k + APG_BATCH_GROUPS - 1) / APG_BATCH_GROUPS);
+  const size_t group = commit_group(k, n);
   const size_t ngroups = (k + group - 1) / group;
   std::vector<const void*> ptrs(cols, cols + k);
   std::vector<size_t> lens(k, n);
@@ -499,7 +512,7 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   for (size_t j0 = 0, gi = 0; j0 < k; j0 += group, ++gi) {
     Ctx& X = *lanes[gi & 1];
     const size_t m = std::min(group, k - j0);
-    const SrsTable* t = commit_table(X, n);
+    const SrsTable* t = srs_table_for(X, n, k);
     if (host) APG_CUDA(cudaStreamWaitEvent(X.stream, landed[gi], 0));
     msm_multi(X, nullptr, t, ptrs.data() + j0, lens.data() + j0, m, false, false, d_out + 64 * j0);
   }
@@ -727,6 +740,7 @@ static size_t ctx_bytes(const Ctx& c) {
   for (const auto& d : c.scratch) b += d.cap;
   for (const auto& t : c.tables)
     if (t.owned) b += (size_t)t.windows * t.n * sizeof(Affine);
+  for (const auto& t : c.retired) b += (size_t)t.windows * t.n * sizeof(Affine);
   if (c.srs && c.srs_owned) b += c.srs_n * sizeof(Affine);
   if (c.lane) b += ctx_bytes(*c.lane);
   return b;
@@ -1145,12 +1159,12 @@ size_t apg_shard_device_bytes(const apg_shard* sh) {
     const size_t n = (size_t)1 << sh->num_vars, k = sh->n_cols;
     size_t b = sh->cols_on_device ? 0 : 32 * n * k;  // the staged columns
     b += gkr_device_bytes_impl(sh->circuit, sh->circuit_len);
-    // The commits' two lanes: a group of ceil(k / 4) columns sorts up to 15
-    // windows a point (4-byte references), and the affine pair rounds hold
+    // The commits' two lanes: a group of columns sorts up to 17 windows a
+    // point (4-byte references; 32 below 2^12 points), and the affine pair rounds hold
     // two point lists and the running products at about half and a quarter
     // of that (capped as msm.cu caps them), plus buckets and levels.
-    const size_t g = (k + 3) / 4;
-    const size_t E = std::min<size_t>((size_t)15 * n * g, (size_t)1 << 28);
+    const size_t g = commit_group(k, n);
+    const size_t E = std::min<size_t>((size_t)(n <= kNarrowTableMax ? 32 : 17) * n * g, (size_t)1 << 28);
     const size_t cap = (size_t)48 << 20;
     size_t lane = 4 * E + ((size_t)96 << 20);
     if (E >= ((size_t)1 << 21))

@@ -127,6 +127,7 @@ struct Ctx {
   size_t srs_n = 0;
   bool srs_owned = true;  // false: borrowed from another context (apg_srs_share)
   std::vector<SrsTable> tables;
+  std::vector<SrsTable> retired;  // owned tables a larger one replaced (srs_table)
   // Window width chosen by apg_msm_autotune per size class (index: ceil of
   // log2 of the point count); 0 = the default rule of srs_table_for.
   int tuned_c[64] = {0};
@@ -221,17 +222,14 @@ void generate_srs(Ctx& c, const uint8_t tau_canonical[32], size_t n, Affine* dst
 // kind 0 trace-like (bits, register words, uniform Fr), kind 1 uniform Fr.
 void synth_column(Ctx& c, uint64_t seed, int kind, size_t n, void* d_out);
 
-// Pippenger over device inputs; the result (canonical affine bytes, 64) is
-// written to device memory `out64` when non-null and returned to `host_out`
-// when non-null.
 struct MsmPlan {
   int c;         // window width
   int windows;   // signed-digit windows
   bool precomp;  // read bases from an SRS window table
+  uint32_t buckets;  // a space: 2^(c-1), or fewer when no digit can reach them
 };
-MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table);
-void msm_device(Ctx& c, const Affine* bases, const SrsTable* table, const void* scalars, bool small_scalars,
-                bool scalars_canonical, size_t n, uint8_t* out64_device, uint8_t* host_out);
+// `bits`: the width of small scalars.
+MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits);
 // k MSMs over the same bases (lens[j] scalars each, device pointers); result
 // j is written to d_out + 64 * j. Columns are processed in groups that share
 // one sort, one accumulation and one bucket reduction.
@@ -239,20 +237,35 @@ struct MsmBatchOpts {
   const size_t* offs = nullptr;  // first base of each column (nullable: all 0)
   bool stack = false;            // one result: the sum of every column's MSM
   int bits = 32;                 // width of small scalars: 32, 16, 8 or 1 (bit-packed u64)
+  bool uniform = false;          // field elements without structure (nearly every digit nonzero)
 };
 void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* const* scalars, const size_t* lens,
                size_t k, bool small_scalars, bool scalars_canonical, uint8_t* d_out,
                const MsmBatchOpts& o = MsmBatchOpts());
+// Pippenger over device inputs; the result (canonical affine bytes, 64) is
+// written to device memory `out64` when non-null and returned to `host_out`
+// when non-null.
+void msm_device(Ctx& c, const Affine* bases, const SrsTable* table, const void* scalars, bool small_scalars,
+                bool scalars_canonical, size_t n, uint8_t* out64_device, uint8_t* host_out,
+                const MsmBatchOpts& o = MsmBatchOpts());
 const SrsTable* srs_table(Ctx& c, int cbits, size_t need);
-// The table an MSM of the first n SRS powers reads: 8-bit windows up to 2^14
-// points (a cheap bucket reduction), 16-bit windows below kWideTableMin and
-// 20-bit windows from there (13 windows instead of 16; the 2^19 buckets a
-// column are amortised over at least 2^20 points). Null if the SRS is short.
+// The table that `cols` MSMs over the first n SRS powers read together: 8-bit
+// windows up to 2^12 points (a cheap bucket reduction), 17-bit windows from
+// kWideTableMin, and between them 15-bit windows for one or two columns and
+// 13-bit ones for more, which pay the reduction of each column's buckets. 15 and
+// 17 divide the 255 bits of a signed scalar (17 and 15 windows: 16 and 18 bits
+// take as many digits over twice the buckets). Measured on a GB300, us: one
+// 2^12-point column 244 at 8 bits, 279 at 13; 2^16 alone 395 at 13, 401 at 15
+// (uniform 578, 532), sixteen 1509, 1711 (uniform 3420, 3496); sixteen of 2^14
+// 930, 1140; sixteen of 2^18 3654 at 13, 4114 at 17, uniform 12024, 10675; 2^20
+// alone 1394 at 17, 1402 at 16, 1881 at 20 (uniform 3142, 3254, 3453); 2^22 3264
+// at 17, 3433 at 16, 3626 at 20 (uniform 10124, 10811, 10108).
 // `tuned`: use the width apg_msm_autotune chose for the size class, if any
 // (commits of the caller's columns); openings commit uniformly random
 // quotient polynomials, for which the default rule is the uniform-scalar one.
-constexpr size_t kWideTableMin = (size_t)1 << 20;
-const SrsTable* srs_table_for(Ctx& c, size_t n, bool tuned = true);
+constexpr size_t kNarrowTableMax = (size_t)1 << 12;
+constexpr size_t kWideTableMin = (size_t)1 << 18;
+const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned = true);
 // Time SRS commits of the first 2^k sample scalars for k in [kmin, kmax] with
 // each candidate width and record the fastest in c.tuned_c (see
 // apg_msm_autotune).

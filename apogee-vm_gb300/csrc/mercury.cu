@@ -228,9 +228,11 @@ void srs_commit(Ctx& c, const Fr* d, size_t len, uint8_t out[64]) {
     memset(out, 0, 64);
     return;
   }
-  const SrsTable* t = srs_table_for(c, len, false);
+  const SrsTable* t = srs_table_for(c, len, 1, false);
   if (!t) throw Error(APG_ERR_SRS_TOO_SMALL, "the SRS holds fewer powers than the polynomial has coefficients");
-  msm_device(c, nullptr, t, d, false, false, len, nullptr, out);
+  MsmBatchOpts o;
+  o.uniform = true;  // an opening's polynomials are combinations at random points
+  msm_device(c, nullptr, t, d, false, false, len, nullptr, out, o);
 }
 
 // Two independent SRS MSMs in one group (one sort, accumulation and bucket
@@ -242,12 +244,14 @@ void srs_commit2(Ctx& c, const Fr* d0, size_t len0, const Fr* d1, size_t len1, u
     srs_commit(c, d1, len1, out1);
     return;
   }
-  const SrsTable* t = srs_table_for(c, std::max(len0, len1), false);
+  const SrsTable* t = srs_table_for(c, std::max(len0, len1), 2, false);
   if (!t) throw Error(APG_ERR_SRS_TOO_SMALL, "the SRS holds fewer powers than the polynomial has coefficients");
   const void* ptrs[2] = {d0, d1};
   const size_t lens[2] = {len0, len1};
   uint8_t* d_out = c.scratch[S_RESULT].as<uint8_t>(128);
-  msm_multi(c, nullptr, t, ptrs, lens, 2, false, false, d_out);
+  MsmBatchOpts o;
+  o.uniform = true;
+  msm_multi(c, nullptr, t, ptrs, lens, 2, false, false, d_out, o);
   uint8_t both[128];
   APG_CUDA(cudaMemcpyAsync(both, d_out, 128, cudaMemcpyDeviceToHost, c.stream));
   c.check_flags();

@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(128) k_accumulate(const uint64_t* sorted, cons
 // addition against 2.3). Measured on a GB300, all levels together: 251 -> 90 us
 // for a 2^16-point commit (155,000 items), 153 -> 38 for a 2^8-point one.
 constexpr int kFoldQuads = 64;
-constexpr int kFoldLastPer = 4;  // items a quad at most in a level of one block
+constexpr int kFoldLastPer = 8;  // items a quad at most in a level of one block
 
 __global__ void __launch_bounds__(4 * kFoldQuads) k_fold_edges(const uint32_t* keys, const Xyzz* pts,
                                                                const uint8_t* pres, size_t len, int per,
@@ -605,8 +605,8 @@ __device__ __forceinline__ uint32_t small_scalar(const void* col, uint32_t i, in
 // window's atomic issued before the first result is awaited (no change in
 // either pass at 2^22).
 template <bool SMALL, bool SCATTER>
-__global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows, int precomp, uint32_t tab_n,
-                                                int canonical_in, uint32_t* cursor, uint32_t* sorted,
+__global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows, int precomp, uint32_t stride,
+                                                uint32_t tab_n, int canonical_in, uint32_t* cursor, uint32_t* sorted,
                                                 uint32_t* flags) {
   const uint32_t col = blockIdx.y;
   const uint32_t n = cols.len[col];
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows
   const uint32_t K = 1u << (c - 1);
   const uint32_t mask = (1u << c) - 1;
   const uint32_t spaces = precomp ? 1u : (uint32_t)windows;
-  const uint32_t key0 = cols.shared ? 0u : col * spaces * K;
+  const uint32_t key0 = cols.shared ? 0u : col * spaces * stride;
   const uint32_t base_i = cols.off[col] + i;
   uint32_t carry = 0;
   for (int w = 0; w < windows; ++w) {
@@ -654,13 +654,13 @@ __global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows
       carry = 1;
     }
     if (!live) mag = 0;
-    if (mag > K) {  // unreachable for values below r; never index past the bucket range
+    if (mag > stride) {  // unreachable for values below r; never index past the bucket range
       if (!SCATTER) raise_flag(flags, DEV_NONCANONICAL);
       mag = 0;
     }
     const unsigned active = __ballot_sync(0xffffffffu, mag != 0);
     if (mag) {
-      const uint32_t key = key0 + (precomp ? 0u : (uint32_t)w * K) + mag - 1;
+      const uint32_t key = key0 + (precomp ? 0u : (uint32_t)w * stride) + mag - 1;
       const unsigned peers = __match_any_sync(active, key);
       const int leader = __ffs(peers) - 1;
       if (SCATTER) {
@@ -673,6 +673,74 @@ __global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows
         atomicAdd(&cursor[key], (uint32_t)__popc(peers));
       }
     }
+  }
+}
+
+// The same digits when a column has few buckets (kFewBins at most: 8-bit
+// windows, a generic-base MSM, a narrow column): a block counts its tile of
+// scalars into a histogram in shared memory and touches each bucket's global
+// counter once, to add its count or, when it places, to reserve that many
+// slots and hand them out from shared memory. The warp-wide form above matches
+// lanes and waits for a global atomic at every window, and with few buckets all
+// warps wait for the same counters (2^20 one-byte scalars: 215 -> 12 us a
+// pass; 2^8 scalars of 32 windows: 12.7 and 18.5 -> 6.5 and 8 us).
+constexpr uint32_t kFewBins = 8192;  // 32 KB of counters
+
+template <bool SMALL, bool SCATTER>
+__global__ void __launch_bounds__(256) k_digits_few(MsmCols cols, int c, int windows, int precomp, uint32_t stride,
+                                                    uint32_t tab_n, int canonical_in, uint32_t tile, uint32_t* cursor,
+                                                    uint32_t* sorted, uint32_t* flags) {
+  extern __shared__ uint32_t bins[];
+  const uint32_t col = blockIdx.y;
+  const uint32_t n = cols.len[col];
+  const uint32_t lo = blockIdx.x * tile, hi = min(lo + tile, n);
+  if (lo >= n) return;
+  const uint32_t spaces = precomp ? 1u : (uint32_t)windows;
+  const uint32_t nb = spaces * stride, key0 = cols.shared ? 0u : col * nb;
+  const uint32_t K = 1u << (c - 1), mask = (1u << c) - 1;
+  for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) bins[b] = 0;
+  __syncthreads();
+  for (int pass = 0; pass < (SCATTER ? 2 : 1); ++pass) {
+    for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+      uint32_t v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = 0;
+      if (SMALL) {
+        v[0] = small_scalar(cols.s[col], i, cols.bits);
+      } else {
+        Fr s = ld_fe(reinterpret_cast<const Fr*>(cols.s[col]) + i);
+        if (!SCATTER && !fe_lt_mod<FrConsts>(s.v)) raise_flag(flags, DEV_NONCANONICAL);
+        if (!canonical_in) s = fe_from_mont(s);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = s.v[k];
+      }
+      uint32_t carry = 0, idx = cols.off[col] + i;
+      for (int w = 0; w < windows; ++w) {
+        const uint32_t coef = (v[0] & mask) + carry;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __funnelshift_r(v[k], k < 7 ? v[k + 1] : 0u, c);
+        const bool neg = w != windows - 1 && coef >= K;  // digit coef - 2^c
+        uint32_t mag = neg ? mask + 1 - coef : coef;
+        carry = neg;
+        if (mag > stride) {  // unreachable for values below r; never index past the bucket range
+          if (!SCATTER) raise_flag(flags, DEV_NONCANONICAL);
+          mag = 0;
+        }
+        if (mag) {
+          uint32_t* bin = &bins[(precomp ? 0u : (uint32_t)w * stride) + mag - 1];
+          if (pass == 0) atomicAdd(bin, 1u);
+          else sorted[atomicAdd(bin, 1u)] = ((uint32_t)neg << 31) | idx;
+        }
+        if (precomp) idx += tab_n;
+      }
+    }
+    __syncthreads();
+    if (pass == 0)
+      for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) {
+        const uint32_t m = bins[b];
+        if (m) bins[b] = atomicAdd(&cursor[key0 + b], m);
+      }
+    __syncthreads();
   }
 }
 
@@ -784,9 +852,18 @@ __global__ void __launch_bounds__(128, APG_ACC_MIN_BLOCKS) k_bucket_acc(const ui
 #define APG_PAIR_ROUNDS 4
 #endif
 constexpr int kPairRounds = APG_PAIR_ROUNDS;
-// Lists shorter than this per group are left to the XYZZ kernel alone (the
-// extra launches would cost more than the products saved).
-constexpr size_t kPairMinEntries = (size_t)1 << 21;
+// Groups of fewer digits are left to the XYZZ kernel alone: the rounds' fixed
+// cost (four inversions and 24 launches, about 450 us) exceeds what they save.
+// Both sides cost the same at about 2^23 digits that are there; the host knows
+// only how many there could be, and a trace column has a quarter of them (bits
+// and 32-bit words), so columns of unknown values take the rounds from twice
+// that. Measured on a GB300 with and without the rounds: one 2^20-point mixed
+// column (16 M possible digits, 4 M real) 1400 and 1160 us, uniform 3133 and
+// 3373; four of 2^18 mixed 1617 and 1366, uniform 3284 and 3597.
+#ifndef APG_PAIR_MIN_ENTRIES
+#define APG_PAIR_MIN_ENTRIES ((size_t)1 << 23)
+#endif
+constexpr size_t kPairMinEntries = APG_PAIR_MIN_ENTRIES;
 // Round 0's output list is held to this many points (64 bytes each).
 constexpr size_t kPairMaxPoints = (size_t)48 << 20;
 
@@ -1352,7 +1429,7 @@ struct FoldLevel {
 inline FoldLevel fold_level(size_t len) {
   const size_t q = kFoldQuads - 1;
   if (len <= q * kFoldLastPer) return {1u, (int)((len + q - 1) / q)};
-  const size_t per = len <= q * q * kFoldLastPer ? 2 : 4;  // (two items leave 2 len / 126 <= 252)
+  const size_t per = len <= q * q * kFoldLastPer ? 2 : 4;  // (two items leave len / 63 <= 504)
   return {(unsigned)((len + q * per - 1) / (q * per)), (int)per};
 }
 
@@ -1447,13 +1524,14 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need) {
   for (auto& t : c.tables)
     if (t.c == cbits && t.n >= need) return &t;
   if (!c.srs || c.srs_n < need) return nullptr;
-  // The wide table covers the whole SRS, a narrow one a 2^16 prefix.
-  size_t n = cbits >= 12 ? c.srs_n : std::min(c.srs_n, (size_t)1 << 16);
+  // A wide table covers the whole SRS, a narrower one the prefix that the
+  // default rule reads it for until a caller needs more. The prefix's table is
+  // then kept until the SRS goes: contexts that share it may still read it.
+  size_t n = cbits >= 16 ? c.srs_n : std::min(c.srs_n, cbits >= 12 ? kWideTableMin : (size_t)1 << 16);
   if (n < need) n = c.srs_n;
   for (auto it = c.tables.begin(); it != c.tables.end(); ++it)
     if (it->c == cbits) {
-      APG_CUDA(cudaStreamSynchronize(c.stream));
-      if (it->owned) cudaFree(it->tab);
+      if (it->owned) c.retired.push_back(*it);
       c.tables.erase(it);
       break;
     }
@@ -1477,21 +1555,17 @@ static int ceil_log2(size_t n) {
   return k;
 }
 
-const SrsTable* srs_table_for(Ctx& c, size_t n, bool tuned) {
+const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned) {
   const int cls = ceil_log2(n);
   if (tuned && cls < 64 && c.tuned_c[cls]) {
     const SrsTable* t = srs_table(c, c.tuned_c[cls], n);
     if (t) return t;
   }
-  if (n <= ((size_t)1 << 14)) {
+  if (n <= kNarrowTableMax) {
     const SrsTable* t = srs_table(c, 8, n);
     if (t) return t;
   }
-  if (n >= kWideTableMin) {
-    const SrsTable* t = srs_table(c, 20, n);
-    if (t) return t;
-  }
-  return srs_table(c, 16, n);
+  return srs_table(c, n >= kWideTableMin ? 17 : cols <= 2 ? 15 : 13, n);
 }
 
 void msm_autotune(Ctx& c, const void* d_sample, size_t sample_len, int kmin, int kmax, const int* cands,
@@ -1532,17 +1606,16 @@ void msm_autotune(Ctx& c, const void* d_sample, size_t sample_len, int kmin, int
   cudaEventDestroy(e1);
 }
 
-MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table) {
+MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits) {
   MsmPlan p;
-  if (table) {
-    p.c = table->c;
-    p.windows = small_scalars ? window_count(32, table->c) : table->windows;
-    p.precomp = true;
-  } else {
-    p.c = default_window(n, small_scalars);
-    p.windows = window_count(small_scalars ? 32 : 254, p.c);
-    p.precomp = false;
-  }
+  p.c = table ? table->c : default_window(n, small_scalars);
+  p.precomp = table != nullptr;
+  p.windows = small_scalars ? window_count(bits, p.c) : table ? table->windows : window_count(254, p.c);
+  // A scalar narrower than the window has one digit, itself, and fills no
+  // bucket past its own range (one-byte columns over 17-bit windows: 2^8 of
+  // 2^16 buckets to scan and reduce).
+  p.buckets = 1u << (p.c - 1);
+  if (small_scalars && bits < p.c) p.buckets = std::min(p.buckets, 1u << bits);
   return p;
 }
 
@@ -1584,18 +1657,15 @@ constexpr size_t kMaxGroupEntries = (size_t)1 << 28;                           /
 
 // The accumulation's slices hold at least this many references: a group too
 // small to fill the resident wave gets fewer, longer slices, trading serial
-// additions a thread against levels of the edge fold. Measured on a GB300 over
-// 2^12 openings and 2^8-2^14-row shards: 4 beat 16 (4.85 -> 4.61 ms an
-// opening at 2^12) and tied 2.
-#ifndef APG_ACC_SEG_MIN
-#define APG_ACC_SEG_MIN 4
-#endif
-constexpr size_t kAccSegMin = APG_ACC_SEG_MIN;
+// additions a thread against items for the edge fold. Measured on a GB300: one
+// 2^8-point uniform column 193 us at four and 215 at eight, one 2^12-point column
+// 242 and 216, two 309 and 258.
+inline size_t acc_slice_min(size_t entries) { return entries <= ((size_t)1 << 15) ? 4 : 8; }
 
 // One group: columns share the plan, the bases and one pass of every kernel.
 void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols& cols, int ncols, size_t nmax,
-               const MsmPlan& p, bool small_scalars, bool scalars_canonical, uint8_t* d_out) {
-  const uint32_t K = 1u << (p.c - 1);
+               const MsmPlan& p, bool small_scalars, bool scalars_canonical, bool uniform, uint8_t* d_out) {
+  const uint32_t K = p.buckets;
   const int spaces_per_col = p.precomp ? 1 : p.windows;
   const int nout = cols.shared ? 1 : ncols;  // results: one per column, or the stack's sum
   const int S = spaces_per_col * nout;
@@ -1612,8 +1682,9 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   uint32_t* sorted = c.scratch[S_SORTED].as<uint32_t>(std::max<size_t>(emax, 1));
   Xyzz* buckets = c.scratch[S_BUCKETS].as<Xyzz>(nbins);
 
+  const size_t slice_min = acc_slice_min(emax);
   const size_t nseg =
-      std::max<size_t>(1, std::min(acc_resident_threads(c), (emax + kAccSegMin - 1) / kAccSegMin));
+      std::max<size_t>(1, std::min(acc_resident_threads(c), (emax + slice_min - 1) / slice_min));
   uint32_t* ikeys[2] = {c.scratch[S_HEAD].as<uint32_t>(2 * nseg), c.scratch[S_TAIL].as<uint32_t>(2 * nseg)};
   Xyzz* ipts[2] = {c.scratch[S_TMP0].as<Xyzz>(2 * nseg), c.scratch[S_TMP1].as<Xyzz>(2 * nseg)};
   uint8_t* ipres[2] = {c.scratch[S_FLAGS].as<uint8_t>(2 * nseg), c.scratch[S_TMP2].as<uint8_t>(2 * nseg)};
@@ -1626,28 +1697,39 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   cudaEvent_t t_total = c.timer_begin();
   APG_CUDA(cudaMemsetAsync(counts, 0, (nbins + 1) * sizeof(uint32_t), c.stream));
   APG_CUDA(cudaMemsetAsync(buckets, 0, nbins * sizeof(Xyzz), c.stream));
-  const dim3 dgrid(blocks_for<int>(std::max<size_t>(nmax, 1), 256), (unsigned)ncols);
   const int canon = scalars_canonical ? 1 : 0;
-  if (small_scalars)
-    launch(c, k_digits<true, false>, dgrid, 256, 0, cols, p.c, p.windows, (int)p.precomp, tab_n, canon, counts,
-           (uint32_t*)nullptr, c.d_flags);
-  else
-    launch(c, k_digits<false, false>, dgrid, 256, 0, cols, p.c, p.windows, (int)p.precomp, tab_n, canon, counts,
-           (uint32_t*)nullptr, c.d_flags);
+  // One pass over the digits: counted (place null) or placed.
+  auto digits = [&](uint32_t* place) {
+    const uint32_t few = (uint32_t)spaces_per_col * K;
+    if (few <= kFewBins) {
+      // Tiles of 256 scalars until they fill the device twice, then up to
+      // eight times as long: a block's counters cost it one pass over them.
+      const size_t tiles = (std::max<size_t>(nmax, 1) + 255) / 256;
+      const uint32_t per = (uint32_t)std::min<size_t>(8, std::max<size_t>(1, tiles * ncols / (2 * (size_t)c.sm_count)));
+      const dim3 grid((unsigned)((tiles + per - 1) / per), (unsigned)ncols);
+      void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t, uint32_t*, uint32_t*, uint32_t*) =
+          small_scalars ? (place ? k_digits_few<true, true> : k_digits_few<true, false>)
+                        : (place ? k_digits_few<false, true> : k_digits_few<false, false>);
+      launch(c, k, grid, 256, few * sizeof(uint32_t), cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, 256 * per,
+             counts, place, c.d_flags);
+    } else {
+      const dim3 grid(blocks_for<int>(std::max<size_t>(nmax, 1), 256), (unsigned)ncols);
+      void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t*, uint32_t*, uint32_t*) =
+          small_scalars ? (place ? k_digits<true, true> : k_digits<true, false>)
+                        : (place ? k_digits<false, true> : k_digits<false, false>);
+      launch(c, k, grid, 256, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place, c.d_flags);
+    }
+  };
+  digits(nullptr);
   launch(c, k_scan_local, (unsigned)scan_blocks, kScanBlock, 0, counts, nbins, blk);
   launch(c, k_scan_blocks, 1, kScanBlock, 0, blk, (int)scan_blocks);
   launch(c, k_scan_add, blocks_for<int>(nbins, 256), 256, 0, counts, nbins, (const uint32_t*)blk, total);
-  if (small_scalars)
-    launch(c, k_digits<true, true>, dgrid, 256, 0, cols, p.c, p.windows, (int)p.precomp, tab_n, canon, counts, sorted,
-           c.d_flags);
-  else
-    launch(c, k_digits<false, true>, dgrid, 256, 0, cols, p.c, p.windows, (int)p.precomp, tab_n, canon, counts,
-           sorted, c.d_flags);
+  digits(sorted);
   cudaEvent_t t_acc = c.timer_begin();
   const uint32_t* pair_mode = nullptr;
   const uint32_t* pair_ends = nullptr;
   const Affine* pair_pts = nullptr;
-  if (kPairRounds > 0 && emax >= kPairMinEntries) {
+  if (kPairRounds > 0 && emax >= kPairMinEntries * (uniform ? 1 : 2)) {
     // Round r's list fits cap[r]: a round keeps ceil(len/2) of each run, so
     // a list never grows and at most halves plus one point per bucket.
     size_t cap[kPairRounds > 0 ? kPairRounds : 1];
@@ -1743,9 +1825,9 @@ void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* c
       const size_t n = lens[j + g];
       if (n >= ((size_t)1 << 31)) throw Error(APG_ERR_INVALID_ARGUMENT, "MSM longer than 2^31 - 1 points");
       const size_t nm = std::max(nmax, n);
-      const MsmPlan q = msm_plan(std::max<size_t>(nm, 1), small_scalars, table);
+      const MsmPlan q = msm_plan(std::max<size_t>(nm, 1), small_scalars, table, o.bits);
       const size_t spaces = q.precomp ? 1 : (size_t)q.windows;
-      const size_t bins = (g + 1) * spaces * ((size_t)1 << (q.c - 1));
+      const size_t bins = (g + 1) * spaces * q.buckets;
       size_t e = 0;
       for (size_t t = 0; t <= g; ++t) e += (size_t)q.windows * lens[j + t];
       if (g > 0 && (bins > kMaxBins || e > kMaxGroupEntries || q.c != p.c || q.windows != p.windows)) break;
@@ -1763,7 +1845,7 @@ void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* c
     cols.shared = o.stack ? 1 : 0;
     cols.bits = o.bits;
     uint8_t* dst = o.stack ? partial + 64 * ngroups : d_out + 64 * j;
-    msm_group(c, bases, table, cols, (int)g, nmax, p, small_scalars, scalars_canonical, dst);
+    msm_group(c, bases, table, cols, (int)g, nmax, p, small_scalars, scalars_canonical, o.uniform, dst);
     ++ngroups;
     j += g;
   }
@@ -1775,14 +1857,14 @@ void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* c
 }
 
 void msm_device(Ctx& c, const Affine* bases, const SrsTable* table, const void* scalars, bool small_scalars,
-                bool scalars_canonical, size_t n, uint8_t* out64_device, uint8_t* host_out) {
+                bool scalars_canonical, size_t n, uint8_t* out64_device, uint8_t* host_out, const MsmBatchOpts& o) {
   if (n == 0) {
     if (out64_device) APG_CUDA(cudaMemsetAsync(out64_device, 0, 64, c.stream));
     if (host_out) memset(host_out, 0, 64);
     return;
   }
   uint8_t* d_out = out64_device ? out64_device : c.scratch[S_RESULT].as<uint8_t>(64);
-  msm_multi(c, bases, table, &scalars, &n, 1, small_scalars, scalars_canonical, d_out);
+  msm_multi(c, bases, table, &scalars, &n, 1, small_scalars, scalars_canonical, d_out, o);
   if (host_out) {
     APG_CUDA(cudaMemcpyAsync(host_out, d_out, 64, cudaMemcpyDeviceToHost, c.stream));
     c.check_flags();

@@ -37,7 +37,7 @@ METRIC = "G1 MSM points/s at 2^22"
 UNIT = "points/s"
 SEED = 20260903
 TAU_SEED = 0x7A75_5EED
-TUNE_WIDTHS = (8, 12, 16, 18, 20)  # window widths the autotuner tries per size class
+TUNE_WIDTHS = (8, 13, 15, 17, 20)  # window widths the autotuner tries per size class
 
 
 def max_over_ranks(x: float, dist, device: str) -> float:
@@ -84,10 +84,10 @@ def algorithmic_fqmul_accumulate(n):
 def own_windows(n, tuned=None):
     """Signed-digit windows of the SRS window table an n-point commit reads:
     the autotuner's width for the size class when it chose one, else the
-    library's default rule (8-bit up to 2^14 points, 16-bit below 2^20,
-    20-bit from 2^20)."""
+    library's default rule for one column (8-bit up to 2^12 points, 15-bit
+    below 2^18, 17-bit from 2^18)."""
     lg = max(0, (n - 1).bit_length())
-    c = (tuned or {}).get(lg) or (8 if n <= 1 << 14 else (16 if n < 1 << 20 else 20))
+    c = (tuned or {}).get(lg) or (8 if n <= 1 << 12 else (15 if n < 1 << 18 else 17))
     return -(-255 // c)
 
 

@@ -55,3 +55,38 @@ def test_reduction_widths_known_tau(ctx, cbits):
     f_tau = sum(c * pow(tau, i, O.P_R) for i, c in enumerate(xs)) % O.P_R
     assert ctx.commit(mem, nv) == O.g1_mul(O.G1_GEN, f_tau)
     assert ctx.commit_batch_device([d.data_ptr()] * 3, nv) == [O.g1_mul(O.G1_GEN, f_tau)] * 3
+
+
+@pytest.mark.parametrize("bits", [1, 8, 16, 32])
+@pytest.mark.parametrize("nv", [2, 8, 12, 14, 18])
+def test_few_bucket_digits_known_tau(ctx, nv, bits):
+    """Narrow columns, whose digits fill few buckets: one scalar a thread, a
+    ragged tile, several tiles a block; random values and all of the largest."""
+    import apogee_gpu as A
+
+    tau, n, p = 0xA5A5A5A5A5, 1 << nv, O.P_R
+    if ctx.srs_len() != 1 << 18:
+        ctx.srs_generate(tau, 1 << 18)
+    rng = random.Random(100 * nv + bits)
+    for vals in ([rng.getrandbits(bits) for _ in range(n)], [(1 << bits) - 1] * n):
+        f_tau, x = 0, 1
+        for v in vals:
+            f_tau, x = (f_tau + v * x) % p, x * tau % p
+        assert ctx.commit_narrow(A.narrow_bytes(vals, bits), bits, nv) == O.g1_mul(O.G1_GEN, f_tau)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "equal"])
+def test_pair_rounds_degenerate_bases(ctx, kind):
+    """2^20 generic bases drawn from {infinity, G, -G, 2G, 3G, 7G}: 17 windows,
+    above the affine pair rounds' least size, so adjacent points of a bucket
+    collide in every way the rounds classify. The value is (sum s_i k_i) G."""
+    import apogee_gpu as A
+
+    rng = random.Random(13)
+    n = 1 << 20
+    ks = [0, 1, O.P_R - 1, 2, 3, 7]
+    pts = {k: (bytes(64) if k == 0 else O.g1_mul(O.G1_GEN, k)) for k in ks}
+    kk = rng.choices(ks, k=n)
+    ss = [rng.randrange(O.P_R)] * n if kind == "equal" else [rng.randrange(O.P_R) for _ in range(n)]
+    want = O.g1_mul(O.G1_GEN, sum(s * k for s, k in zip(ss, kk)) % O.P_R)
+    assert ctx.msm(b"".join(pts[k] for k in kk), A.to_mont_bytes(ss)) == want
