@@ -170,7 +170,7 @@ int accumulator_msms(Ctx& c, const uint8_t* sides, const uint8_t* scalars, const
   const size_t lens[2] = {n, n};
   uint8_t* d_out = c.scratch[S_RESULT].as<uint8_t>(128);
   msm_multi(c, d_pts, nullptr, cols, lens, 2, false, false, d_out);
-  uint8_t* h = static_cast<uint8_t*>(c.host_pinned());
+  uint8_t* h = c.host_pinned() + Ctx::kPinnedTables;
   APG_CUDA(cudaMemcpyAsync(h, d_out, 128, cudaMemcpyDeviceToHost, c.stream));
   c.check_flags();
   memcpy(a_out, h, 64);

@@ -311,9 +311,14 @@ struct Transcript {
     out[out_len] = fzero();
     return r;
   }
-  void absorb(uint64_t tag, const F* xs, size_t n) {
+  // A message of n elements: its tag and length, then the elements. The
+  // first part does not wait for the elements.
+  void open(uint64_t tag, size_t n) {
     observe(from_u64(tag));
     observe(from_u64((uint64_t)n));
+  }
+  void absorb(uint64_t tag, const F* xs, size_t n) {
+    open(tag, n);
     for (size_t i = 0; i < n; ++i) observe(xs[i]);
   }
   void absorb(uint64_t tag, const std::vector<F>& xs) { absorb(tag, xs.data(), xs.size()); }

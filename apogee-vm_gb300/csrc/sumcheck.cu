@@ -42,7 +42,9 @@ struct RoundArgs {
   int slots_step0;           // first step slot
   int n_val_slots;           // nd + nv
   unsigned* done;            // blocks finished this round (zero between rounds)
-  Fr* out;                   // the round's 4 sums, written by the last block
+  Fr* out;                   // the round's sums at nodes 0..2 (pinned host memory), by the last block
+  uint32_t* flag;            // set to seq (pinned host memory) once they are there
+  uint32_t seq;
   int xsplit;                // one thread per (pair, node X) instead of per pair
   const uint8_t* src_bits;   // stored width of each src table (null: all Fr)
   int nodes;                 // bit X set: evaluate the summand at node X (0..2)
@@ -107,38 +109,76 @@ __device__ __forceinline__ Fr at_node(const Fr& lo, const Fr& step, int x) {
   return v;
 }
 
-// After every block has published its 4 partial sums: the last block to
-// finish (it takes the last ticket) adds them all into A.out and re-arms the
-// counter for the next round.
-__device__ __forceinline__ void round_total(const RoundArgs& A, const Fr* partials, Fr* red) {
+// The sum of a value over the warp's (or the narrower block's) lanes, in every lane.
+__device__ __forceinline__ Fr warp_sum(Fr a, int width, unsigned mask) {
+#pragma unroll 1
+  for (int off = width >> 1; off > 0; off >>= 1) {
+    Fr o;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) o.v[w] = __shfl_xor_sync(mask, a.v[w], off);
+    a = fe_add(a, o);
+  }
+  return a;
+}
+
+// The end of a round kernel: warp w's sums at the round's nodes stand in
+// ws[3 w + x]. One thread a node adds them up; with several blocks they go to
+// `partials`, and the last block to finish (it takes the last ticket) adds every
+// block's, a warp a node. The sums land in pinned host memory, then the flag the
+// host spins on; whatever the kernel stored before (a level of tables the host
+// is to read) is visible with it.
+__device__ __forceinline__ void round_finish(const RoundArgs& A, const Fr* ws, int nwarps, Fr* partials) {
   __shared__ bool last;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(A.done, 1u) == gridDim.x - 1;
+  const int x = threadIdx.x;
+  __threadfence_system();
+  __syncthreads();
+  if (x < 3) {
+    Fr a = ws[x];
+    for (int w = 1; w < nwarps; ++w) a = fe_add(a, ws[3 * w + x]);
+    st_fe(gridDim.x == 1 ? &A.out[x] : &partials[(size_t)blockIdx.x * 4 + x], a);
+    __threadfence_system();
   }
   __syncthreads();
+  if (x == 0) last = gridDim.x == 1 || atomicAdd(A.done, 1u) == gridDim.x - 1;
+  __syncthreads();
   if (!last) return;
-  __threadfence();
-  for (int x = 0; x < 4; ++x) {
-    Fr a = fe_zero<FrConsts>();
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-      const uint4* q = reinterpret_cast<const uint4*>(&partials[(size_t)b * 4 + x]);
-      const uint4 u0 = __ldcg(q), u1 = __ldcg(q + 1);
-      Fr v;
-      v.v[0] = u0.x, v.v[1] = u0.y, v.v[2] = u0.z, v.v[3] = u0.w;
-      v.v[4] = u1.x, v.v[5] = u1.y, v.v[6] = u1.z, v.v[7] = u1.w;
-      a = fe_add(a, v);
+  if (gridDim.x > 1) {
+    __threadfence();
+    const int width = min(32, (int)blockDim.x), lane = threadIdx.x & 31;
+    const unsigned mask = width == 32 ? 0xffffffffu : (1u << width) - 1;
+    for (int node = threadIdx.x >> 5; node < 3; node += max(1, (int)blockDim.x >> 5)) {
+      Fr a = fe_zero<FrConsts>();
+      for (unsigned b = lane; b < gridDim.x; b += width) {
+        const uint4* q = reinterpret_cast<const uint4*>(&partials[(size_t)b * 4 + node]);
+        const uint4 u0 = __ldcg(q), u1 = __ldcg(q + 1);
+        Fr v;
+        v.v[0] = u0.x, v.v[1] = u0.y, v.v[2] = u0.z, v.v[3] = u0.w;
+        v.v[4] = u1.x, v.v[5] = u1.y, v.v[6] = u1.z, v.v[7] = u1.w;
+        a = fe_add(a, v);
+      }
+      a = warp_sum(a, width, mask);
+      if (lane == 0) st_fe(&A.out[node], a);
     }
-    red[threadIdx.x] = a;
-    __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-      if (threadIdx.x < (unsigned)off) red[threadIdx.x] = fe_add(red[threadIdx.x], red[threadIdx.x + off]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) st_fe(&A.out[x], red[0]);
+    __threadfence_system();
     __syncthreads();
   }
-  if (threadIdx.x == 0) *A.done = 0;
+  if (x == 0) {
+    *A.done = 0;
+    __threadfence_system();
+    *reinterpret_cast<volatile uint32_t*>(A.flag) = A.seq;
+  }
+}
+
+// Every thread's sums at the three nodes, reduced a warp at a time.
+__device__ __forceinline__ void round_finish_threads(const RoundArgs& A, const Fr acc[3], Fr* ws, Fr* partials) {
+  const int width = min(32, (int)blockDim.x);
+  const unsigned mask = width == 32 ? 0xffffffffu : (1u << width) - 1;
+#pragma unroll 1
+  for (int x = 0; x < 3; ++x) {
+    const Fr a = warp_sum(acc[x], width, mask);
+    if ((threadIdx.x & 31) == 0) ws[3 * (threadIdx.x >> 5) + x] = a;
+  }
+  round_finish(A, ws, max(1, (int)blockDim.x >> 5), partials);
 }
 
 // Resident blocks a SM k_round is compiled for (1: the compiler's choice).
@@ -149,10 +189,10 @@ __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_MIN_BLOCKS)
     k_round(RoundArgs A, DevProgram P, VirtualRound V, Fr* partials) {
   extern __shared__ uint32_t sm_raw[];
   const Slots sm = thread_slots(sm_raw);
-  __shared__ Fr red[kRoundThreads];
-  Fr acc[4];
+  __shared__ Fr ws[3 * kRoundThreads / 32];
+  Fr acc[3];
 #pragma unroll
-  for (int x = 0; x < 4; ++x) acc[x] = fe_zero<FrConsts>();
+  for (int x = 0; x < 3; ++x) acc[x] = fe_zero<FrConsts>();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   if (A.xsplit) {
     // Small rounds: thread t evaluates pair t / 4 at node X = t % 4 alone
@@ -178,15 +218,10 @@ __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_MIN_BLOCKS)
       load_line(A, A.nd, i, e_lo, e_hi, x == 0);
       acc[0] = fe_add(acc[0], fe_mul(fe_add(e_lo, e_hi), eval_summand(P, sm)));
     }
-    // Reduce over threads of the same node: strides that are multiples of 4.
-    red[threadIdx.x] = acc[0];
-    __syncthreads();
-    for (int off = blockDim.x / 2; off >= 4; off >>= 1) {
-      if (threadIdx.x < (unsigned)off) red[threadIdx.x] = fe_add(red[threadIdx.x], red[threadIdx.x + off]);
-      __syncthreads();
+    if (x == 1 || x == 2) {
+      acc[x == 1 ? 1 : 2] = acc[0];
+      acc[0] = fe_zero<FrConsts>();
     }
-    if (threadIdx.x < 4) st_fe(&partials[(size_t)blockIdx.x * 4 + threadIdx.x], red[threadIdx.x]);
-    __syncthreads();
   } else {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < A.npairs; i += stride) {
     Fr lo, hi;
@@ -219,137 +254,94 @@ __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_MIN_BLOCKS)
       }
     }
   }
-  // Block reduction, one node at a time through shared memory.
-  for (int x = 0; x < 4; ++x) {
-    red[threadIdx.x] = acc[x];
-    __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-      if (threadIdx.x < (unsigned)off) red[threadIdx.x] = fe_add(red[threadIdx.x], red[threadIdx.x + off]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) st_fe(&partials[(size_t)blockIdx.x * 4 + x], red[0]);
-    __syncthreads();
   }
-  }
-  round_total(A, partials, red);
+  round_finish_threads(A, acc, ws, partials);
 }
 
-// A summand S = sum_j c_j T_{a_j} T_{b_j} over data tables only (halving
-// lists of tree gates, a zerocheck's product gate): thread per pair, each
-// term's two lines read (and folded with the previous challenge) straight
-// into registers and multiplied at the round's nodes, with no operand slots
-// and no interpreter. Tables no term reads are folded too, so every table
-// is bound each round as the generic kernel binds it.
+// The terms of a short quadratic form (HostPairTerms) on the device.
 struct PairTerms {
   const uint16_t* a;
   const uint16_t* b;
   const Fr* c;
   const uint8_t* unit;  // c_j == 1: its product is skipped
-  const uint16_t* rest;
-  int n, nrest;
+  int n;
 };
 
-// Four resident blocks a SM (128 registers a thread, no spills): the
-// two-table zerocheck's rounds take 16 % less time than at the compiler's
-// choice (166 registers, three blocks); five and six spill. The products are
-// the interpreter's out-of-line rmul: inlined, the rounds took 15 % longer.
-#ifndef APG_PAIRS_MIN_BLOCKS
-#define APG_PAIRS_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(kRoundThreads, APG_PAIRS_MIN_BLOCKS) k_round_pairs(RoundArgs A, PairTerms T, Fr* partials) {
-  __shared__ Fr red[kRoundThreads];
-  const bool n1 = (A.nodes >> 1) & 1;
-  Fr acc0 = fe_zero<FrConsts>(), acc1 = fe_zero<FrConsts>(), acc2 = fe_zero<FrConsts>();
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < A.npairs; i += stride) {
-    Fr lo, hi;
-    for (int r = 0; r < T.nrest; ++r) load_line(A, T.rest[r], i, lo, hi);
-    Fr s0 = fe_zero<FrConsts>(), s1 = fe_zero<FrConsts>(), s2 = fe_zero<FrConsts>();
-    for (int j = 0; j < T.n; ++j) {
-      Fr alo, ahi, blo, bhi;
-      load_line(A, T.a[j], i, alo, ahi);
-      load_line(A, T.b[j], i, blo, bhi);
-      Fr p0 = rmul(alo, blo);
-      Fr p2 = rmul(fe_sub(fe_add(ahi, ahi), alo), fe_sub(fe_add(bhi, bhi), blo));  // the lines at X = 2
-      Fr p1 = n1 ? rmul(ahi, bhi) : fe_zero<FrConsts>();
-      if (!T.unit[j]) {
-        const Fr cj = ld_fe(&T.c[j]);
-        p0 = rmul(cj, p0);
-        p2 = rmul(cj, p2);
-        if (n1) p1 = rmul(cj, p1);
-      }
-      s0 = fe_add(s0, p0);
-      s2 = fe_add(s2, p2);
-      if (n1) s1 = fe_add(s1, p1);
-    }
-    Fr e_lo, e_hi;
-    load_line(A, A.nd, i, e_lo, e_hi);
-    const Fr w = fe_add(e_lo, e_hi);  // the pair's eq weight without the current variable's factor
-    acc0 = fe_add(acc0, rmul(w, s0));
-    acc2 = fe_add(acc2, rmul(w, s2));
-    if (n1) acc1 = fe_add(acc1, rmul(w, s1));
-  }
-  const Fr accs[4] = {acc0, acc1, acc2, fe_zero<FrConsts>()};
-  for (int x = 0; x < 4; ++x) {
-    red[threadIdx.x] = accs[x];
-    __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-      if (threadIdx.x < (unsigned)off) red[threadIdx.x] = fe_add(red[threadIdx.x], red[threadIdx.x + off]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) st_fe(&partials[(size_t)blockIdx.x * 4 + x], red[0]);
-    __syncthreads();
-  }
-  round_total(A, partials, red);
+// A round of a short quadratic form, staged through shared memory. A block
+// takes P pairs at a time: its threads fold the pairs' entries of every table
+// with the previous challenge, one entry a thread, into shared memory (and the
+// level they bind); then a thread a (pair, node, share of the terms) multiplies
+// its terms' lines and weighs their sum. In a small round a thread's chain is
+// a fold, a product, its coefficient and the pair's weight, four products, and
+// the kernel's code is short (one out-of-line product: a launch runs its code
+// once, from a cold instruction cache): 11-14 us a round of up to 2^11 pairs of
+// ten terms on a GB300, where a thread a (pair, term) took 34. Entries lie as 16-byte halves, lo and
+// hi of a pair apart, so that threads of consecutive pairs read consecutive
+// 16 bytes.
+constexpr int kTermThreads = 256;
+
+__device__ __forceinline__ Fr term_ld(const uint4* line, int k, int h, int i, int P) {
+  const uint4 u = line[((k * 2 + h) * 2) * P + i], v = line[((k * 2 + h) * 2 + 1) * P + i];
+  Fr r;
+  r.v[0] = u.x, r.v[1] = u.y, r.v[2] = u.z, r.v[3] = u.w;
+  r.v[4] = v.x, r.v[5] = v.y, r.v[6] = v.z, r.v[7] = v.w;
+  return r;
 }
 
-// The same summand in rounds with few pairs (the tops of halving lists): one
-// thread per (pair, term), or per (pair, table no term reads), which only
-// folds, so a pair's folds and products run side by side instead of as one
-// thread's chain of a hundred products. Each term thread weighs its own term
-// by c_j and the pair's eq weight; the block sums them all. The pair's eq
-// line is stored by its first term's thread; a table two terms share is
-// stored twice with the same value.
-__global__ void __launch_bounds__(kRoundThreads) k_round_pairs_small(RoundArgs A, PairTerms T, Fr* partials) {
-  __shared__ Fr red[kRoundThreads];
-  const bool n1 = (A.nodes >> 1) & 1;
-  const size_t per = (size_t)T.n + T.nrest;
-  Fr acc0 = fe_zero<FrConsts>(), acc1 = fe_zero<FrConsts>(), acc2 = fe_zero<FrConsts>();
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < A.npairs * per; t += stride) {
-    const size_t i = t / per;
-    const int j = (int)(t - i * per);
-    if (j >= T.n) {
-      Fr lo, hi;
-      load_line<APG_SMALL_OUTLINE>(A, T.rest[j - T.n], i, lo, hi);
-      continue;
+// Table k's line at node x of pair i (1 when there is no table).
+__device__ __forceinline__ Fr term_at(const uint4* line, uint16_t k, int i, int P, int x) {
+  if (k == kNoTable) return fe_one<FrConsts>();
+  if (x == 0) return term_ld(line, k, 0, i, P);
+  const Fr hi = term_ld(line, k, 1, i, P);
+  return x == 1 ? hi : fe_sub(fe_add(hi, hi), term_ld(line, k, 0, i, P));
+}
+
+__global__ void __launch_bounds__(kTermThreads) k_round_terms(RoundArgs A, PairTerms T, int logP, Fr* partials) {
+  extern __shared__ uint4 line[];
+  __shared__ Fr ws[3 * kTermThreads / 32];
+  const int P = 1 << logP, nt = A.nd + 1, three = (A.nodes >> 1) & 1;
+  // Threads of node 0, then 2 (or 0, 1, 2): a group of 128 (64) each.
+  const int G = three ? kTermThreads / 4 : kTermThreads / 2, group = threadIdx.x / G, share = G >> logP;
+  const int x = three ? group : 2 * group, i = threadIdx.x & (P - 1), j0 = (threadIdx.x % G) >> logP;
+  const bool on = x < 3 && j0 < T.n;
+  Fr acc = fe_zero<FrConsts>();
+  for (size_t p0 = (size_t)blockIdx.x << logP; p0 < A.npairs; p0 += (size_t)gridDim.x << logP) {
+    for (int t = threadIdx.x; t < nt << (logP + 1); t += kTermThreads) {
+      const int k = t >> (logP + 1), e = t & (2 * P - 1);
+      const size_t at = 2 * p0 + e;
+      if (at >= 2 * A.npairs) continue;
+      const Fr* in = table_in(A, k);
+      const int bits = A.in_is_src && A.src_bits ? A.src_bits[k] : 0;
+      Fr v;
+      if (!A.bind) {
+        v = bits ? narrow_entry(in, bits, at) : ld_fe(&in[at]);
+      } else {
+        const Fr v0 = bits ? narrow_entry(in, bits, 2 * at) : ld_fe(&in[2 * at]);
+        const Fr v1 = bits ? narrow_entry(in, bits, 2 * at + 1) : ld_fe(&in[2 * at + 1]);
+        v = fe_add(v0, rmul(A.c, fe_sub(v1, v0)));
+        st_fe(&A.out_base[(size_t)k * (A.in_len / 2) + at], v);
+      }
+      uint4* o = &line[((k * 2 + (e & 1)) * 2) * P + (e >> 1)];
+      o[0] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+      o[P] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
     }
-    Fr alo, ahi, blo, bhi, e_lo, e_hi;
-    load_line<APG_SMALL_OUTLINE>(A, T.a[j], i, alo, ahi);
-    load_line<APG_SMALL_OUTLINE>(A, T.b[j], i, blo, bhi);
-    load_line<APG_SMALL_OUTLINE>(A, A.nd, i, e_lo, e_hi, j == 0);
-    Fr cw = fe_add(e_lo, e_hi);  // the pair's eq weight without the current variable's factor
-    // The term's products at X = 0 and 2 (the lines at X = 2 are 2 hi - lo)
-    // and its weight, two at a time.
-    const FrPair p = rmul2(alo, blo, fe_sub(fe_add(ahi, ahi), alo), fe_sub(fe_add(bhi, bhi), blo));
-    if (!T.unit[j]) cw = rmul(ld_fe(&T.c[j]), cw);
-    const FrPair wp = rmul2(cw, p.a, cw, p.b);
-    acc0 = fe_add(acc0, wp.a);
-    acc2 = fe_add(acc2, wp.b);
-    if (n1) acc1 = fe_add(acc1, rmul(cw, rmul(ahi, bhi)));
-  }
-  const Fr accs[4] = {acc0, acc1, acc2, fe_zero<FrConsts>()};
-  for (int x = 0; x < 4; ++x) {
-    red[threadIdx.x] = accs[x];
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-      if (threadIdx.x < (unsigned)off) red[threadIdx.x] = fe_add(red[threadIdx.x], red[threadIdx.x + off]);
-      __syncthreads();
+    if (on && p0 + i < A.npairs) {
+      Fr s = fe_zero<FrConsts>();
+      for (int j = j0; j < T.n; j += share) {
+        Fr p = term_at(line, T.a[j], i, P, x);
+        if (T.b[j] != kNoTable) p = rmul(p, term_at(line, T.b[j], i, P, x));
+        if (!T.unit[j]) p = rmul(ld_fe(&T.c[j]), p);
+        s = fe_add(s, p);
+      }
+      // The pair's eq weight without the current variable's factor.
+      acc = fe_add(acc, rmul(fe_add(term_ld(line, A.nd, 0, i, P), term_ld(line, A.nd, 1, i, P)), s));
     }
-    if (threadIdx.x == 0) st_fe(&partials[(size_t)blockIdx.x * 4 + x], red[0]);
     __syncthreads();
   }
-  round_total(A, partials, red);
+  acc = warp_sum(acc, 32, 0xffffffffu);
+  if ((threadIdx.x & 31) < 3) ws[3 * (threadIdx.x >> 5) + (threadIdx.x & 31)] = (threadIdx.x & 31) == x ? acc : fe_zero<FrConsts>();
+  round_finish(A, ws, kTermThreads / 32, partials);
 }
 
 // Wide gate lists (many gates, many tables): one warp per pair. The pair's
@@ -365,14 +357,14 @@ template <bool OUTLINE>
 __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_WARP_MIN_BLOCKS) k_round_warp(RoundArgs A, DevProgram P, VirtualRound V,
                                                               Fr* partials) {
   extern __shared__ uint32_t sm_raw[];
-  __shared__ Fr red[kRoundThreads];
+  __shared__ Fr ws[3 * kRoundThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int per_warp = A.slots_step0 + A.n_val_slots + 2;
   const Slots S = warp_slots(sm_raw + (size_t)warp * per_warp * 8, per_warp);
   const int eq_slot = per_warp - 2;
-  Fr acc[4];
+  Fr acc[3];
 #pragma unroll
-  for (int x = 0; x < 4; ++x) acc[x] = fe_zero<FrConsts>();
+  for (int x = 0; x < 3; ++x) acc[x] = fe_zero<FrConsts>();
   const size_t wstride = (size_t)gridDim.x * nwarps;
   for (size_t i = (size_t)blockIdx.x * nwarps + warp; i < A.npairs; i += wstride) {
     Fr lo, hi;
@@ -420,36 +412,32 @@ __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_WARP_MIN_BLOCKS) k_ro
       __syncwarp();
     }
   }
-  // Per node: the block's warps' sums (lane 0 of each), then the cross-block total.
-  for (int x = 0; x < 4; ++x) {
-    red[threadIdx.x] = lane == 0 ? acc[x] : fe_zero<FrConsts>();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      Fr a = fe_zero<FrConsts>();
-      for (int w = 0; w < nwarps; ++w) a = fe_add(a, red[32 * w]);
-      st_fe(&partials[(size_t)blockIdx.x * 4 + x], a);
-    }
-    __syncthreads();
-  }
-  round_total(A, partials, red);
+  if (lane == 0)
+#pragma unroll
+    for (int x = 0; x < 3; ++x) ws[3 * warp + x] = acc[x];
+  round_finish(A, ws, nwarps, partials);
 }
 
 // Tables of length 2 -> their bound value (the last round's fold).
 // With no rounds at all (a one-entry table) c is ignored and the entry itself
 // is the value.
+// One block; the values and then the flag go to pinned host memory.
 __global__ void k_final_bind(const Fr* const* src, const uint8_t* src_bits, const Fr* in_base, size_t in_len,
-                             int in_is_src, int nt, Fr c, int no_rounds, Fr* out) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nt) return;
-  const Fr* t = in_is_src ? src[k] : in_base + (size_t)k * in_len;
-  const int bits = in_is_src && src_bits ? src_bits[k] : 0;
-  const Fr a0 = bits ? narrow_entry(t, bits, 0) : ld_fe(&t[0]);
-  if (no_rounds) {
-    st_fe(&out[k], a0);
-    return;
+                             int in_is_src, int nt, Fr c, int no_rounds, Fr* out, uint32_t* flag, uint32_t seq) {
+  for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+    const Fr* t = in_is_src ? src[k] : in_base + (size_t)k * in_len;
+    const int bits = in_is_src && src_bits ? src_bits[k] : 0;
+    const Fr a0 = bits ? narrow_entry(t, bits, 0) : ld_fe(&t[0]);
+    if (no_rounds) {
+      st_fe(&out[k], a0);
+      continue;
+    }
+    const Fr a1 = bits ? narrow_entry(t, bits, 1) : ld_fe(&t[1]);
+    st_fe(&out[k], fe_add(a0, rmul(c, fe_sub(a1, a0))));
   }
-  const Fr a1 = bits ? narrow_entry(t, bits, 1) : ld_fe(&t[1]);
-  st_fe(&out[k], fe_add(a0, fe_mul(c, fe_sub(a1, a0))));
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t*>(flag) = seq;
 }
 
 __global__ void k_lift(const void* p, int bits, size_t n, Fr* out) {
@@ -541,6 +529,30 @@ static VirtualRound virtual_round(const std::vector<F>& point, int nvars) {
   return V;
 }
 
+// k_round_terms' pairs a block: in small rounds as many as give a thread one
+// entry to fold, growing (for the shares' evenness) while the blocks still fill
+// the device four times and shared memory leaves four blocks an SM.
+struct TermsShape {
+  int log_pairs;
+  unsigned blocks;
+  size_t smem;
+};
+#ifndef APG_TERMS_SMEM
+#define APG_TERMS_SMEM (56 * 1024)
+#endif
+static TermsShape terms_shape(size_t npairs, int nt, int sm_count) {
+  TermsShape s;
+  s.log_pairs = 0;
+  auto smem = [&](int lp) { return (size_t)nt * 64 << lp; };
+  while (s.log_pairs < 6 && ((size_t)nt << (s.log_pairs + 2)) <= (size_t)kTermThreads) ++s.log_pairs;
+  while (s.log_pairs < 6 && smem(s.log_pairs + 1) <= (size_t)(APG_TERMS_SMEM) &&
+         (npairs >> (s.log_pairs + 1)) >= (size_t)sm_count * 4)
+    ++s.log_pairs;
+  s.blocks = (unsigned)std::min<size_t>((npairs + ((size_t)1 << s.log_pairs) - 1) >> s.log_pairs, (size_t)sm_count * 8);
+  s.smem = smem(s.log_pairs);
+  return s;
+}
+
 void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint8_t>& vkinds, int n_cached,
                   const std::vector<const Fr*>& src, const std::vector<F>& eq_point, host::Transcript& tr,
                   std::vector<std::array<F, 4>>& rounds, std::vector<F>& point, std::vector<F>& finals,
@@ -606,23 +618,25 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
   if (small_warp_ok)
     APG_CUDA(cudaFuncSetAttribute(k_round_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   const int warp_max_blocks = c.sm_count * 16;
+  APG_CUDA(cudaFuncSetAttribute(k_round_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   Fr* partials = c.scratch[S_TMP6].as<Fr>((size_t)std::max(max_blocks, warp_max_blocks) * 4);
-  Fr* d_out = c.scratch[S_RESULT].as<Fr>(4);
   unsigned* done = c.scratch[S_ROUND].as<unsigned>(1);
   APG_CUDA(cudaMemsetAsync(done, 0, sizeof(unsigned), c.stream));
-  F* sums = reinterpret_cast<F*>(c.host_pinned());
+  uint8_t* pinned = c.host_pinned();
+  const F* sums = reinterpret_cast<const F*>(pinned + Ctx::kPinnedSums);
+  Fr* host_tables = reinterpret_cast<Fr*>(pinned + Ctx::kPinnedTables);
   DevProgram P = prog;
   P.cached_slot0 = n_val;
-  // The pair-term kernel's tables on the device (when the summand has that form).
+  // The terms on the device (when the summand is a short quadratic form).
   PairTerms PT;
   memset(&PT, 0, sizeof(PT));
-  const bool use_pairs = pairs && vkinds.empty() && n_cached == 0 && !pairs->a.empty();
-  if (use_pairs) {
-    const size_t nt_ = pairs->a.size(), nr = pairs->rest.size();
-    const size_t cb = 32 * nt_, ab = 2 * nt_, rb = 2 * std::max<size_t>(nr, 1), ub = nt_;
-    const size_t total = cb + 2 * ab + rb + ub + 4 * 32;
+  const bool use_terms = pairs && vkinds.empty() && n_cached == 0 && !pairs->a.empty() && (size_t)nt * 64 <= 200 * 1024;
+  std::vector<uint8_t> h;  // (lives until the copy from it has surely run: the first round's end)
+  if (use_terms) {
+    const size_t nt_ = pairs->a.size();
+    const size_t cb = 32 * nt_, ab = 2 * nt_, total = cb + 2 * ab + nt_ + 4 * 32;
     uint8_t* d = c.scratch[S_PAIR_TERMS].as<uint8_t>(total);
-    std::vector<uint8_t> h(total, 0);
+    h.assign(total, 0);
     size_t off = 0;
     auto put = [&](const void* p, size_t n) {
       const size_t at = (off + 31) & ~(size_t)31;
@@ -635,12 +649,9 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     PT.c = reinterpret_cast<const Fr*>(put(pairs->c.data(), cb));
     PT.a = reinterpret_cast<const uint16_t*>(put(pairs->a.data(), ab));
     PT.b = reinterpret_cast<const uint16_t*>(put(pairs->b.data(), ab));
-    PT.rest = reinterpret_cast<const uint16_t*>(put(pairs->rest.data(), 2 * nr));
-    PT.unit = put(unit.data(), ub);
+    PT.unit = put(unit.data(), nt_);
     PT.n = (int)nt_;
-    PT.nrest = (int)nr;
     APG_CUDA(cudaMemcpyAsync(d, h.data(), total, cudaMemcpyHostToDevice, c.stream));
-    APG_CUDA(cudaStreamSynchronize(c.stream));  // `h` is a host temporary
   }
 
   // 1/r_j for every nonzero eq coordinate, from one inversion (Montgomery's
@@ -657,6 +668,46 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     }
   }
   F chal = host::fzero();
+  // The round polynomial factors as s(X) = eq_r(X) q(X): eq's factor for this
+  // variable, eq_r(X) = (1 - r_r)(1 - X) + r_r X, is common to every pair, and
+  // the rest of a pair's eq weight is e(2i) + e(2i + 1). q has degree 2 and is
+  // summed at nodes 0 and 2; from the second round on q(1) follows from s(0) +
+  // s(1) = s_{r-1}(c_{r-1}), which holds for any tables because the bound tables
+  // are the lines at c. Round 0, and a round whose eq coordinate is 0, sum at
+  // node 1 as well.
+  auto needs_one = [&](int r) { return r == 0 || eq_point[r].zero(); };
+  // A round from its sums q(0), q(1) (when needed) and q(2): the cubic onto the
+  // transcript (whose tag and length have been absorbed), the next challenge.
+  auto close_round = [&](int r, F q[4]) {
+    const F rr = eq_point[r], one_m_r = host::fsub(host::fone(), rr);
+    if (!needs_one(r)) {
+      const auto& gp = rounds.back();  // s_{r-1}(X), ascending coefficients
+      const F claim = host::fadd(
+          gp[0], host::fmul(chal, host::fadd(gp[1], host::fmul(chal, host::fadd(gp[2], host::fmul(chal, gp[3]))))));
+      q[1] = host::fmul(host::fsub(claim, host::fmul(one_m_r, q[0])), inv_r[r]);
+    }
+    // q(3) = q(0) - 3 q(1) + 3 q(2); s(X) = eq_r(X) q(X) with eq_r(X) = 1 - r - X + 2 r X.
+    const F three = host::from_u64(3);
+    q[3] = host::fadd(q[0], host::fmul(three, host::fsub(q[2], q[1])));
+    F sv[4];
+    F eqx = one_m_r;                          // eq_r(0)
+    const F step = host::fsub(host::fadd(rr, rr), host::fone());  // eq_r(X + 1) - eq_r(X) = 2r - 1
+    for (int x = 0; x < 4; ++x) {
+      sv[x] = host::fmul(eqx, q[x]);
+      eqx = host::fadd(eqx, step);
+    }
+    auto g = host::cubic_through(sv);
+    for (const F& v : g) tr.observe(v);
+    chal = tr.challenge(host::T_SUMCHECK_CHALLENGE);
+    rounds.push_back(g);
+    point.push_back(chal);
+  };
+  typedef std::chrono::steady_clock Clock;
+  auto count_host = [&](Clock::time_point t0) {
+    if (!c.timers.on) return;  // the host's share of a round: interpolation and the transcript step
+    c.timers.ms[APG_TIMER_HOST_ROUND] += std::chrono::duration<double, std::milli>(Clock::now() - t0).count();
+    c.timers.count[APG_TIMER_HOST_ROUND] += 1;
+  };
   for (int r = 0; r < n; ++r) {
     RoundArgs A;
     memset(&A, 0, sizeof(A));
@@ -674,84 +725,54 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     A.slots_step0 = n_val + n_cached;
     A.n_val_slots = n_val;
     A.done = done;
-    A.out = d_out;
+    A.out = reinterpret_cast<Fr*>(pinned + Ctx::kPinnedSums);
+    A.flag = reinterpret_cast<uint32_t*>(pinned);
+    A.seq = ++c.flag_seq;
     VirtualRound V = virtual_round(point, n);
     // Rounds too small to fill the device evaluate the nodes of a pair on
     // threads of their own.
     A.xsplit = A.npairs * 4 <= (size_t)threads * max_blocks ? 1 : 0;
     A.src_bits = d_bits;
-    // The round polynomial factors as s(X) = eq_r(X) q(X): eq's factor for
-    // this variable, eq_r(X) = (1 - r_r)(1 - X) + r_r X, is common to every
-    // pair, and the rest of a pair's eq weight is e(2i) + e(2i + 1). The
-    // device sums q at nodes 0 and 2 (q has degree 2); from the second round
-    // on q(1) follows from s(0) + s(1) = s_{r-1}(c_{r-1}), which holds for any
-    // tables because the bound tables are the lines at c. Round 0, and a round
-    // whose eq coordinate is 0, evaluate node 1 as well.
-    const F rr = eq_point[r];
-    const bool need1 = r == 0 || rr.zero();
-    A.nodes = need1 ? 7 : 5;
+    A.nodes = needs_one(r) ? 7 : 5;
     const size_t work = A.xsplit ? A.npairs * 4 : A.npairs;
     const int blocks = warp_mode
                            ? (int)std::min<size_t>((A.npairs + kRoundThreads / 32 - 1) / (kRoundThreads / 32),
                                                    (size_t)warp_max_blocks)
                            : (int)std::min<size_t>((work + threads - 1) / threads, (size_t)max_blocks);
     cudaEvent_t t0 = c.timer_begin();
-    if (use_pairs && !A.xsplit)
-      launch(c, k_round_pairs, (int)std::min<size_t>((A.npairs + kRoundThreads - 1) / kRoundThreads,
-                                                     (size_t)c.sm_count * 8),
-             kRoundThreads, 0, A, PT, partials);
-    else if (use_pairs && PT.n + PT.nrest >= 4)  // (one or two terms: the node-split generic rounds were faster)
-      launch(c, k_round_pairs_small,
-             (int)std::min<size_t>((A.npairs * (size_t)(PT.n + PT.nrest) + kRoundThreads - 1) / kRoundThreads,
-                                   (size_t)c.sm_count * 8),
-             kRoundThreads, 0, A, PT, partials);
+    if (use_terms) {
+      const TermsShape t = terms_shape(A.npairs, nt, c.sm_count);
+      launch(c, k_round_terms, t.blocks, kTermThreads, t.smem, A, PT, t.log_pairs, partials);
+    }
     else if (small_warp_ok && A.npairs * 32 <= (size_t)kRoundThreads * c.sm_count * 4)
       launch(c, k_round_warp<true>, (int)((A.npairs + kRoundThreads / 32 - 1) / (kRoundThreads / 32)), kRoundThreads,
              warp_smem, A, P, V, partials);
     else if (warp_mode) launch(c, k_round_warp<false>, blocks, kRoundThreads, warp_smem, A, P, V, partials);
     else launch(c, k_round, blocks, threads, smem, A, P, V, partials);
     c.timer_end(APG_TIMER_SUMCHECK_ROUND, t0);
-    APG_CUDA(cudaMemcpyAsync(sums, d_out, 128, cudaMemcpyDeviceToHost, c.stream));
-    APG_CUDA(cudaStreamSynchronize(c.stream));
-    const auto host0 = std::chrono::steady_clock::now();
+    // While the device works: the message's tag and length need no sums.
+    tr.open(host::T_SUMCHECK_ROUND, 4);
+    c.wait_flag();
+    const auto host0 = Clock::now();
     F q[4] = {sums[0], sums[1], sums[2], host::fzero()};
-    const F one_m_r = host::fsub(host::fone(), rr);
-    if (!need1) {
-      const auto& gp = rounds.back();  // s_{r-1}(X), ascending coefficients
-      const F claim = host::fadd(
-          gp[0], host::fmul(chal, host::fadd(gp[1], host::fmul(chal, host::fadd(gp[2], host::fmul(chal, gp[3]))))));
-      q[1] = host::fmul(host::fsub(claim, host::fmul(one_m_r, q[0])), inv_r[r]);
-    }
-    // q(3) = q(0) - 3 q(1) + 3 q(2); s(X) = eq_r(X) q(X) with eq_r(X) = 1 - r - X + 2 r X.
-    const F three = host::from_u64(3);
-    q[3] = host::fadd(q[0], host::fmul(three, host::fsub(q[2], q[1])));
-    F sv[4];
-    F eqx = one_m_r;                          // eq_r(0)
-    const F step = host::fsub(host::fadd(rr, rr), host::fone());  // eq_r(X + 1) - eq_r(X) = 2r - 1
-    for (int x = 0; x < 4; ++x) {
-      sv[x] = host::fmul(eqx, q[x]);
-      eqx = host::fadd(eqx, step);
-    }
-    auto g = host::cubic_through(sv);
-    tr.absorb(host::T_SUMCHECK_ROUND, g.data(), 4);
-    chal = tr.challenge(host::T_SUMCHECK_CHALLENGE);
-    rounds.push_back(g);
-    point.push_back(chal);
-    if (c.timers.on) {  // the host's share of a round: interpolation and the transcript step
-      c.timers.ms[APG_TIMER_HOST_ROUND] +=
-          std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host0).count();
-      c.timers.count[APG_TIMER_HOST_ROUND] += 1;
-    }
+    close_round(r, q);
+    count_host(host0);
   }
   // The last fold: every table bound to the full point.
-  Fr* d_fin = c.scratch[S_TMP7].as<Fr>(nt);
   if (nd > 0) {
     const Fr* base = n >= 2 ? lvl[(n - 1) & 1] : nullptr;
-    launch(c, k_final_bind, (unsigned)((nd + 63) / 64), 64, 0, (const Fr* const*)d_src, d_bits, base, (size_t)2,
-           n <= 1 ? 1 : 0, nd, to_dev(chal), n == 0 ? 1 : 0, d_fin);
-    APG_CUDA(cudaMemcpyAsync(finals.data(), d_fin, 32 * (size_t)nd, cudaMemcpyDeviceToHost, c.stream));
+    const bool in_pinned = (size_t)nd * 32 <= Ctx::kPinnedBytes - Ctx::kPinnedTables;
+    Fr* d_fin = in_pinned ? host_tables : c.scratch[S_TMP7].as<Fr>(nt);
+    launch(c, k_final_bind, 1, 256, 0, (const Fr* const*)d_src, d_bits, base, (size_t)2, n <= 1 ? 1 : 0, nd,
+           to_dev(chal), n == 0 ? 1 : 0, d_fin, reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
+    if (!in_pinned)
+      APG_CUDA(cudaMemcpyAsync(finals.data(), d_fin, 32 * (size_t)nd, cudaMemcpyDeviceToHost, c.stream));
+    c.wait_flag();
+    if (in_pinned) memcpy(finals.data(), host_tables, 32 * (size_t)nd);
+    else APG_CUDA(cudaStreamSynchronize(c.stream));
+  } else {
+    APG_CUDA(cudaStreamSynchronize(c.stream));
   }
-  APG_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 // A device copy of a resolved gate list.
@@ -907,11 +928,11 @@ bool pair_terms_of(const HostProgram& hp, int nd, HostPairTerms& out) {
   out = HostPairTerms();
   if (hp.n_cached != 0 || hp.n_weighted <= 0) return false;
   const F one = host::fone(), zero = host::fzero();
-  // Terms over the same two tables merge (exact arithmetic: the sum is the
-  // same at every node).
+  // Terms over the same tables merge (exact arithmetic: the sum is the same at
+  // every node). kNoTable sorts last: a linear term is (a, none).
   std::map<std::pair<uint16_t, uint16_t>, F> merged;
   auto term = [&](uint16_t a, uint16_t b, const F& cf) {
-    if (a >= nd || b >= nd) return false;
+    if ((a >= nd && a != kNoTable) || (b >= nd && b != kNoTable)) return false;
     const auto k = a < b ? std::make_pair(a, b) : std::make_pair(b, a);
     auto it = merged.find(k);
     if (it == merged.end()) merged.emplace(k, cf);
@@ -934,17 +955,16 @@ bool pair_terms_of(const HostProgram& hp, int nd, HostPairTerms& out) {
       case G_TREE_CROSS:  // v0 v3 + v1 v2
         ok = g.nops == 4 && term(op[0], op[3], W) && term(op[1], op[2], W);
         break;
-      case G_QUADRATIC:  // c0 + linear + products: products only
-        ok = g.p1 == 0 && cf[0] == zero && g.nops == 2 * g.p2;
-        for (uint32_t u = 0; ok && u < g.p2; ++u) ok = term(op[2 * u], op[2 * u + 1], host::fmul(cf[1 + u], W));
+      case G_QUADRATIC:  // c0 + linear + products
+        ok = hp.n_weighted < kWarpModeGates && g.nops == g.p1 + 2 * g.p2 && term(kNoTable, kNoTable, host::fmul(cf[0], W));
+        for (uint32_t u = 0; ok && u < g.p1; ++u) ok = term(op[u], kNoTable, host::fmul(cf[1 + u], W));
+        for (uint32_t u = 0; ok && u < g.p2; ++u)
+          ok = term(op[g.p1 + 2 * u], op[g.p1 + 2 * u + 1], host::fmul(cf[1 + g.p1 + u], W));
         break;
       default:
         ok = false;
     }
-    if (!ok) {
-      out = HostPairTerms();
-      return false;
-    }
+    if (!ok) return false;
   }
   for (auto& kv : merged) {
     if (kv.second == zero) continue;
@@ -952,14 +972,10 @@ bool pair_terms_of(const HostProgram& hp, int nd, HostPairTerms& out) {
     out.b.push_back(kv.first.second);
     out.c.push_back(kv.second);
   }
-  if (out.a.empty() || out.a.size() > 4096) {
+  if (out.a.empty() || out.a.size() > 4096 || nd >= kNoTable) {
     out = HostPairTerms();
     return false;
   }
-  std::vector<char> used(nd, 0);
-  for (size_t j = 0; j < out.a.size(); ++j) used[out.a[j]] = used[out.b[j]] = 1;
-  for (int k = 0; k < nd; ++k)
-    if (!used[k]) out.rest.push_back((uint16_t)k);
   return true;
 }
 

@@ -71,17 +71,17 @@ void build_eq_table(Ctx& c, const std::vector<host::F>& r, Fr* out);
 // `src_bits` (empty: every table Fr) gives each data table's stored width;
 // narrow tables are read through the lift in the first two rounds and the
 // first bind writes Fr (the lazy lift of crates/poly/src/lib.rs:156-185).
-// A summand that is a weighted sum of products of two data tables,
-// S = sum_j c_j T_{a_j} T_{b_j} (halving lists of TreeProduct / TreeCross
-// gates, a zerocheck's product gate): the round kernel for it reads each
-// term's two lines and multiplies, with no interpreter between. `rest` lists
-// the data tables no term reads (they are still bound every round).
+// A summand that is a short quadratic form in the data tables,
+// S = sum_j c_j T_{a_j} T_{b_j} with either factor or both absent (halving lists
+// of TreeProduct / TreeCross gates, a zerocheck's gate): its round kernels read
+// each term's lines and multiply, with no interpreter between.
+constexpr uint16_t kNoTable = 0xffff;
 struct HostPairTerms {
-  std::vector<uint16_t> a, b, rest;
+  std::vector<uint16_t> a, b;  // b absent: a linear term; both: the constant
   std::vector<host::F> c;
 };
-// The program's terms, when every weighted gate is such a product of data
-// tables (slots below nd) and nothing is cached; false otherwise.
+// The program's terms, when every weighted gate expands to such terms over
+// data tables (slots below nd) and nothing is cached; false otherwise.
 bool pair_terms_of(const HostProgram& hp, int nd, HostPairTerms& out);
 
 void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint8_t>& vkinds, int n_cached,
