@@ -440,6 +440,20 @@ __global__ void k_final_bind(const Fr* const* src, const uint8_t* src_bits, cons
   if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t*>(flag) = seq;
 }
 
+// The source tables' entries, table after table, into pinned host memory, then
+// the flag (one block: the few entries the host takes over).
+__global__ void k_gather(const Fr* const* src, const uint8_t* src_bits, int nt, size_t len, Fr* out, uint32_t* flag,
+                         uint32_t seq) {
+  for (size_t t = threadIdx.x; t < nt * len; t += blockDim.x) {
+    const int k = (int)(t / len);
+    const int bits = src_bits ? src_bits[k] : 0;
+    st_fe(&out[t], bits ? narrow_entry(src[k], bits, t - k * len) : ld_fe(&src[k][t - k * len]));
+  }
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t*>(flag) = seq;
+}
+
 __global__ void k_lift(const void* p, int bits, size_t n, Fr* out) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) st_fe(&out[i], narrow_entry(p, bits, i));
@@ -527,6 +541,25 @@ static VirtualRound virtual_round(const std::vector<F>& point, int nvars) {
   V.ram_q = to_dev(q);
   V.pow2_b = to_dev(pw);
   return V;
+}
+
+// How many of a short quadratic form's last rounds run on the host. Both sides
+// pay the transcript's permutations (6 us each: three a round on the device's
+// way, which hides one, four on the host's); a device round adds its launch, a
+// kernel of about 10 us and the flag, a host round its products at 20 ns: two a
+// table to bind and up to two a term and node. So the host takes the rounds of
+// up to kHostTailProducts products; its tables then fit the pinned buffer.
+// Measured on a GB300 at 0, 200, 600 and 1500: a 2^8-row zerocheck of a*b 396,
+// 352, 356, 381 us, 2^16 rows 807, 754, 743, 774, the GKR proof of a 7-column
+// 2^12-row shard 4528, 4290, 4343, 4496.
+constexpr size_t kHostTailProducts = 200;
+static int host_tail_rounds(int n, int nd, const HostPairTerms& t) {
+  const size_t nt = (size_t)nd + 1, per_pair = 2 * nt + 4 * t.a.size() + 2;
+  int k = 0;
+  while (k < n && (per_pair << k) <= kHostTailProducts) ++k;
+  if (n == k + 1) ++k;  // round 0 binds nothing: a list this short is gathered whole
+  while (k > 0 && (nt << (k + 1)) * 32 > Ctx::kPinnedBytes - Ctx::kPinnedTables) --k;
+  return n == k + 1 ? 0 : k;
 }
 
 // k_round_terms' pairs a block: in small rounds as many as give a thread one
@@ -631,8 +664,9 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
   PairTerms PT;
   memset(&PT, 0, sizeof(PT));
   const bool use_terms = pairs && vkinds.empty() && n_cached == 0 && !pairs->a.empty() && (size_t)nt * 64 <= 200 * 1024;
+  const int host_rounds = use_terms ? host_tail_rounds(n, nd, *pairs) : 0;
   std::vector<uint8_t> h;  // (lives until the copy from it has surely run: the first round's end)
-  if (use_terms) {
+  if (use_terms && host_rounds < n) {
     const size_t nt_ = pairs->a.size();
     const size_t cb = 32 * nt_, ab = 2 * nt_, total = cb + 2 * ab + nt_ + 4 * 32;
     uint8_t* d = c.scratch[S_PAIR_TERMS].as<uint8_t>(total);
@@ -708,7 +742,8 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     c.timers.ms[APG_TIMER_HOST_ROUND] += std::chrono::duration<double, std::milli>(Clock::now() - t0).count();
     c.timers.count[APG_TIMER_HOST_ROUND] += 1;
   };
-  for (int r = 0; r < n; ++r) {
+  const int dev_rounds = n - host_rounds;
+  for (int r = 0; r < dev_rounds; ++r) {
     RoundArgs A;
     memset(&A, 0, sizeof(A));
     A.nd = nd;
@@ -720,7 +755,8 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     A.in_is_src = r <= 1;
     A.in_len = (size_t)1 << (n - r + (r > 0 ? 1 : 0));
     A.in_base = r >= 2 ? lvl[(r - 1) & 1] : nullptr;
-    A.out_base = r >= 1 ? lvl[r & 1] : nullptr;
+    // (the last level before the host's rounds lands where the host reads it)
+    A.out_base = r < 1 ? nullptr : host_rounds && r == dev_rounds - 1 ? host_tables : lvl[r & 1];
     A.npairs = (size_t)1 << (n - r - 1);
     A.slots_step0 = n_val + n_cached;
     A.n_val_slots = n_val;
@@ -757,6 +793,55 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     F q[4] = {sums[0], sums[1], sums[2], host::fzero()};
     close_round(r, q);
     count_host(host0);
+  }
+  if (host_rounds > 0) {
+    if (dev_rounds == 0) {
+      launch(c, k_gather, 1, 256, 0, (const Fr* const*)d_src, d_bits, nt, len0, host_tables,
+             reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
+      c.wait_flag();
+    }
+    // Level dev_rounds - 1 (or the source tables), still to be bound with the last challenge.
+    const F* t0 = reinterpret_cast<const F*>(host_tables);
+    size_t len = (size_t)1 << (host_rounds + (dev_rounds > 0 ? 1 : 0));
+    std::vector<F> tab(t0, t0 + nt * len);
+    auto bind = [&]() {
+      for (size_t k = 0; k < (size_t)nt; ++k)
+        for (size_t i = 0; i < len / 2; ++i) {
+          const F lo = tab[k * len + 2 * i], hi = tab[k * len + 2 * i + 1];
+          tab[k * (len / 2) + i] = host::fadd(lo, host::fmul(chal, host::fsub(hi, lo)));
+        }
+      len /= 2;
+    };
+    if (dev_rounds > 0) bind();
+    for (int r = dev_rounds; r < n; ++r) {
+      const auto host0 = Clock::now();
+      F q[4] = {host::fzero(), host::fzero(), host::fzero(), host::fzero()};
+      for (size_t i = 0; i < len / 2; ++i) {
+        const F* e = tab.data() + nd * len + 2 * i;
+        const F w = host::fadd(e[0], e[1]);
+        for (int x = 0; x < 3; ++x) {
+          if (x == 1 && !needs_one(r)) continue;
+          auto at = [&](uint16_t k) {
+            const F* t = tab.data() + k * len + 2 * i;
+            return x == 0 ? t[0] : x == 1 ? t[1] : host::fsub(host::fadd(t[1], t[1]), t[0]);
+          };
+          F s = host::fzero();
+          for (size_t j = 0; j < pairs->a.size(); ++j) {
+            F v = pairs->c[j];
+            if (pairs->a[j] != kNoTable) v = v == host::fone() ? at(pairs->a[j]) : host::fmul(v, at(pairs->a[j]));
+            if (pairs->b[j] != kNoTable) v = host::fmul(v, at(pairs->b[j]));
+            s = host::fadd(s, v);
+          }
+          q[x] = host::fadd(q[x], host::fmul(w, s));
+        }
+      }
+      tr.open(host::T_SUMCHECK_ROUND, 4);
+      close_round(r, q);
+      bind();
+      count_host(host0);
+    }
+    for (int k = 0; k < nd; ++k) finals[k] = tab[k];
+    return;
   }
   // The last fold: every table bound to the full point.
   if (nd > 0) {

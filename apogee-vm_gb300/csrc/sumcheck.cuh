@@ -74,7 +74,8 @@ void build_eq_table(Ctx& c, const std::vector<host::F>& r, Fr* out);
 // A summand that is a short quadratic form in the data tables,
 // S = sum_j c_j T_{a_j} T_{b_j} with either factor or both absent (halving lists
 // of TreeProduct / TreeCross gates, a zerocheck's gate): its round kernels read
-// each term's lines and multiply, with no interpreter between.
+// each term's lines and multiply, with no interpreter between, and its last few
+// rounds run on the host.
 constexpr uint16_t kNoTable = 0xffff;
 struct HostPairTerms {
   std::vector<uint16_t> a, b;  // b absent: a linear term; both: the constant
