@@ -516,6 +516,123 @@ __device__ __forceinline__ Fe<C> fe_sqr(const Fe<C>& a) {
   return r;
 }
 
+// Sums of up to fifteen products, reduced once: each product costs its 64 wide
+// products and an addition of 16 words, and the sum one set of reduction rows.
+// Fifteen products of values below m stay below 2^512 (m^2 < 2^507.2), and
+// their reduced value below 15 * 0.19 m + m < 4 m.
+constexpr int kWideProducts = 15;
+
+template <class C>
+struct FeWide {
+  uint32_t w[16];
+};
+
+template <class C>
+__device__ __forceinline__ FeWide<C> wide_zero() {
+  FeWide<C> r;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) r.w[k] = 0;
+  return r;
+}
+
+// acc += a b.
+template <class C>
+__device__ __forceinline__ void wide_mac(FeWide<C>& acc, const Fe<C>& a, const Fe<C>& b) {
+  uint32_t e[8], o[8], t[16], cy;
+  eo_first(e, o, a.v, b.v[0]);
+  t[0] = e[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    eo_mul_row(e, o, a.v, b.v[i]);
+    t[i] = e[0];
+  }
+  eo_merge(t + 8, e, o);
+  asm("add.cc.u32  %0, %0, %9;\n\t"
+      "addc.cc.u32 %1, %1, %10;\n\t"
+      "addc.cc.u32 %2, %2, %11;\n\t"
+      "addc.cc.u32 %3, %3, %12;\n\t"
+      "addc.cc.u32 %4, %4, %13;\n\t"
+      "addc.cc.u32 %5, %5, %14;\n\t"
+      "addc.cc.u32 %6, %6, %15;\n\t"
+      "addc.cc.u32 %7, %7, %16;\n\t"
+      "addc.u32    %8, 0, 0;"
+      : "+r"(acc.w[0]), "+r"(acc.w[1]), "+r"(acc.w[2]), "+r"(acc.w[3]), "+r"(acc.w[4]), "+r"(acc.w[5]), "+r"(acc.w[6]),
+        "+r"(acc.w[7]), "=&r"(cy)
+      : "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]), "r"(t[7]));
+  asm("{\n\t"
+      ".reg .u32 x;\n\t"
+      "add.cc.u32  x, %16, 0xffffffff;\n\t"  // the carry back into the flag
+      "addc.cc.u32 %0, %0, %8;\n\t"
+      "addc.cc.u32 %1, %1, %9;\n\t"
+      "addc.cc.u32 %2, %2, %10;\n\t"
+      "addc.cc.u32 %3, %3, %11;\n\t"
+      "addc.cc.u32 %4, %4, %12;\n\t"
+      "addc.cc.u32 %5, %5, %13;\n\t"
+      "addc.cc.u32 %6, %6, %14;\n\t"
+      "addc.u32    %7, %7, %15;\n\t"
+      "}"
+      : "+r"(acc.w[8]), "+r"(acc.w[9]), "+r"(acc.w[10]), "+r"(acc.w[11]), "+r"(acc.w[12]), "+r"(acc.w[13]),
+        "+r"(acc.w[14]), "+r"(acc.w[15])
+      : "r"(t[8]), "r"(t[9]), "r"(t[10]), "r"(t[11]), "r"(t[12]), "r"(t[13]), "r"(t[14]), "r"(t[15]), "r"(cy));
+}
+
+// r = a - 2m if a >= 2m.
+template <class C>
+__device__ __forceinline__ void fe_sub_twice_if(uint32_t r[8]) {
+  constexpr uint32_t q[8] = {C::P0 << 1,
+                             (C::P1 << 1) | (C::P0 >> 31),
+                             (C::P2 << 1) | (C::P1 >> 31),
+                             (C::P3 << 1) | (C::P2 >> 31),
+                             (C::P4 << 1) | (C::P3 >> 31),
+                             (C::P5 << 1) | (C::P4 >> 31),
+                             (C::P6 << 1) | (C::P5 >> 31),
+                             (C::P7 << 1) | (C::P6 >> 31)};
+  uint32_t s0, s1, s2, s3, s4, s5, s6, s7, br;
+  asm("sub.cc.u32  %0, %9, %17;\n\t"
+      "subc.cc.u32 %1, %10, %18;\n\t"
+      "subc.cc.u32 %2, %11, %19;\n\t"
+      "subc.cc.u32 %3, %12, %20;\n\t"
+      "subc.cc.u32 %4, %13, %21;\n\t"
+      "subc.cc.u32 %5, %14, %22;\n\t"
+      "subc.cc.u32 %6, %15, %23;\n\t"
+      "subc.cc.u32 %7, %16, %24;\n\t"
+      "subc.u32    %8, 0, 0;"
+      : "=r"(s0), "=r"(s1), "=r"(s2), "=r"(s3), "=r"(s4), "=r"(s5), "=r"(s6), "=r"(s7), "=r"(br)
+      : "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "n"(q[0]), "n"(q[1]),
+        "n"(q[2]), "n"(q[3]), "n"(q[4]), "n"(q[5]), "n"(q[6]), "n"(q[7]));
+  const bool keep = br != 0;
+  r[0] = keep ? r[0] : s0;
+  r[1] = keep ? r[1] : s1;
+  r[2] = keep ? r[2] : s2;
+  r[3] = keep ? r[3] : s3;
+  r[4] = keep ? r[4] : s4;
+  r[5] = keep ? r[5] : s5;
+  r[6] = keep ? r[6] : s6;
+  r[7] = keep ? r[7] : s7;
+}
+
+// The sum's value times 2^-256 mod m.
+template <class C>
+__device__ __forceinline__ Fe<C> fe_from_wide(const FeWide<C>& a) {
+  uint32_t lo[8];
+  eo_redc<C>(lo, a.w);
+  Fe<C> r;
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+      : "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]), "r"(a.w[8]),
+        "r"(a.w[9]), "r"(a.w[10]), "r"(a.w[11]), "r"(a.w[12]), "r"(a.w[13]), "r"(a.w[14]), "r"(a.w[15]));
+  fe_sub_twice_if<C>(r.v);
+  fe_reduce_once<C>(r.v);
+  return r;
+}
+
 // Montgomery form -> canonical limbs (multiply by 1), and back (multiply by R^2).
 template <class C>
 __device__ __forceinline__ Fe<C> fe_from_mont(const Fe<C>& a) {

@@ -316,7 +316,7 @@ GkrValues* gkr_forward_impl(Ctx& c, const uint8_t* blob, size_t blob_len, const 
     APG_CUDA(cudaMallocAsync((void**)&V->layers[k + 1], 32 * rows * std::max<uint32_t>(L.width, 1), c.stream));
     HostProgram hp = layer_program(C, k, ch, false, {});
     DevProgram P;
-    upload_program(c, hp, P, 0);
+    upload_program(c, hp, P);
     const int w = (int)C.width(k);
     const int nv = L.halving ? 0 : (int)C.virtuals.size();
     P.cached_slot0 = L.halving ? 2 * w : w + nv;
@@ -417,8 +417,6 @@ int gkr_prove_impl(Ctx& c, const uint8_t* blob, size_t blob_len, GkrValues* V, c
       acc = host::fmul(acc, lambda);
     }
     HostProgram hp = layer_program(C, kk, ch, true, weights);
-    DevProgram P;
-    upload_program(c, hp, P, 0);
     // L2: the tables, child 0 then child 1 of every column for a halving list.
     const uint32_t w = C.width(kk);
     std::vector<const Fr*> src;
@@ -438,10 +436,7 @@ int gkr_prove_impl(Ctx& c, const uint8_t* blob, size_t blob_len, GkrValues* V, c
     }
     std::vector<std::array<F, 4>> rounds;
     std::vector<F> rho, finals;
-    HostPairTerms pairs;
-    const bool by_pairs = pair_terms_of(hp, (int)src.size(), pairs);
-    run_sumcheck(c, P, (int)src.size(), vkinds, (int)L.cached.size(), src, point, tr, rounds, rho, finals,
-                 src_bits, by_pairs ? &pairs : nullptr);
+    run_sumcheck(c, hp, (int)src.size(), vkinds, src, point, tr, rounds, rho, finals, src_bits);
     // L3.
     std::vector<F> claims;
     if (L.halving) {
@@ -522,8 +517,6 @@ int gkr_prove_sumcheck_impl(Ctx& c, const uint8_t* blob, size_t blob_len, size_t
     return APG_ERR_INVALID_ARGUMENT;
   }
   HostProgram hp = layer_program(C, layer, ch, true, w);
-  DevProgram P;
-  upload_program(c, hp, P, 0);
   std::vector<const Fr*> src;
   std::vector<uint8_t> vkinds;
   for (size_t x = 0; x < width; ++x) src.push_back(static_cast<const Fr*>(d_lower[x]));
@@ -533,10 +526,7 @@ int gkr_prove_sumcheck_impl(Ctx& c, const uint8_t* blob, size_t blob_len, size_t
     for (auto k : C.virtuals) vkinds.push_back((uint8_t)k);
   std::vector<std::array<F, 4>> rounds;
   std::vector<F> rho, finals;
-  HostPairTerms pairs;
-  const bool by_pairs = pair_terms_of(hp, (int)src.size(), pairs);
-  run_sumcheck(c, P, (int)src.size(), vkinds, (int)L.cached.size(), src, point, tr, rounds, rho, finals, {},
-               by_pairs ? &pairs : nullptr);
+  run_sumcheck(c, hp, (int)src.size(), vkinds, src, point, tr, rounds, rho, finals);
   for (size_t r = 0; r < rounds.size(); ++r) memcpy(rounds_out + 128 * r, rounds[r].data(), 128);
   memcpy(point_out, rho.data(), 32 * rho.size());
   memcpy(finals_out, finals.data(), 32 * finals.size());

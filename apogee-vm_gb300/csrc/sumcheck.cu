@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <chrono>
 #include <map>
+#include <set>
 #include <tuple>
 
 #include "sumcheck.cuh"
@@ -25,7 +26,7 @@ namespace apg {
 namespace {
 
 constexpr int kRoundThreads = 128;
-constexpr int kWarpModeGates = 16;  // weighted gates from which a list goes one pair per warp
+constexpr int kWarpModeGates = 16;  // weighted gates from which an interpreted list goes one pair per warp
 
 struct RoundArgs {
   int nd;                    // data tables (eq is separate)
@@ -258,90 +259,163 @@ __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_MIN_BLOCKS)
   round_finish_threads(A, acc, ws, partials);
 }
 
-// The terms of a short quadratic form (HostPairTerms) on the device.
-struct PairTerms {
-  const uint16_t* a;
-  const uint16_t* b;
-  const Fr* c;
-  const uint8_t* unit;  // c_j == 1: its product is skipped
-  int n;
+// A summand as a factored quadratic form in its tables,
+//   S = sum_g T_{a_g} (d_g + sum_t B_gt T_{b_gt}),
+// a group's factor or its constant possibly absent (kNoTable: 1; kNoConst: 0).
+// What most summands are: a halving list's products, a zerocheck's gate, a
+// family circuit's 131 gates merged (QuadForm, below).
+constexpr uint16_t kNoTable = 0xffff;
+constexpr uint32_t kNoConst = 0xffffffffu;
+enum TermKind : uint16_t { TERM_MUL = 0, TERM_PLUS = 1, TERM_MINUS = 2 };  // B, 1, -1
+
+struct FormGroup {
+  uint16_t a, n;
+  uint32_t off, d;  // first term (and its coefficient); the constant's coefficient
+};
+struct FormTerm {
+  uint16_t b, kind;
+};
+struct DevForm {
+  const FormGroup* groups;
+  const FormTerm* terms;
+  const Fr* coeffs;
+  int ng;
 };
 
-// A round of a short quadratic form, staged through shared memory. A block
-// takes P pairs at a time: its threads fold the pairs' entries of every table
-// with the previous challenge, one entry a thread, into shared memory (and the
-// level they bind); then a thread a (pair, node, share of the terms) multiplies
-// its terms' lines and weighs their sum. In a small round a thread's chain is
-// a fold, a product, its coefficient and the pair's weight, four products, and
-// the kernel's code is short (one out-of-line product: a launch runs its code
-// once, from a cold instruction cache): 11-14 us a round of up to 2^11 pairs of
-// ten terms on a GB300, where a thread a (pair, term) took 34. Entries lie as 16-byte halves, lo and
-// hi of a pair apart, so that threads of consecutive pairs read consecutive
-// 16 bytes.
-constexpr int kTermThreads = 256;
+// A round of a factored quadratic form, staged through shared memory. A block
+// takes 2^log_pp pairs at a time: its threads fold the pairs' lines of every
+// table with the previous challenge (a line a thread) and leave each line's
+// values at the round's nodes in shared memory; then a warp takes every
+// nshare-th group for a tile of pairs, so its lanes run the same terms and read
+// the same coefficients. Both the inner sums and the sum over the groups stay
+// unreduced (wide_mac): 64 products a term instead of 136. A tile is 16 pairs at
+// two nodes; at three nodes 32 pairs in three passes (two of 16 pairs at nodes 0
+// and 2, one of 32 at node 1) or, where so many pairs' values are too much shared
+// memory, 8 pairs at three nodes and a quarter of the lanes idle. The small
+// rounds' chain is two folds, a share of the groups and the pair's weight; a
+// value's 16-byte halves lie apart so that lanes of consecutive pairs read
+// consecutive 16 bytes. Measured on a GB300: the first rounds of a shard circuit's
+// row-wise list over 2^21 rows 2791 and 1287 us with the interpreter, 1669 and
+// 721 so; of add_sub's list 0 (131 gates, 69 columns) over 2^16 992 us a pair a
+// warp, 396 so; small rounds of such lists 42-83 -> 18-45 us.
+constexpr int kFormMaxWarps = 16;
 
-__device__ __forceinline__ Fr term_ld(const uint4* line, int k, int h, int i, int P) {
-  const uint4 u = line[((k * 2 + h) * 2) * P + i], v = line[((k * 2 + h) * 2 + 1) * P + i];
+__device__ __forceinline__ Fr form_ld(const uint4* val, int at, int pp) {
+  const uint4 u = val[at], v = val[at + pp];
   Fr r;
   r.v[0] = u.x, r.v[1] = u.y, r.v[2] = u.z, r.v[3] = u.w;
   r.v[4] = v.x, r.v[5] = v.y, r.v[6] = v.z, r.v[7] = v.w;
   return r;
 }
 
-// Table k's line at node x of pair i (1 when there is no table).
-__device__ __forceinline__ Fr term_at(const uint4* line, uint16_t k, int i, int P, int x) {
-  if (k == kNoTable) return fe_one<FrConsts>();
-  if (x == 0) return term_ld(line, k, 0, i, P);
-  const Fr hi = term_ld(line, k, 1, i, P);
-  return x == 1 ? hi : fe_sub(fe_add(hi, hi), term_ld(line, k, 0, i, P));
+__device__ __forceinline__ void form_st(uint4* val, int at, int pp, const Fr& a) {
+  val[at] = make_uint4(a.v[0], a.v[1], a.v[2], a.v[3]);
+  val[at + pp] = make_uint4(a.v[4], a.v[5], a.v[6], a.v[7]);
 }
 
-__global__ void __launch_bounds__(kTermThreads) k_round_terms(RoundArgs A, PairTerms T, int logP, Fr* partials) {
-  extern __shared__ uint4 line[];
-  __shared__ Fr ws[3 * kTermThreads / 32];
-  const int P = 1 << logP, nt = A.nd + 1, three = (A.nodes >> 1) & 1;
-  // Threads of node 0, then 2 (or 0, 1, 2): a group of 128 (64) each.
-  const int G = three ? kTermThreads / 4 : kTermThreads / 2, group = threadIdx.x / G, share = G >> logP;
-  const int x = three ? group : 2 * group, i = threadIdx.x & (P - 1), j0 = (threadIdx.x % G) >> logP;
-  const bool on = x < 3 && j0 < T.n;
-  Fr acc = fe_zero<FrConsts>();
-  for (size_t p0 = (size_t)blockIdx.x << logP; p0 < A.npairs; p0 += (size_t)gridDim.x << logP) {
-    for (int t = threadIdx.x; t < nt << (logP + 1); t += kTermThreads) {
-      const int k = t >> (logP + 1), e = t & (2 * P - 1);
-      const size_t at = 2 * p0 + e;
-      if (at >= 2 * A.npairs) continue;
-      const Fr* in = table_in(A, k);
-      const int bits = A.in_is_src && A.src_bits ? A.src_bits[k] : 0;
-      Fr v;
-      if (!A.bind) {
-        v = bits ? narrow_entry(in, bits, at) : ld_fe(&in[at]);
+// WARPS: the most a block has. At 8 the registers (128, no spills; three
+// blocks of 80 spill and are 7 % slower) leave two blocks of 256 threads an SM, at
+// 16 (small rounds, where a block's shares count) one of 512.
+template <int WARPS, int BLOCKS>
+__global__ void __launch_bounds__(32 * WARPS, BLOCKS)
+    k_round_form(RoundArgs A, DevForm F, VirtualRound V, int nshare, int log_pp, int passes, Fr* partials) {
+  extern __shared__ uint4 val[];  // node xi of table k, pair i, half q: ((k nn + xi) 2 + q) pp + i
+  __shared__ Fr ws[3 * WARPS];
+  const int three = (A.nodes >> 1) & 1, nn = 2 + three, pp = 1 << log_pp;
+  const int ns = A.nd + A.nv;  // slots; eq's weights stand in slot ns, node 0
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  // Lanes of a pass: 2^log_l pairs a node, the nodes from lane slot 0 on (the
+  // idle quarter of the 8-pair tile repeats the last node).
+  const int log_l = three && passes == 1 ? 3 : 4, slot = lane >> log_l;
+  const int share = warp % nshare, tile = (warp / nshare) << (passes == 3 ? 5 : log_l);
+  Fr acc = fe_zero<FrConsts>(), acc1 = fe_zero<FrConsts>();  // (acc1: node 1 of the third pass)
+  for (size_t p0 = (size_t)blockIdx.x << log_pp; p0 < A.npairs; p0 += (size_t)gridDim.x << log_pp) {
+    for (int t = threadIdx.x; t < (ns + 1) << log_pp; t += blockDim.x) {
+      const int k = t >> log_pp, at = t & (pp - 1);
+      const size_t pair = p0 + at;
+      if (pair >= A.npairs) continue;
+      Fr lo, hi;
+      if (k < A.nd || k == ns) {
+        load_line<true>(A, k == ns ? A.nd : k, pair, lo, hi);
       } else {
-        const Fr v0 = bits ? narrow_entry(in, bits, 2 * at) : ld_fe(&in[2 * at]);
-        const Fr v1 = bits ? narrow_entry(in, bits, 2 * at + 1) : ld_fe(&in[2 * at + 1]);
-        v = fe_add(v0, rmul(A.c, fe_sub(v1, v0)));
-        st_fe(&A.out_base[(size_t)k * (A.in_len / 2) + at], v);
+        virtual_line_dev(V, A.vkinds[k - A.nd], pair, lo, hi);
+        hi = fe_add(lo, hi);
       }
-      uint4* o = &line[((k * 2 + (e & 1)) * 2) * P + (e >> 1)];
-      o[0] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
-      o[P] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+      uint4* o = val + (size_t)(k * nn) * 2 * pp;
+      if (k == ns) {
+        form_st(o, at, pp, fe_add(lo, hi));  // the pair's weight without the current variable's factor
+        continue;
+      }
+      form_st(o, at, pp, lo);
+      if (three) form_st(o, 2 * pp + at, pp, hi);
+      form_st(o, (nn - 1) * 2 * pp + at, pp, fe_sub(fe_add(hi, hi), lo));
     }
     __syncthreads();
-    if (on && p0 + i < A.npairs) {
+    for (int pass = 0; pass < passes; ++pass) {
+      const int i = tile + (pass == 2 ? lane : (pass << 4) + (lane & ((1 << log_l) - 1)));
+      const int xi = pass == 2 ? 1 : passes == 3 ? 2 * slot : min(slot, nn - 1);
+      if (i >= pp || p0 + i >= A.npairs) continue;
+      const uint4* mine = val + xi * 2 * pp + i;
+      const int step = nn * 2 * pp;  // between tables
       Fr s = fe_zero<FrConsts>();
-      for (int j = j0; j < T.n; j += share) {
-        Fr p = term_at(line, T.a[j], i, P, x);
-        if (T.b[j] != kNoTable) p = rmul(p, term_at(line, T.b[j], i, P, x));
-        if (!T.unit[j]) p = rmul(ld_fe(&T.c[j]), p);
-        s = fe_add(s, p);
+      FeWide<FrConsts> outer = wide_zero<FrConsts>();
+      int no = 0;
+      for (int g = share; g < F.ng; g += nshare) {
+        const FormGroup G = F.groups[g];
+        Fr in = G.d == kNoConst ? fe_zero<FrConsts>() : ld_fe(&F.coeffs[G.d]);
+        FeWide<FrConsts> sum = wide_zero<FrConsts>();
+        int ni = 0;
+        for (uint32_t t = G.off; t < G.off + G.n; ++t) {
+          const FormTerm T = F.terms[t];
+          const Fr v = form_ld(mine, T.b * step, pp);
+          if (T.kind == TERM_PLUS) in = fe_add(in, v);
+          else if (T.kind == TERM_MINUS) in = fe_sub(in, v);
+          else {
+            wide_mac(sum, ld_fe(&F.coeffs[t]), v);
+            ++ni;
+          }
+          if (ni == kWideProducts || (ni > 0 && t + 1 == G.off + G.n)) {
+            in = fe_add(in, fe_from_wide(sum));
+            sum = wide_zero<FrConsts>();
+            ni = 0;
+          }
+        }
+        if (G.a == kNoTable) {
+          s = fe_add(s, in);
+        } else {
+          wide_mac(outer, form_ld(mine, G.a * step, pp), in);
+          ++no;
+        }
+        if (no == kWideProducts || (no > 0 && g + nshare >= F.ng)) {
+          s = fe_add(s, fe_from_wide(outer));
+          outer = wide_zero<FrConsts>();
+          no = 0;
+        }
       }
-      // The pair's eq weight without the current variable's factor.
-      acc = fe_add(acc, rmul(fe_add(term_ld(line, A.nd, 0, i, P), term_ld(line, A.nd, 1, i, P)), s));
+      s = rmul(form_ld(val + i, ns * step, pp), s);
+      if (pass == 2) acc1 = fe_add(acc1, s);
+      else if (slot < nn) acc = fe_add(acc, s);
     }
     __syncthreads();
   }
-  acc = warp_sum(acc, 32, 0xffffffffu);
-  if ((threadIdx.x & 31) < 3) ws[3 * (threadIdx.x >> 5) + (threadIdx.x & 31)] = (threadIdx.x & 31) == x ? acc : fe_zero<FrConsts>();
-  round_finish(A, ws, kTermThreads / 32, partials);
+  // The warp's sum a node, from the slot's first lane.
+#pragma unroll 1
+  for (int off = 1; off < 1 << log_l; off <<= 1) {
+    Fr o;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) o.v[w] = __shfl_xor_sync(0xffffffffu, acc.v[w], off);
+    acc = fe_add(acc, o);
+  }
+  if (passes == 3) acc1 = warp_sum(acc1, 32, 0xffffffffu);
+  const int node = three && passes == 1 ? slot : 2 * slot;
+  if (lane == 0 && !(three && passes == 1)) ws[3 * warp + 1] = acc1;  // (zero at two nodes)
+  if ((lane & ((1 << log_l) - 1)) == 0 && slot < nn) ws[3 * warp + node] = acc;
+  round_finish(A, ws, nwarps, partials);
+}
+
+typedef void (*FormKernel)(RoundArgs, DevForm, VirtualRound, int, int, int, Fr*);
+inline FormKernel form_kernel(unsigned threads) {
+  return threads <= 256 ? k_round_form<8, 2> : k_round_form<kFormMaxWarps, 1>;
 }
 
 // Wide gate lists (many gates, many tables): one warp per pair. The pair's
@@ -459,23 +533,44 @@ __global__ void k_lift(const void* p, int bits, size_t n, Fr* out) {
   if (i < n) st_fe(&out[i], narrow_entry(p, bits, i));
 }
 
-// eq(r, y) for every y < 2^n: prod_j (y_j ? r_j : 1 - r_j).
-__global__ void k_eq_table(const Fr* r, int n, size_t len, Fr* out) {
-  size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (y >= len) return;
-  Fr acc = fe_one<FrConsts>();
-  for (int j = 0; j < n; ++j) {
-    Fr rj = ld_fe(&r[j]);
-    acc = fe_mul(acc, ((y >> j) & 1) ? rj : fe_sub(fe_one<FrConsts>(), rj));
-  }
-  st_fe(&out[y], acc);
-}
+// eq(r, y) = prod_j (y_j ? r_j : 1 - r_j) for every y < 2^n, a block 1024
+// consecutive y: the low ten variables as the product of two tables of five, the
+// others one factor for the block, folded into the first table. About eleven
+// products after one another whatever n, and one an entry (chains of n products
+// with their factors in device memory, three launches above 2^12: 345 us over the
+// 22 lists of a 10-column 2^21-row proof on a GB300, now 226).
+struct EqPoint {
+  Fr r[40];
+};
+constexpr int kEqLow = 10;
 
-// out[y] = lo[y mod 2^nlo] * hi[y >> nlo]: eq(r, y) split at bit nlo.
-__global__ void k_eq_combine(const Fr* lo, const Fr* hi, int nlo, size_t len, Fr* out) {
-  size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (y >= len) return;
-  st_fe(&out[y], fe_mul(ld_fe(&lo[y & (((size_t)1 << nlo) - 1)]), ld_fe(&hi[y >> nlo])));
+__device__ __forceinline__ Fr eq_factor(const Fr& r, bool bit) { return bit ? r : fe_sub(fe_one<FrConsts>(), r); }
+
+__global__ void __launch_bounds__(256) k_eq_table(const __grid_constant__ EqPoint P, int n, Fr* out) {
+  __shared__ Fr tab[2][1 << (kEqLow / 2)], high;
+  const int nl = min(n, kEqLow), na = nl / 2, t = threadIdx.x, lane = t & 31;
+  if (t < 64) {
+    const int h = t >> 5, first = h ? na : 0, bits = h ? nl - na : na;
+    if (lane < 1 << bits) {
+      Fr a = fe_one<FrConsts>();
+      for (int j = 0; j < bits; ++j) a = rmul(a, eq_factor(P.r[first + j], (lane >> j) & 1));
+      tab[h][lane] = a;
+    }
+  } else if (t < 96) {
+    Fr a = nl + lane < n ? eq_factor(P.r[nl + lane], (blockIdx.x >> lane) & 1) : fe_one<FrConsts>();
+    for (int off = 1; off < n - nl; off <<= 1) {
+      Fr o;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) o.v[w] = __shfl_down_sync(0xffffffffu, a.v[w], off);
+      if (lane + off < 32) a = rmul(a, o);
+    }
+    if (lane == 0) high = a;
+  }
+  __syncthreads();
+  if (n > nl && t < 1 << na) tab[0][t] = rmul(tab[0][t], high);
+  __syncthreads();
+  for (int e = t; e < 1 << nl; e += 256)
+    st_fe(&out[((size_t)blockIdx.x << nl) + e], rmul(tab[0][e & ((1 << na) - 1)], tab[1][e >> na]));
 }
 
 }  // namespace
@@ -492,30 +587,17 @@ static Fr to_dev(const F& a) {
   return r;
 }
 
-// eq(r, y) for every y < 2^|r|. Up to 12 variables each entry is its own
-// product of |r| factors; beyond, the two halves' tables (2^(n/2) entries
-// each) are built that way and every entry is one product of the two.
 void lift_column(Ctx& c, const void* p, int bits, size_t n, Fr* out) {
   if (n) launch(c, k_lift, (unsigned)((n + 255) / 256), 256, 0, p, bits, n, out);
 }
 
 void build_eq_table(Ctx& c, const std::vector<F>& r, Fr* out) {
   const int n = (int)r.size();
-  const size_t len = (size_t)1 << n;
-  const int nlo = n / 2, nhi = n - nlo;
-  const bool split = n > 12;
-  const size_t lo_len = (size_t)1 << nlo, hi_len = (size_t)1 << nhi;
-  Fr* d_r = c.scratch[S_TMP4].as<Fr>(std::max<size_t>(n, 1) + (split ? lo_len + hi_len : 0));
-  if (n) APG_CUDA(cudaMemcpyAsync(d_r, r.data(), 32 * (size_t)n, cudaMemcpyHostToDevice, c.stream));
-  if (!split) {
-    launch(c, k_eq_table, (unsigned)((len + 255) / 256), 256, 0, (const Fr*)d_r, n, len, out);
-    return;
-  }
-  Fr* lo = d_r + n;
-  Fr* hi = lo + lo_len;
-  launch(c, k_eq_table, (unsigned)((lo_len + 255) / 256), 256, 0, (const Fr*)d_r, nlo, lo_len, lo);
-  launch(c, k_eq_table, (unsigned)((hi_len + 255) / 256), 256, 0, (const Fr*)(d_r + nlo), nhi, hi_len, hi);
-  launch(c, k_eq_combine, (unsigned)((len + 255) / 256), 256, 0, (const Fr*)lo, (const Fr*)hi, nlo, len, out);
+  EqPoint p;
+  if (n > (int)(sizeof(p.r) / sizeof(Fr))) throw Error(APG_ERR_INVALID_ARGUMENT, "an eq table of more than 40 variables");
+  memset(&p, 0, sizeof(p));
+  if (n) memcpy(p.r, r.data(), 32 * (size_t)n);
+  launch(c, k_eq_table, 1u << std::max(0, n - kEqLow), 256, 0, p, n, out);
 }
 
 static VirtualRound virtual_round(const std::vector<F>& point, int nvars) {
@@ -543,7 +625,17 @@ static VirtualRound virtual_round(const std::vector<F>& point, int nvars) {
   return V;
 }
 
-// How many of a short quadratic form's last rounds run on the host. Both sides
+// The host's side of a factored quadratic form (k_round_form).
+struct HostForm {
+  std::vector<FormGroup> groups;  // by falling cost
+  std::vector<FormTerm> terms;
+  std::vector<F> coeffs;  // one a term, then the groups' constants
+  size_t cost = 0;        // wide products a node
+  size_t muls = 0;        // products a node
+};
+bool quadratic_form(const HostProgram& hp, int slots, HostForm& out);
+
+// How many of a short form's last rounds run on the host. Both sides
 // pay the transcript's permutations (6 us each: three a round on the device's
 // way, which hides one, four on the host's); a device round adds its launch, a
 // kernel of about 10 us and the flag, a host round its products at 20 ns: two a
@@ -553,8 +645,8 @@ static VirtualRound virtual_round(const std::vector<F>& point, int nvars) {
 // 352, 356, 381 us, 2^16 rows 807, 754, 743, 774, the GKR proof of a 7-column
 // 2^12-row shard 4528, 4290, 4343, 4496.
 constexpr size_t kHostTailProducts = 200;
-static int host_tail_rounds(int n, int nd, const HostPairTerms& t) {
-  const size_t nt = (size_t)nd + 1, per_pair = 2 * nt + 4 * t.a.size() + 2;
+static int host_tail_rounds(int n, int nd, const HostForm& f) {
+  const size_t nt = (size_t)nd + 1, per_pair = 2 * nt + 2 * f.muls + 2;
   int k = 0;
   while (k < n && (per_pair << k) <= kHostTailProducts) ++k;
   if (n == k + 1) ++k;  // round 0 binds nothing: a list this short is gathered whole
@@ -562,62 +654,100 @@ static int host_tail_rounds(int n, int nd, const HostPairTerms& t) {
   return n == k + 1 ? 0 : k;
 }
 
-// k_round_terms' pairs a block: in small rounds as many as give a thread one
-// entry to fold, growing (for the shares' evenness) while the blocks still fill
-// the device four times and shared memory leaves four blocks an SM.
-struct TermsShape {
-  int log_pairs;
-  unsigned blocks;
+// k_round_form's block: `share` warps split the groups of each tile of pairs.
+struct FormShape {
+  int share, log_pp, passes;
+  unsigned threads, blocks;
   size_t smem;
 };
-#ifndef APG_TERMS_SMEM
-#define APG_TERMS_SMEM (56 * 1024)
-#endif
-static TermsShape terms_shape(size_t npairs, int nt, int sm_count) {
-  TermsShape s;
-  s.log_pairs = 0;
-  auto smem = [&](int lp) { return (size_t)nt * 64 << lp; };
-  while (s.log_pairs < 6 && ((size_t)nt << (s.log_pairs + 2)) <= (size_t)kTermThreads) ++s.log_pairs;
-  while (s.log_pairs < 6 && smem(s.log_pairs + 1) <= (size_t)(APG_TERMS_SMEM) &&
-         (npairs >> (s.log_pairs + 1)) >= (size_t)sm_count * 4)
-    ++s.log_pairs;
-  s.blocks = (unsigned)std::min<size_t>((npairs + ((size_t)1 << s.log_pairs) - 1) >> s.log_pairs, (size_t)sm_count * 8);
-  s.smem = smem(s.log_pairs);
+constexpr size_t kFormSmemMax = 200 * 1024;
+constexpr size_t kFormSmem = 48 * 1024;       // (20, 28, 36, 72, 100 KB: within 1 % or up to 6 % slower)
+constexpr size_t kFormSmemThree = 40 * 1024;  // (three passes: zerochecks 5 % faster, 21-table lists 1 % slower)
+constexpr size_t kFormShareCost = 2000;       // (500, 1000: a 10-column 2^21-row GKR proof 17 %, 5 % slower)
+static FormShape form_shape(const HostForm& f, size_t npairs, int slots, bool three, int sm_count) {
+  const size_t line = (size_t)(slots + 1) * (three ? 3 : 2) * sizeof(Fr);  // a pair's values
+  FormShape s;
+  s.passes = three && line * 32 <= kFormSmemThree ? 3 : 1;
+  const int log_p = s.passes == 3 ? 5 : three ? 3 : 4;  // a tile
+  s.log_pp = log_p;
+  if (npairs <= ((size_t)sm_count * 2 << 4)) {
+    // About a tile a block: every warp a share of its own, and few enough lines
+    // a block that a thread folds one or two.
+    s.share = f.groups.size() > 16 ? kFormMaxWarps : 8;
+    s.threads = 32 * s.share;
+    while (s.log_pp > 0 && ((size_t)1 << (s.log_pp - 1)) >= npairs) --s.log_pp;
+    while (s.log_pp > 0 && ((size_t)(slots + 1) << s.log_pp) > 2 * s.threads && (npairs >> (s.log_pp - 1)) <= (size_t)sm_count)
+      --s.log_pp;
+  } else {
+    // As many tiles as the shared memory of four blocks an SM takes, and a
+    // share for every two thousand wide products (a share costs its own weight
+    // and reduction, 270).
+    int tiles = 1, share = 1;
+    while (tiles < 8 && line * ((size_t)2 * tiles << log_p) <= kFormSmem) tiles *= 2;
+    while (share * tiles < 8 && ((size_t)share * 2 * kFormShareCost <= f.cost || share * tiles < 4)) share *= 2;
+    s.share = share;
+    s.threads = 32 * share * tiles;
+    for (int t = tiles; t > 1; t /= 2) ++s.log_pp;
+  }
+  while (s.log_pp > 0 && (line << s.log_pp) > kFormSmemMax) {
+    --s.log_pp;
+    if (s.log_pp >= log_p) s.threads /= 2;
+  }
+  s.smem = line << s.log_pp;
+  s.blocks = (unsigned)std::min<size_t>((npairs + ((size_t)1 << s.log_pp) - 1) >> s.log_pp, (size_t)sm_count * 8);
   return s;
 }
 
-void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint8_t>& vkinds, int n_cached,
+void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8_t>& vkinds,
                   const std::vector<const Fr*>& src, const std::vector<F>& eq_point, host::Transcript& tr,
                   std::vector<std::array<F, 4>>& rounds, std::vector<F>& point, std::vector<F>& finals,
-                  const std::vector<uint8_t>& src_bits, const HostPairTerms* pairs) {
+                  const std::vector<uint8_t>& src_bits) {
   const int n = (int)eq_point.size();
   const int nt = nd + 1;  // with eq
   if (vkinds.size() > 8) throw Error(APG_ERR_BAD_CIRCUIT, "more than 8 virtual tables");
   rounds.clear();
   point.clear();
   finals.assign(nd, host::fzero());
-
-  // Round-0 sources: the data tables, then eq built from the eq point.
   const size_t len0 = (size_t)1 << n;
   Fr* eq = c.scratch[S_TMP3].as<Fr>(len0);
   build_eq_table(c, eq_point, eq);
-  std::vector<const Fr*> srcs(src);
-  srcs.push_back(eq);
-  const Fr** d_src = c.scratch[S_TMP5].as<const Fr*>(nt);
-  APG_CUDA(cudaMemcpyAsync(d_src, srcs.data(), sizeof(Fr*) * nt, cudaMemcpyHostToDevice, c.stream));
-  // Stored widths of the data tables, when any is narrow (eq is Fr).
-  const uint8_t* d_bits = nullptr;
+
+  const int n_val = nd + (int)vkinds.size(), n_cached = hp.n_cached;
+  HostForm form;
+  const bool use_form = (size_t)(n_val + 1) * 3 * sizeof(Fr) <= kFormSmemMax && quadratic_form(hp, n_val, form);
+  const int host_rounds = use_form && vkinds.empty() ? host_tail_rounds(n, nd, form) : 0;
+
+  // One upload: the counter of finished blocks (zero), the round-0 sources (the
+  // data tables, then eq), their stored widths when any is narrow (eq is Fr)
+  // and the form. `up` lives until the copy from it has surely run (the rounds).
   bool narrow = false;
   for (uint8_t b : src_bits) narrow |= b != 0;
-  if (narrow) {
-    if ((int)src_bits.size() != nd) throw Error(APG_ERR_INTERNAL, "one width per data table");
-    std::vector<uint8_t> bits(src_bits);
-    bits.push_back(0);
-    uint8_t* db = c.scratch[S_ENTRIES].as<uint8_t>(nt);
-    APG_CUDA(cudaMemcpyAsync(db, bits.data(), nt, cudaMemcpyHostToDevice, c.stream));
-    APG_CUDA(cudaStreamSynchronize(c.stream));  // `bits` is a host temporary
-    d_bits = db;
-  }
+  if (narrow && (int)src_bits.size() != nd) throw Error(APG_ERR_INTERNAL, "one width per data table");
+  std::vector<const Fr*> srcs(src);
+  srcs.push_back(eq);
+  std::vector<uint8_t> bits(narrow ? src_bits : std::vector<uint8_t>());
+  if (narrow) bits.push_back(0);
+  std::vector<uint8_t> up(32, 0);
+  auto put = [&](const void* p, size_t len) {
+    const size_t at = (up.size() + 31) & ~(size_t)31;
+    up.resize(at + len);
+    if (len) memcpy(up.data() + at, p, len);
+    return at;
+  };
+  const size_t at_src = put(srcs.data(), sizeof(Fr*) * nt), at_bits = put(bits.data(), bits.size()),
+               at_g = put(form.groups.data(), form.groups.size() * sizeof(FormGroup)),
+               at_t = put(form.terms.data(), form.terms.size() * sizeof(FormTerm)),
+               at_c = put(form.coeffs.data(), form.coeffs.size() * 32);
+  uint8_t* d_up = c.scratch[S_PAIR_TERMS].as<uint8_t>(up.size());
+  APG_CUDA(cudaMemcpyAsync(d_up, up.data(), up.size(), cudaMemcpyHostToDevice, c.stream));
+  unsigned* done = reinterpret_cast<unsigned*>(d_up);
+  const Fr** d_src = reinterpret_cast<const Fr**>(d_up + at_src);
+  const uint8_t* d_bits = narrow ? d_up + at_bits : nullptr;
+  DevForm DF;
+  DF.groups = reinterpret_cast<const FormGroup*>(d_up + at_g);
+  DF.terms = reinterpret_cast<const FormTerm*>(d_up + at_t);
+  DF.coeffs = reinterpret_cast<const Fr*>(d_up + at_c);
+  DF.ng = (int)form.groups.size();
 
   // Level buffers: level r (r >= 1) holds nt tables of 2^(n-r) entries.
   Fr* lvl[2] = {nullptr, nullptr};
@@ -625,73 +755,50 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     lvl[1] = c.scratch[S_LEVEL_A].as<Fr>((size_t)nt * (len0 / 2));
     lvl[0] = c.scratch[S_LEVEL_B].as<Fr>((size_t)nt * (len0 / 4 > 0 ? len0 / 4 : 1));
   }
-  const int n_val = nd + (int)vkinds.size();
-  const int slots = 2 * n_val + n_cached;
+  // The interpreter's shapes (gate lists that are no quadratic form).
   // Wide gate lists get narrower blocks (a power of two, for the reduction
   // tree) so that every thread's slots still fit in shared memory.
   // (Down to 8 threads a block for the widest lists, e.g. 130-column ones.)
+  const int slots = 2 * n_val + n_cached;
   int threads = kRoundThreads;
   while (threads > 8 && (size_t)std::max(slots, 1) * 32 * threads > 200 * 1024) threads /= 2;
   const size_t smem = (size_t)std::max(slots, 1) * 32 * threads;
   // Lists of many gates go one pair per warp (k_round_warp): the pair's
   // tables are stored once for the warp instead of once per thread.
-  const bool warp_mode = prog.n_weighted >= kWarpModeGates;
-  if (!warp_mode && smem > 200 * 1024) throw Error(APG_ERR_BAD_CIRCUIT, "gate list too wide for one thread block");
-  APG_CUDA(cudaFuncSetAttribute(k_round, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  const bool warp_mode = hp.n_weighted >= kWarpModeGates;
   const int max_blocks = c.sm_count * 8 * (kRoundThreads / threads);  // the same thread count in smaller blocks
   const int warp_slots = n_val + n_cached + n_val + 2;
   const size_t warp_smem = (size_t)(kRoundThreads / 32) * warp_slots * 32;
-  if (warp_mode && warp_smem > 200 * 1024) throw Error(APG_ERR_BAD_CIRCUIT, "gate list too wide for one thread block");
-  if (warp_mode) APG_CUDA(cudaFuncSetAttribute(k_round_warp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   // Rounds with few enough pairs for one warp each in a single wave run one
-  // pair per warp whatever the list's width (APG_SMALL_WARP): the lanes fold
-  // the tables and evaluate the gates side by side, so a round's latency is a
-  // fold and a gate, not one thread's chain through every fold and gate.
-  const bool small_warp_ok = APG_SMALL_WARP && warp_smem <= 200 * 1024;
-  if (small_warp_ok)
-    APG_CUDA(cudaFuncSetAttribute(k_round_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  // pair per warp whatever the list's width: the lanes fold the tables and
+  // evaluate the gates side by side, so a round's latency is a fold and a gate,
+  // not one thread's chain through every fold and gate.
+  const bool small_warp_ok = warp_smem <= 200 * 1024;
   const int warp_max_blocks = c.sm_count * 16;
-  APG_CUDA(cudaFuncSetAttribute(k_round_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  DevProgram P;
+  memset(&P, 0, sizeof(P));
+  if (use_form) {
+    for (auto k : {form_kernel(256), form_kernel(512)})
+      APG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFormSmemMax));
+  } else {
+    if ((warp_mode ? warp_smem : smem) > 200 * 1024)
+      throw Error(APG_ERR_BAD_CIRCUIT, "gate list too wide for one thread block");
+    upload_program(c, hp, P);
+    P.cached_slot0 = n_val;
+    APG_CUDA(cudaFuncSetAttribute(k_round, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    APG_CUDA(cudaFuncSetAttribute(k_round_warp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    APG_CUDA(cudaFuncSetAttribute(k_round_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  }
   Fr* partials = c.scratch[S_TMP6].as<Fr>((size_t)std::max(max_blocks, warp_max_blocks) * 4);
-  unsigned* done = c.scratch[S_ROUND].as<unsigned>(1);
-  APG_CUDA(cudaMemsetAsync(done, 0, sizeof(unsigned), c.stream));
   uint8_t* pinned = c.host_pinned();
   const F* sums = reinterpret_cast<const F*>(pinned + Ctx::kPinnedSums);
   Fr* host_tables = reinterpret_cast<Fr*>(pinned + Ctx::kPinnedTables);
-  DevProgram P = prog;
-  P.cached_slot0 = n_val;
-  // The terms on the device (when the summand is a short quadratic form).
-  PairTerms PT;
-  memset(&PT, 0, sizeof(PT));
-  const bool use_terms = pairs && vkinds.empty() && n_cached == 0 && !pairs->a.empty() && (size_t)nt * 64 <= 200 * 1024;
-  const int host_rounds = use_terms ? host_tail_rounds(n, nd, *pairs) : 0;
-  std::vector<uint8_t> h;  // (lives until the copy from it has surely run: the first round's end)
-  if (use_terms && host_rounds < n) {
-    const size_t nt_ = pairs->a.size();
-    const size_t cb = 32 * nt_, ab = 2 * nt_, total = cb + 2 * ab + nt_ + 4 * 32;
-    uint8_t* d = c.scratch[S_PAIR_TERMS].as<uint8_t>(total);
-    h.assign(total, 0);
-    size_t off = 0;
-    auto put = [&](const void* p, size_t n) {
-      const size_t at = (off + 31) & ~(size_t)31;
-      if (n) memcpy(h.data() + at, p, n);
-      off = at + n;
-      return d + at;
-    };
-    std::vector<uint8_t> unit(nt_);
-    for (size_t j = 0; j < nt_; ++j) unit[j] = pairs->c[j] == host::fone() ? 1 : 0;
-    PT.c = reinterpret_cast<const Fr*>(put(pairs->c.data(), cb));
-    PT.a = reinterpret_cast<const uint16_t*>(put(pairs->a.data(), ab));
-    PT.b = reinterpret_cast<const uint16_t*>(put(pairs->b.data(), ab));
-    PT.unit = put(unit.data(), nt_);
-    PT.n = (int)nt_;
-    APG_CUDA(cudaMemcpyAsync(d, h.data(), total, cudaMemcpyHostToDevice, c.stream));
-  }
 
   // 1/r_j for every nonzero eq coordinate, from one inversion (Montgomery's
-  // batch trick): the rounds divide by their coordinate.
+  // batch trick): the rounds divide by their coordinate. Found while the device
+  // works on round 0, which needs none.
   std::vector<F> inv_r(n, host::fzero());
-  {
+  auto invert_coordinates = [&]() {
     std::vector<F> pre(n + 1, host::fone());
     for (int j = 0; j < n; ++j) pre[j + 1] = eq_point[j].zero() ? pre[j] : host::fmul(pre[j], eq_point[j]);
     F inv = host::finv(pre[n]);
@@ -700,7 +807,7 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
       inv_r[j] = host::fmul(inv, pre[j]);
       inv = host::fmul(inv, eq_point[j]);
     }
-  }
+  };
   F chal = host::fzero();
   // The round polynomial factors as s(X) = eq_r(X) q(X): eq's factor for this
   // variable, eq_r(X) = (1 - r_r)(1 - X) + r_r X, is common to every pair, and
@@ -776,9 +883,9 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
                                                    (size_t)warp_max_blocks)
                            : (int)std::min<size_t>((work + threads - 1) / threads, (size_t)max_blocks);
     cudaEvent_t t0 = c.timer_begin();
-    if (use_terms) {
-      const TermsShape t = terms_shape(A.npairs, nt, c.sm_count);
-      launch(c, k_round_terms, t.blocks, kTermThreads, t.smem, A, PT, t.log_pairs, partials);
+    if (use_form) {
+      const FormShape f = form_shape(form, A.npairs, n_val, needs_one(r), c.sm_count);
+      launch(c, form_kernel(f.threads), f.blocks, f.threads, f.smem, A, DF, V, f.share, f.log_pp, f.passes, partials);
     }
     else if (small_warp_ok && A.npairs * 32 <= (size_t)kRoundThreads * c.sm_count * 4)
       launch(c, k_round_warp<true>, (int)((A.npairs + kRoundThreads / 32 - 1) / (kRoundThreads / 32)), kRoundThreads,
@@ -788,6 +895,7 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     c.timer_end(APG_TIMER_SUMCHECK_ROUND, t0);
     // While the device works: the message's tag and length need no sums.
     tr.open(host::T_SUMCHECK_ROUND, 4);
+    if (r == 0 && n > 1) invert_coordinates();
     c.wait_flag();
     const auto host0 = Clock::now();
     F q[4] = {sums[0], sums[1], sums[2], host::fzero()};
@@ -798,6 +906,7 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
     if (dev_rounds == 0) {
       launch(c, k_gather, 1, 256, 0, (const Fr* const*)d_src, d_bits, nt, len0, host_tables,
              reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
+      if (n > 1) invert_coordinates();
       c.wait_flag();
     }
     // Level dev_rounds - 1 (or the source tables), still to be bound with the last challenge.
@@ -826,11 +935,15 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
             return x == 0 ? t[0] : x == 1 ? t[1] : host::fsub(host::fadd(t[1], t[1]), t[0]);
           };
           F s = host::fzero();
-          for (size_t j = 0; j < pairs->a.size(); ++j) {
-            F v = pairs->c[j];
-            if (pairs->a[j] != kNoTable) v = v == host::fone() ? at(pairs->a[j]) : host::fmul(v, at(pairs->a[j]));
-            if (pairs->b[j] != kNoTable) v = host::fmul(v, at(pairs->b[j]));
-            s = host::fadd(s, v);
+          for (const FormGroup& G : form.groups) {
+            F in = G.d == kNoConst ? host::fzero() : form.coeffs[G.d];
+            for (uint32_t t = G.off; t < G.off + G.n; ++t) {
+              const F v = at(form.terms[t].b);
+              const uint16_t kind = form.terms[t].kind;
+              in = kind == TERM_MINUS ? host::fsub(in, v)
+                                      : host::fadd(in, kind == TERM_PLUS ? v : host::fmul(form.coeffs[t], v));
+            }
+            s = host::fadd(s, G.a == kNoTable ? in : host::fmul(at(G.a), in));
           }
           q[x] = host::fadd(q[x], host::fmul(w, s));
         }
@@ -863,211 +976,216 @@ void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint
 // A device copy of a resolved gate list.
 namespace {
 
-// A summed gate list without cached entries is one quadratic form in its
-// slots: S = sum_j w_j g_j = C + sum_i A_i x_i + sum_{a<=b} B_ab x_a x_b.
-// Expanding every gate into those monomials (weights applied on the host)
-// and merging equal monomials across gates needs fewer products per node
-// than evaluating the gates one by one when the gates share operands (the
-// reference's family circuits: about 30 % fewer). The form is emitted as
-// quadratic gates of at most kLinChunk coefficients, weight 1, so the lanes
-// of a warp still split the work and every coefficient is under the 0/1/-1
-// masks. Exact field arithmetic: the sum is the same at every node.
-constexpr int kLinChunk = 31;
-
-bool linearize(HostProgram& hp) {
-  if (!hp.summed || hp.n_cached != 0 || hp.n_weighted < kWarpModeGates) return false;
-  const F one = host::fone(), zero = host::fzero(), minus_one = host::fneg(host::fone());
-  auto triv = [&](const F& v) { return v == zero || v == one || v == minus_one; };
-  F cst = zero;
-  std::map<uint16_t, F> lin;
-  std::map<std::pair<uint16_t, uint16_t>, F> quad;
-  auto add_lin = [&](uint16_t a, const F& v) { lin[a] = host::fadd(lin.count(a) ? lin[a] : zero, v); };
-  auto add_quad = [&](uint16_t a, uint16_t b, const F& v) {
+// A polynomial of degree two at most in the slots: terms keyed by their two
+// slots, lower first, kNoTable for an absent second one.
+struct QuadPoly {
+  F c = host::fzero();
+  std::map<std::pair<uint16_t, uint16_t>, F> m;
+  void add(uint16_t a, uint16_t b, const F& v) {
     const auto k = a < b ? std::make_pair(a, b) : std::make_pair(b, a);
-    quad[k] = host::fadd(quad.count(k) ? quad[k] : zero, v);
+    auto it = m.emplace(k, v);
+    if (!it.second) it.first->second = host::fadd(it.first->second, v);
+  }
+};
+
+// Adds w times the gate's value to `out`; operands at `slots` and above are the
+// cached entries' polynomials. False when the degree passes two.
+bool add_gate(const HostProgram& hp, const DevGate& g, const F& w, int slots, const std::vector<QuadPoly>& cached,
+              QuadPoly& out) {
+  const F* c = hp.coeffs.data() + g.cf_off;
+  const uint16_t* o = hp.ops.data() + g.op_off;
+  auto linear = [&](uint16_t a, const F& v) {
+    if (a < slots) {
+      out.add(a, kNoTable, v);
+      return;
+    }
+    const QuadPoly& p = cached[a - slots];
+    out.c = host::fadd(out.c, host::fmul(v, p.c));
+    for (auto& t : p.m) out.add(t.first.first, t.first.second, host::fmul(v, t.second));
   };
-  long now = 0;  // products a node as the gates stand
-  for (int j = 0; j < hp.n_weighted; ++j) {
-    const DevGate& g = hp.gates[j];
-    const F w = j < (int)hp.weights.size() ? hp.weights[j] : one;
-    const F* c = hp.coeffs.data() + g.cf_off;
-    const uint16_t* o = hp.ops.data() + g.op_off;
-    const int t = g.p1, u = g.p2;
-    now += w == one ? 0 : 1;
-    switch (g.kind) {
-      case G_LINEAR:
-        for (int i = 0; i < t; ++i) add_lin(o[i], host::fmul(w, c[i])), now += triv(c[i]) ? 0 : 1;
-        cst = host::fadd(cst, host::fmul(w, c[t]));
-        break;
-      case G_PRODUCT:
-        add_quad(o[0], o[1], host::fmul(w, c[0]));
-        now += 1 + (triv(c[0]) ? 0 : 1);
-        break;
-      case G_MASK:  // x m + 1 - m
-        add_quad(o[0], o[1], w);
-        add_lin(o[1], host::fneg(w));
-        cst = host::fadd(cst, w);
-        now += 1;
-        break;
-      case G_AFFINE: {  // (sum l_i x_i + l_t)(sum r_k y_k + r_u)
-        const F lt = c[t], ru = c[t + 1 + u];
-        for (int i = 0; i < t; ++i) {
-          for (int k = 0; k < u; ++k) add_quad(o[i], o[t + k], host::fmul(w, host::fmul(c[i], c[t + 1 + k])));
-          add_lin(o[i], host::fmul(w, host::fmul(c[i], ru)));
-          now += triv(c[i]) ? 0 : 1;
-        }
-        for (int k = 0; k < u; ++k) {
-          add_lin(o[t + k], host::fmul(w, host::fmul(lt, c[t + 1 + k])));
-          now += triv(c[t + 1 + k]) ? 0 : 1;
-        }
-        cst = host::fadd(cst, host::fmul(w, host::fmul(lt, ru)));
-        now += 1;
-        break;
+  auto product = [&](uint16_t a, uint16_t b, const F& v) {
+    if (a < slots && b < slots) {
+      out.add(a, b, v);
+      return true;
+    }
+    QuadPoly pa, pb;
+    if (a < slots) pa.add(a, kNoTable, host::fone());
+    else pa = cached[a - slots];
+    if (b < slots) pb.add(b, kNoTable, host::fone());
+    else pb = cached[b - slots];
+    out.c = host::fadd(out.c, host::fmul(v, host::fmul(pa.c, pb.c)));
+    for (auto& t : pa.m) out.add(t.first.first, t.first.second, host::fmul(v, host::fmul(t.second, pb.c)));
+    for (auto& t : pb.m) out.add(t.first.first, t.first.second, host::fmul(v, host::fmul(t.second, pa.c)));
+    for (auto& t : pa.m)
+      for (auto& u : pb.m) {
+        if (t.first.second != kNoTable || u.first.second != kNoTable) return false;
+        out.add(t.first.first, u.first.first, host::fmul(v, host::fmul(t.second, u.second)));
       }
-      case G_TREE_PRODUCT:
-        add_quad(o[0], o[1], w);
-        now += 1;
-        break;
-      case G_TREE_CROSS:
-        add_quad(o[0], o[3], w);
-        add_quad(o[1], o[2], w);
-        now += 2;
-        break;
-      case G_QUADRATIC:
-        cst = host::fadd(cst, host::fmul(w, c[0]));
-        for (int i = 0; i < t; ++i) add_lin(o[i], host::fmul(w, c[1 + i])), now += triv(c[1 + i]) ? 0 : 1;
-        for (int k = 0; k < u; ++k) {
-          if (c[1 + t + k] == zero) continue;
-          add_quad(o[t + 2 * k], o[t + 2 * k + 1], host::fmul(w, c[1 + t + k]));
-          now += 1 + (triv(c[1 + t + k]) ? 0 : 1);
-        }
-        break;
-      default:
-        return false;
+    return true;
+  };
+  const int t = g.p1, u = g.p2;
+  switch (g.kind) {
+    case G_LINEAR:
+      for (int i = 0; i < t; ++i) linear(o[i], host::fmul(w, c[i]));
+      out.c = host::fadd(out.c, host::fmul(w, c[t]));
+      return true;
+    case G_PRODUCT:
+      return product(o[0], o[1], host::fmul(w, c[0]));
+    case G_MASK:  // x m + 1 - m
+      linear(o[1], host::fneg(w));
+      out.c = host::fadd(out.c, w);
+      return product(o[0], o[1], w);
+    case G_AFFINE: {  // (sum l_i x_i + l_t)(sum r_k y_k + r_u)
+      const F lt = host::fmul(w, c[t]), ru = host::fmul(w, c[t + 1 + u]);
+      for (int i = 0; i < t; ++i) {
+        const F li = host::fmul(w, c[i]);
+        for (int k = 0; k < u; ++k)
+          if (!product(o[i], o[t + k], host::fmul(li, c[t + 1 + k]))) return false;
+        linear(o[i], host::fmul(ru, c[i]));
+      }
+      for (int k = 0; k < u; ++k) linear(o[t + k], host::fmul(lt, c[t + 1 + k]));
+      out.c = host::fadd(out.c, host::fmul(lt, c[t + 1 + u]));
+      return true;
     }
+    case G_TREE_PRODUCT:
+      return product(o[0], o[1], w);
+    case G_TREE_CROSS:
+      return product(o[0], o[3], w) && product(o[1], o[2], w);
+    case G_QUADRATIC:
+      out.c = host::fadd(out.c, host::fmul(w, c[0]));
+      for (int i = 0; i < t; ++i) linear(o[i], host::fmul(w, c[1 + i]));
+      for (int k = 0; k < u; ++k)
+        if (!product(o[t + 2 * k], o[t + 2 * k + 1], host::fmul(w, c[1 + t + k]))) return false;
+      return true;
   }
-  std::vector<std::pair<uint16_t, F>> L;
-  std::vector<std::pair<std::pair<uint16_t, uint16_t>, F>> Q;
-  long lin_cost = 0;
-  for (auto& e : lin)
-    if (e.second != zero) L.push_back(e), lin_cost += triv(e.second) ? 0 : 1;
-  for (auto& e : quad)
-    if (e.second != zero) Q.push_back(e), lin_cost += 1 + (triv(e.second) ? 0 : 1);
-  if (lin_cost >= now) return false;
-  // Chunks of at most kLinChunk coefficients (the constant rides in chunk 0),
-  // at least one a lane of the warp.
-  const size_t terms = L.size() + Q.size();
-// At least 96 chunks (about three a lane): measured 3-5 % faster than 32, 64,
-// 128 or 192 on the reference's add_sub and shift_bitwise circuits.
-#ifndef APG_LIN_MIN_CHUNKS
-#define APG_LIN_MIN_CHUNKS 96
-#endif
-  const size_t chunks = std::max<size_t>((terms + kLinChunk - 2) / (kLinChunk - 1), APG_LIN_MIN_CHUNKS);
-  const size_t per = std::max<size_t>(1, (terms + chunks - 1) / chunks);
-  std::vector<DevGate> gates;
-  std::vector<uint16_t> ops;
-  std::vector<F> coeffs;
-  size_t li = 0, qi = 0;
-  bool first = true;
-  while (first || li < L.size() || qi < Q.size()) {
-    DevGate d;
-    memset(&d, 0, sizeof(d));
-    d.kind = G_QUADRATIC;
-    d.op_off = (uint32_t)ops.size();
-    d.cf_off = (uint32_t)coeffs.size();
-    coeffs.push_back(first ? cst : zero);
-    first = false;
-    size_t take = per;
-    int t = 0, u = 0;
-    std::vector<F> qc;
-    std::vector<uint16_t> qo;
-    while (take && li < L.size()) {
-      ops.push_back(L[li].first);
-      coeffs.push_back(L[li].second);
-      ++li, ++t, --take;
-    }
-    while (take && qi < Q.size()) {
-      qo.push_back(Q[qi].first.first);
-      qo.push_back(Q[qi].first.second);
-      qc.push_back(Q[qi].second);
-      ++qi, ++u, --take;
-    }
-    ops.insert(ops.end(), qo.begin(), qo.end());
-    coeffs.insert(coeffs.end(), qc.begin(), qc.end());
-    d.p1 = (uint16_t)t;
-    d.p2 = (uint16_t)u;
-    d.nops = (uint16_t)(t + 2 * u);
-    gates.push_back(d);
+  return false;
+}
+
+// The products a node takes gate by gate, and the terms its expansion may have.
+void gate_size(const HostProgram& hp, const DevGate& g, size_t& products, size_t& expanded) {
+  const F one = host::fone(), minus_one = host::fneg(one), zero = host::fzero();
+  const size_t t = g.p1, u = g.p2;
+  const size_t ncoef = g.kind == G_LINEAR ? t : g.kind == G_PRODUCT ? 1 : g.kind == G_AFFINE ? t + u + 1 : g.kind == G_QUADRATIC ? 1 + t + u : 0;
+  for (size_t i = 0; i < ncoef; ++i) {
+    const F& v = hp.coeffs[g.cf_off + i];
+    products += v == one || v == minus_one || v == zero ? 0 : 1;
   }
-  hp.gates = gates;
-  hp.ops = ops;
-  hp.coeffs = coeffs;
-  hp.n_weighted = (int)gates.size();
-  hp.weights.assign(gates.size(), one);
-  return true;
+  products += g.kind == G_LINEAR ? 0 : g.kind == G_QUADRATIC ? u : g.kind == G_TREE_CROSS ? 2 : 1;
+  expanded += g.kind == G_AFFINE ? (t + 1) * (u + 1) : 1 + t + u;
 }
 
 }  // namespace
 
-bool pair_terms_of(const HostProgram& hp, int nd, HostPairTerms& out) {
-  out = HostPairTerms();
-  if (hp.n_cached != 0 || hp.n_weighted <= 0) return false;
-  const F one = host::fone(), zero = host::fzero();
-  // Terms over the same tables merge (exact arithmetic: the sum is the same at
-  // every node). kNoTable sorts last: a linear term is (a, none).
-  std::map<std::pair<uint16_t, uint16_t>, F> merged;
-  auto term = [&](uint16_t a, uint16_t b, const F& cf) {
-    if ((a >= nd && a != kNoTable) || (b >= nd && b != kNoTable)) return false;
-    const auto k = a < b ? std::make_pair(a, b) : std::make_pair(b, a);
-    auto it = merged.find(k);
-    if (it == merged.end()) merged.emplace(k, cf);
-    else it->second = host::fadd(it->second, cf);
-    return true;
-  };
+// The summed gate list as one factored quadratic form: every gate expanded with
+// its weight and its cached operands' polynomials, equal monomials merged
+// (exact arithmetic: the sum is the same at every node), then grouped greedily
+// by the slot that the most remaining products share, whose linear term becomes
+// its group's constant. False when the degree passes two, or when the gates as
+// they stand take fewer products than the form.
+bool quadratic_form(const HostProgram& hp, int slots, HostForm& out) {
+  out = HostForm();
+  if (!hp.summed || slots >= kNoTable) return false;
+  size_t products = 0, expanded = 0;
+  for (const DevGate& g : hp.gates) gate_size(hp, g, products, expanded);
+  if (expanded > 20000) return false;
+  std::vector<QuadPoly> cached(hp.n_cached);
+  const F one = host::fone(), minus_one = host::fneg(one);
+  for (int j = 0; j < hp.n_cached; ++j) {
+    if (!add_gate(hp, hp.gates[j], one, slots, cached, cached[j])) return false;
+    if (cached[j].m.size() > 256) return false;
+  }
+  QuadPoly s;
   for (int j = 0; j < hp.n_weighted; ++j) {
-    const DevGate& g = hp.gates[j];
-    const F W = j < (int)hp.weights.size() ? hp.weights[j] : one;
-    const uint16_t* op = hp.ops.data() + g.op_off;
-    const F* cf = hp.coeffs.data() + g.cf_off;
-    bool ok = false;
-    switch (g.kind) {
-      case G_TREE_PRODUCT:  // v0 v1
-        ok = g.nops == 2 && term(op[0], op[1], W);
-        break;
-      case G_PRODUCT:  // c v0 v1
-        ok = g.nops == 2 && term(op[0], op[1], host::fmul(cf[0], W));
-        break;
-      case G_TREE_CROSS:  // v0 v3 + v1 v2
-        ok = g.nops == 4 && term(op[0], op[3], W) && term(op[1], op[2], W);
-        break;
-      case G_QUADRATIC:  // c0 + linear + products
-        ok = hp.n_weighted < kWarpModeGates && g.nops == g.p1 + 2 * g.p2 && term(kNoTable, kNoTable, host::fmul(cf[0], W));
-        for (uint32_t u = 0; ok && u < g.p1; ++u) ok = term(op[u], kNoTable, host::fmul(cf[1 + u], W));
-        for (uint32_t u = 0; ok && u < g.p2; ++u)
-          ok = term(op[g.p1 + 2 * u], op[g.p1 + 2 * u + 1], host::fmul(cf[1 + g.p1 + u], W));
-        break;
-      default:
-        ok = false;
+    const F w = j < (int)hp.weights.size() ? hp.weights[j] : one;
+    products += w == one ? 0 : 1;
+    if (!add_gate(hp, hp.gates[hp.n_cached + j], w, slots, cached, s)) return false;
+  }
+  // The products by slot; the linear terms apart.
+  struct Edge {
+    uint16_t a, b;
+    F v;
+    bool used;
+  };
+  std::vector<Edge> edges;
+  std::vector<std::vector<int>> at(slots);
+  std::vector<F> lin(slots, host::fzero());
+  for (auto& t : s.m) {
+    if (t.second.zero()) continue;
+    const uint16_t a = t.first.first, b = t.first.second;
+    if (b == kNoTable) {
+      lin[a] = t.second;
+      continue;
     }
-    if (!ok) return false;
+    at[a].push_back((int)edges.size());
+    if (b != a) at[b].push_back((int)edges.size());
+    edges.push_back({a, b, t.second, false});
   }
-  for (auto& kv : merged) {
-    if (kv.second == zero) continue;
-    out.a.push_back(kv.first.first);
-    out.b.push_back(kv.first.second);
-    out.c.push_back(kv.second);
+  struct Group {
+    uint16_t a;
+    F d;
+    std::vector<std::pair<uint16_t, F>> terms;
+    size_t cost;
+  };
+  std::vector<Group> groups;
+  auto weigh = [&](Group& g) {
+    size_t mul = 0;
+    for (auto& t : g.terms) mul += t.second == one || t.second == minus_one ? 0 : 1;
+    out.muls += mul + (g.a == kNoTable ? 0 : 1);
+    g.cost = 8 + 8 * g.terms.size() + 64 * mul + (mul ? 72 : 0) + (g.a == kNoTable ? 0 : 64);
+    out.cost += g.cost;
+  };
+  std::set<std::pair<int, int>> open;  // (-remaining products, slot)
+  std::vector<int> left(slots);
+  for (int k = 0; k < slots; ++k)
+    if ((left[k] = (int)at[k].size()) > 0) open.insert({-left[k], k});
+  while (!open.empty()) {
+    const int a = open.begin()->second;
+    Group g{(uint16_t)a, lin[a], {}, 0};
+    lin[a] = host::fzero();
+    for (int e : at[a]) {
+      Edge& E = edges[e];
+      if (E.used) continue;
+      E.used = true;
+      const uint16_t b = E.a == a ? E.b : E.a;
+      g.terms.push_back({b, E.v});
+      if (b != a) {
+        open.erase({-left[b], b});
+        if (--left[b] > 0) open.insert({-left[b], b});
+      }
+    }
+    open.erase({-left[a], a});
+    left[a] = 0;
+    weigh(g);
+    groups.push_back(std::move(g));
   }
-  if (out.a.empty() || out.a.size() > 4096 || nd >= kNoTable) {
-    out = HostPairTerms();
+  Group rest{kNoTable, s.c, {}, 0};
+  for (int k = 0; k < slots; ++k)
+    if (!lin[k].zero()) rest.terms.push_back({(uint16_t)k, lin[k]});
+  if (!rest.terms.empty() || !rest.d.zero()) {
+    weigh(rest);
+    groups.push_back(std::move(rest));
+  }
+  if (out.cost > 136 * products + 1000) {
+    out = HostForm();
     return false;
   }
+  std::stable_sort(groups.begin(), groups.end(), [](const Group& x, const Group& y) { return x.cost > y.cost; });
+  for (const Group& g : groups) {
+    out.groups.push_back({g.a, (uint16_t)g.terms.size(), (uint32_t)out.terms.size(), kNoConst});
+    for (auto& t : g.terms) {
+      out.terms.push_back({t.first, (uint16_t)(t.second == one ? TERM_PLUS : t.second == minus_one ? TERM_MINUS : TERM_MUL)});
+      out.coeffs.push_back(t.second);
+    }
+  }
+  for (size_t k = 0; k < groups.size(); ++k)
+    if (!groups[k].d.zero()) {
+      out.groups[k].d = (uint32_t)out.coeffs.size();
+      out.coeffs.push_back(groups[k].d);
+    }
   return true;
 }
 
-void upload_program(Ctx& c, const HostProgram& hp_in, DevProgram& P, int slot_cap) {
-  (void)slot_cap;
-  HostProgram hp = hp_in;
-  linearize(hp);
+void upload_program(Ctx& c, const HostProgram& hp, DevProgram& P) {
   std::vector<DevGate> gates = hp.gates;
   const std::vector<F>& coeffs = hp.coeffs;
   std::vector<F> weights = hp.weights;

@@ -61,35 +61,22 @@ __device__ __forceinline__ Fr narrow_entry(const void* p, int bits, size_t i) {
 // The first n entries of a column, lifted into an Fr table.
 void lift_column(Ctx& c, const void* p, int bits, size_t n, Fr* out);
 
-void upload_program(Ctx& c, const HostProgram& hp, DevProgram& P, int slot_cap);
+void upload_program(Ctx& c, const HostProgram& hp, DevProgram& P);
+// eq(r, y) for every y < 2^|r| (|r| at most 40).
 void build_eq_table(Ctx& c, const std::vector<host::F>& r, Fr* out);
 
 // Prove sum_y eq(eq_point, y) * S(y) over `src` tables (nd of them, each
-// 2^|eq_point| entries, device memory), drawing challenges from `tr`. Returns
+// 2^|eq_point| entries, device memory) and the virtual tables, S being the
+// weighted sum of the program's gates, drawing challenges from `tr`. Returns
 // the rounds' ascending coefficients, the bound point and each data table's
 // final value.
 // `src_bits` (empty: every table Fr) gives each data table's stored width;
 // narrow tables are read through the lift in the first two rounds and the
 // first bind writes Fr (the lazy lift of crates/poly/src/lib.rs:156-185).
-// A summand that is a short quadratic form in the data tables,
-// S = sum_j c_j T_{a_j} T_{b_j} with either factor or both absent (halving lists
-// of TreeProduct / TreeCross gates, a zerocheck's gate): its round kernels read
-// each term's lines and multiply, with no interpreter between, and its last few
-// rounds run on the host.
-constexpr uint16_t kNoTable = 0xffff;
-struct HostPairTerms {
-  std::vector<uint16_t> a, b;  // b absent: a linear term; both: the constant
-  std::vector<host::F> c;
-};
-// The program's terms, when every weighted gate expands to such terms over
-// data tables (slots below nd) and nothing is cached; false otherwise.
-bool pair_terms_of(const HostProgram& hp, int nd, HostPairTerms& out);
-
-void run_sumcheck(Ctx& c, const DevProgram& prog, int nd, const std::vector<uint8_t>& vkinds, int n_cached,
+void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8_t>& vkinds,
                   const std::vector<const Fr*>& src, const std::vector<host::F>& eq_point, host::Transcript& tr,
                   std::vector<std::array<host::F, 4>>& rounds, std::vector<host::F>& point,
-                  std::vector<host::F>& finals, const std::vector<uint8_t>& src_bits = {},
-                  const HostPairTerms* pairs = nullptr);
+                  std::vector<host::F>& finals, const std::vector<uint8_t>& src_bits = {});
 
 // `bits` (null: all Fr) is each table's stored width.
 int prove_zerocheck_impl(Ctx& c, size_t arity, const uint8_t* coefs, const uint32_t* ta, const uint32_t* tb,

@@ -45,6 +45,7 @@ static HostProgram zerocheck_program(const std::vector<F>& coefs, const uint32_t
   hp.weights.push_back(host::fone());
   hp.n_cached = 0;
   hp.n_weighted = 1;
+  hp.summed = true;
   return hp;
 }
 
@@ -110,13 +111,9 @@ int prove_zerocheck_impl(Ctx& c, size_t arity, const uint8_t* coefs, const uint3
   std::vector<F> r(num_vars);
   for (size_t j = 0; j < num_vars; ++j) r[j] = tr.challenge(host::T_SUMCHECK_CHALLENGE);
   HostProgram hp = zerocheck_program(cf, ta, tb, nterms);
-  DevProgram P;
-  upload_program(c, hp, P, 0);
   std::vector<std::array<F, 4>> rounds;
   std::vector<F> point, finals;
-  HostPairTerms pairs;
-  const bool by_pairs = pair_terms_of(hp, (int)arity, pairs);
-  run_sumcheck(c, P, (int)arity, {}, 0, src, r, tr, rounds, point, finals, src_bits, by_pairs ? &pairs : nullptr);
+  run_sumcheck(c, hp, (int)arity, {}, src, r, tr, rounds, point, finals, src_bits);
   for (auto& f : finals)
     if (!host::below_p(f.w)) throw Error(APG_ERR_INTERNAL, "non-canonical device value");
   tr.absorb(host::T_SUMCHECK_FINAL_EVALS, finals);
