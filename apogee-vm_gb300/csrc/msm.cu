@@ -92,6 +92,17 @@ __global__ void k_points_out(const Affine* src, size_t n, uint4* raw) {
   raw[4 * i + 3] = make_uint4(y.v[4], y.v[5], y.v[6], y.v[7]);
 }
 
+// words of a result and the error flags into pinned host memory, then the flag
+// the host waits for.
+__global__ void k_publish(const uint32_t* src, uint32_t words, const uint32_t* err, uint32_t* dst, uint32_t* head,
+                          uint32_t seq) {
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  if (threadIdx.x == 0) head[1] = *err;
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t*>(head) = seq;
+}
+
 }  // namespace
 
 // Canonical Fr -> Montgomery in place, flagging values >= p.
@@ -202,7 +213,7 @@ __global__ void k_recode(const void* scalars, size_t n, int c, int windows, int 
   }
 }
 
-// ---- exclusive scan (u32), three passes ------------------------------------
+// ---- exclusive scan (u32), two passes ------------------------------------
 
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;  // per thread
@@ -234,26 +245,28 @@ __global__ void k_scan_local(uint32_t* data, size_t n, uint32_t* block_sums) {
   if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = sh[threadIdx.x];
 }
 
-// Exclusive scan of up to kScanBlock block sums in one block; total at [nb].
-__global__ void k_scan_blocks(uint32_t* block_sums, int nb) {
-  __shared__ uint32_t sh[kScanBlock];
-  uint32_t v = threadIdx.x < (unsigned)nb ? block_sums[threadIdx.x] : 0;
-  sh[threadIdx.x] = v;
+// Adds to each k_scan_local block's entries the sums of the blocks before it,
+// which every block adds up for itself (kScanBlock of them at most); the total
+// goes to *total_out. One block's scan (its total already in block_sums[0])
+// needs no such launch.
+__global__ void __launch_bounds__(256) k_scan_add(uint32_t* data, size_t n, const uint32_t* block_sums,
+                                                  uint32_t* total_out) {
+  __shared__ uint32_t part[8];
+  uint32_t before = 0;
+  for (unsigned b = threadIdx.x; b < blockIdx.x; b += 256) before += block_sums[b];
+  for (int off = 16; off > 0; off >>= 1) before += __shfl_xor_sync(0xffffffffu, before, off);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = before;
   __syncthreads();
-  for (int off = 1; off < kScanBlock; off <<= 1) {
-    uint32_t t = threadIdx.x >= (unsigned)off ? sh[threadIdx.x - off] : 0;
-    __syncthreads();
-    sh[threadIdx.x] += t;
-    __syncthreads();
+  before = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) before += part[w];
+  const size_t base = (size_t)blockIdx.x * kScanBlock * kScanItems;
+#pragma unroll
+  for (int k = 0; k < kScanBlock * kScanItems / 256; ++k) {
+    const size_t i = base + k * 256 + threadIdx.x;
+    if (i < n) data[i] += before;
   }
-  if (threadIdx.x < (unsigned)nb) block_sums[threadIdx.x] = sh[threadIdx.x] - v;
-  if (threadIdx.x == kScanBlock - 1) block_sums[nb] = sh[threadIdx.x];
-}
-
-__global__ void k_scan_add(uint32_t* data, size_t n, const uint32_t* block_sums, uint32_t* total_out) {
-  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) data[i] += block_sums[i / (kScanBlock * kScanItems)];
-  if (i == 0) *total_out = block_sums[(n + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems)];
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_out = before + block_sums[blockIdx.x];
 }
 
 __global__ void k_scatter(const uint64_t* entries, size_t e_count, uint32_t* cursor, uint64_t* sorted) {
@@ -550,9 +563,11 @@ __global__ void __launch_bounds__(32) k_finish(const Xyzz* tsum, int spaces, int
     for (int j = 0; j < c; ++j) total = quad_dbl(total);
     total = quad_add(total, quad_ld(&in[w], l));
   }
-  const Affine a = xyzz_to_affine(quad_gather(total, lane), flags);
+  // (X / ZZ, Y / ZZZ) with 1 / (ZZ ZZZ) from one inversion, x and y in lanes 0 and 1.
+  const Xyzz t = quad_gather(total, lane);
+  const Fq inv = fe_inverse(cmul(t.zz, t.zzz), flags);  // (0 at infinity: the result is (0, 0))
+  const Fq r = fe_from_mont(cmul(l == 1 ? t.y : t.x, cmul(inv, l == 1 ? t.zz : t.zzz)));
   if (lane >= 2) return;
-  const Fq r = fe_from_mont(lane ? a.y : a.x);
   uint32_t* o = out64 + 16 * (size_t)blockIdx.x + 8 * lane;
 #pragma unroll
   for (int k = 0; k < 8; ++k) o[k] = r.v[k];
@@ -1472,6 +1487,21 @@ inline unsigned blocks_for(size_t n, int threads) {
 // Host side
 // ---------------------------------------------------------------------------
 
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host) {
+  uint8_t* pinned = c.host_pinned();
+  if (bytes > Ctx::kPinnedBytes - Ctx::kPinnedTables || bytes % 4) {
+    APG_CUDA(cudaMemcpyAsync(host, d_src, bytes, cudaMemcpyDeviceToHost, c.stream));
+    c.check_flags();
+    return;
+  }
+  uint32_t* head = reinterpret_cast<uint32_t*>(pinned);
+  launch(c, k_publish, 1, 256, 0, (const uint32_t*)d_src, (uint32_t)(bytes / 4), (const uint32_t*)c.d_flags,
+         reinterpret_cast<uint32_t*>(pinned + Ctx::kPinnedTables), head, ++c.flag_seq);
+  c.wait_flag();
+  memcpy(host, pinned + Ctx::kPinnedTables, bytes);
+  if (head[1]) c.check_flags();  // clears the flags and throws
+}
+
 void upload_points_async(Ctx& c, const uint8_t* host, size_t n, Affine* dst) {
   if (n == 0) return;
   uint4* raw = c.scratch[S_TMP7].as<uint4>(4 * n);
@@ -1652,7 +1682,7 @@ size_t pair_resident_threads(Ctx& c) {
   return (size_t)c.sm_count * (size_t)per_sm * kPairThreads;
 }
 
-constexpr size_t kMaxBins = (size_t)(kScanBlock - 1) * kScanBlock * kScanItems;  // one pass of the 3-kernel scan
+constexpr size_t kMaxBins = (size_t)(kScanBlock - 1) * kScanBlock * kScanItems;  // one pass of the scan
 constexpr size_t kMaxGroupEntries = (size_t)1 << 28;                           // 1 GiB of sorted references
 
 // The accumulation's slices hold at least this many references: a group too
@@ -1675,12 +1705,14 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   const Affine* src = p.precomp ? table->tab : bases;
   const uint32_t tab_n = p.precomp ? (uint32_t)table->n : 0;
 
-  uint32_t* counts = c.scratch[S_COUNTS].as<uint32_t>(nbins + 1);
   const size_t scan_blocks = (nbins + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
   uint32_t* blk = c.scratch[S_SCANBLK].as<uint32_t>(kScanBlock + 1);
-  uint32_t* total = c.scratch[S_OFFSETS].as<uint32_t>(1);
+  uint32_t* total = scan_blocks > 1 ? blk + kScanBlock : blk;
   uint32_t* sorted = c.scratch[S_SORTED].as<uint32_t>(std::max<size_t>(emax, 1));
-  Xyzz* buckets = c.scratch[S_BUCKETS].as<Xyzz>(nbins);
+  // The buckets and, after them, their counts: what a group must find at zero.
+  const size_t zero_bytes = nbins * sizeof(Xyzz) + (nbins + 1) * sizeof(uint32_t);
+  Xyzz* buckets = reinterpret_cast<Xyzz*>(c.scratch[S_BUCKETS].get(zero_bytes));
+  uint32_t* counts = reinterpret_cast<uint32_t*>(buckets + nbins);
 
   const size_t slice_min = acc_slice_min(emax);
   const size_t nseg =
@@ -1695,8 +1727,7 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   Xyzz* lvlR = c.scratch[S_LEVEL_A].as<Xyzz>((size_t)S * rp.blocks);
 
   cudaEvent_t t_total = c.timer_begin();
-  APG_CUDA(cudaMemsetAsync(counts, 0, (nbins + 1) * sizeof(uint32_t), c.stream));
-  APG_CUDA(cudaMemsetAsync(buckets, 0, nbins * sizeof(Xyzz), c.stream));
+  APG_CUDA(cudaMemsetAsync(buckets, 0, zero_bytes, c.stream));
   const int canon = scalars_canonical ? 1 : 0;
   // One pass over the digits: counted (place null) or placed.
   auto digits = [&](uint32_t* place) {
@@ -1722,8 +1753,8 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   };
   digits(nullptr);
   launch(c, k_scan_local, (unsigned)scan_blocks, kScanBlock, 0, counts, nbins, blk);
-  launch(c, k_scan_blocks, 1, kScanBlock, 0, blk, (int)scan_blocks);
-  launch(c, k_scan_add, blocks_for<int>(nbins, 256), 256, 0, counts, nbins, (const uint32_t*)blk, total);
+  if (scan_blocks > 1)
+    launch(c, k_scan_add, (unsigned)scan_blocks, 256, 0, counts, nbins, (const uint32_t*)blk, total);
   digits(sorted);
   cudaEvent_t t_acc = c.timer_begin();
   const uint32_t* pair_mode = nullptr;
@@ -1755,8 +1786,7 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
       uint32_t* st = cnt + (size_t)r * scan_n;
       launch(c, k_halve_counts, blocks_for<int>(scan_n, 256), 256, 0, ends_in, (uint32_t)nbins, st);
       launch(c, k_scan_local, sblocks, kScanBlock, 0, st, scan_n, blk);
-      launch(c, k_scan_blocks, 1, kScanBlock, 0, blk, (int)sblocks);
-      launch(c, k_scan_add, blocks_for<int>(scan_n, 256), 256, 0, st, scan_n, (const uint32_t*)blk, mode + 1);
+      if (sblocks > 1) launch(c, k_scan_add, sblocks, 256, 0, st, scan_n, (const uint32_t*)blk, mode + 1);
       const uint32_t* rr = r == 0 ? (const uint32_t*)sorted : (const uint32_t*)nullptr;
       const Affine* in = r == 0 ? src : lst[(r - 1) & 1];
       if (r == 0) {
@@ -1866,8 +1896,7 @@ void msm_device(Ctx& c, const Affine* bases, const SrsTable* table, const void* 
   uint8_t* d_out = out64_device ? out64_device : c.scratch[S_RESULT].as<uint8_t>(64);
   msm_multi(c, bases, table, &scalars, &n, 1, small_scalars, scalars_canonical, d_out, o);
   if (host_out) {
-    APG_CUDA(cudaMemcpyAsync(host_out, d_out, 64, cudaMemcpyDeviceToHost, c.stream));
-    c.check_flags();
+    fetch_checked(c, d_out, 64, host_out);
   }
 }
 
@@ -2004,8 +2033,8 @@ int msm_noalloc(const void* d_bases, const void* d_scalars, size_t n, void* d_ou
                                                             flags);
   APG_NA_LAUNCH();
   k_scan_local<<<(unsigned)scan_blocks, kScanBlock, 0, st>>>(counts, nbins, blk);
-  k_scan_blocks<<<1, kScanBlock, 0, st>>>(blk, (int)scan_blocks);
-  k_scan_add<<<blocks_for<int>(nbins, 256), 256, 0, st>>>(counts, nbins, (const uint32_t*)blk, total);
+  static_assert(kNoAllocBins > (size_t)kScanBlock * kScanItems, "one block's scan leaves its total elsewhere");
+  k_scan_add<<<(unsigned)scan_blocks, 256, 0, st>>>(counts, nbins, (const uint32_t*)blk, total);
   k_scatter<<<blocks_for<int>(E, 256), 256, 0, st>>>((const uint64_t*)entries, E, counts, sorted);
   APG_NA_LAUNCH();
   k_accumulate<<<blocks_for<int>(nseg, 128), 128, 0, st>>>((const uint64_t*)sorted, (const uint32_t*)total,
