@@ -224,6 +224,79 @@ __global__ void __launch_bounds__(kFwdThreads) k_forward(DevProgram P, int w, in
   for (int j = 0; j < width; ++j) st_fe(&out[(size_t)j * rows + y], eval_gate_dev(P, P.n_cached + j, sm));
 }
 
+// A halving list's gates over Fr layers: out[y] = a[y] a[y + rows], or with a
+// second column (TreeCross) a[y] b[y + rows] + a[y + rows] b[y]. A thread a gate
+// and row, no interpreter: the layer is read and written once (on a GB300, ten
+// columns over 2^21 rows: the first list 510 us in the staged interpreter, 207 so,
+// the 21 lists 1371 and 478).
+struct TreeGate {
+  const Fr* a;
+  const Fr* b;  // null: a product of a's halves
+};
+struct TreeLayer {
+  const TreeGate* gates;
+  Fr* out;
+  size_t rows;
+  int width;
+};
+
+__device__ __forceinline__ void tree_row(const TreeGate& G, size_t y, size_t rows, Fr* out) {
+  const Fr a0 = ld_fe(&G.a[y]), a1 = ld_fe(&G.a[y + rows]);
+  Fr v;
+  if (!G.b) {
+    v = fe_mul(a0, a1);
+  } else {
+    const Fr b0 = ld_fe(&G.b[y]), b1 = ld_fe(&G.b[y + rows]);
+    FeWide<FrConsts> s = wide_zero<FrConsts>();
+    wide_mac(s, a0, b1);
+    wide_mac(s, a1, b0);
+    v = fe_from_wide(s);
+  }
+  st_fe(out, v);
+}
+
+__global__ void __launch_bounds__(256) k_forward_tree(TreeLayer L) {
+  const TreeGate G = L.gates[blockIdx.y];
+  for (size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x; y < L.rows; y += (size_t)gridDim.x * blockDim.x)
+    tree_row(G, y, L.rows, &L.out[(size_t)blockIdx.y * L.rows + y]);
+}
+
+// The remaining halving lists, one after another in one block, once a list is
+// small (a launch a list costs more than its few rows).
+constexpr size_t kTreeTailCells = 4096;
+
+__global__ void __launch_bounds__(1024) k_forward_tree_tail(const TreeLayer* layers, int n) {
+  for (int k = 0; k < n; ++k) {
+    const TreeLayer L = layers[k];
+    const size_t cells = L.rows * L.width;
+    for (size_t t = threadIdx.x; t < cells; t += blockDim.x) {
+      const size_t g = t / L.rows;
+      tree_row(L.gates[g], t - g * L.rows, L.rows, &L.out[t]);
+    }
+    __syncthreads();
+  }
+}
+
+// Column x of the base into its place, a block row of the grid a column (the
+// columns of one upload's list: source, destination, bytes).
+struct ColumnCopy {
+  const uint8_t* src;
+  uint8_t* dst;
+  size_t bytes;
+};
+
+__global__ void __launch_bounds__(256) k_copy_columns(const ColumnCopy* cols) {
+  const ColumnCopy C = cols[blockIdx.y];
+  const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  size_t words = 0;
+  if (((uintptr_t)C.src & 15) == 0) {  // (the destination is 256-byte aligned)
+    words = C.bytes / 16;
+    for (size_t i = i0; i < words; i += stride)
+      reinterpret_cast<uint4*>(C.dst)[i] = reinterpret_cast<const uint4*>(C.src)[i];
+  }
+  for (size_t i = 16 * words + i0; i < C.bytes; i += stride) C.dst[i] = C.src[i];
+}
+
 }  // namespace
 
 // Layer k >= 1: width(k) Fr columns of 2^vars(k), contiguous. Layer 0, the
@@ -238,15 +311,15 @@ __global__ void __launch_bounds__(kFwdThreads) k_forward(DevProgram P, int w, in
 struct GkrValues {
   Ctx* ctx = nullptr;
   Circuit circuit;
-  std::vector<Fr*> layers;
+  uint8_t* pool = nullptr;   // every layer
+  std::vector<Fr*> layers;   // within it
   std::vector<size_t> base_off;
   std::vector<uint8_t> base_bits;
   bool base_narrow = false;
   Fr* lifted = nullptr;
   ~GkrValues() {
     cudaStream_t st = ctx ? ctx->stream : nullptr;
-    for (auto p : layers)
-      if (p) cudaFreeAsync(p, st);
+    if (pool) cudaFreeAsync(pool, st);
     if (lifted) cudaFreeAsync(lifted, st);
   }
   const void* base_raw(size_t x) const { return reinterpret_cast<const uint8_t*>(layers[0]) + base_off[x]; }
@@ -299,60 +372,125 @@ GkrValues* gkr_forward_impl(Ctx& c, const uint8_t* blob, size_t blob_len, const 
     V->base_off[x] = total;
     total += (narrow_bytes(V->base_bits[x], n0) + 255) / 256 * 256;
   }
-  APG_CUDA(cudaMallocAsync((void**)&V->layers[0], std::max<size_t>(total, 256), c.stream));
-  for (size_t x = 0; x < C.n_committed; ++x)
-    APG_CUDA(cudaMemcpyAsync(reinterpret_cast<uint8_t*>(V->layers[0]) + V->base_off[x], base[x],
-                             narrow_bytes(V->base_bits[x], n0),
-                             base_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.stream));
-  const uint8_t* d_bits = nullptr;
-  if (V->base_narrow) {
-    uint8_t* db = c.scratch[S_ENTRIES].as<uint8_t>(C.n_committed);
-    APG_CUDA(cudaMemcpyAsync(db, V->base_bits.data(), C.n_committed, cudaMemcpyHostToDevice, c.stream));
-    d_bits = db;
+  // Every layer in one allocation, the base first.
+  std::vector<size_t> layer_off(C.layers.size() + 1, 0);
+  for (size_t k = 0; k < C.layers.size(); ++k) {
+    layer_off[k + 1] = total;
+    total += (32 * ((size_t)1 << C.layers[k].num_vars) * std::max<uint32_t>(C.layers[k].width, 1) + 255) / 256 * 256;
   }
+  APG_CUDA(cudaMallocAsync((void**)&V->pool, std::max<size_t>(total, 256), c.stream));
+  for (size_t k = 0; k < V->layers.size(); ++k) V->layers[k] = reinterpret_cast<Fr*>(V->pool + layer_off[k]);
+
+  // What the host prepares for all layers goes up at once: the base's copies,
+  // its widths, the row-wise programs and column lists, the halving lists' gates.
+  struct Step {
+    bool tree = false;
+    PackedProgram prog{};
+    size_t cols = 0, gates = 0;
+  };
+  Packer up;
+  std::vector<Step> steps(C.layers.size());
+  std::vector<ColumnCopy> copies(C.n_committed);
+  for (size_t x = 0; x < C.n_committed; ++x)
+    copies[x] = {static_cast<const uint8_t*>(base[x]), V->pool + V->base_off[x], narrow_bytes(V->base_bits[x], n0)};
+  const size_t at_copies = up.put(copies.data(), copies.size() * sizeof(ColumnCopy));
+  const size_t at_bits = up.put(V->base_bits.data(), V->base_bits.size());
+  size_t first_tail = C.layers.size();
+  for (size_t k = 0; k < C.layers.size(); ++k) {
+    const CLayer& L = C.layers[k];
+    const size_t w = C.width(k);
+    std::vector<const Fr*> cols(w);
+    for (size_t x = 0; x < w; ++x) cols[x] = k == 0 ? reinterpret_cast<const Fr*>(V->base_raw(x)) : V->col(k, x);
+    steps[k].tree = L.halving && (k > 0 || !V->base_narrow);
+    if (steps[k].tree) {
+      std::vector<TreeGate> gates;
+      for (const CGate& G : L.producing)
+        gates.push_back({cols[G.ops[0].second], G.kind == G_TREE_CROSS ? cols[G.ops[1].second] : nullptr});
+      steps[k].gates = up.put(gates.data(), gates.size() * sizeof(TreeGate));
+    } else {
+      steps[k].prog = pack_program(layer_program(C, k, ch, false, {}), up);
+      steps[k].cols = up.put(cols.data(), cols.size() * sizeof(Fr*));
+    }
+  }
+  // The run of small halving lists at the top, one launch.
+  while (first_tail > 0) {
+    const CLayer& L = C.layers[first_tail - 1];
+    if (!steps[first_tail - 1].tree || ((size_t)L.width << L.num_vars) > kTreeTailCells) break;
+    --first_tail;
+  }
+  const size_t at_tail = up.put(nullptr, 0), tail_n = C.layers.size() - first_tail;
+  up.bytes.resize(at_tail + tail_n * sizeof(TreeLayer));
+  uint8_t* d_up = c.scratch[S_TMP2].as<uint8_t>(up.bytes.size());
+  auto tree_layer = [&](size_t k) {
+    return TreeLayer{reinterpret_cast<const TreeGate*>(d_up + steps[k].gates), V->layers[k + 1],
+                     (size_t)1 << C.layers[k].num_vars, (int)C.layers[k].width};
+  };
+  for (size_t k = first_tail; k < C.layers.size(); ++k) {
+    const TreeLayer t = tree_layer(k);
+    memcpy(up.bytes.data() + at_tail + (k - first_tail) * sizeof(TreeLayer), &t, sizeof(t));
+  }
+  APG_CUDA(cudaMemcpyAsync(d_up, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, c.stream));
+  if (base_on_device) {
+    const size_t most = 32 * n0, per = (most / 16 + 255) / 256;
+    const unsigned bx = (unsigned)std::max<size_t>(1, std::min(per, (size_t)c.sm_count * 16 / C.n_committed + 1));
+    for (size_t x = 0; x < C.n_committed; x += 32768)
+      launch(c, k_copy_columns, dim3(bx, (unsigned)std::min<size_t>(32768, C.n_committed - x)), 256, 0,
+             reinterpret_cast<const ColumnCopy*>(d_up + at_copies) + x);
+  } else {
+    for (size_t x = 0; x < C.n_committed; ++x)
+      APG_CUDA(cudaMemcpyAsync(copies[x].dst, copies[x].src, copies[x].bytes, cudaMemcpyHostToDevice, c.stream));
+  }
+  const uint8_t* d_bits = V->base_narrow ? d_up + at_bits : nullptr;
   for (size_t k = 0; k < C.layers.size(); ++k) {
     const CLayer& L = C.layers[k];
     const size_t rows = (size_t)1 << L.num_vars;
-    APG_CUDA(cudaMallocAsync((void**)&V->layers[k + 1], 32 * rows * std::max<uint32_t>(L.width, 1), c.stream));
-    HostProgram hp = layer_program(C, k, ch, false, {});
-    DevProgram P;
-    upload_program(c, hp, P);
+    cudaEvent_t t0 = c.timer_begin();
+    if (k == first_tail) {
+      launch(c, k_forward_tree_tail, 1, 1024, 0, reinterpret_cast<const TreeLayer*>(d_up + at_tail), (int)tail_n);
+      c.timer_end(APG_TIMER_GKR_FORWARD, t0);
+      break;
+    }
+    if (steps[k].tree) {
+      for (uint32_t g = 0; g < L.width; g += 32768) {
+        TreeLayer t = tree_layer(k);
+        t.gates += g;
+        t.out += (size_t)g * rows;
+        const size_t bx = std::min<size_t>((rows + 255) / 256, (size_t)c.sm_count * 32);
+        launch(c, k_forward_tree, dim3((unsigned)bx, std::min<uint32_t>(32768, L.width - g)), 256, 0, t);
+      }
+      c.timer_end(APG_TIMER_GKR_FORWARD, t0);
+      continue;
+    }
+    DevProgram P = steps[k].prog.on_device(d_up);
     const int w = (int)C.width(k);
     const int nv = L.halving ? 0 : (int)C.virtuals.size();
     P.cached_slot0 = L.halving ? 2 * w : w + nv;
     VirtualKinds vk;
     memset(&vk, 0, sizeof(vk));
     for (int v = 0; v < nv; ++v) vk.k[v] = (uint8_t)C.virtuals[v];
-    std::vector<const Fr*> cols(w);
-    for (int x = 0; x < w; ++x)
-      cols[x] = k == 0 ? reinterpret_cast<const Fr*>(V->base_raw(x)) : V->col(k, x);
-    const Fr** d_cols = c.scratch[S_TMP5].as<const Fr*>(w);
-    APG_CUDA(cudaMemcpyAsync(d_cols, cols.data(), sizeof(Fr*) * w, cudaMemcpyHostToDevice, c.stream));
     // A row-wise list over an Fr layer reads the layer in place; a halving
-    // list (two rows of a column a slot pair) or a narrow base is staged.
+    // list over a narrow base (two rows of a column a slot pair) is staged.
     const bool in_place = !L.halving && (k > 0 || !V->base_narrow) && w > 0;
     const size_t slots_n = (size_t)P.cached_slot0 + L.cached.size() - (in_place ? (size_t)w : 0);
     int threads = kFwdThreads;
     while (threads > 8 && std::max<size_t>(slots_n, 1) * 32 * threads > 200 * 1024) threads /= 2;
     const size_t smem = std::max<size_t>(slots_n, 1) * 32 * threads;
     if (smem > 200 * 1024) throw Error(APG_ERR_BAD_CIRCUIT, "gate list too wide for one thread block");
-    cudaEvent_t t0 = c.timer_begin();
     if (L.width && in_place) {
       APG_CUDA(cudaFuncSetAttribute(k_forward_g, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       // Columns of the layer lie a fixed stride apart (the base's at its
       // 256-byte-aligned offsets, later layers back to back).
-      const size_t stride = w > 1 ? (size_t)(cols[1] - cols[0]) : 0;
-      launch(c, k_forward_g, (unsigned)((rows + threads - 1) / threads), threads, smem, P, w, nv, vk, cols[0],
-             stride, rows, (int)L.width, V->layers[k + 1]);
+      const Fr* col0 = V->col(k, 0);
+      const size_t stride = w > 1 ? (size_t)(V->col(k, 1) - col0) : 0;
+      launch(c, k_forward_g, (unsigned)((rows + threads - 1) / threads), threads, smem, P, w, nv, vk, col0, stride,
+             rows, (int)L.width, V->layers[k + 1]);
     } else if (L.width) {
       APG_CUDA(cudaFuncSetAttribute(k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       launch(c, k_forward, (unsigned)((rows + threads - 1) / threads), threads, smem, P, w, nv, vk,
-             (const Fr* const*)d_cols, k == 0 ? d_bits : (const uint8_t*)nullptr, rows, L.halving ? 1 : 0,
-             (int)L.width, V->layers[k + 1]);
+             reinterpret_cast<const Fr* const*>(d_up + steps[k].cols), k == 0 ? d_bits : (const uint8_t*)nullptr, rows,
+             L.halving ? 1 : 0, (int)L.width, V->layers[k + 1]);
     }
     c.timer_end(APG_TIMER_GKR_FORWARD, t0);
-    // The program and column list buffers are reused by the next layer.
-    APG_CUDA(cudaStreamSynchronize(c.stream));
   }
   c.check_flags();
   return V.release();

@@ -719,7 +719,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
 
   // One upload: the counter of finished blocks (zero), the round-0 sources (the
   // data tables, then eq), their stored widths when any is narrow (eq is Fr)
-  // and the form. `up` lives until the copy from it has surely run (the rounds).
+  // and the form or the program. `up` lives until the copy from it has surely run (the rounds).
   bool narrow = false;
   for (uint8_t b : src_bits) narrow |= b != 0;
   if (narrow && (int)src_bits.size() != nd) throw Error(APG_ERR_INTERNAL, "one width per data table");
@@ -727,19 +727,17 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
   srcs.push_back(eq);
   std::vector<uint8_t> bits(narrow ? src_bits : std::vector<uint8_t>());
   if (narrow) bits.push_back(0);
-  std::vector<uint8_t> up(32, 0);
-  auto put = [&](const void* p, size_t len) {
-    const size_t at = (up.size() + 31) & ~(size_t)31;
-    up.resize(at + len);
-    if (len) memcpy(up.data() + at, p, len);
-    return at;
-  };
-  const size_t at_src = put(srcs.data(), sizeof(Fr*) * nt), at_bits = put(bits.data(), bits.size()),
-               at_g = put(form.groups.data(), form.groups.size() * sizeof(FormGroup)),
-               at_t = put(form.terms.data(), form.terms.size() * sizeof(FormTerm)),
-               at_c = put(form.coeffs.data(), form.coeffs.size() * 32);
-  uint8_t* d_up = c.scratch[S_PAIR_TERMS].as<uint8_t>(up.size());
-  APG_CUDA(cudaMemcpyAsync(d_up, up.data(), up.size(), cudaMemcpyHostToDevice, c.stream));
+  Packer up;
+  const uint32_t zero[8] = {0};
+  up.put(zero, sizeof(zero));
+  const size_t at_src = up.put(srcs.data(), sizeof(Fr*) * nt), at_bits = up.put(bits.data(), bits.size()),
+               at_g = up.put(form.groups.data(), form.groups.size() * sizeof(FormGroup)),
+               at_t = up.put(form.terms.data(), form.terms.size() * sizeof(FormTerm)),
+               at_c = up.put(form.coeffs.data(), form.coeffs.size() * 32);
+  PackedProgram packed{};
+  if (!use_form) packed = pack_program(hp, up);
+  uint8_t* d_up = c.scratch[S_PAIR_TERMS].as<uint8_t>(up.bytes.size());
+  APG_CUDA(cudaMemcpyAsync(d_up, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, c.stream));
   unsigned* done = reinterpret_cast<unsigned*>(d_up);
   const Fr** d_src = reinterpret_cast<const Fr**>(d_up + at_src);
   const uint8_t* d_bits = narrow ? d_up + at_bits : nullptr;
@@ -783,7 +781,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
   } else {
     if ((warp_mode ? warp_smem : smem) > 200 * 1024)
       throw Error(APG_ERR_BAD_CIRCUIT, "gate list too wide for one thread block");
-    upload_program(c, hp, P);
+    P = packed.on_device(d_up);
     P.cached_slot0 = n_val;
     APG_CUDA(cudaFuncSetAttribute(k_round, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     APG_CUDA(cudaFuncSetAttribute(k_round_warp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -1185,7 +1183,7 @@ bool quadratic_form(const HostProgram& hp, int slots, HostForm& out) {
   return true;
 }
 
-void upload_program(Ctx& c, const HostProgram& hp, DevProgram& P) {
+PackedProgram pack_program(const HostProgram& hp, Packer& out) {
   std::vector<DevGate> gates = hp.gates;
   const std::vector<F>& coeffs = hp.coeffs;
   std::vector<F> weights = hp.weights;
@@ -1230,27 +1228,26 @@ void upload_program(Ctx& c, const HostProgram& hp, DevProgram& P) {
     for (int j = 0; j < nw; ++j) gates[n0 + j] = wg[j];
     weights = ww;
   }
-  const size_t gb = gates.size() * sizeof(DevGate);
-  const size_t ob = hp.ops.size() * sizeof(uint16_t);
-  const size_t cb = coeffs.size() * 32;
-  const size_t wb = weights.size() * 32;
-  const size_t total = gb + ob + cb + wb + 256;
-  uint8_t* d = c.scratch[S_TMP2].as<uint8_t>(total);
-  std::vector<uint8_t> h(total, 0);
-  size_t off = 0;
-  auto put = [&](const void* p, size_t n) {
-    size_t at = (off + 31) & ~(size_t)31;
-    if (n) memcpy(h.data() + at, p, n);
-    off = at + n;
-    return d + at;
-  };
-  P.gates = (const DevGate*)put(gates.data(), gb);
-  P.ops = (const uint16_t*)put(hp.ops.data(), ob);
-  P.coeffs = (const Fr*)put(coeffs.data(), cb);
-  P.weights = (const Fr*)put(weights.data(), wb);
+  PackedProgram P;
+  P.gates = out.put(gates.data(), gates.size() * sizeof(DevGate));
+  P.ops = out.put(hp.ops.data(), hp.ops.size() * sizeof(uint16_t));
+  P.coeffs = out.put(coeffs.data(), coeffs.size() * 32);
+  P.weights = out.put(weights.data(), weights.size() * 32);
   P.n_cached = hp.n_cached;
   P.n_weighted = hp.n_weighted;
-  APG_CUDA(cudaMemcpyAsync(d, h.data(), off, cudaMemcpyHostToDevice, c.stream));
+  return P;
+}
+
+DevProgram PackedProgram::on_device(const uint8_t* base) const {
+  DevProgram P;
+  P.gates = reinterpret_cast<const DevGate*>(base + gates);
+  P.ops = reinterpret_cast<const uint16_t*>(base + ops);
+  P.coeffs = reinterpret_cast<const Fr*>(base + coeffs);
+  P.weights = reinterpret_cast<const Fr*>(base + weights);
+  P.n_cached = n_cached;
+  P.n_weighted = n_weighted;
+  P.cached_slot0 = 0;
+  return P;
 }
 
 }  // namespace apg

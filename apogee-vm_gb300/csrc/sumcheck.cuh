@@ -61,7 +61,23 @@ __device__ __forceinline__ Fr narrow_entry(const void* p, int bits, size_t i) {
 // The first n entries of a column, lifted into an Fr table.
 void lift_column(Ctx& c, const void* p, int bits, size_t n, Fr* out);
 
-void upload_program(Ctx& c, const HostProgram& hp, DevProgram& P);
+// Tables the host prepares, packed for one upload: every part 32-byte aligned.
+struct Packer {
+  std::vector<uint8_t> bytes;
+  size_t put(const void* p, size_t n) {
+    const size_t at = (bytes.size() + 31) & ~(size_t)31;
+    bytes.resize(at + n);
+    if (n) memcpy(bytes.data() + at, p, n);
+    return at;
+  }
+};
+// A gate list packed; on_device gives its tables under the upload's address.
+struct PackedProgram {
+  size_t gates, ops, coeffs, weights;
+  int n_cached, n_weighted;
+  DevProgram on_device(const uint8_t* base) const;
+};
+PackedProgram pack_program(const HostProgram& hp, Packer& out);
 // eq(r, y) for every y < 2^|r| (|r| at most 40).
 void build_eq_table(Ctx& c, const std::vector<host::F>& r, Fr* out);
 
