@@ -138,6 +138,7 @@ void apg_ctx_destroy(apg_ctx* ctx) {
     if (c.stream) cudaStreamSynchronize(c.stream);
     release_lane(c);
     for (auto& b : c.scratch) b.release();
+    for (auto& b : c.fft_tw) b.release();
     for (auto& t : c.tables)
       if (t.owned) cudaFree(t.tab);
     for (auto& t : c.retired) cudaFree(t.tab);
@@ -748,6 +749,7 @@ int apg_mercury_batch_open_stacked_device(apg_ctx* ctx, const void* const* d_col
 static size_t ctx_bytes(const Ctx& c) {
   size_t b = 0;
   for (const auto& d : c.scratch) b += d.cap;
+  for (const auto& d : c.fft_tw) b += d.cap;
   for (const auto& t : c.tables)
     if (t.owned) b += (size_t)t.windows * t.n * sizeof(Affine);
   for (const auto& t : c.retired) b += (size_t)t.windows * t.n * sizeof(Affine);

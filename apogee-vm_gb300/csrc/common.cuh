@@ -133,6 +133,7 @@ struct Ctx {
   // log2 of the point count); 0 = the default rule of srs_table_for.
   int tuned_c[64] = {0};
   DevBuf scratch[S_COUNT];
+  DevBuf fft_tw[16];  // twiddles of the one-block transforms, by log2 of the size (mercury.cu)
   uint32_t* d_flags = nullptr;  // device error flags (DeviceFlag bits)
   uint64_t launches = 0;        // kernels launched on this context
   Timers timers;

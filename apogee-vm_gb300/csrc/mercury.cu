@@ -31,34 +31,52 @@ Fr dv(const F& a) {
   return r;
 }
 
-// h_j = sum_i eq1[i] * f[j*b + i]: one warp per row.
-__global__ void k_row_dot(const Fr* f, const Fr* eq1, size_t b, size_t rows, Fr* h) {
-  const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) / 32;
-  const int lane = threadIdx.x & 31;
-  if (warp >= rows) return;
+// A lane's share of sum_i a[i] b[i], i from `first` in steps of `step`: fifteen
+// products to a reduction.
+__device__ __forceinline__ Fr dot_share(const Fr* a, const Fr* b, size_t n, size_t first, size_t step) {
   Fr acc = fe_zero<FrConsts>();
-  for (size_t i = lane; i < b; i += 32) acc = fe_add(acc, fe_mul(ld_fe(&eq1[i]), ld_fe(&f[warp * b + i])));
+  for (size_t i = first; i < n;) {
+    FeWide<FrConsts> w = wide_zero<FrConsts>();
+    for (int k = 0; k < kWideProducts && i < n; ++k, i += step) wide_mac(w, ld_fe(&a[i]), ld_fe(&b[i]));
+    acc = fe_add(acc, fe_from_wide(w));
+  }
+  return acc;
+}
+
+__device__ __forceinline__ Fr warp_total(Fr acc) {  // in lane 0
   for (int off = 16; off > 0; off >>= 1) {
     Fr o;
 #pragma unroll
     for (int w = 0; w < 8; ++w) o.v[w] = __shfl_down_sync(0xffffffffu, acc.v[w], off);
     acc = fe_add(acc, o);
   }
-  if (lane == 0) st_fe(&h[warp], acc);
+  return acc;
 }
 
-// out[0] = sum_i a[i] * b[i] (one block).
-__global__ void k_dot(const Fr* a, const Fr* b, size_t n, Fr* out) {
-  __shared__ Fr red[256];
-  Fr acc = fe_zero<FrConsts>();
-  for (size_t i = threadIdx.x; i < n; i += blockDim.x) acc = fe_add(acc, fe_mul(ld_fe(&a[i]), ld_fe(&b[i])));
-  red[threadIdx.x] = acc;
+// h_j = sum_i eq1[i] * f[j*b + i], one warp per row, for the columns of a table
+// (`one`, when not null, in their place). Bound by its products: unreduced sums
+// and all columns in one launch took 16 columns of 2^22 from 1.65 to 0.63 ms on a
+// GB300.
+__global__ void __launch_bounds__(256) k_row_dot(const Fr* const* cols, const Fr* one, const Fr* eq1, size_t b,
+                                                 size_t rows, Fr* h) {
+  const size_t row = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) / 32;
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const Fr* f = one ? one : cols[blockIdx.y];
+  const Fr acc = warp_total(dot_share(eq1, f + row * b, b, lane, 32));
+  if (lane == 0) st_fe(&h[blockIdx.y * rows + row], acc);
+}
+
+// out[j] = sum_i a[i] * b[j * n + i], a block each.
+__global__ void __launch_bounds__(256) k_dot(const Fr* a, const Fr* b, size_t n, Fr* out) {
+  __shared__ Fr red[8];
+  const Fr acc = warp_total(dot_share(a, b + blockIdx.x * n, n, threadIdx.x, blockDim.x));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < (unsigned)off) red[threadIdx.x] = fe_add(red[threadIdx.x], red[threadIdx.x + off]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) st_fe(out, red[0]);
+  if (threadIdx.x != 0) return;
+  Fr s = red[0];
+  for (int w = 1; w < 8; ++w) s = fe_add(s, red[w]);
+  st_fe(&out[blockIdx.x], s);
 }
 
 // Suffix Horner over `count` positions of `cols` interleaved columns
@@ -80,10 +98,17 @@ __global__ void k_suffix_local(const Fr* in, Fr* out, size_t stride, size_t coun
   st_fe(&agg[seg * cols + col], acc);
 }
 
+// The powers a level takes with its launch: r^0 .. r^L for the fix, or r^(2^s)
+// for the scan.
+constexpr int kSuffixMax = 32;
+struct SuffixPowers {
+  Fr p[kSuffixMax + 1];
+};
+
 // Pass 2: with upper[s] = acc at the bottom of segment s (the next level's
 // result), acc_j = local_j + r^(lo_{s+1} - j) * upper[s+1].
 __global__ void k_suffix_fix(Fr* out, size_t stride, size_t count, size_t cols, int L, const Fr* upper,
-                             const Fr* pows) {
+                             const __grid_constant__ SuffixPowers pows) {
   const size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (id >= count * cols) return;
   const size_t j = id / cols, col = id % cols;
@@ -93,7 +118,26 @@ __global__ void k_suffix_fix(Fr* out, size_t stride, size_t count, size_t cols, 
   const size_t next = (seg + 1) * L;
   Fr carry = ld_fe(&upper[(seg + 1) * cols + col]);
   Fr* p = &out[j * stride + col];
-  st_fe(p, fe_add(ld_fe(p), fe_mul(ld_fe(&pows[next - j]), carry)));
+  st_fe(p, fe_add(ld_fe(p), fe_mul(pows.p[next - j], carry)));
+}
+
+// A column of up to 1024 positions by one block, a thread a position:
+// acc_j += r^(2^s) acc_{j + 2^s} for s = 0, 1, ..., log2(count) products after one
+// another instead of a segment's length and a level's launches.
+constexpr size_t kSuffixScanMax = 1024;
+__global__ void __launch_bounds__(1024) k_suffix_scan(const Fr* in, Fr* out, size_t stride, int count,
+                                                      const __grid_constant__ SuffixPowers pows) {
+  __shared__ Fr sh[kSuffixScanMax];
+  const int j = threadIdx.x;
+  const size_t at = j * stride + blockIdx.x;
+  Fr acc = j < count ? ld_fe(&in[at]) : fe_zero<FrConsts>();
+  for (int s = 0, off = 1; off < count; ++s, off <<= 1) {
+    sh[j] = acc;
+    __syncthreads();
+    if (j + off < count) acc = fe_add(acc, fe_mul(pows.p[s], sh[j + off]));
+    __syncthreads();
+  }
+  if (j < count) st_fe(&out[at], acc);
 }
 
 // out[i] = base^i.
@@ -129,6 +173,83 @@ __global__ void k_fft_stage(Fr* a, size_t m, size_t half, const Fr* tw) {
   Fr lo = ld_fe(&a[start + k]), hi = fe_mul(ld_fe(&a[start + k + half]), w);
   st_fe(&a[start + k], fe_add(lo, hi));
   st_fe(&a[start + k + half], fe_sub(lo, hi));
+}
+
+// ---- transforms of up to 2^12 points in one block ------------------------------
+//
+// 4096 elements are 128 KB of shared memory, so a transform is one block and one
+// launch: a launch a stage cost 4 us each, 60 of them in a 2^22 opening. Element
+// i's 16-byte halves stand at sh[i] and sh[m + i].
+constexpr size_t kFftBlockMax = 4096;
+
+__device__ __forceinline__ Fr fft_ld(const uint4* sh, size_t m, size_t i) {
+  const uint4 u = sh[i], v = sh[m + i];
+  Fr r;
+  r.v[0] = u.x, r.v[1] = u.y, r.v[2] = u.z, r.v[3] = u.w;
+  r.v[4] = v.x, r.v[5] = v.y, r.v[6] = v.z, r.v[7] = v.w;
+  return r;
+}
+__device__ __forceinline__ void fft_st(uint4* sh, size_t m, size_t i, const Fr& a) {
+  sh[i] = make_uint4(a.v[0], a.v[1], a.v[2], a.v[3]);
+  sh[m + i] = make_uint4(a.v[4], a.v[5], a.v[6], a.v[7]);
+}
+
+// The decimation-in-time stages over bit-reversed input. tw holds w^k for
+// k < m/2; the inverse transform's w^-k is 1 or -w^(m/2 - k).
+__device__ __forceinline__ void fft_stages(uint4* sh, size_t m, const Fr* tw, bool inverse) {
+  for (size_t half = 1; half < m; half *= 2) {
+    __syncthreads();
+    for (size_t t = threadIdx.x; t < m / 2; t += blockDim.x) {
+      const size_t k = t & (half - 1), at = 2 * (t - k) + k, e = k * (m / (2 * half));
+      const Fr lo = fft_ld(sh, m, at);
+      Fr hi = fft_ld(sh, m, at + half);
+      if (e) hi = rmul(hi, ld_fe(&tw[inverse ? m / 2 - e : e]));
+      if (e && inverse) hi = fe_neg(hi);
+      fft_st(sh, m, at, fe_add(lo, hi));
+      fft_st(sh, m, at + half, fe_sub(lo, hi));
+    }
+  }
+  __syncthreads();
+}
+
+// The transforms of g, rev(eq1), h and rev(eq2), each b long in m = 2b, block q
+// the q-th: out[q m ..].
+struct SymOperands {
+  const Fr* src[4];
+};
+__global__ void __launch_bounds__(1024) k_sym_fft(SymOperands S, size_t b, int bits, const Fr* tw, Fr* out) {
+  extern __shared__ uint4 sh_fft[];
+  const size_t m = 2 * b, q = blockIdx.x;
+  const Fr* src = S.src[q];
+  for (size_t i = threadIdx.x; i < m; i += blockDim.x) {
+    const Fr v = i < b ? ld_fe(&src[q & 1 ? b - 1 - i : i]) : fe_zero<FrConsts>();
+    fft_st(sh_fft, m, __brevll((unsigned long long)i) >> (64 - bits), v);
+  }
+  fft_stages(sh_fft, m, tw, false);
+  for (size_t i = threadIdx.x; i < m; i += blockDim.x) st_fe(&out[q * m + i], fft_ld(sh_fft, m, i));
+}
+
+// R = IFFT(G P1 + gamma H P2), then S and D and symmetric_witness's two
+// assertions (k_sym_out, k_reverse). scale = 1/m.
+__global__ void __launch_bounds__(1024) k_sym_ifft(const Fr* t, size_t b, int bits, const Fr* tw, Fr gamma, Fr scale,
+                                                   Fr expect_mid, const Fr* g, Fr* S, Fr* D, uint32_t* flags) {
+  extern __shared__ uint4 sh_fft[];
+  const size_t m = 2 * b;
+  for (size_t i = threadIdx.x; i < m; i += blockDim.x) {
+    FeWide<FrConsts> s = wide_zero<FrConsts>();
+    wide_mac(s, ld_fe(&t[i]), ld_fe(&t[m + i]));
+    wide_mac(s, gamma, rmul(ld_fe(&t[2 * m + i]), ld_fe(&t[3 * m + i])));
+    fft_st(sh_fft, m, __brevll((unsigned long long)i) >> (64 - bits), fe_from_wide(s));
+  }
+  fft_stages(sh_fft, m, tw, true);
+  if (threadIdx.x == 0 &&
+      (!fe_is_zero(fft_ld(sh_fft, m, m - 1)) || !fe_eq(rmul(scale, fft_ld(sh_fft, m, b - 1)), expect_mid)))
+    atomicOr(flags, (uint32_t)DEV_NONZERO_REM);
+  for (size_t i = threadIdx.x; i < b; i += blockDim.x) {
+    if (i + 1 < b)
+      st_fe(&S[i], rmul(scale, fe_add(fft_ld(sh_fft, m, b + i), fft_ld(sh_fft, m, b - 2 - i))));
+    st_fe(&D[i], ld_fe(&g[b - 1 - i]));
+  }
 }
 
 // The four padded operands of S: g, rev(eq1), h, rev(eq2), each b long in 2b.
@@ -186,16 +307,21 @@ __global__ void k_numerator(const Fr* f, const Fr* q, size_t n, size_t nq, Fr c,
 
 // f* = sum_j w_j stack_j: stack j's column in slot s (cols[j * maxlen + s],
 // null past the stack's end) covers entries [s * 2^width, (s + 1) * 2^width).
-__global__ void k_combine_stacked(const Fr* const* cols, const Fr* w, int nstacks, size_t maxlen, int width,
+// Unreduced sums: 16 columns of 2^22 998 -> 664 us on a GB300.
+__global__ void __launch_bounds__(256) k_combine_stacked(const Fr* const* cols, const Fr* w, int nstacks, size_t maxlen, int width,
                                   size_t n, Fr* out) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const size_t slot = i >> width, row = i & (((size_t)1 << width) - 1);
   Fr acc = fe_zero<FrConsts>();
   if (slot < maxlen)
-    for (int j = 0; j < nstacks; ++j) {
-      const Fr* col = cols[(size_t)j * maxlen + slot];
-      if (col) acc = fe_add(acc, fe_mul(ld_fe(&w[j]), ld_fe(&col[row])));
+    for (int j = 0; j < nstacks;) {
+      FeWide<FrConsts> s = wide_zero<FrConsts>();
+      for (int k = 0; k < kWideProducts && j < nstacks; ++k, ++j) {
+        const Fr* col = cols[(size_t)j * maxlen + slot];
+        if (col) wide_mac(s, ld_fe(&w[j]), ld_fe(&col[row]));
+      }
+      acc = fe_add(acc, fe_from_wide(s));
     }
   st_fe(&out[i], acc);
 }
@@ -256,24 +382,39 @@ void srs_commit2(Ctx& c, const Fr* d0, size_t len0, const Fr* d1, size_t len1, u
   memcpy(out1, both + 64, 64);
 }
 
-// acc_j = sum_{k >= j} x_k r^(k - j) for every position, in place or not.
-void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, size_t cols, const F& r,
-                   int depth = 0) {
+// acc_j = sum_{k >= j} x_k r^(k - j) for every position, in place or not: one
+// block scan a column where a column fits a block; else segments (32 positions
+// where there are enough to fill the device, 8 where the chain is what counts),
+// the same over their aggregates, and a fix.
+void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, size_t cols, const F& r) {
   if (count == 0) return;
-  const int L = 32;
+  SuffixPowers pows;
+  if (count <= kSuffixScanMax && cols < ((size_t)1 << 31)) {
+    F p = r;
+    for (int s = 0; s < 11; ++s) {
+      pows.p[s] = dv(p);
+      p = host::fsqr(p);
+    }
+    const unsigned threads = (unsigned)std::max<size_t>(32, (count + 31) / 32 * 32);
+    launch(c, k_suffix_scan, (unsigned)cols, threads, 0, in, out, stride, (int)count, pows);
+    return;
+  }
+  const int L = count * cols >= ((size_t)1 << 20) ? kSuffixMax : 8;
   const size_t nseg = (count + L - 1) / L;
-  // Scratch per level: aggregates (nseg x cols) and the power table r^0..r^L,
-  // stream-ordered so every recursion level owns its own.
+  // Scratch per level: aggregates (nseg x cols), stream-ordered so every
+  // recursion level owns its own.
   Fr* agg;
-  APG_CUDA(cudaMallocAsync((void**)&agg, 32 * nseg * cols + 32 * (L + 1), c.stream));
-  Fr* pows = agg + nseg * cols;
-  launch(c, k_powers, 1, L + 1, 0, dv(r), (size_t)(L + 1), pows);
+  APG_CUDA(cudaMallocAsync((void**)&agg, 32 * nseg * cols, c.stream));
   launch(c, k_suffix_local, nb(nseg * cols, 128), 128, 0, in, out, stride, count, cols, L, dv(r), agg);
   if (nseg > 1) {
+    F p = host::fone();
+    for (int k = 0; k <= L; ++k) {
+      pows.p[k] = dv(p);
+      p = host::fmul(p, r);
+    }
     F rL = host::fpow_u64(r, L);
-    suffix_horner(c, agg, agg, cols, nseg, cols, rL, depth + 1);
-    launch(c, k_suffix_fix, nb(count * cols, 256), 256, 0, out, stride, count, cols, L, (const Fr*)agg,
-           (const Fr*)pows);
+    suffix_horner(c, agg, agg, cols, nseg, cols, rL);
+    launch(c, k_suffix_fix, nb(count * cols, 256), 256, 0, out, stride, count, cols, L, (const Fr*)agg, pows);
   }
   APG_CUDA(cudaFreeAsync(agg, c.stream));
 }
@@ -286,6 +427,20 @@ F two_adic_root() {
     e[3] >>= 1;
   }
   return host::fpow(host::from_u64(5), e);
+}
+
+// w^k for k < m/2, w of order m = 2^log_m: kept by the context for the sizes that
+// transform in one block (64 KB at most each).
+const Fr* twiddles(Ctx& c, int log_m) {
+  DevBuf& b = c.fft_tw[log_m];
+  if (!b.p) {
+    F w = two_adic_root();
+    for (int i = log_m; i < 28; ++i) w = host::fsqr(w);
+    const size_t half = (size_t)1 << (log_m - 1);
+    Fr* tw = b.as<Fr>(half);
+    launch(c, k_powers, nb(half, 256), 256, 0, dv(w), half, tw);
+  }
+  return static_cast<const Fr*>(b.p);
 }
 
 void fft_inplace(Ctx& c, Fr* a, size_t m, const Fr* tw) {
@@ -735,7 +890,7 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   // Step 1: h, v.
   build_eq_table(c, u1, eq1);
   build_eq_table(c, u2, eq2);
-  launch(c, k_row_dot, nb(b * 32, 256), 256, 0, d_f, (const Fr*)eq1, b, b, h);
+  launch(c, k_row_dot, nb(b * 32, 256), 256, 0, (const Fr* const*)nullptr, d_f, (const Fr*)eq1, b, b, h);
   launch(c, k_dot, 1, 256, 0, (const Fr*)eq2, (const Fr*)h, b, tmp);
   F v = read_fr(c, tmp);
   uint8_t pts[8][64];
@@ -767,22 +922,34 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
     const size_t m = 2 * b;
     int k = 0;
     while (((size_t)1 << k) < m) ++k;
-    F w = two_adic_root();
-    for (int i = k; i < 28; ++i) w = fsqr(w);
-    launch(c, k_sym_pad, nb(m, 256), 256, 0, (const Fr*)g, (const Fr*)eq1, (const Fr*)h, (const Fr*)eq2, b, TG, TP1,
-           TH, TP2);
-    launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(w), m / 2, tw);
-    fft_inplace(c, TG, m, tw);
-    fft_inplace(c, TP1, m, tw);
-    fft_inplace(c, TH, m, tw);
-    fft_inplace(c, TP2, m, tw);
-    launch(c, k_sym_mix, nb(m, 256), 256, 0, (const Fr*)TG, (const Fr*)TP1, (const Fr*)TH, (const Fr*)TP2, m,
-           dv(gamma), TG);
-    launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(finv(w)), m / 2, tw);
-    fft_inplace(c, TG, m, tw);
-    launch(c, k_scale, nb(m, 256), 256, 0, TG, m, dv(finv(from_u64(m))));
-    launch(c, k_sym_out, nb(b, 256), 256, 0, (const Fr*)TG, b, dv(fadd(h_alpha, fmul(gamma, v))), S, c.d_flags);
-    launch(c, k_reverse, nb(b, 256), 256, 0, (const Fr*)g, b, D);
+    const F mid = fadd(h_alpha, fmul(gamma, v));
+    if (m <= kFftBlockMax) {
+      const Fr* tws = twiddles(c, k);
+      const unsigned threads = (unsigned)std::min<size_t>(1024, std::max<size_t>(32, m / 2));
+      const size_t smem = 32 * m;
+      APG_CUDA(cudaFuncSetAttribute(k_sym_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)kFftBlockMax));
+      APG_CUDA(cudaFuncSetAttribute(k_sym_ifft, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)kFftBlockMax));
+      launch(c, k_sym_fft, 4, threads, smem, SymOperands{{g, eq1, h, eq2}}, b, k, tws, TG);
+      launch(c, k_sym_ifft, 1, threads, smem, (const Fr*)TG, b, k, tws, dv(gamma), dv(finv(from_u64(m))), dv(mid),
+             (const Fr*)g, S, D, c.d_flags);
+    } else {
+      F w = two_adic_root();
+      for (int i = k; i < 28; ++i) w = fsqr(w);
+      launch(c, k_sym_pad, nb(m, 256), 256, 0, (const Fr*)g, (const Fr*)eq1, (const Fr*)h, (const Fr*)eq2, b, TG, TP1,
+             TH, TP2);
+      launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(w), m / 2, tw);
+      fft_inplace(c, TG, m, tw);
+      fft_inplace(c, TP1, m, tw);
+      fft_inplace(c, TH, m, tw);
+      fft_inplace(c, TP2, m, tw);
+      launch(c, k_sym_mix, nb(m, 256), 256, 0, (const Fr*)TG, (const Fr*)TP1, (const Fr*)TH, (const Fr*)TP2, m,
+             dv(gamma), TG);
+      launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(finv(w)), m / 2, tw);
+      fft_inplace(c, TG, m, tw);
+      launch(c, k_scale, nb(m, 256), 256, 0, TG, m, dv(finv(from_u64(m))));
+      launch(c, k_sym_out, nb(b, 256), 256, 0, (const Fr*)TG, b, dv(mid), S, c.d_flags);
+      launch(c, k_reverse, nb(b, 256), 256, 0, (const Fr*)g, b, D);
+    }
   }
   srs_commit2(c, S, b - 1, D, b, pts[3], pts[4]);
   tr.absorb_g1(T_PCS_OPENING, &pts[3][0], 2);
@@ -893,19 +1060,29 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   const size_t w1 = width / 2, b1 = (size_t)1 << w1, b2 = (size_t)1 << (width - w1);
   std::vector<F> u1(u.begin(), u.begin() + w1), u2(u.begin() + w1, u.end());
   Fr* work;
-  const size_t words = b1 + 2 * b2 + ncols + nstacks + n;
+  const size_t words = b1 + b2 + ncols * b2 + ncols + nstacks + n;
   APG_CUDA(cudaMallocAsync((void**)&work, 32 * words, c.stream));
   struct Guard {
     Ctx& c;
     Fr* p;
     ~Guard() { cudaFreeAsync(p, c.stream); }
   } guard{c, work};
-  Fr *eq1 = work, *eq2 = eq1 + b1, *h = eq2 + b2, *cv = h + b2, *w = cv + ncols, *fstar = w + nstacks;
+  Fr *eq1 = work, *eq2 = eq1 + b1, *h = eq2 + b2, *cv = h + ncols * b2, *w = cv + ncols, *fstar = w + nstacks;
   build_eq_table(c, u1, eq1);
   build_eq_table(c, u2, eq2);
-  for (size_t col = 0; col < ncols; ++col) {
-    launch(c, k_row_dot, nb(b2 * 32, 256), 256, 0, d_cols[col], (const Fr*)eq1, b1, b2, h);
-    launch(c, k_dot, 1, 256, 0, (const Fr*)eq2, (const Fr*)h, b2, cv + col);
+  // The columns' addresses: stack after stack, then by (stack, slot), null past a
+  // stack's end.
+  std::vector<const Fr*> table(d_cols, d_cols + ncols);
+  table.resize(ncols + nstacks * maxlen, nullptr);
+  for (size_t j = 0, idx = 0; j < nstacks; ++j)
+    for (size_t s = 0; s < stack_lens[j]; ++s) table[ncols + j * maxlen + s] = d_cols[idx++];
+  const Fr** d_table = c.scratch[S_TMP5].as<const Fr*>(table.size());
+  APG_CUDA(cudaMemcpyAsync(d_table, table.data(), sizeof(Fr*) * table.size(), cudaMemcpyHostToDevice, c.stream));
+  for (size_t c0 = 0; c0 < ncols; c0 += 32768) {
+    const unsigned cn = (unsigned)std::min<size_t>(32768, ncols - c0);
+    launch(c, k_row_dot, dim3(nb(b2 * 32, 256), cn), 256, 0, (const Fr* const*)(d_table + c0), (const Fr*)nullptr,
+           (const Fr*)eq1, b1, b2, h + c0 * b2);
+    launch(c, k_dot, cn, 256, 0, (const Fr*)eq2, (const Fr*)(h + c0 * b2), b2, cv + c0);
   }
   const std::vector<F> vals = read_frs(c, cv, ncols);
   vs.assign(nstacks, fzero());
@@ -941,12 +1118,7 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
     host::g1::msm_small(cms, wts.data(), nstacks, cm_star);
   else
     msm_device(c, d_cms, nullptr, w, false, false, nstacks, nullptr, cm_star);
-  std::vector<const Fr*> table(nstacks * maxlen, nullptr);
-  for (size_t j = 0, idx = 0; j < nstacks; ++j)
-    for (size_t s = 0; s < stack_lens[j]; ++s) table[j * maxlen + s] = d_cols[idx++];
-  const Fr** d_table = c.scratch[S_TMP5].as<const Fr*>(table.size());
-  APG_CUDA(cudaMemcpyAsync(d_table, table.data(), sizeof(Fr*) * table.size(), cudaMemcpyHostToDevice, c.stream));
-  launch(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)d_table, (const Fr*)w, (int)nstacks, maxlen,
+  launch(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)(d_table + ncols), (const Fr*)w, (int)nstacks, maxlen,
          (int)width, n, fstar);
   F v;
   int st = mercury_open_impl(c, fstar, nv, cm_star, point, tr, v, proof_out);
