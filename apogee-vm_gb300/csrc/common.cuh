@@ -235,6 +235,10 @@ __global__ void k_fr_to_mont(Fr* v, size_t n, uint32_t* flags);
 // kernel stores both in pinned memory and the host waits for its flag (instead of
 // two copies and a synchronisation: about 15 us less a result on a GB300).
 void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host);
+// The same in two halves: publish on the stream (work may follow), collect before
+// anything else is published.
+uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes);
+void collect_checked(Ctx& c, uint32_t seq, size_t bytes, void* host);
 // Canonical 64-byte points (host) -> device affine Montgomery, validated.
 void upload_points(Ctx& c, const uint8_t* host, size_t n, Affine* dst);
 // The same without waiting: the flags are the caller's to check.

@@ -340,9 +340,15 @@ struct Transcript {
   }
   // A G1 point list as one message of 4 limbs a point (g1_limbs).
   void absorb_g1(uint64_t tag, const uint8_t* pts, size_t n) {
-    std::vector<F> limbs(4 * n);
-    for (size_t k = 0; k < n; ++k) g1_limbs(pts + 64 * k, &limbs[4 * k]);
-    absorb(tag, limbs);
+    open(tag, 4 * n);
+    observe_g1(pts, n);
+  }
+  void observe_g1(const uint8_t* pts, size_t n) {
+    for (size_t k = 0; k < n; ++k) {
+      F limbs[4];
+      g1_limbs(pts + 64 * k, limbs);
+      for (const F& x : limbs) observe(x);
+    }
   }
 
   bool load(const uint8_t b[226]) {

@@ -175,6 +175,56 @@ __global__ void k_fft_stage(Fr* a, size_t m, size_t half, const Fr* tw) {
   st_fe(&a[start + k + half], fe_sub(lo, hi));
 }
 
+// ---- the O(b) polynomials of the BDFG step ---------------------------------------
+
+// out[q] = poly_q(x_q), a block each: a thread runs Horner over a run of `run`
+// coefficients, then the runs fold by doubling distances; pw[q] holds x and
+// x^(run 2^s) for s = 0..7.
+constexpr int kEvals = 6;
+struct EvalArgs {
+  const Fr* poly[kEvals];
+  uint32_t len[kEvals];
+  Fr pw[kEvals][9];
+};
+__global__ void __launch_bounds__(256) k_eval(const __grid_constant__ EvalArgs E, uint32_t run, Fr* out) {
+  __shared__ Fr sh[256];
+  const int q = blockIdx.x, t = threadIdx.x;
+  const Fr* p = E.poly[q];
+  const uint32_t lo = t * run, hi = min(lo + run, E.len[q]);
+  Fr acc = fe_zero<FrConsts>();
+  for (uint32_t i = hi; i-- > lo && lo < hi;) acc = fe_add(ld_fe(&p[i]), rmul(E.pw[q][0], acc));
+  for (int s = 0; s < 8; ++s) {
+    sh[t] = acc;
+    __syncthreads();
+    if (t + (1 << s) < 256) acc = fe_add(acc, rmul(E.pw[q][s + 1], sh[t + (1 << s)]));
+    __syncthreads();
+  }
+  if (t == 0) st_fe(&out[q], acc);
+}
+
+// out[k] = sum_i sum_j mul[i][j] poly_i[k - j] + low[k]: the combination F of the
+// four openings' numerators (multipliers of up to three coefficients, the
+// interpolants folded into the five lowest), and with one coefficient each the
+// linearization.
+struct BdfgArgs {
+  const Fr* poly[5];
+  uint32_t len[5];
+  Fr mul[5][3];
+  int nmul[5];
+  Fr low[5];
+};
+__global__ void __launch_bounds__(256) k_bdfg(const __grid_constant__ BdfgArgs B, uint32_t n, Fr* out) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  FeWide<FrConsts> s = wide_zero<FrConsts>();  // (at most fourteen products)
+  for (int i = 0; i < 5; ++i)
+    for (int j = 0; j < B.nmul[i]; ++j)
+      if (k >= (uint32_t)j && k - j < B.len[i]) wide_mac(s, B.mul[i][j], ld_fe(&B.poly[i][k - j]));
+  Fr v = fe_from_wide(s);
+  if (k < 5) v = fe_add(v, B.low[k]);
+  st_fe(&out[k], v);
+}
+
 // ---- transforms of up to 2^12 points in one block ------------------------------
 //
 // 4096 elements are 128 KB of shared memory, so a transform is one block and one
@@ -232,7 +282,8 @@ __global__ void __launch_bounds__(1024) k_sym_fft(SymOperands S, size_t b, int b
 // R = IFFT(G P1 + gamma H P2), then S and D and symmetric_witness's two
 // assertions (k_sym_out, k_reverse). scale = 1/m.
 __global__ void __launch_bounds__(1024) k_sym_ifft(const Fr* t, size_t b, int bits, const Fr* tw, Fr gamma, Fr scale,
-                                                   Fr expect_mid, const Fr* g, Fr* S, Fr* D, uint32_t* flags) {
+                                                   const Fr* h_alpha, Fr gamma_v, const Fr* g, Fr* S, Fr* D,
+                                                   uint32_t* flags) {
   extern __shared__ uint4 sh_fft[];
   const size_t m = 2 * b;
   for (size_t i = threadIdx.x; i < m; i += blockDim.x) {
@@ -243,7 +294,8 @@ __global__ void __launch_bounds__(1024) k_sym_ifft(const Fr* t, size_t b, int bi
   }
   fft_stages(sh_fft, m, tw, true);
   if (threadIdx.x == 0 &&
-      (!fe_is_zero(fft_ld(sh_fft, m, m - 1)) || !fe_eq(rmul(scale, fft_ld(sh_fft, m, b - 1)), expect_mid)))
+      (!fe_is_zero(fft_ld(sh_fft, m, m - 1)) ||
+       !fe_eq(rmul(scale, fft_ld(sh_fft, m, b - 1)), fe_add(ld_fe(h_alpha), gamma_v))))
     atomicOr(flags, (uint32_t)DEV_NONZERO_REM);
   for (size_t i = threadIdx.x; i < b; i += blockDim.x) {
     if (i + 1 < b)
@@ -279,10 +331,10 @@ __global__ void k_scale(Fr* a, size_t m, Fr s) {
 
 // S[k - b] = R[k] + R[2b - 2 - k] for k in [b, 2b - 1); checks R[2b-1] = 0 and
 // R[b-1] = h(alpha) + gamma v (symmetric_witness's two assertions).
-__global__ void k_sym_out(const Fr* R, size_t b, Fr expect_mid, Fr* S, uint32_t* flags) {
+__global__ void k_sym_out(const Fr* R, size_t b, const Fr* h_alpha, Fr gamma_v, Fr* S, uint32_t* flags) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i == 0) {
-    if (!fe_is_zero(ld_fe(&R[2 * b - 1])) || !fe_eq(ld_fe(&R[b - 1]), expect_mid))
+    if (!fe_is_zero(ld_fe(&R[2 * b - 1])) || !fe_eq(ld_fe(&R[b - 1]), fe_add(ld_fe(h_alpha), gamma_v)))
       atomicOr(flags, (uint32_t)DEV_NONZERO_REM);
   }
   if (i >= b - 1) return;
@@ -326,19 +378,14 @@ __global__ void __launch_bounds__(256) k_combine_stacked(const Fr* const* cols, 
   st_fe(&out[i], acc);
 }
 
+// The remainders x[0 .. n) of exact divisions.
 __global__ void k_expect_zero(const Fr* x, uint32_t* flags) {
-  if (!fe_is_zero(ld_fe(x))) atomicOr(flags, (uint32_t)DEV_NONZERO_REM);
+  if (!fe_is_zero(ld_fe(&x[threadIdx.x]))) atomicOr(flags, (uint32_t)DEV_NONZERO_REM);
 }
 
 inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // ---- host helpers -------------------------------------------------------------
-
-F read_fr(Ctx& c, const Fr* d) {
-  F x;
-  fetch_checked(c, d, 32, x.w);
-  return x;
-}
 
 std::vector<F> read_frs(Ctx& c, const Fr* d, size_t n) {
   std::vector<F> v(n);
@@ -346,40 +393,21 @@ std::vector<F> read_frs(Ctx& c, const Fr* d, size_t n) {
   return v;
 }
 
-// MSM of the first `len` SRS powers against device scalars, canonical bytes.
-void srs_commit(Ctx& c, const Fr* d, size_t len, uint8_t out[64]) {
-  if (len == 0) {
-    memset(out, 0, 64);
-    return;
-  }
-  const SrsTable* t = srs_table_for(c, len, 1, false);
+// One or two MSMs of the first SRS powers against device scalars, two in one
+// group (one sort, accumulation and bucket reduction for both): launched, and
+// later fetched as canonical bytes, so that the transcript takes what it already
+// has while they run. Openings' scalars are combinations at random points.
+const uint8_t* srs_commit_start(Ctx& c, const Fr* d0, size_t len0, const Fr* d1 = nullptr, size_t len1 = 0) {
+  const size_t k = d1 ? 2 : 1;
+  const SrsTable* t = srs_table_for(c, std::max(len0, len1), k, false);
   if (!t) throw Error(APG_ERR_SRS_TOO_SMALL, "the SRS holds fewer powers than the polynomial has coefficients");
   MsmBatchOpts o;
-  o.uniform = true;  // an opening's polynomials are combinations at random points
-  msm_device(c, nullptr, t, d, false, false, len, nullptr, out, o);
-}
-
-// Two independent SRS MSMs in one group (one sort, accumulation and bucket
-// reduction for both).
-void srs_commit2(Ctx& c, const Fr* d0, size_t len0, const Fr* d1, size_t len1, uint8_t out0[64],
-                 uint8_t out1[64]) {
-  if (len0 == 0 || len1 == 0) {
-    srs_commit(c, d0, len0, out0);
-    srs_commit(c, d1, len1, out1);
-    return;
-  }
-  const SrsTable* t = srs_table_for(c, std::max(len0, len1), 2, false);
-  if (!t) throw Error(APG_ERR_SRS_TOO_SMALL, "the SRS holds fewer powers than the polynomial has coefficients");
+  o.uniform = true;
   const void* ptrs[2] = {d0, d1};
   const size_t lens[2] = {len0, len1};
   uint8_t* d_out = c.scratch[S_RESULT].as<uint8_t>(128);
-  MsmBatchOpts o;
-  o.uniform = true;
-  msm_multi(c, nullptr, t, ptrs, lens, 2, false, false, d_out, o);
-  uint8_t both[128];
-  fetch_checked(c, d_out, 128, both);
-  memcpy(out0, both, 64);
-  memcpy(out1, both + 64, 64);
+  msm_multi(c, nullptr, t, ptrs, lens, k, false, false, d_out, o);
+  return d_out;
 }
 
 // acc_j = sum_{k >= j} x_k r^(k - j) for every position, in place or not: one
@@ -417,6 +445,26 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
     launch(c, k_suffix_fix, nb(count * cols, 256), 256, 0, out, stride, count, cols, L, (const Fr*)agg, pows);
   }
   APG_CUDA(cudaFreeAsync(agg, c.stream));
+}
+
+// out[q] = poly_q(x_q) for up to kEvals polynomials.
+void eval_polys(Ctx& c, int n, const Fr* const* poly, const size_t* len, const F* x, Fr* out) {
+  EvalArgs E;
+  memset(&E, 0, sizeof(E));
+  size_t most = 1;
+  for (int q = 0; q < n; ++q) most = std::max(most, len[q]);
+  const size_t run = (most + 255) / 256;
+  for (int q = 0; q < n; ++q) {
+    E.poly[q] = poly[q];
+    E.len[q] = (uint32_t)len[q];
+    E.pw[q][0] = dv(x[q]);
+    F p = host::fpow_u64(x[q], run);
+    for (int s = 0; s < 8; ++s) {
+      E.pw[q][s + 1] = dv(p);
+      p = host::fsqr(p);
+    }
+  }
+  launch(c, k_eval, (unsigned)n, 256, 0, E, (uint32_t)run, out);
 }
 
 F two_adic_root() {
@@ -492,17 +540,6 @@ Poly uinterpolate(const std::vector<std::pair<F, F>>& pts) {
     uadd_scaled(out, num, host::fmul(pts[i].second, host::finv(den)));
   }
   return out;
-}
-
-std::pair<Poly, F> udiv_linear(const Poly& p, const F& r) {
-  if (p.empty()) return {{}, host::fzero()};
-  Poly q(p.size() - 1);
-  F acc = p.back();
-  for (size_t i = p.size() - 1; i-- > 0;) {
-    q[i] = acc;
-    acc = host::fadd(p[i], host::fmul(acc, r));
-  }
-  return {q, acc};
 }
 
 F tensor_eval(const std::vector<F>& u, F x) {
@@ -887,20 +924,24 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   Fr *eq1 = work, *eq2 = eq1 + b, *h = eq2 + b, *g = h + b, *S = g + b, *D = S + b, *acc = D + b, *num = acc + n;
   Fr *TG = num + n, *TP1 = TG + 2 * b, *TH = TP1 + 2 * b, *TP2 = TH + 2 * b, *tw = TP2 + 2 * b, *tmp = tw + b;
 
-  // Step 1: h, v.
+  // Step 1: h, v. The claim goes into the transcript while h is committed.
   build_eq_table(c, u1, eq1);
   build_eq_table(c, u2, eq2);
   launch(c, k_row_dot, nb(b * 32, 256), 256, 0, (const Fr* const*)nullptr, d_f, (const Fr*)eq1, b, b, h);
   launch(c, k_dot, 1, 256, 0, (const Fr*)eq2, (const Fr*)h, b, tmp);
-  F v = read_fr(c, tmp);
+  const uint32_t v_there = publish_checked(c, tmp, 32);
   uint8_t pts[8][64];
-  srs_commit(c, h, b, pts[0]);
+  const uint8_t* d_pts = srs_commit_start(c, h, b);
   tr.absorb(T_MERCURY_INSTANCE, std::vector<F>{from_u64(n)});
   tr.absorb_g1(T_COMMITMENT, cm, 1);
+  F v;
+  collect_checked(c, v_there, 32, v.w);
   std::vector<F> claim = u;
   claim.push_back(v);
   tr.absorb(T_EVALUATION_CLAIM, claim);
-  tr.absorb_g1(T_PCS_OPENING, pts[0], 1);
+  tr.open(T_PCS_OPENING, 4);
+  fetch_checked(c, d_pts, 64, pts[0]);
+  tr.observe_g1(pts[0], 1);
   F alpha = tr.challenge(T_MERCURY_ALPHA);
 
   // Step 2: the fold. acc rows: acc_j = sum_{k>=j} alpha^(k-j) row_k; q is
@@ -911,18 +952,23 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   APG_CUDA(cudaMemcpyAsync(g, acc, 32 * b, cudaMemcpyDeviceToDevice, c.stream));
   const Fr* q = acc + b;
   const size_t nq = n - b;
-  srs_commit2(c, q, nq, g, b, pts[1], pts[2]);
-  tr.absorb_g1(T_PCS_OPENING, &pts[1][0], 2);
+  d_pts = srs_commit_start(c, q, nq, g, b);
+  Fr *d_halpha = tmp + 1, *d_ev = tmp + 2;  // h(alpha), then the six values
+  {
+    const Fr* hp[1] = {h};
+    eval_polys(c, 1, hp, &b, &alpha, d_halpha);
+  }
+  tr.open(T_PCS_OPENING, 8);
+  fetch_checked(c, d_pts, 128, pts[1]);
+  tr.observe_g1(pts[1], 2);
   F gamma = tr.challenge(T_MERCURY_GAMMA);
 
   // Step 3: S and D.
-  std::vector<F> hh = read_frs(c, h, b);
-  F h_alpha = ueval(hh, alpha);
   {
     const size_t m = 2 * b;
     int k = 0;
     while (((size_t)1 << k) < m) ++k;
-    const F mid = fadd(h_alpha, fmul(gamma, v));
+    const Fr gamma_v = dv(fmul(gamma, v));
     if (m <= kFftBlockMax) {
       const Fr* tws = twiddles(c, k);
       const unsigned threads = (unsigned)std::min<size_t>(1024, std::max<size_t>(32, m / 2));
@@ -930,8 +976,8 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
       APG_CUDA(cudaFuncSetAttribute(k_sym_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)kFftBlockMax));
       APG_CUDA(cudaFuncSetAttribute(k_sym_ifft, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)kFftBlockMax));
       launch(c, k_sym_fft, 4, threads, smem, SymOperands{{g, eq1, h, eq2}}, b, k, tws, TG);
-      launch(c, k_sym_ifft, 1, threads, smem, (const Fr*)TG, b, k, tws, dv(gamma), dv(finv(from_u64(m))), dv(mid),
-             (const Fr*)g, S, D, c.d_flags);
+      launch(c, k_sym_ifft, 1, threads, smem, (const Fr*)TG, b, k, tws, dv(gamma), dv(finv(from_u64(m))),
+             (const Fr*)d_halpha, gamma_v, (const Fr*)g, S, D, c.d_flags);
     } else {
       F w = two_adic_root();
       for (int i = k; i < 28; ++i) w = fsqr(w);
@@ -947,12 +993,15 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
       launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(finv(w)), m / 2, tw);
       fft_inplace(c, TG, m, tw);
       launch(c, k_scale, nb(m, 256), 256, 0, TG, m, dv(finv(from_u64(m))));
-      launch(c, k_sym_out, nb(b, 256), 256, 0, (const Fr*)TG, b, dv(mid), S, c.d_flags);
+      launch(c, k_sym_out, nb(b, 256), 256, 0, (const Fr*)TG, b, (const Fr*)d_halpha, gamma_v, S,
+             c.d_flags);
       launch(c, k_reverse, nb(b, 256), 256, 0, (const Fr*)g, b, D);
     }
   }
-  srs_commit2(c, S, b - 1, D, b, pts[3], pts[4]);
-  tr.absorb_g1(T_PCS_OPENING, &pts[3][0], 2);
+  d_pts = srs_commit_start(c, S, b - 1, D, b);
+  tr.open(T_PCS_OPENING, 8);
+  fetch_checked(c, d_pts, 128, pts[3]);
+  tr.observe_g1(pts[3], 2);
   F z;
   do {
     z = tr.challenge(T_MERCURY_Z);
@@ -964,17 +1013,26 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   F zi = finv(z);
 
   // Step 4: the six values, the numerator and its quotient by (X - z).
-  std::vector<F> gg = read_frs(c, g, b), ss = read_frs(c, S, b - 1);
-  F ev[6] = {ueval(gg, z), ueval(gg, zi), ueval(hh, z), ueval(hh, zi), ueval(ss, z), ueval(ss, zi)};
-  tr.absorb(T_PCS_OPENING, ev, 6);
+  {
+    const Fr* polys[6] = {g, g, h, h, S, S};
+    const size_t lens[6] = {b, b, b, b, b - 1, b - 1};
+    const F at[6] = {z, zi, z, zi, z, zi};
+    eval_polys(c, 6, polys, lens, at, d_ev);
+  }
+  const std::vector<F> evs = read_frs(c, d_halpha, 7);
+  const F h_alpha = evs[0];
+  const F* ev = evs.data() + 1;
   F zb = fpow_u64(z, b);
   launch(c, k_numerator, nb(n, 256), 256, 0, d_f, q, n, nq, dv(fsub(zb, alpha)), dv(ev[0]), num);
   tp = c.timer_begin();
   suffix_horner(c, num, num, 1, n, 1, z);
   c.timer_end(APG_TIMER_MERCURY_PASS, tp);
   launch(c, k_expect_zero, 1, 1, 0, (const Fr*)num, c.d_flags);  // the remainder f(z) - ... = 0
-  srs_commit(c, num + 1, n - 1, pts[5]);
-  tr.absorb_g1(T_PCS_OPENING, pts[5], 1);
+  d_pts = srs_commit_start(c, num + 1, n - 1);
+  tr.absorb(T_PCS_OPENING, ev, 6);
+  tr.open(T_PCS_OPENING, 4);
+  fetch_checked(c, d_pts, 64, pts[5]);
+  tr.observe_g1(pts[5], 1);
 
   // Step 4(e): BDFG20 over T = {z, 1/z, alpha} (crates/pcs-verify/src/bdfg.rs).
   F two_inv = finv(from_u64(2));
@@ -989,46 +1047,60 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   Poly zc[4] = {wa, Poly{fone()}, wa, uvanishing({zi, alpha})};
   Poly rr[4] = {uinterpolate({{z, ev[0]}, {zi, ev[1]}}), uinterpolate({{z, ev[2]}, {zi, ev[3]}, {alpha, h_alpha}}),
                 uinterpolate({{z, ev[4]}, {zi, ev[5]}}), Poly{d_z}};
-  Poly dd(gg.rbegin(), gg.rend());
-  const Poly* polys[4] = {&gg, &hh, &ss, &dd};
-  F delta = tr.challenge(T_BDFG_BATCH);
-  Poly f;
-  F pw = fone();
+  const F delta = tr.challenge(T_BDFG_BATCH);
+  // F = sum_i delta^i Z_i (poly_i - r_i), b + 2 coefficients, and W = F / Z_T by
+  // its three roots in turn: after a root's suffix Horner the remainder stands
+  // first and the quotient after it.
+  BdfgArgs B;
+  memset(&B, 0, sizeof(B));
+  const Fr* polys[4] = {g, h, S, D};
+  const uint32_t lens[4] = {(uint32_t)b, (uint32_t)b, (uint32_t)(b - 1), (uint32_t)b};
+  F low[5] = {fzero(), fzero(), fzero(), fzero(), fzero()}, pw = fone();
   for (int i = 0; i < 4; ++i) {
-    Poly sh = *polys[i];
-    uadd_scaled(sh, rr[i], fneg(fone()));
-    uadd_scaled(f, umul(zc[i], sh), pw);
+    B.poly[i] = polys[i];
+    B.len[i] = lens[i];
+    B.nmul[i] = (int)zc[i].size();
+    for (size_t j = 0; j < zc[i].size(); ++j) B.mul[i][j] = dv(fmul(pw, zc[i][j]));
+    const Poly zr = umul(zc[i], rr[i]);
+    for (size_t k = 0; k < zr.size(); ++k) low[k] = fsub(low[k], fmul(pw, zr[k]));
     pw = fmul(pw, delta);
   }
-  Poly W = f;
-  for (auto& root : tset) {
-    auto d = udiv_linear(W, root);
-    if (!d.second.zero()) throw Error(APG_ERR_INTERNAL, "F is not divisible by Z_T");
-    W = d.first;
-  }
-  Fr* dW = TH;  // reuse a transform buffer (2b >= |W|)
-  APG_CUDA(cudaMemcpyAsync(dW, W.data(), 32 * W.size(), cudaMemcpyHostToDevice, c.stream));
-  srs_commit(c, dW, W.size(), pts[6]);
-  tr.absorb_g1(T_PCS_OPENING, pts[6], 1);
+  for (int k = 0; k < 5; ++k) B.low[k] = dv(low[k]);
+  Fr* dF = TH;  // reuse a transform buffer (2b >= b + 2)
+  launch(c, k_bdfg, nb(b + 2, 256), 256, 0, B, (uint32_t)(b + 2), dF);
+  for (int r = 0; r < 3; ++r) suffix_horner(c, dF + r, dF + r, 1, b + 2 - r, 1, tset[r]);
+  launch(c, k_expect_zero, 1, 3, 0, (const Fr*)dF, c.d_flags);
+  const Fr* dW = dF + 3;
+  d_pts = srs_commit_start(c, dW, b - 1);
+  tr.open(T_PCS_OPENING, 4);
+  fetch_checked(c, d_pts, 64, pts[6]);
+  tr.observe_g1(pts[6], 1);
   F zp = tr.challenge(T_BDFG_POINT);
-  Poly Lp;
+  // The linearization - Z_T(z') W + sum_i c_i poly_i - constant, and W' = it / (X - z').
+  memset(&B, 0, sizeof(B));
   F cst = fzero();
-  uadd_scaled(Lp, W, fneg(ueval(uvanishing(tset), zp)));
   for (int i = 0; i < 4; ++i) {
     F cc = fmul(fpow_u64(delta, i), ueval(zc[i], zp));
-    uadd_scaled(Lp, *polys[i], cc);
+    B.poly[i] = polys[i];
+    B.len[i] = lens[i];
+    B.nmul[i] = 1;
+    B.mul[i][0] = dv(cc);
     cst = fadd(cst, fmul(cc, ueval(rr[i], zp)));
   }
-  if (Lp.empty()) Lp.push_back(fzero());
-  Lp[0] = fsub(Lp[0], cst);
-  auto wp = udiv_linear(Lp, zp);
-  if (!wp.second.zero()) throw Error(APG_ERR_INTERNAL, "the linearization does not vanish at z'");
-  Fr* dWp = TP2;
-  APG_CUDA(cudaMemcpyAsync(dWp, wp.first.data(), 32 * wp.first.size(), cudaMemcpyHostToDevice, c.stream));
-  srs_commit(c, dWp, wp.first.size(), pts[7]);
-  tr.absorb_g1(T_PCS_OPENING, pts[7], 1);
+  B.poly[4] = dW;
+  B.len[4] = (uint32_t)(b - 1);
+  B.nmul[4] = 1;
+  B.mul[4][0] = dv(fneg(ueval(uvanishing(tset), zp)));
+  B.low[0] = dv(fneg(cst));
+  Fr* dL = TP2;
+  launch(c, k_bdfg, nb(b, 256), 256, 0, B, (uint32_t)b, dL);
+  suffix_horner(c, dL, dL, 1, b, 1, zp);
+  launch(c, k_expect_zero, 1, 1, 0, (const Fr*)dL, c.d_flags);
+  d_pts = srs_commit_start(c, dL + 1, b - 1);
+  tr.open(T_PCS_OPENING, 4);
+  fetch_checked(c, d_pts, 64, pts[7]);
+  tr.observe_g1(pts[7], 1);
   (void)tr.challenge(T_PAIRING_MERGE);
-  c.check_flags();
 
   v_out = v;
   for (int i = 0; i < 8; ++i) memcpy(proof_out + 64 * i, pts[i], 64);
@@ -1084,6 +1156,7 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
            (const Fr*)eq1, b1, b2, h + c0 * b2);
     launch(c, k_dot, cn, 256, 0, (const Fr*)eq2, (const Fr*)(h + c0 * b2), b2, cv + c0);
   }
+  tr.absorb_g1(T_COMMITMENT, cms, nstacks);  // (while the columns are evaluated)
   const std::vector<F> vals = read_frs(c, cv, ncols);
   vs.assign(nstacks, fzero());
   for (size_t j = 0, idx = 0; j < nstacks; ++j)
@@ -1094,7 +1167,6 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
     }
   std::vector<F> point = u;
   point.insert(point.end(), r.begin(), r.end());
-  tr.absorb_g1(T_COMMITMENT, cms, nstacks);
   std::vector<F> claim = point;
   claim.insert(claim.end(), vs.begin(), vs.end());
   tr.absorb(T_EVALUATION_CLAIM, claim);
@@ -1113,13 +1185,13 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   Affine* d_cms = c.scratch[S_BASES].as<Affine>(nstacks);
   upload_points(c, cms, nstacks, d_cms);
   APG_CUDA(cudaMemcpyAsync(w, wts.data(), 32 * nstacks, cudaMemcpyHostToDevice, c.stream));
+  launch(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)(d_table + ncols), (const Fr*)w, (int)nstacks, maxlen,
+         (int)width, n, fstar);
   uint8_t cm_star[64];
   if (nstacks <= kHostMsmMax)
     host::g1::msm_small(cms, wts.data(), nstacks, cm_star);
   else
     msm_device(c, d_cms, nullptr, w, false, false, nstacks, nullptr, cm_star);
-  launch(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)(d_table + ncols), (const Fr*)w, (int)nstacks, maxlen,
-         (int)width, n, fstar);
   F v;
   int st = mercury_open_impl(c, fstar, nv, cm_star, point, tr, v, proof_out);
   if (st) return st;

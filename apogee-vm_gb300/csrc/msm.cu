@@ -92,11 +92,11 @@ __global__ void k_points_out(const Affine* src, size_t n, uint4* raw) {
   raw[4 * i + 3] = make_uint4(y.v[4], y.v[5], y.v[6], y.v[7]);
 }
 
-// words of a result and the error flags into pinned host memory, then the flag
-// the host waits for.
-__global__ void k_publish(const uint32_t* src, uint32_t words, const uint32_t* err, uint32_t* dst, uint32_t* head,
-                          uint32_t seq) {
-  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+// A result (16-byte pieces) and the error flags into pinned host memory, then the
+// flag the host waits for.
+__global__ void __launch_bounds__(512) k_publish(const uint4* src, uint32_t n, const uint32_t* err, uint4* dst,
+                                                 uint32_t* head, uint32_t seq) {
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
   if (threadIdx.x == 0) head[1] = *err;
   __threadfence_system();
   __syncthreads();
@@ -1487,19 +1487,28 @@ inline unsigned blocks_for(size_t n, int threads) {
 // Host side
 // ---------------------------------------------------------------------------
 
-void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host) {
+uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes) {
   uint8_t* pinned = c.host_pinned();
-  if (bytes > Ctx::kPinnedBytes - Ctx::kPinnedTables || bytes % 4) {
-    APG_CUDA(cudaMemcpyAsync(host, d_src, bytes, cudaMemcpyDeviceToHost, c.stream));
-    c.check_flags();
+  if (bytes > Ctx::kPinnedBytes - Ctx::kPinnedTables || bytes % 16) throw Error(APG_ERR_INTERNAL, "an odd result");
+  launch(c, k_publish, 1, 512, 0, (const uint4*)d_src, (uint32_t)(bytes / 16), (const uint32_t*)c.d_flags,
+         reinterpret_cast<uint4*>(pinned + Ctx::kPinnedTables), reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
+  return c.flag_seq;
+}
+
+void collect_checked(Ctx& c, uint32_t seq, size_t bytes, void* host) {
+  if (seq != c.flag_seq) throw Error(APG_ERR_INTERNAL, "a result collected after another was published");
+  c.wait_flag();
+  memcpy(host, c.host_pinned() + Ctx::kPinnedTables, bytes);
+  if (reinterpret_cast<const uint32_t*>(c.host_pinned())[1]) c.check_flags();  // clears the flags and throws
+}
+
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host) {
+  if (bytes <= Ctx::kPinnedBytes - Ctx::kPinnedTables && bytes % 16 == 0) {
+    collect_checked(c, publish_checked(c, d_src, bytes), bytes, host);
     return;
   }
-  uint32_t* head = reinterpret_cast<uint32_t*>(pinned);
-  launch(c, k_publish, 1, 256, 0, (const uint32_t*)d_src, (uint32_t)(bytes / 4), (const uint32_t*)c.d_flags,
-         reinterpret_cast<uint32_t*>(pinned + Ctx::kPinnedTables), head, ++c.flag_seq);
-  c.wait_flag();
-  memcpy(host, pinned + Ctx::kPinnedTables, bytes);
-  if (head[1]) c.check_flags();  // clears the flags and throws
+  APG_CUDA(cudaMemcpyAsync(host, d_src, bytes, cudaMemcpyDeviceToHost, c.stream));
+  c.check_flags();
 }
 
 void upload_points_async(Ctx& c, const uint8_t* host, size_t n, Affine* dst) {
