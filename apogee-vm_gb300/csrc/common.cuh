@@ -82,7 +82,8 @@ struct SrsTable {
 enum ScratchSlot {
   S_ENTRIES, S_SORTED, S_SCANBLK, S_BUCKETS, S_HEAD, S_TAIL, S_FLAGS, S_LEVEL_A,
   S_LEVEL_B, S_LEVEL_T, S_TSUM, S_RESULT, S_BASES, S_SCALARS, S_TMP0, S_TMP1, S_TMP2, S_TMP3, S_TMP4,
-  S_TMP5, S_TMP6, S_TMP7, S_ROUND, S_PAIR_A, S_PAIR_B, S_PAIR_PP, S_PAIR_CNT, S_PAIR_TERMS, S_COUNT
+  S_TMP5, S_TMP6, S_TMP7, S_ROUND, S_PAIR_A, S_PAIR_B, S_PAIR_PP, S_PAIR_CNT, S_PAIR_TERMS,
+  S_SPLIT_BASES, S_SPLIT_SCALARS, S_COUNT
 };
 
 // Per-kernel CUDA-event timers (ids are public: APG_TIMER_* in the header).
@@ -258,7 +259,7 @@ struct MsmPlan {
   uint32_t buckets;  // a space: 2^(c-1), or fewer when no digit can reach them
 };
 // `bits`: the width of small scalars.
-MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits);
+MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits, int full_bits = 254);
 // k MSMs over the same bases (lens[j] scalars each, device pointers); result
 // j is written to d_out + 64 * j. Columns are processed in groups that share
 // one sort, one accumulation and one bucket reduction.
@@ -267,6 +268,7 @@ struct MsmBatchOpts {
   bool stack = false;            // one result: the sum of every column's MSM
   int bits = 32;                 // width of small scalars: 32, 16, 8 or 1 (bit-packed u64)
   bool uniform = false;          // field elements without structure (nearly every digit nonzero)
+  int full_bits = 254;           // width of the other scalars
 };
 void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* const* scalars, const size_t* lens,
                size_t k, bool small_scalars, bool scalars_canonical, uint8_t* d_out,

@@ -2,6 +2,7 @@
 //
 // Pipeline for a group of columns over the same bases, all on the context's
 // stream (msm_group):
+//  0. k_split       without an SRS table: scalars as two halves over P and phi(P).
 //  1. k_digits      one thread per scalar: Montgomery -> canonical, signed
 //                   c-bit digits in [-2^(c-1), 2^(c-1)] (the reference's
 //                   recoding rule, msm.rs:180-198) and a histogram of bucket
@@ -23,7 +24,6 @@
 // The allocation-free variant at the end of this file keeps the first
 // single-MSM form of the sort and the accumulation (k_recode, k_scatter,
 // k_accumulate).
-// single-MSM form of the pipeline (k_recode, k_scatter, k_accumulate, k_finish).
 #include "common.cuh"
 #include "curve_quad.cuh"
 
@@ -606,6 +606,102 @@ __device__ __forceinline__ uint32_t small_scalar(const void* col, uint32_t i, in
       return reinterpret_cast<const uint16_t*>(col)[i];
     default:
       return reinterpret_cast<const uint32_t*>(col)[i];
+  }
+}
+
+// ---- scalars in two halves ----------------------------------------------------
+//
+// BN254 has the endomorphism phi(x, y) = (beta x, y) = lambda (x, y), with beta and
+// lambda cube roots of one in Fq and Fr (Gallant, Lambert and Vanstone, "Faster point
+// multiplication on elliptic curves with efficient endomorphisms", 2001): a scalar
+// splits as k = k1 + lambda k2 with |k1|, |k2| < 2^127, so n products become 2n of half
+// the length and the windows' Horner chain half as deep. (a1, -b1), (a2, b2) is the
+// short basis of {(x, y): x + lambda y = 0 mod r} that the extended Euclidean algorithm
+// gives, and g1, g2 are round(2^256 b2 / r), round(2^256 b1 / r).
+__device__ constexpr uint32_t kSplitA1[2] = {0x94d213e3u, 0x89d32568u};  // (b2 is the same)
+__device__ constexpr uint32_t kSplitA2[4] = {0x1221250bu, 0x0be4e154u, 0xeeb859fdu, 0x6f4d8248u};
+__device__ constexpr uint32_t kSplitB1[4] = {0x7d4f1128u, 0x8211bbebu, 0xeeb859fcu, 0x6f4d8248u};
+__device__ constexpr uint32_t kSplitG1[3] = {0xc7e0b3d7u, 0xd91d232eu, 0x00000002u};
+__device__ constexpr uint32_t kSplitG2[5] = {0x391eb18eu, 0x7a7bd9d4u, 0xa773d2cfu, 0x4ccef014u, 0x00000002u};
+__device__ constexpr uint32_t kSplitBeta[8] = {0xd782e155u, 0x71930c11u, 0xffbe3323u, 0xa6bb947cu, 0xd4741444u, 0xaa303344u, 0x26594943u, 0x2c3b3f0du};  // Montgomery form
+
+// The NO words of a * b from word LO on.
+template <int NA, int NB, int LO, int NO>
+__device__ __forceinline__ void product_words(const uint32_t* a, const uint32_t* b, uint32_t* out) {
+  uint32_t t[NA + NB];
+#pragma unroll
+  for (int i = 0; i < NA + NB; ++i) t[i] = 0;
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    uint64_t carry = 0;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      carry += (uint64_t)a[i] * b[j] + t[i + j];
+      t[i + j] = (uint32_t)carry;
+      carry >>= 32;
+    }
+    t[i + NB] = (uint32_t)carry;
+  }
+#pragma unroll
+  for (int i = 0; i < NO; ++i) out[i] = i + LO < NA + NB ? t[i + LO] : 0u;
+}
+
+// out = a - b over five words, modulo 2^160.
+__device__ __forceinline__ void sub160(const uint32_t* a, const uint32_t* b, uint32_t* out) {
+  uint64_t borrow = 0;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const uint64_t d = (uint64_t)a[i] - b[i] - borrow;
+    out[i] = (uint32_t)d;
+    borrow = d >> 63;
+  }
+}
+
+// Scalar i of column j leaves |k1| at 2 off + i and |k2| len further on, over P and
+// phi(P) with the halves' signs folded into the points: columns of twice the length
+// for the ordinary kernels (`at` holds the columns' first places).
+struct SplitCols {
+  MsmCols in;
+  uint32_t at[kMaxCols];
+};
+__global__ void __launch_bounds__(128) k_split(const __grid_constant__ SplitCols S, const Affine* bases,
+                                               int canonical_in, Affine* out_bases, Fr* out_scalars,
+                                               uint32_t* flags) {
+  const uint32_t col = blockIdx.y, n = S.in.len[col], i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  Fr k = ld_fe(reinterpret_cast<const Fr*>(S.in.s[col]) + i);
+  if (!fe_lt_mod<FrConsts>(k.v)) raise_flag(flags, DEV_NONCANONICAL);
+  if (!canonical_in) k = fe_from_mont(k);
+  uint32_t c1[2], c2[4], x[5], y[5], k1[5], k2[5];
+  product_words<8, 3, 8, 2>(k.v, kSplitG1, c1);
+  product_words<8, 5, 8, 4>(k.v, kSplitG2, c2);
+  product_words<2, 2, 0, 5>(c1, kSplitA1, x);
+  sub160(k.v, x, k1);
+  product_words<4, 4, 0, 5>(c2, kSplitA2, y);
+  sub160(k1, y, k1);
+  product_words<2, 4, 0, 5>(c1, kSplitB1, x);
+  product_words<4, 2, 0, 5>(c2, kSplitA1, y);
+  sub160(x, y, k2);
+  const Affine p = ld_affine(&bases[S.in.off[col] + i]);
+  Fq beta;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) beta.v[w] = kSplitBeta[w];
+  const uint32_t zero[5] = {0, 0, 0, 0, 0};
+  Fr half;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) half.v[w] = 0;
+  const size_t o = (size_t)S.at[col] + i;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t* v = h ? k2 : k1;
+    const bool neg = v[4] >> 31;
+    if (neg) sub160(zero, v, v);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) half.v[w] = v[w];
+    const size_t to = o + (h ? n : 0);
+    st_fe(&out_scalars[to], half);
+    st_fe(&out_bases[to].x, h ? fe_mul(p.x, beta) : p.x);
+    st_fe(&out_bases[to].y, neg ? fe_neg(p.y) : p.y);
   }
 }
 
@@ -1557,6 +1653,14 @@ static int default_window(size_t n, bool small) {
   return cb;
 }
 
+// Window width for n half scalars (127 bits). Eight bits make sixteen windows exactly.
+// Swept on a GB300, us a call from host points and scalars, by the whole scalars'
+// count: 2^12 at 7/8/9/12 bits 510/494/551/544, 2^14 at 8/12/13 639/621/633, 2^16 at
+// 12/13/14 876/866/928, 2^18 at 12/13/16 1900/1746/1735.
+static int split_window(size_t n) {
+  return n < ((size_t)1 << 15) ? 8 : n < ((size_t)1 << 17) ? 12 : n < ((size_t)1 << 19) ? 13 : 16;
+}
+
 static int window_count(int bits, int cb) { return (bits + 1 + cb - 1) / cb; }
 
 const SrsTable* srs_table(Ctx& c, int cbits, size_t need) {
@@ -1645,11 +1749,11 @@ void msm_autotune(Ctx& c, const void* d_sample, size_t sample_len, int kmin, int
   cudaEventDestroy(e1);
 }
 
-MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits) {
+MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits, int full_bits) {
   MsmPlan p;
-  p.c = table ? table->c : default_window(n, small_scalars);
+  p.c = table ? table->c : full_bits < 254 ? split_window(n) : default_window(n, small_scalars);
   p.precomp = table != nullptr;
-  p.windows = small_scalars ? window_count(bits, p.c) : table ? table->windows : window_count(254, p.c);
+  p.windows = small_scalars ? window_count(bits, p.c) : table ? table->windows : window_count(full_bits, p.c);
   // A scalar narrower than the window has one digit, itself, and fills no
   // bucket past its own range (one-byte columns over 17-bit windows: 2^8 of
   // 2^16 buckets to scan and reduce).
@@ -1659,6 +1763,15 @@ MsmPlan msm_plan(size_t n, bool small_scalars, const SrsTable* table, int bits) 
 }
 
 namespace {
+
+// Scalars over the caller's own bases are split (k_split) up to this many halves. A
+// call without a window table ends in Horner's chain over the windows, one doubling
+// after another whatever the size: 254 of them took 520 us of the 750 that a GB300
+// needed for 2484 points, half of that when split. us a call, whole -> split: 2^4
+// 796 -> 412, 2^12 801 -> 494, 2^16 1140 -> 866, 2^19 2980 -> 2694; at 2^20 the gain
+// is down to 5 % for twice the memory of the bases.
+constexpr int kSplitBits = 127;
+constexpr size_t kSplitMax = (size_t)1 << 20;
 
 // Threads of k_bucket_acc resident on the whole device (one wave).
 size_t acc_resident_threads(Ctx& c) {
@@ -1849,6 +1962,37 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
 
 void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* const* scalars, const size_t* lens,
                size_t k, bool small_scalars, bool scalars_canonical, uint8_t* d_out, const MsmBatchOpts& o) {
+  // Field elements over the caller's bases: as halves, while they are few enough.
+  if (!table && !small_scalars && o.full_bits == 254 && k <= (size_t)kMaxCols) {
+    size_t n2 = 0, nmax = 0;
+    for (size_t j = 0; j < k; ++j) {
+      n2 = lens[j] > kSplitMax ? kSplitMax + 1 : std::min(kSplitMax + 1, n2 + 2 * lens[j]);
+      nmax = std::max(nmax, lens[j]);
+    }
+    if (n2 > 0 && n2 <= kSplitMax) {
+      Affine* sb = c.scratch[S_SPLIT_BASES].as<Affine>(n2);
+      Fr* ss = c.scratch[S_SPLIT_SCALARS].as<Fr>(n2);
+      SplitCols S{};
+      const void* ptrs[kMaxCols];
+      size_t len2[kMaxCols], offs[kMaxCols], at = 0;
+      for (size_t j = 0; j < k; ++j) {
+        S.in.s[j] = scalars[j];
+        S.in.len[j] = (uint32_t)lens[j];
+        S.in.off[j] = o.offs ? (uint32_t)o.offs[j] : 0u;
+        S.at[j] = (uint32_t)at;
+        ptrs[j] = ss + at;
+        len2[j] = 2 * lens[j];
+        offs[j] = at;
+        at += len2[j];
+      }
+      launch(c, k_split, dim3(blocks_for<int>(nmax, 128), (unsigned)k), 128, 0, S, bases, scalars_canonical ? 1 : 0, sb,
+             ss, c.d_flags);
+      MsmBatchOpts o2 = o;
+      o2.offs = offs;
+      o2.full_bits = kSplitBits;
+      return msm_multi(c, sb, nullptr, ptrs, len2, k, false, true, d_out, o2);
+    }
+  }
   // A stack sums its columns: every group writes one partial result, added
   // at the end when there is more than one.
   uint8_t* partial = nullptr;
@@ -1864,7 +2008,7 @@ void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* c
       const size_t n = lens[j + g];
       if (n >= ((size_t)1 << 31)) throw Error(APG_ERR_INVALID_ARGUMENT, "MSM longer than 2^31 - 1 points");
       const size_t nm = std::max(nmax, n);
-      const MsmPlan q = msm_plan(std::max<size_t>(nm, 1), small_scalars, table, o.bits);
+      const MsmPlan q = msm_plan(std::max<size_t>(nm, 1), small_scalars, table, o.bits, o.full_bits);
       const size_t spaces = q.precomp ? 1 : (size_t)q.windows;
       const size_t bins = (g + 1) * spaces * q.buckets;
       size_t e = 0;
