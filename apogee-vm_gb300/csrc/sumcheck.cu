@@ -283,11 +283,11 @@ struct DevForm {
 };
 
 // A round of a factored quadratic form, staged through shared memory. A block
-// takes 2^log_pp pairs at a time: its threads fold the pairs' lines of every
-// table with the previous challenge (a line a thread) and leave each line's
-// values at the round's nodes in shared memory; then a warp takes every
-// nshare-th group for a tile of pairs, so its lanes run the same terms and read
-// the same coefficients. Both the inner sums and the sum over the groups stay
+// takes 2^log_pp pairs at a time, nshare warps a tile of them: they fold the tile's
+// lines of every table with the previous challenge (a line a thread) and leave each
+// line's values at the round's nodes in shared memory; then each takes every
+// nshare-th group of terms, so its lanes run the same terms and read the same
+// coefficients. Both the inner sums and the sum over the groups stay
 // unreduced (wide_mac): 64 products a term instead of 136. A tile is 16 pairs at
 // two nodes; at three nodes 32 pairs in three passes (two of 16 pairs at nodes 0
 // and 2, one of 32 at node 1) or, where so many pairs' values are too much shared
@@ -327,11 +327,17 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
   // Lanes of a pass: 2^log_l pairs a node, the nodes from lane slot 0 on (the
   // idle quarter of the 8-pair tile repeats the last node).
   const int log_l = three && passes == 1 ? 3 : 4, slot = lane >> log_l;
-  const int share = warp % nshare, tile = (warp / nshare) << (passes == 3 ? 5 : log_l);
+  const int log_t = passes == 3 ? 5 : log_l, log_tp = min(log_pp, log_t);
+  const int share = warp % nshare, group = warp / nshare, tile = group << log_t;
+  // The warps of a tile are a group: they fold its lines and wait for one another only.
+  auto group_sync = [&]() {
+    if (nshare == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(32 * nshare) : "memory");
+  };
   Fr acc = fe_zero<FrConsts>(), acc1 = fe_zero<FrConsts>();  // (acc1: node 1 of the third pass)
   for (size_t p0 = (size_t)blockIdx.x << log_pp; p0 < A.npairs; p0 += (size_t)gridDim.x << log_pp) {
-    for (int t = threadIdx.x; t < (ns + 1) << log_pp; t += blockDim.x) {
-      const int k = t >> log_pp, at = t & (pp - 1);
+    for (int t = 32 * share + lane; t < (ns + 1) << log_tp; t += 32 * nshare) {
+      const int k = t >> log_tp, at = tile + (t & ((1 << log_tp) - 1));
       const size_t pair = p0 + at;
       if (pair >= A.npairs) continue;
       Fr lo, hi;
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
       if (three) form_st(o, 2 * pp + at, pp, hi);
       form_st(o, (nn - 1) * 2 * pp + at, pp, fe_sub(fe_add(hi, hi), lo));
     }
-    __syncthreads();
+    group_sync();
     for (int pass = 0; pass < passes; ++pass) {
       const int i = tile + (pass == 2 ? lane : (pass << 4) + (lane & ((1 << log_l) - 1)));
       const int xi = pass == 2 ? 1 : passes == 3 ? 2 * slot : min(slot, nn - 1);
@@ -396,7 +402,7 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
       if (pass == 2) acc1 = fe_add(acc1, s);
       else if (slot < nn) acc = fe_add(acc, s);
     }
-    __syncthreads();
+    group_sync();
   }
   // The warp's sum a node, from the slot's first lane.
 #pragma unroll 1
@@ -681,10 +687,14 @@ static FormShape form_shape(const HostForm& f, size_t npairs, int slots, bool th
   } else {
     // As many tiles as the shared memory of four blocks an SM takes, and a
     // share for every two thousand wide products (a share costs its own weight
-    // and reduction, 270).
+    // and reduction, 270). Blocks of four warps, four to an SM, where the values
+    // fit: their folds, which wait for memory, run beside others' products
+    // (zerochecks of 2^21 rows 1485 and 1783 us with two blocks of eight, 1445 and
+    // 1711 so).
     int tiles = 1, share = 1;
-    while (tiles < 8 && line * ((size_t)2 * tiles << log_p) <= kFormSmem) tiles *= 2;
-    while (share * tiles < 8 && ((size_t)share * 2 * kFormShareCost <= f.cost || share * tiles < 4)) share *= 2;
+    const int warps = (line << log_p) * 4 <= kFormSmemMax ? 4 : 8;
+    while (tiles < warps && line * ((size_t)2 * tiles << log_p) <= kFormSmem) tiles *= 2;
+    while (share * tiles < warps && ((size_t)share * 2 * kFormShareCost <= f.cost || share * tiles < 4)) share *= 2;
     s.share = share;
     s.threads = 32 * share * tiles;
     for (int t = tiles; t > 1; t /= 2) ++s.log_pp;
