@@ -706,24 +706,94 @@ __global__ void __launch_bounds__(128) k_split(const __grid_constant__ SplitCols
 }
 
 // Digits of one scalar, counted (SCATTER = false) or placed (SCATTER = true).
-// Lanes of a warp that hit the same bucket share one atomic: the leader adds
-// the group's size and hands each peer its rank, so a bucket that a large
-// share of the scalars hit (digit 1 from {0,1} columns and from the carries of
-// 32-bit values) costs one atomic per warp, not one per scalar. Measured and
-// not kept: aggregating only the lanes that share the first active lane's
-// bucket, with plain atomics for the rest (13 % slower on mixed columns), and
-// the window width compiled in with the window loop unrolled and every
-// window's atomic issued before the first result is awaited (no change in
-// either pass at 2^22).
+//
+// A block takes 256 scalars. Its threads first run the windows of a scalar's low 32
+// bits; scalars with anything above those go to shared memory, close together, and
+// the block's warps run their other windows, so that a column of mostly narrow values
+// doesn't walk whole warps through every window for the few wide ones. Lanes of a warp
+// that hit the same bucket share one atomic where that is common: those of digit 1
+// ({0,1} columns, carries of 32-bit values) and, when the first other lane's bucket is
+// shared, all lanes' (columns of few distinct values). Matching every lane with every
+// other one at every window takes longer than the atomics it saves and kept both
+// passes at it (the shuffle queue full nine cycles in ten); now a uniform column is
+// bound by its scattered accesses in L2, about 170 G a second. A placed digit is
+// stored one window later, when its cursor's atomic has come back. Measured on a
+// GB300, counted and placed: four mixed columns of 2^20 196 + 297 -> 134 + 212 us, four
+// uniform ones 461 + 929 -> 383 + 776.
+constexpr int kDigitThreads = 256;
+
+struct DigitOut {
+  uint32_t* cursor;
+  uint32_t* sorted;
+  uint32_t* flags;
+  uint32_t stride;
+};
+
+template <bool SCATTER>
+struct DigitStep {
+  uint32_t base = 0, ref = 0;  // the digit placed last: its group's first place (in the leader), its reference
+  unsigned peers = 0;          // its group; 0: none
+
+  __device__ __forceinline__ void flush(const DigitOut& o, unsigned lane) {
+    if (!SCATTER) return;
+    const uint32_t b = __shfl_sync(0xffffffffu, base, peers ? __ffs(peers) - 1 : 0);
+    if (peers) o.sorted[b + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = ref;
+    peers = 0;
+  }
+
+  // One window of the warp's scalars: digit mag (0: none) of bucket range key0.
+  __device__ __forceinline__ void put(const DigitOut& o, unsigned lane, uint32_t mag, uint32_t key0, uint32_t r) {
+    if (mag > o.stride) {  // unreachable for values below r; never index past the bucket range
+      if (!SCATTER) raise_flag(o.flags, DEV_NONCANONICAL);
+      mag = 0;
+    }
+    const unsigned some = __ballot_sync(0xffffffffu, mag != 0);
+    if (!some) return;
+    const uint32_t key = key0 + mag - 1;
+    const unsigned ones = __ballot_sync(0xffffffffu, mag == 1), left = some & ~ones;
+    unsigned group = mag == 1 ? ones : mag ? 1u << lane : 0u;
+    if (left) {
+      const uint32_t k = __shfl_sync(0xffffffffu, mag, __ffs(left) - 1);
+      const unsigned same = __ballot_sync(0xffffffffu, mag == k);
+      if (mag == k) group = same;
+      if ((same & (same - 1)) && left != same) {
+        const unsigned peers = __match_any_sync(0xffffffffu, mag);
+        if (mag) group = peers;
+      }
+    }
+    const bool lead = group && (int)lane == __ffs(group) - 1;
+    uint32_t b = 0;
+    if (lead) {
+      if (SCATTER) b = atomicAdd(&o.cursor[key], (uint32_t)__popc(group));
+      else atomicAdd(&o.cursor[key], (uint32_t)__popc(group));
+    }
+    if (SCATTER) {
+      flush(o, lane);
+      base = b;
+      peers = group;
+      ref = r;
+    }
+  }
+};
+
+// The signed digit of a window's c bits and the carry into it: its size, the sign and
+// the next carry in neg.
+__device__ __forceinline__ uint32_t signed_digit(uint32_t coef, uint32_t K, bool top, uint32_t& neg) {
+  neg = !top && coef >= K;
+  return neg ? 2 * K - coef : coef;  // coef - 2^c < 0
+}
+
 template <bool SMALL, bool SCATTER>
-__global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows, int precomp, uint32_t stride,
-                                                uint32_t tab_n, int canonical_in, uint32_t* cursor, uint32_t* sorted,
-                                                uint32_t* flags) {
+__global__ void __launch_bounds__(kDigitThreads) k_digits(MsmCols cols, int c, int windows, int precomp,
+                                                          uint32_t stride, uint32_t tab_n, int canonical_in,
+                                                          uint32_t* cursor, uint32_t* sorted, uint32_t* flags) {
+  __shared__ uint32_t wide[SMALL ? 1 : 9][kDigitThreads];  // limbs, then the place in the block and the carry
+  __shared__ uint32_t nwide;
   const uint32_t col = blockIdx.y;
   const uint32_t n = cols.len[col];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i0 = blockIdx.x * kDigitThreads, i = i0 + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31u;
-  if (i - lane >= n) return;  // the whole warp lies past the column's end
+  if (i0 >= n) return;  // the whole block lies past the column's end
   const bool live = i < n;
   uint32_t limbs[8];
 #pragma unroll
@@ -739,52 +809,62 @@ __global__ void __launch_bounds__(256) k_digits(MsmCols cols, int c, int windows
       for (int k = 0; k < 8; ++k) limbs[k] = s.v[k];
     }
   }
-  const uint32_t K = 1u << (c - 1);
-  const uint32_t mask = (1u << c) - 1;
+  const uint32_t K = 1u << (c - 1), mask = (1u << c) - 1;
   const uint32_t spaces = precomp ? 1u : (uint32_t)windows;
   const uint32_t key0 = cols.shared ? 0u : col * spaces * stride;
-  const uint32_t base_i = cols.off[col] + i;
-  uint32_t carry = 0;
-  for (int w = 0; w < windows; ++w) {
-    const int off = w * c;
-    uint32_t raw = 0;
-    if (off < 256) {
-      const int limb = off >> 5, sh = off & 31;
-      uint64_t v = limbs[limb] >> sh;
-      if (limb + 1 < 8) v |= (uint64_t)limbs[limb + 1] << (32 - sh);
-      raw = (uint32_t)v & mask;
+  const uint32_t key_step = precomp ? 0u : stride, ref_step = precomp ? tab_n : 0u;
+  const DigitOut out = {cursor, sorted, flags, stride};
+  DigitStep<SCATTER> st;
+  const int low = min(windows, (32 + c) / c);  // 33 bits: a 32-bit value and its carry
+  uint32_t carry = 0, ref = cols.off[col] + i, key = key0;
+  uint64_t v = limbs[0] | (uint64_t)limbs[1] << 32;
+  for (int w = 0; w < low; ++w) {
+    uint32_t neg;
+    const uint32_t mag = signed_digit(((uint32_t)v & mask) + carry, K, w == windows - 1, neg);
+    st.put(out, lane, live ? mag : 0u, key, (neg << 31) | ref);
+    v >>= c;
+    carry = neg;
+    key += key_step;
+    ref += ref_step;
+  }
+  if (!SMALL && low < windows) {
+    if (threadIdx.x == 0) nwide = 0;
+    __syncthreads();
+    uint32_t above = carry | (uint32_t)v | (uint32_t)(v >> 32);
+#pragma unroll
+    for (int k = 2; k < 8; ++k) above |= limbs[k];
+    const unsigned some = __ballot_sync(0xffffffffu, above != 0);
+    uint32_t at = 0;
+    if (lane == 0 && some) at = atomicAdd(&nwide, (uint32_t)__popc(some));
+    at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(some & ((1u << lane) - 1u));
+    if (above) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) wide[k][at] = limbs[k];
+      wide[8][at] = threadIdx.x | carry << 31;
     }
-    const uint32_t coef = raw + carry;
-    uint32_t mag, neg = 0;
-    if (w == windows - 1 || coef < K) {
-      mag = coef;
-      carry = 0;
-    } else {
-      mag = (1u << c) - coef;  // digit coef - 2^c < 0
-      neg = 1;
-      carry = 1;
-    }
-    if (!live) mag = 0;
-    if (mag > stride) {  // unreachable for values below r; never index past the bucket range
-      if (!SCATTER) raise_flag(flags, DEV_NONCANONICAL);
-      mag = 0;
-    }
-    const unsigned active = __ballot_sync(0xffffffffu, mag != 0);
-    if (mag) {
-      const uint32_t key = key0 + (precomp ? 0u : (uint32_t)w * stride) + mag - 1;
-      const unsigned peers = __match_any_sync(active, key);
-      const int leader = __ffs(peers) - 1;
-      if (SCATTER) {
-        uint32_t base = 0;
-        if ((int)lane == leader) base = atomicAdd(&cursor[key], (uint32_t)__popc(peers));
-        base = __shfl_sync(peers, base, leader);
-        const uint32_t idx = precomp ? (uint32_t)w * tab_n + base_i : base_i;
-        sorted[base + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = (neg << 31) | idx;
-      } else if ((int)lane == leader) {
-        atomicAdd(&cursor[key], (uint32_t)__popc(peers));
+    __syncthreads();
+    if (threadIdx.x - lane < nwide) {
+      const bool on = threadIdx.x < nwide;
+      const uint32_t who = on ? wide[8][threadIdx.x] : 0u;
+      carry = who >> 31;
+      ref = cols.off[col] + i0 + (who & 0x7fffffffu) + (uint32_t)low * ref_step;
+      for (int w = low; w < windows; ++w) {
+        const int off = w * c, limb = off >> 5;
+        uint32_t raw = 0;
+        if (on && limb < 8) {
+          const uint32_t a = wide[limb][threadIdx.x], b = limb < 7 ? wide[limb + 1][threadIdx.x] : 0u;
+          raw = __funnelshift_r(a, b, off & 31) & mask;
+        }
+        uint32_t neg;
+        const uint32_t mag = signed_digit(raw + carry, K, w == windows - 1, neg);
+        st.put(out, lane, mag, key, (neg << 31) | ref);
+        carry = neg;
+        key += key_step;
+        ref += ref_step;
       }
     }
   }
+  st.flush(out, lane);
 }
 
 // The same digits when a column has few buckets (kFewBins at most: 8-bit
@@ -1866,11 +1946,12 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
       launch(c, k, grid, 256, few * sizeof(uint32_t), cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, 256 * per,
              counts, place, c.d_flags);
     } else {
-      const dim3 grid(blocks_for<int>(std::max<size_t>(nmax, 1), 256), (unsigned)ncols);
+      const dim3 grid(blocks_for<int>(std::max<size_t>(nmax, 1), kDigitThreads), (unsigned)ncols);
       void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t*, uint32_t*, uint32_t*) =
           small_scalars ? (place ? k_digits<true, true> : k_digits<true, false>)
                         : (place ? k_digits<false, true> : k_digits<false, false>);
-      launch(c, k, grid, 256, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place, c.d_flags);
+      launch(c, k, grid, kDigitThreads, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place,
+             c.d_flags);
     }
   };
   digits(nullptr);
