@@ -367,7 +367,8 @@ __global__ void __launch_bounds__(128) k_accumulate(const uint64_t* sorted, cons
 constexpr int kFoldQuads = 64;
 constexpr int kFoldLastPer = 8;  // items a quad at most in a level of one block
 
-__global__ void __launch_bounds__(4 * kFoldQuads) k_fold_edges(const uint32_t* keys, const Xyzz* pts,
+template <int BLOCKS>
+__global__ void __launch_bounds__(4 * kFoldQuads, BLOCKS) k_fold_edges(const uint32_t* keys, const Xyzz* pts,
                                                                const uint8_t* pres, size_t len, int per,
                                                                Xyzz* buckets, uint32_t* okeys, Xyzz* opts,
                                                                uint8_t* opres) {
@@ -502,7 +503,8 @@ __global__ void __launch_bounds__(4 * kFoldQuads) k_fold_edges(const uint32_t* k
 // of 2^19 (bound by the products) 1.9 -> 1.65 ms.
 constexpr int kReduceQuads = 64;  // a block at most: two warps a scheduler (see kFoldQuads)
 
-__global__ void __launch_bounds__(4 * kReduceQuads) k_reduce(const Xyzz* R, const Xyzz* T, int M, int lf, int scale,
+template <int BLOCKS>
+__global__ void __launch_bounds__(4 * kReduceQuads, BLOCKS) k_reduce(const Xyzz* R, const Xyzz* T, int M, int lf, int scale,
                                                              int last, Xyzz* outT, Xyzz* outR) {
   extern __shared__ uint4 sm_points[];
   Fq* sh = reinterpret_cast<Fq*>(sm_points);
@@ -1650,6 +1652,13 @@ inline ReducePlan reduce_plan(uint32_t K, int S, int sm_count) {
   p.last_quads = std::max(8, p.last_m >> p.last_lf);  // whole warps
   return p;
 }
+// The tails' kernels hold about 170 registers, one block an SM; where there are more
+// blocks than SMs, a form of 128 (some spilled) lets two share one: four 2^12-point
+// columns 285 -> 264 us, 2^20 one-byte scalars 470 -> 451, but 2^8 points 176 -> 178.
+template <class K>
+inline K tail_kernel(K one, K two, size_t blocks, int sm_count) {
+  return blocks > (size_t)sm_count ? two : one;
+}
 inline size_t reduce_smem(int quads) { return (size_t)quads * sizeof(Xyzz); }
 
 template <class T>
@@ -2024,15 +2033,16 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   c.timer_end(APG_TIMER_MSM_ACCUMULATE, t_acc);
   for (size_t len = 2 * nseg, cur = 0; len > 2; cur ^= 1) {
     const FoldLevel f = fold_level(len);
-    launch(c, k_fold_edges, f.blocks, 4 * kFoldQuads, 0, (const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
+    launch(c, tail_kernel(k_fold_edges<1>, k_fold_edges<2>, f.blocks, c.sm_count), f.blocks, 4 * kFoldQuads, 0, (const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
            (const uint8_t*)ipres[cur], len, f.per, buckets, ikeys[cur ^ 1], ipts[cur ^ 1], ipres[cur ^ 1]);
     len = 2 * (size_t)f.blocks;
   }
   const bool two_levels = rp.last_scale > 0;
   if (two_levels)
-    launch(c, k_reduce, dim3(rp.blocks, S), 4 * kReduceQuads, reduce_smem(kReduceQuads), (const Xyzz*)buckets,
+    launch(c, tail_kernel(k_reduce<1>, k_reduce<2>, (size_t)rp.blocks * S, c.sm_count), dim3(rp.blocks, S),
+           4 * kReduceQuads, reduce_smem(kReduceQuads), (const Xyzz*)buckets,
            (const Xyzz*)nullptr, (int)K, rp.lf, 0, 0, lvlT, lvlR);
-  launch(c, k_reduce, dim3(1, S), 4 * rp.last_quads, reduce_smem(rp.last_quads),
+  launch(c, tail_kernel(k_reduce<1>, k_reduce<2>, S, c.sm_count), dim3(1, S), 4 * rp.last_quads, reduce_smem(rp.last_quads),
          (const Xyzz*)(two_levels ? lvlR : buckets), (const Xyzz*)(two_levels ? lvlT : nullptr), rp.last_m, rp.last_lf,
          rp.last_scale, 1, tsum, (Xyzz*)nullptr);
   launch(c, k_finish, (unsigned)nout, 32, 0, (const Xyzz*)tsum, spaces_per_col, p.c, (uint32_t*)d_out, c.d_flags);
@@ -2277,13 +2287,13 @@ int msm_noalloc(const void* d_bases, const void* d_scalars, size_t n, void* d_ou
   APG_NA_LAUNCH();
   for (size_t len = 2 * nseg, cur = 0; len > 2; cur ^= 1) {
     const FoldLevel f = fold_level(len);
-    k_fold_edges<<<f.blocks, 4 * kFoldQuads, 0, st>>>((const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
+    k_fold_edges<1><<<f.blocks, 4 * kFoldQuads, 0, st>>>((const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
                                                       (const uint8_t*)ipres[cur], len, f.per, buckets, ikeys[cur ^ 1],
                                                       ipts[cur ^ 1], ipres[cur ^ 1]);
     APG_NA_LAUNCH();
     len = 2 * (size_t)f.blocks;
   }
-  k_reduce<<<dim3(1, spaces), 4 * kReduceQuads, reduce_smem(kReduceQuads), st>>>(
+  k_reduce<1><<<dim3(1, spaces), 4 * kReduceQuads, reduce_smem(kReduceQuads), st>>>(
       (const Xyzz*)buckets, (const Xyzz*)nullptr, K, 2, 0, 1, tsum, (Xyzz*)nullptr);
   APG_NA_LAUNCH();
   k_finish<<<1, 32, 0, st>>>((const Xyzz*)tsum, spaces, kNoAllocC, (uint32_t*)d_out, flags);
