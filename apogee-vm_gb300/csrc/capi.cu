@@ -527,7 +527,7 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   APG_CUDA(cudaStreamWaitEvent(c.stream, ev, 0));
   APG_CUDA(cudaEventDestroy(ev));
   try {
-    fetch_checked(c, d_out, 64 * k, out);
+    fetch_checked(c, d_out, 64 * k, out, false);  // (follows the other lane's event)
   } catch (...) {  // the lane's own flags must not outlive this call
     cudaMemsetAsync(L.d_flags, 0, 4, L.stream);
     cudaStreamSynchronize(L.stream);

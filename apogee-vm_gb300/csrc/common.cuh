@@ -225,6 +225,39 @@ inline void launch(Ctx& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size
   }
 }
 
+// The same for a kernel that begins with chain_begin() and follows another kernel
+// on the stream: its blocks may be set up while that one's last blocks still run
+// (programmatic stream serialization), and wait there for it to end. Every kernel of a
+// chain waits, so each sees all that stands before it. What follows an event or a
+// memory operation is launched plainly. Measured on a GB300, the chains of an MSM and an
+// opening launched so: commitments of four 2^8-point columns 178 -> 160 us, a stacked
+// 2^16-variable opening (93 launches) 2359 -> 2176.
+template <class... KArgs, class... Args>
+inline void launch_chained(Ctx& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  if (c.timers.on) return launch(c, kernel, grid, block, smem, args...);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c.stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  APG_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+  ++c.launches;
+}
+
+#ifdef __CUDACC__
+// The first thing that a kernel of launch_chained does, before it reads or writes
+// memory: wait for the kernel before it, then let the one after it be set up.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // Entry points implemented in the .cu files.
 // ---------------------------------------------------------------------------
@@ -235,10 +268,10 @@ __global__ void k_fr_to_mont(Fr* v, size_t n, uint32_t* flags);
 // `bytes` of a result on the stream to the host, the error flags checked: a
 // kernel stores both in pinned memory and the host waits for its flag (instead of
 // two copies and a synchronisation: about 15 us less a result on a GB300).
-void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host);
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host, bool chained = true);
 // The same in two halves: publish on the stream (work may follow), collect before
 // anything else is published.
-uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes);
+uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes, bool chained = true);
 void collect_checked(Ctx& c, uint32_t seq, size_t bytes, void* host);
 // Canonical 64-byte points (host) -> device affine Montgomery, validated.
 void upload_points(Ctx& c, const uint8_t* host, size_t n, Affine* dst);

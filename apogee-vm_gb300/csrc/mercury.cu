@@ -59,6 +59,7 @@ __device__ __forceinline__ Fr warp_total(Fr acc) {  // in lane 0
 // GB300.
 __global__ void __launch_bounds__(256) k_row_dot(const Fr* const* cols, const Fr* one, const Fr* eq1, size_t b,
                                                  size_t rows, Fr* h) {
+  chain_begin();
   const size_t row = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(256) k_row_dot(const Fr* const* cols, const Fr
 
 // out[j] = sum_i a[i] * b[j * n + i], a block each.
 __global__ void __launch_bounds__(256) k_dot(const Fr* a, const Fr* b, size_t n, Fr* out) {
+  chain_begin();
   __shared__ Fr red[8];
   const Fr acc = warp_total(dot_share(a, b + blockIdx.x * n, n, threadIdx.x, blockDim.x));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(256) k_dot(const Fr* a, const Fr* b, size_t n,
 // its bottom value as the segment's aggregate.
 __global__ void k_suffix_local(const Fr* in, Fr* out, size_t stride, size_t count, size_t cols, int L, Fr r,
                                Fr* agg) {
+  chain_begin();
   const size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t nseg = (count + L - 1) / L;
   if (id >= nseg * cols) return;
@@ -109,6 +112,7 @@ struct SuffixPowers {
 // result), acc_j = local_j + r^(lo_{s+1} - j) * upper[s+1].
 __global__ void k_suffix_fix(Fr* out, size_t stride, size_t count, size_t cols, int L, const Fr* upper,
                              const __grid_constant__ SuffixPowers pows) {
+  chain_begin();
   const size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (id >= count * cols) return;
   const size_t j = id / cols, col = id % cols;
@@ -127,6 +131,7 @@ __global__ void k_suffix_fix(Fr* out, size_t stride, size_t count, size_t cols, 
 constexpr size_t kSuffixScanMax = 1024;
 __global__ void __launch_bounds__(1024) k_suffix_scan(const Fr* in, Fr* out, size_t stride, int count,
                                                       const __grid_constant__ SuffixPowers pows) {
+  chain_begin();
   __shared__ Fr sh[kSuffixScanMax];
   const int j = threadIdx.x;
   const size_t at = j * stride + blockIdx.x;
@@ -142,6 +147,7 @@ __global__ void __launch_bounds__(1024) k_suffix_scan(const Fr* in, Fr* out, siz
 
 // out[i] = base^i.
 __global__ void k_powers(Fr base, size_t count, Fr* out) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= count) return;
   Fr acc = fe_one<FrConsts>(), b = base;
@@ -153,6 +159,7 @@ __global__ void k_powers(Fr base, size_t count, Fr* out) {
 }
 
 __global__ void k_bitrev(Fr* a, size_t m, int bits) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= m) return;
   size_t j = __brevll((unsigned long long)i) >> (64 - bits);
@@ -166,6 +173,7 @@ __global__ void k_bitrev(Fr* a, size_t m, int bits) {
 // One radix-2 decimation-in-time stage at half-width `half` (the reference's
 // butterflies, crates/pcs/src/fft.rs:100-134): tw holds w^k for k < m/2.
 __global__ void k_fft_stage(Fr* a, size_t m, size_t half, const Fr* tw) {
+  chain_begin();
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= m / 2) return;
   size_t start = (t / half) * 2 * half, k = t % half;
@@ -187,6 +195,7 @@ struct EvalArgs {
   Fr pw[kEvals][9];
 };
 __global__ void __launch_bounds__(256) k_eval(const __grid_constant__ EvalArgs E, uint32_t run, Fr* out) {
+  chain_begin();
   __shared__ Fr sh[256];
   const int q = blockIdx.x, t = threadIdx.x;
   const Fr* p = E.poly[q];
@@ -214,6 +223,7 @@ struct BdfgArgs {
   Fr low[5];
 };
 __global__ void __launch_bounds__(256) k_bdfg(const __grid_constant__ BdfgArgs B, uint32_t n, Fr* out) {
+  chain_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   FeWide<FrConsts> s = wide_zero<FrConsts>();  // (at most fourteen products)
@@ -268,6 +278,7 @@ struct SymOperands {
   const Fr* src[4];
 };
 __global__ void __launch_bounds__(1024) k_sym_fft(SymOperands S, size_t b, int bits, const Fr* tw, Fr* out) {
+  chain_begin();
   extern __shared__ uint4 sh_fft[];
   const size_t m = 2 * b, q = blockIdx.x;
   const Fr* src = S.src[q];
@@ -284,6 +295,7 @@ __global__ void __launch_bounds__(1024) k_sym_fft(SymOperands S, size_t b, int b
 __global__ void __launch_bounds__(1024) k_sym_ifft(const Fr* t, size_t b, int bits, const Fr* tw, Fr gamma, Fr scale,
                                                    const Fr* h_alpha, Fr gamma_v, const Fr* g, Fr* S, Fr* D,
                                                    uint32_t* flags) {
+  chain_begin();
   extern __shared__ uint4 sh_fft[];
   const size_t m = 2 * b;
   for (size_t i = threadIdx.x; i < m; i += blockDim.x) {
@@ -307,6 +319,7 @@ __global__ void __launch_bounds__(1024) k_sym_ifft(const Fr* t, size_t b, int bi
 // The four padded operands of S: g, rev(eq1), h, rev(eq2), each b long in 2b.
 __global__ void k_sym_pad(const Fr* g, const Fr* eq1, const Fr* h, const Fr* eq2, size_t b, Fr* G, Fr* P1, Fr* H,
                           Fr* P2) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= 2 * b) return;
   const Fr z = fe_zero<FrConsts>();
@@ -317,6 +330,7 @@ __global__ void k_sym_pad(const Fr* g, const Fr* eq1, const Fr* h, const Fr* eq2
 }
 
 __global__ void k_sym_mix(const Fr* G, const Fr* P1, const Fr* H, const Fr* P2, size_t m, Fr gamma, Fr* R) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= m) return;
   Fr a = fe_mul(ld_fe(&G[i]), ld_fe(&P1[i]));
@@ -325,6 +339,7 @@ __global__ void k_sym_mix(const Fr* G, const Fr* P1, const Fr* H, const Fr* P2, 
 }
 
 __global__ void k_scale(Fr* a, size_t m, Fr s) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < m) st_fe(&a[i], fe_mul(ld_fe(&a[i]), s));
 }
@@ -332,6 +347,7 @@ __global__ void k_scale(Fr* a, size_t m, Fr s) {
 // S[k - b] = R[k] + R[2b - 2 - k] for k in [b, 2b - 1); checks R[2b-1] = 0 and
 // R[b-1] = h(alpha) + gamma v (symmetric_witness's two assertions).
 __global__ void k_sym_out(const Fr* R, size_t b, const Fr* h_alpha, Fr gamma_v, Fr* S, uint32_t* flags) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i == 0) {
     if (!fe_is_zero(ld_fe(&R[2 * b - 1])) || !fe_eq(ld_fe(&R[b - 1]), fe_add(ld_fe(h_alpha), gamma_v)))
@@ -343,12 +359,14 @@ __global__ void k_sym_out(const Fr* R, size_t b, const Fr* h_alpha, Fr gamma_v, 
 }
 
 __global__ void k_reverse(const Fr* src, size_t b, Fr* dst) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < b) st_fe(&dst[i], ld_fe(&src[b - 1 - i]));
 }
 
 // numerator = f - (z^b - alpha) q - g(z), with q the n - b coefficients.
 __global__ void k_numerator(const Fr* f, const Fr* q, size_t n, size_t nq, Fr c, Fr gz, Fr* out) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   Fr v = ld_fe(&f[i]);
@@ -362,6 +380,7 @@ __global__ void k_numerator(const Fr* f, const Fr* q, size_t n, size_t nq, Fr c,
 // Unreduced sums: 16 columns of 2^22 998 -> 664 us on a GB300.
 __global__ void __launch_bounds__(256) k_combine_stacked(const Fr* const* cols, const Fr* w, int nstacks, size_t maxlen, int width,
                                   size_t n, Fr* out) {
+  chain_begin();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const size_t slot = i >> width, row = i & (((size_t)1 << width) - 1);
@@ -380,6 +399,7 @@ __global__ void __launch_bounds__(256) k_combine_stacked(const Fr* const* cols, 
 
 // The remainders x[0 .. n) of exact divisions.
 __global__ void k_expect_zero(const Fr* x, uint32_t* flags) {
+  chain_begin();
   if (!fe_is_zero(ld_fe(&x[threadIdx.x]))) atomicOr(flags, (uint32_t)DEV_NONZERO_REM);
 }
 
@@ -424,7 +444,7 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
       p = host::fsqr(p);
     }
     const unsigned threads = (unsigned)std::max<size_t>(32, (count + 31) / 32 * 32);
-    launch(c, k_suffix_scan, (unsigned)cols, threads, 0, in, out, stride, (int)count, pows);
+    launch_chained(c, k_suffix_scan, (unsigned)cols, threads, 0, in, out, stride, (int)count, pows);
     return;
   }
   const int L = count * cols >= ((size_t)1 << 20) ? kSuffixMax : 8;
@@ -433,7 +453,7 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
   // recursion level owns its own.
   Fr* agg;
   APG_CUDA(cudaMallocAsync((void**)&agg, 32 * nseg * cols, c.stream));
-  launch(c, k_suffix_local, nb(nseg * cols, 128), 128, 0, in, out, stride, count, cols, L, dv(r), agg);
+  launch_chained(c, k_suffix_local, nb(nseg * cols, 128), 128, 0, in, out, stride, count, cols, L, dv(r), agg);
   if (nseg > 1) {
     F p = host::fone();
     for (int k = 0; k <= L; ++k) {
@@ -442,7 +462,7 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
     }
     F rL = host::fpow_u64(r, L);
     suffix_horner(c, agg, agg, cols, nseg, cols, rL);
-    launch(c, k_suffix_fix, nb(count * cols, 256), 256, 0, out, stride, count, cols, L, (const Fr*)agg, pows);
+    launch_chained(c, k_suffix_fix, nb(count * cols, 256), 256, 0, out, stride, count, cols, L, (const Fr*)agg, pows);
   }
   APG_CUDA(cudaFreeAsync(agg, c.stream));
 }
@@ -464,7 +484,7 @@ void eval_polys(Ctx& c, int n, const Fr* const* poly, const size_t* len, const F
       p = host::fsqr(p);
     }
   }
-  launch(c, k_eval, (unsigned)n, 256, 0, E, (uint32_t)run, out);
+  launch_chained(c, k_eval, (unsigned)n, 256, 0, E, (uint32_t)run, out);
 }
 
 F two_adic_root() {
@@ -486,7 +506,7 @@ const Fr* twiddles(Ctx& c, int log_m) {
     for (int i = log_m; i < 28; ++i) w = host::fsqr(w);
     const size_t half = (size_t)1 << (log_m - 1);
     Fr* tw = b.as<Fr>(half);
-    launch(c, k_powers, nb(half, 256), 256, 0, dv(w), half, tw);
+    launch_chained(c, k_powers, nb(half, 256), 256, 0, dv(w), half, tw);
   }
   return static_cast<const Fr*>(b.p);
 }
@@ -494,8 +514,8 @@ const Fr* twiddles(Ctx& c, int log_m) {
 void fft_inplace(Ctx& c, Fr* a, size_t m, const Fr* tw) {
   int bits = 0;
   while (((size_t)1 << bits) < m) ++bits;
-  launch(c, k_bitrev, nb(m, 256), 256, 0, a, m, bits);
-  for (size_t half = 1; half < m; half *= 2) launch(c, k_fft_stage, nb(m / 2, 256), 256, 0, a, m, half, tw);
+  launch_chained(c, k_bitrev, nb(m, 256), 256, 0, a, m, bits);
+  for (size_t half = 1; half < m; half *= 2) launch_chained(c, k_fft_stage, nb(m / 2, 256), 256, 0, a, m, half, tw);
 }
 
 // ---- univariate helpers on the host (O(b), crates/pcs-verify/src/uni.rs) -------
@@ -927,8 +947,8 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   // Step 1: h, v. The claim goes into the transcript while h is committed.
   build_eq_table(c, u1, eq1);
   build_eq_table(c, u2, eq2);
-  launch(c, k_row_dot, nb(b * 32, 256), 256, 0, (const Fr* const*)nullptr, d_f, (const Fr*)eq1, b, b, h);
-  launch(c, k_dot, 1, 256, 0, (const Fr*)eq2, (const Fr*)h, b, tmp);
+  launch_chained(c, k_row_dot, nb(b * 32, 256), 256, 0, (const Fr* const*)nullptr, d_f, (const Fr*)eq1, b, b, h);
+  launch_chained(c, k_dot, 1, 256, 0, (const Fr*)eq2, (const Fr*)h, b, tmp);
   const uint32_t v_there = publish_checked(c, tmp, 32);
   uint8_t pts[8][64];
   const uint8_t* d_pts = srs_commit_start(c, h, b);
@@ -975,27 +995,27 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
       const size_t smem = 32 * m;
       APG_CUDA(cudaFuncSetAttribute(k_sym_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)kFftBlockMax));
       APG_CUDA(cudaFuncSetAttribute(k_sym_ifft, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)kFftBlockMax));
-      launch(c, k_sym_fft, 4, threads, smem, SymOperands{{g, eq1, h, eq2}}, b, k, tws, TG);
-      launch(c, k_sym_ifft, 1, threads, smem, (const Fr*)TG, b, k, tws, dv(gamma), dv(finv(from_u64(m))),
+      launch_chained(c, k_sym_fft, 4, threads, smem, SymOperands{{g, eq1, h, eq2}}, b, k, tws, TG);
+      launch_chained(c, k_sym_ifft, 1, threads, smem, (const Fr*)TG, b, k, tws, dv(gamma), dv(finv(from_u64(m))),
              (const Fr*)d_halpha, gamma_v, (const Fr*)g, S, D, c.d_flags);
     } else {
       F w = two_adic_root();
       for (int i = k; i < 28; ++i) w = fsqr(w);
-      launch(c, k_sym_pad, nb(m, 256), 256, 0, (const Fr*)g, (const Fr*)eq1, (const Fr*)h, (const Fr*)eq2, b, TG, TP1,
+      launch_chained(c, k_sym_pad, nb(m, 256), 256, 0, (const Fr*)g, (const Fr*)eq1, (const Fr*)h, (const Fr*)eq2, b, TG, TP1,
              TH, TP2);
-      launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(w), m / 2, tw);
+      launch_chained(c, k_powers, nb(m / 2, 256), 256, 0, dv(w), m / 2, tw);
       fft_inplace(c, TG, m, tw);
       fft_inplace(c, TP1, m, tw);
       fft_inplace(c, TH, m, tw);
       fft_inplace(c, TP2, m, tw);
-      launch(c, k_sym_mix, nb(m, 256), 256, 0, (const Fr*)TG, (const Fr*)TP1, (const Fr*)TH, (const Fr*)TP2, m,
+      launch_chained(c, k_sym_mix, nb(m, 256), 256, 0, (const Fr*)TG, (const Fr*)TP1, (const Fr*)TH, (const Fr*)TP2, m,
              dv(gamma), TG);
-      launch(c, k_powers, nb(m / 2, 256), 256, 0, dv(finv(w)), m / 2, tw);
+      launch_chained(c, k_powers, nb(m / 2, 256), 256, 0, dv(finv(w)), m / 2, tw);
       fft_inplace(c, TG, m, tw);
-      launch(c, k_scale, nb(m, 256), 256, 0, TG, m, dv(finv(from_u64(m))));
-      launch(c, k_sym_out, nb(b, 256), 256, 0, (const Fr*)TG, b, (const Fr*)d_halpha, gamma_v, S,
+      launch_chained(c, k_scale, nb(m, 256), 256, 0, TG, m, dv(finv(from_u64(m))));
+      launch_chained(c, k_sym_out, nb(b, 256), 256, 0, (const Fr*)TG, b, (const Fr*)d_halpha, gamma_v, S,
              c.d_flags);
-      launch(c, k_reverse, nb(b, 256), 256, 0, (const Fr*)g, b, D);
+      launch_chained(c, k_reverse, nb(b, 256), 256, 0, (const Fr*)g, b, D);
     }
   }
   d_pts = srs_commit_start(c, S, b - 1, D, b);
@@ -1023,11 +1043,11 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   const F h_alpha = evs[0];
   const F* ev = evs.data() + 1;
   F zb = fpow_u64(z, b);
-  launch(c, k_numerator, nb(n, 256), 256, 0, d_f, q, n, nq, dv(fsub(zb, alpha)), dv(ev[0]), num);
+  launch_chained(c, k_numerator, nb(n, 256), 256, 0, d_f, q, n, nq, dv(fsub(zb, alpha)), dv(ev[0]), num);
   tp = c.timer_begin();
   suffix_horner(c, num, num, 1, n, 1, z);
   c.timer_end(APG_TIMER_MERCURY_PASS, tp);
-  launch(c, k_expect_zero, 1, 1, 0, (const Fr*)num, c.d_flags);  // the remainder f(z) - ... = 0
+  launch_chained(c, k_expect_zero, 1, 1, 0, (const Fr*)num, c.d_flags);  // the remainder f(z) - ... = 0
   d_pts = srs_commit_start(c, num + 1, n - 1);
   tr.absorb(T_PCS_OPENING, ev, 6);
   tr.open(T_PCS_OPENING, 4);
@@ -1067,9 +1087,9 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   }
   for (int k = 0; k < 5; ++k) B.low[k] = dv(low[k]);
   Fr* dF = TH;  // reuse a transform buffer (2b >= b + 2)
-  launch(c, k_bdfg, nb(b + 2, 256), 256, 0, B, (uint32_t)(b + 2), dF);
+  launch_chained(c, k_bdfg, nb(b + 2, 256), 256, 0, B, (uint32_t)(b + 2), dF);
   for (int r = 0; r < 3; ++r) suffix_horner(c, dF + r, dF + r, 1, b + 2 - r, 1, tset[r]);
-  launch(c, k_expect_zero, 1, 3, 0, (const Fr*)dF, c.d_flags);
+  launch_chained(c, k_expect_zero, 1, 3, 0, (const Fr*)dF, c.d_flags);
   const Fr* dW = dF + 3;
   d_pts = srs_commit_start(c, dW, b - 1);
   tr.open(T_PCS_OPENING, 4);
@@ -1093,9 +1113,9 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   B.mul[4][0] = dv(fneg(ueval(uvanishing(tset), zp)));
   B.low[0] = dv(fneg(cst));
   Fr* dL = TP2;
-  launch(c, k_bdfg, nb(b, 256), 256, 0, B, (uint32_t)b, dL);
+  launch_chained(c, k_bdfg, nb(b, 256), 256, 0, B, (uint32_t)b, dL);
   suffix_horner(c, dL, dL, 1, b, 1, zp);
-  launch(c, k_expect_zero, 1, 1, 0, (const Fr*)dL, c.d_flags);
+  launch_chained(c, k_expect_zero, 1, 1, 0, (const Fr*)dL, c.d_flags);
   d_pts = srs_commit_start(c, dL + 1, b - 1);
   tr.open(T_PCS_OPENING, 4);
   fetch_checked(c, d_pts, 64, pts[7]);
@@ -1152,9 +1172,9 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   APG_CUDA(cudaMemcpyAsync(d_table, table.data(), sizeof(Fr*) * table.size(), cudaMemcpyHostToDevice, c.stream));
   for (size_t c0 = 0; c0 < ncols; c0 += 32768) {
     const unsigned cn = (unsigned)std::min<size_t>(32768, ncols - c0);
-    launch(c, k_row_dot, dim3(nb(b2 * 32, 256), cn), 256, 0, (const Fr* const*)(d_table + c0), (const Fr*)nullptr,
+    launch_chained(c, k_row_dot, dim3(nb(b2 * 32, 256), cn), 256, 0, (const Fr* const*)(d_table + c0), (const Fr*)nullptr,
            (const Fr*)eq1, b1, b2, h + c0 * b2);
-    launch(c, k_dot, cn, 256, 0, (const Fr*)eq2, (const Fr*)(h + c0 * b2), b2, cv + c0);
+    launch_chained(c, k_dot, cn, 256, 0, (const Fr*)eq2, (const Fr*)(h + c0 * b2), b2, cv + c0);
   }
   tr.absorb_g1(T_COMMITMENT, cms, nstacks);  // (while the columns are evaluated)
   const std::vector<F> vals = read_frs(c, cv, ncols);
@@ -1185,7 +1205,7 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   Affine* d_cms = c.scratch[S_BASES].as<Affine>(nstacks);
   upload_points(c, cms, nstacks, d_cms);
   APG_CUDA(cudaMemcpyAsync(w, wts.data(), 32 * nstacks, cudaMemcpyHostToDevice, c.stream));
-  launch(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)(d_table + ncols), (const Fr*)w, (int)nstacks, maxlen,
+  launch_chained(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)(d_table + ncols), (const Fr*)w, (int)nstacks, maxlen,
          (int)width, n, fstar);
   uint8_t cm_star[64];
   if (nstacks <= kHostMsmMax)

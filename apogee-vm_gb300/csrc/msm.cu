@@ -96,6 +96,7 @@ __global__ void k_points_out(const Affine* src, size_t n, uint4* raw) {
 // flag the host waits for.
 __global__ void __launch_bounds__(512) k_publish(const uint4* src, uint32_t n, const uint32_t* err, uint4* dst,
                                                  uint32_t* head, uint32_t seq) {
+  chain_begin();
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
   if (threadIdx.x == 0) head[1] = *err;
   __threadfence_system();
@@ -219,6 +220,7 @@ constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;  // per thread
 
 __global__ void k_scan_local(uint32_t* data, size_t n, uint32_t* block_sums) {
+  chain_begin();
   __shared__ uint32_t sh[kScanBlock];
   size_t base = (size_t)blockIdx.x * kScanBlock * kScanItems + (size_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
@@ -251,6 +253,7 @@ __global__ void k_scan_local(uint32_t* data, size_t n, uint32_t* block_sums) {
 // needs no such launch.
 __global__ void __launch_bounds__(256) k_scan_add(uint32_t* data, size_t n, const uint32_t* block_sums,
                                                   uint32_t* total_out) {
+  chain_begin();
   __shared__ uint32_t part[8];
   uint32_t before = 0;
   for (unsigned b = threadIdx.x; b < blockIdx.x; b += 256) before += block_sums[b];
@@ -372,6 +375,7 @@ __global__ void __launch_bounds__(4 * kFoldQuads, BLOCKS) k_fold_edges(const uin
                                                                const uint8_t* pres, size_t len, int per,
                                                                Xyzz* buckets, uint32_t* okeys, Xyzz* opts,
                                                                uint8_t* opres) {
+  chain_begin();
   __shared__ Fq sv[4 * kFoldQuads];
   __shared__ uint32_t skey[kFoldQuads];
   __shared__ uint8_t slive[kFoldQuads], spres[kFoldQuads];
@@ -506,6 +510,7 @@ constexpr int kReduceQuads = 64;  // a block at most: two warps a scheduler (see
 template <int BLOCKS>
 __global__ void __launch_bounds__(4 * kReduceQuads, BLOCKS) k_reduce(const Xyzz* R, const Xyzz* T, int M, int lf, int scale,
                                                              int last, Xyzz* outT, Xyzz* outR) {
+  chain_begin();
   extern __shared__ uint4 sm_points[];
   Fq* sh = reinterpret_cast<Fq*>(sm_points);
   const int l = threadIdx.x & 3, q = threadIdx.x >> 2, Q = blockDim.x >> 2, sp = blockIdx.y;
@@ -558,6 +563,7 @@ __global__ void __launch_bounds__(4 * kReduceQuads, BLOCKS) k_reduce(const Xyzz*
 // over a quad (2,484 points: 1243 -> 522 us).
 __global__ void __launch_bounds__(32) k_finish(const Xyzz* tsum, int spaces, int c, uint32_t* out64,
                                                uint32_t* flags) {
+  chain_begin();
   const int lane = threadIdx.x & 31, l = lane & 3;
   const Xyzz* in = tsum + (size_t)blockIdx.x * spaces;
   Fq total = quad_ld(&in[spaces - 1], l);
@@ -789,6 +795,7 @@ template <bool SMALL, bool SCATTER>
 __global__ void __launch_bounds__(kDigitThreads) k_digits(MsmCols cols, int c, int windows, int precomp,
                                                           uint32_t stride, uint32_t tab_n, int canonical_in,
                                                           uint32_t* cursor, uint32_t* sorted, uint32_t* flags) {
+  chain_begin();
   __shared__ uint32_t wide[SMALL ? 1 : 9][kDigitThreads];  // limbs, then the place in the block and the carry
   __shared__ uint32_t nwide;
   const uint32_t col = blockIdx.y;
@@ -883,6 +890,7 @@ template <bool SMALL, bool SCATTER>
 __global__ void __launch_bounds__(256) k_digits_few(MsmCols cols, int c, int windows, int precomp, uint32_t stride,
                                                     uint32_t tab_n, int canonical_in, uint32_t tile, uint32_t* cursor,
                                                     uint32_t* sorted, uint32_t* flags) {
+  chain_begin();
   extern __shared__ uint32_t bins[];
   const uint32_t col = blockIdx.y;
   const uint32_t n = cols.len[col];
@@ -955,6 +963,7 @@ __global__ void __launch_bounds__(128, APG_ACC_MIN_BLOCKS) k_bucket_acc(const ui
                                                     Xyzz* buckets, uint32_t* okeys, Xyzz* opts, uint8_t* opres,
                                                     const uint32_t* mode, const uint32_t* pair_ends,
                                                     const Affine* pair_pts) {
+  chain_begin();
   const size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (s >= nseg) return;
   const bool direct = mode && *mode == 0;
@@ -1672,11 +1681,15 @@ inline unsigned blocks_for(size_t n, int threads) {
 // Host side
 // ---------------------------------------------------------------------------
 
-uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes) {
+uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes, bool chained) {
   uint8_t* pinned = c.host_pinned();
   if (bytes > Ctx::kPinnedBytes - Ctx::kPinnedTables || bytes % 16) throw Error(APG_ERR_INTERNAL, "an odd result");
-  launch(c, k_publish, 1, 512, 0, (const uint4*)d_src, (uint32_t)(bytes / 16), (const uint32_t*)c.d_flags,
-         reinterpret_cast<uint4*>(pinned + Ctx::kPinnedTables), reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
+  auto go = [&](auto... args) {
+    if (chained) launch_chained(c, k_publish, 1, 512, 0, args...);
+    else launch(c, k_publish, 1, 512, 0, args...);
+  };
+  go((const uint4*)d_src, (uint32_t)(bytes / 16), (const uint32_t*)c.d_flags,
+     reinterpret_cast<uint4*>(pinned + Ctx::kPinnedTables), reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
   return c.flag_seq;
 }
 
@@ -1687,9 +1700,9 @@ void collect_checked(Ctx& c, uint32_t seq, size_t bytes, void* host) {
   if (reinterpret_cast<const uint32_t*>(c.host_pinned())[1]) c.check_flags();  // clears the flags and throws
 }
 
-void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host) {
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host, bool chained) {
   if (bytes <= Ctx::kPinnedBytes - Ctx::kPinnedTables && bytes % 16 == 0) {
-    collect_checked(c, publish_checked(c, d_src, bytes), bytes, host);
+    collect_checked(c, publish_checked(c, d_src, bytes, chained), bytes, host);
     return;
   }
   APG_CUDA(cudaMemcpyAsync(host, d_src, bytes, cudaMemcpyDeviceToHost, c.stream));
@@ -1942,6 +1955,10 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   const int canon = scalars_canonical ? 1 : 0;
   // One pass over the digits: counted (place null) or placed.
   auto digits = [&](uint32_t* place) {
+    auto go = [&](auto k, dim3 grid, int threads, size_t smem, auto... args) {
+      if (place) launch_chained(c, k, grid, threads, smem, args...);
+      else launch(c, k, grid, threads, smem, args...);  // (follows the memset)
+    };
     const uint32_t few = (uint32_t)spaces_per_col * K;
     if (few <= kFewBins) {
       // Tiles of 256 scalars until they fill the device twice, then up to
@@ -1952,21 +1969,20 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
       void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t, uint32_t*, uint32_t*, uint32_t*) =
           small_scalars ? (place ? k_digits_few<true, true> : k_digits_few<true, false>)
                         : (place ? k_digits_few<false, true> : k_digits_few<false, false>);
-      launch(c, k, grid, 256, few * sizeof(uint32_t), cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, 256 * per,
-             counts, place, c.d_flags);
+      go(k, grid, 256, few * sizeof(uint32_t), cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, 256 * per, counts,
+         place, c.d_flags);
     } else {
       const dim3 grid(blocks_for<int>(std::max<size_t>(nmax, 1), kDigitThreads), (unsigned)ncols);
       void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t*, uint32_t*, uint32_t*) =
           small_scalars ? (place ? k_digits<true, true> : k_digits<true, false>)
                         : (place ? k_digits<false, true> : k_digits<false, false>);
-      launch(c, k, grid, kDigitThreads, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place,
-             c.d_flags);
+      go(k, grid, kDigitThreads, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place, c.d_flags);
     }
   };
   digits(nullptr);
-  launch(c, k_scan_local, (unsigned)scan_blocks, kScanBlock, 0, counts, nbins, blk);
+  launch_chained(c, k_scan_local, (unsigned)scan_blocks, kScanBlock, 0, counts, nbins, blk);
   if (scan_blocks > 1)
-    launch(c, k_scan_add, (unsigned)scan_blocks, 256, 0, counts, nbins, (const uint32_t*)blk, total);
+    launch_chained(c, k_scan_add, (unsigned)scan_blocks, 256, 0, counts, nbins, (const uint32_t*)blk, total);
   digits(sorted);
   cudaEvent_t t_acc = c.timer_begin();
   const uint32_t* pair_mode = nullptr;
@@ -1997,8 +2013,8 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
     for (int r = 0; r < kPairRounds; ++r) {
       uint32_t* st = cnt + (size_t)r * scan_n;
       launch(c, k_halve_counts, blocks_for<int>(scan_n, 256), 256, 0, ends_in, (uint32_t)nbins, st);
-      launch(c, k_scan_local, sblocks, kScanBlock, 0, st, scan_n, blk);
-      if (sblocks > 1) launch(c, k_scan_add, sblocks, 256, 0, st, scan_n, (const uint32_t*)blk, mode + 1);
+      launch_chained(c, k_scan_local, sblocks, kScanBlock, 0, st, scan_n, blk);
+      if (sblocks > 1) launch_chained(c, k_scan_add, sblocks, 256, 0, st, scan_n, (const uint32_t*)blk, mode + 1);
       const uint32_t* rr = r == 0 ? (const uint32_t*)sorted : (const uint32_t*)nullptr;
       const Affine* in = r == 0 ? src : lst[(r - 1) & 1];
       if (r == 0) {
@@ -2027,25 +2043,26 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
     pair_ends = ends_in;
     pair_pts = lst[(kPairRounds - 1) & 1];
   }
-  launch(c, k_bucket_acc, blocks_for<int>(nseg, 128), 128, 0, (const uint32_t*)sorted, (const uint32_t*)counts,
+  launch_chained(c, k_bucket_acc, blocks_for<int>(nseg, 128), 128, 0, (const uint32_t*)sorted, (const uint32_t*)counts,
          (uint32_t)nbins, (const uint32_t*)total, nseg, src, buckets, ikeys[0], ipts[0], ipres[0], pair_mode,
          pair_ends, pair_pts);
   c.timer_end(APG_TIMER_MSM_ACCUMULATE, t_acc);
   for (size_t len = 2 * nseg, cur = 0; len > 2; cur ^= 1) {
     const FoldLevel f = fold_level(len);
-    launch(c, tail_kernel(k_fold_edges<1>, k_fold_edges<2>, f.blocks, c.sm_count), f.blocks, 4 * kFoldQuads, 0, (const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur],
-           (const uint8_t*)ipres[cur], len, f.per, buckets, ikeys[cur ^ 1], ipts[cur ^ 1], ipres[cur ^ 1]);
+    launch_chained(c, tail_kernel(k_fold_edges<1>, k_fold_edges<2>, f.blocks, c.sm_count), f.blocks, 4 * kFoldQuads, 0,
+                   (const uint32_t*)ikeys[cur], (const Xyzz*)ipts[cur], (const uint8_t*)ipres[cur], len, f.per, buckets,
+                   ikeys[cur ^ 1], ipts[cur ^ 1], ipres[cur ^ 1]);
     len = 2 * (size_t)f.blocks;
   }
   const bool two_levels = rp.last_scale > 0;
   if (two_levels)
-    launch(c, tail_kernel(k_reduce<1>, k_reduce<2>, (size_t)rp.blocks * S, c.sm_count), dim3(rp.blocks, S),
+    launch_chained(c, tail_kernel(k_reduce<1>, k_reduce<2>, (size_t)rp.blocks * S, c.sm_count), dim3(rp.blocks, S),
            4 * kReduceQuads, reduce_smem(kReduceQuads), (const Xyzz*)buckets,
            (const Xyzz*)nullptr, (int)K, rp.lf, 0, 0, lvlT, lvlR);
-  launch(c, tail_kernel(k_reduce<1>, k_reduce<2>, S, c.sm_count), dim3(1, S), 4 * rp.last_quads, reduce_smem(rp.last_quads),
+  launch_chained(c, tail_kernel(k_reduce<1>, k_reduce<2>, S, c.sm_count), dim3(1, S), 4 * rp.last_quads, reduce_smem(rp.last_quads),
          (const Xyzz*)(two_levels ? lvlR : buckets), (const Xyzz*)(two_levels ? lvlT : nullptr), rp.last_m, rp.last_lf,
          rp.last_scale, 1, tsum, (Xyzz*)nullptr);
-  launch(c, k_finish, (unsigned)nout, 32, 0, (const Xyzz*)tsum, spaces_per_col, p.c, (uint32_t*)d_out, c.d_flags);
+  launch_chained(c, k_finish, (unsigned)nout, 32, 0, (const Xyzz*)tsum, spaces_per_col, p.c, (uint32_t*)d_out, c.d_flags);
   c.timer_end(APG_TIMER_MSM_TOTAL, t_total);
 }
 

@@ -319,6 +319,7 @@ __device__ __forceinline__ void form_st(uint4* val, int at, int pp, const Fr& a)
 template <int WARPS, int BLOCKS>
 __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
     k_round_form(RoundArgs A, DevForm F, VirtualRound V, int nshare, int log_pp, int passes, Fr* partials) {
+  chain_begin();
   extern __shared__ uint4 val[];  // node xi of table k, pair i, half q: ((k nn + xi) 2 + q) pp + i
   __shared__ Fr ws[3 * WARPS];
   const int three = (A.nodes >> 1) & 1, nn = 2 + three, pp = 1 << log_pp;
@@ -504,6 +505,7 @@ __global__ void __launch_bounds__(kRoundThreads, APG_ROUND_WARP_MIN_BLOCKS) k_ro
 // One block; the values and then the flag go to pinned host memory.
 __global__ void k_final_bind(const Fr* const* src, const uint8_t* src_bits, const Fr* in_base, size_t in_len,
                              int in_is_src, int nt, Fr c, int no_rounds, Fr* out, uint32_t* flag, uint32_t seq) {
+  chain_begin();
   for (int k = threadIdx.x; k < nt; k += blockDim.x) {
     const Fr* t = in_is_src ? src[k] : in_base + (size_t)k * in_len;
     const int bits = in_is_src && src_bits ? src_bits[k] : 0;
@@ -524,6 +526,7 @@ __global__ void k_final_bind(const Fr* const* src, const uint8_t* src_bits, cons
 // the flag (one block: the few entries the host takes over).
 __global__ void k_gather(const Fr* const* src, const uint8_t* src_bits, int nt, size_t len, Fr* out, uint32_t* flag,
                          uint32_t seq) {
+  chain_begin();
   for (size_t t = threadIdx.x; t < nt * len; t += blockDim.x) {
     const int k = (int)(t / len);
     const int bits = src_bits ? src_bits[k] : 0;
@@ -553,6 +556,7 @@ constexpr int kEqLow = 10;
 __device__ __forceinline__ Fr eq_factor(const Fr& r, bool bit) { return bit ? r : fe_sub(fe_one<FrConsts>(), r); }
 
 __global__ void __launch_bounds__(256) k_eq_table(const __grid_constant__ EqPoint P, int n, Fr* out) {
+  chain_begin();
   __shared__ Fr tab[2][1 << (kEqLow / 2)], high;
   const int nl = min(n, kEqLow), na = nl / 2, t = threadIdx.x, lane = t & 31;
   if (t < 64) {
@@ -603,7 +607,7 @@ void build_eq_table(Ctx& c, const std::vector<F>& r, Fr* out) {
   if (n > (int)(sizeof(p.r) / sizeof(Fr))) throw Error(APG_ERR_INVALID_ARGUMENT, "an eq table of more than 40 variables");
   memset(&p, 0, sizeof(p));
   if (n) memcpy(p.r, r.data(), 32 * (size_t)n);
-  launch(c, k_eq_table, 1u << std::max(0, n - kEqLow), 256, 0, p, n, out);
+  launch_chained(c, k_eq_table, 1u << std::max(0, n - kEqLow), 256, 0, p, n, out);
 }
 
 static VirtualRound virtual_round(const std::vector<F>& point, int nvars) {
@@ -893,7 +897,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
     cudaEvent_t t0 = c.timer_begin();
     if (use_form) {
       const FormShape f = form_shape(form, A.npairs, n_val, needs_one(r), c.sm_count);
-      launch(c, form_kernel(f.threads), f.blocks, f.threads, f.smem, A, DF, V, f.share, f.log_pp, f.passes, partials);
+      launch_chained(c, form_kernel(f.threads), f.blocks, f.threads, f.smem, A, DF, V, f.share, f.log_pp, f.passes, partials);
     }
     else if (small_warp_ok && A.npairs * 32 <= (size_t)kRoundThreads * c.sm_count * 4)
       launch(c, k_round_warp<true>, (int)((A.npairs + kRoundThreads / 32 - 1) / (kRoundThreads / 32)), kRoundThreads,
@@ -912,7 +916,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
   }
   if (host_rounds > 0) {
     if (dev_rounds == 0) {
-      launch(c, k_gather, 1, 256, 0, (const Fr* const*)d_src, d_bits, nt, len0, host_tables,
+      launch_chained(c, k_gather, 1, 256, 0, (const Fr* const*)d_src, d_bits, nt, len0, host_tables,
              reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
       if (n > 1) invert_coordinates();
       c.wait_flag();
@@ -969,7 +973,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
     const Fr* base = n >= 2 ? lvl[(n - 1) & 1] : nullptr;
     const bool in_pinned = (size_t)nd * 32 <= Ctx::kPinnedBytes - Ctx::kPinnedTables;
     Fr* d_fin = in_pinned ? host_tables : c.scratch[S_TMP7].as<Fr>(nt);
-    launch(c, k_final_bind, 1, 256, 0, (const Fr* const*)d_src, d_bits, base, (size_t)2, n <= 1 ? 1 : 0, nd,
+    launch_chained(c, k_final_bind, 1, 256, 0, (const Fr* const*)d_src, d_bits, base, (size_t)2, n <= 1 ? 1 : 0, nd,
            to_dev(chal), n == 0 ? 1 : 0, d_fin, reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
     if (!in_pinned)
       APG_CUDA(cudaMemcpyAsync(finals.data(), d_fin, 32 * (size_t)nd, cudaMemcpyDeviceToHost, c.stream));
