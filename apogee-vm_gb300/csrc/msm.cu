@@ -1931,7 +1931,7 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
 
   const size_t scan_blocks = (nbins + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
   uint32_t* blk = c.scratch[S_SCANBLK].as<uint32_t>(kScanBlock + 1);
-  uint32_t* total = scan_blocks > 1 ? blk + kScanBlock : blk;
+  uint32_t* total = blk + kScanBlock;  // (its own word: the pair rounds scan through blk as well)
   uint32_t* sorted = c.scratch[S_SORTED].as<uint32_t>(std::max<size_t>(emax, 1));
   // The buckets and, after them, their counts: what a group must find at zero.
   const size_t zero_bytes = nbins * sizeof(Xyzz) + (nbins + 1) * sizeof(uint32_t);
@@ -1980,7 +1980,7 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
     }
   };
   digits(nullptr);
-  launch_chained(c, k_scan_local, (unsigned)scan_blocks, kScanBlock, 0, counts, nbins, blk);
+  launch_chained(c, k_scan_local, (unsigned)scan_blocks, kScanBlock, 0, counts, nbins, scan_blocks > 1 ? blk : total);
   if (scan_blocks > 1)
     launch_chained(c, k_scan_add, (unsigned)scan_blocks, 256, 0, counts, nbins, (const uint32_t*)blk, total);
   digits(sorted);
