@@ -271,7 +271,8 @@ int apg_srs_prepare(apg_ctx* ctx, int cbits) {
   return guarded(ctx, [&](Ctx& c) {
     if (!c.srs) return (int)APG_ERR_NO_SRS;
     if (cbits == 0) {
-      srs_table(c, 8, std::min(c.srs_n, kNarrowTableMax));
+      for (size_t n : {std::min(c.srs_n, (size_t)1 << 8), std::min(c.srs_n, kNarrowTableMax)})
+        srs_table(c, narrow_window(n), n);
       if (c.srs_n > kNarrowTableMax)
         for (int w : {13, 15}) srs_table(c, w, std::min(c.srs_n, kWideTableMin));
       if (c.srs_n >= kWideTableMin) srs_table(c, 17, c.srs_n);
@@ -1172,11 +1173,12 @@ size_t apg_shard_device_bytes(const apg_shard* sh) {
     size_t b = sh->cols_on_device ? 0 : 32 * n * k;  // the staged columns
     b += gkr_device_bytes_impl(sh->circuit, sh->circuit_len);
     // The commits' two lanes: a group of columns sorts up to 17 windows a
-    // point (4-byte references; 32 below 2^12 points), and the affine pair rounds hold
-    // two point lists and the running products at about half and a quarter
-    // of that (capped as msm.cu caps them), plus buckets and levels.
+    // point (4-byte references; 37 or 43 up to 2^12 points), and the affine
+    // pair rounds hold two point lists and the running products at about half
+    // and a quarter of that (capped as msm.cu caps them), plus buckets and
+    // levels.
     const size_t g = commit_group(k, n);
-    const size_t E = std::min<size_t>((size_t)(n <= kNarrowTableMax ? 32 : 17) * n * g, (size_t)1 << 28);
+    const size_t E = std::min<size_t>((size_t)(n <= kNarrowTableMax ? 43 : 17) * n * g, (size_t)1 << 28);
     const size_t cap = (size_t)48 << 20;
     size_t lane = 4 * E + ((size_t)96 << 20);
     if (E >= ((size_t)1 << 21))

@@ -313,13 +313,15 @@ void msm_device(Ctx& c, const Affine* bases, const SrsTable* table, const void* 
                 bool scalars_canonical, size_t n, uint8_t* out64_device, uint8_t* host_out,
                 const MsmBatchOpts& o = MsmBatchOpts());
 const SrsTable* srs_table(Ctx& c, int cbits, size_t need);
-// The table that `cols` MSMs over the first n SRS powers read together: 8-bit
-// windows up to 2^12 points (a cheap bucket reduction), 17-bit windows from
-// kWideTableMin, and between them 15-bit windows for one or two columns and
-// 13-bit ones for more, which pay the reduction of each column's buckets. 15 and
-// 17 divide the 255 bits of a signed scalar (17 and 15 windows: 16 and 18 bits
-// take as many digits over twice the buckets). Measured on a GB300, us: one
-// 2^12-point column 244 at 8 bits, 279 at 13; 2^16 alone 395 at 13, 401 at 15
+// The table that `cols` MSMs over the first n SRS powers read together: 6-bit
+// windows up to 2^8 points and 7-bit ones up to 2^12 (a short bucket reduction),
+// 17-bit windows from kWideTableMin, and between them 15-bit windows for one or two
+// columns and 13-bit ones for more, which pay the reduction of each column's buckets.
+// 15 and 17 divide the 255 bits of a signed scalar (17 and 15 windows: 16 and 18 bits
+// take as many digits over twice the buckets). Measured on a GB300, us: four 2^8-point
+// columns 138 at 6 bits, 146 at 7, 156 at 8 (uniform 165, 172, 168); four of 2^10 167,
+// 161, 166 (205, 188, 193); one of 2^12 169, 158, 166 and 223 at 13 (uniform 205, 184,
+// 191, 248); 2^16 alone 395 at 13, 401 at 15
 // (uniform 578, 532), sixteen 1509, 1711 (uniform 3420, 3496); sixteen of 2^14
 // 930, 1140; sixteen of 2^18 3654 at 13, 4114 at 17, uniform 12024, 10675; 2^20
 // alone 1394 at 17, 1402 at 16, 1881 at 20 (uniform 3142, 3254, 3453); 2^22 3264
@@ -328,6 +330,7 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need);
 // (commits of the caller's columns); openings commit uniformly random
 // quotient polynomials, for which the default rule is the uniform-scalar one.
 constexpr size_t kNarrowTableMax = (size_t)1 << 12;
+constexpr int narrow_window(size_t n) { return n <= ((size_t)1 << 8) ? 6 : 7; }
 constexpr size_t kWideTableMin = (size_t)1 << 18;
 const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned = true);
 // Time SRS commits of the first 2^k sample scalars for k in [kmin, kmax] with

@@ -1772,7 +1772,7 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need) {
   // A wide table covers the whole SRS, a narrower one the prefix that the
   // default rule reads it for until a caller needs more. The prefix's table is
   // then kept until the SRS goes: contexts that share it may still read it.
-  size_t n = cbits >= 16 ? c.srs_n : std::min(c.srs_n, cbits >= 12 ? kWideTableMin : (size_t)1 << 16);
+  size_t n = cbits >= 16 ? c.srs_n : std::min(c.srs_n, cbits >= 12 ? kWideTableMin : (size_t)1 << (cbits >= 7 ? 16 : 12));
   if (n < need) n = c.srs_n;
   for (auto it = c.tables.begin(); it != c.tables.end(); ++it)
     if (it->c == cbits) {
@@ -1807,7 +1807,7 @@ const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned) {
     if (t) return t;
   }
   if (n <= kNarrowTableMax) {
-    const SrsTable* t = srs_table(c, 8, n);
+    const SrsTable* t = srs_table(c, narrow_window(n), n);
     if (t) return t;
   }
   return srs_table(c, n >= kWideTableMin ? 17 : cols <= 2 ? 15 : 13, n);

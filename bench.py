@@ -84,10 +84,10 @@ def algorithmic_fqmul_accumulate(n):
 def own_windows(n, tuned=None):
     """Signed-digit windows of the SRS window table an n-point commit reads:
     the autotuner's width for the size class when it chose one, else the
-    library's default rule for one column (8-bit up to 2^12 points, 15-bit
-    below 2^18, 17-bit from 2^18)."""
+    library's default rule for one column (6-bit up to 2^8 points, 7-bit up
+    to 2^12, 15-bit below 2^18, 17-bit from 2^18)."""
     lg = max(0, (n - 1).bit_length())
-    c = (tuned or {}).get(lg) or (8 if n <= 1 << 12 else (15 if n < 1 << 18 else 17))
+    c = (tuned or {}).get(lg) or (6 if n <= 1 << 8 else 7 if n <= 1 << 12 else 15 if n < 1 << 18 else 17)
     return -(-255 // c)
 
 
