@@ -125,24 +125,46 @@ __global__ void k_suffix_fix(Fr* out, size_t stride, size_t count, size_t cols, 
   st_fe(p, fe_add(ld_fe(p), fe_mul(pows.p[next - j], carry)));
 }
 
-// A column of up to 1024 positions by one block, a thread a position:
-// acc_j += r^(2^s) acc_{j + 2^s} for s = 0, 1, ..., log2(count) products after one
-// another instead of a segment's length and a level's launches.
+// A column of up to 1024 positions by one block: a thread runs Horner over its R
+// positions, the threads' sums are scanned (acc_t += r^(R 2^s) acc_{t + 2^s} for s = 0,
+// 1, ...) and what follows a thread's positions is added to them. One position a thread
+// up to 256; four above, where a step over all positions would be eight warps a
+// scheduler (1024 positions: 28 us, four a thread 14). pows holds r^(2^s), then r^3.
 constexpr size_t kSuffixScanMax = 1024;
-__global__ void __launch_bounds__(1024) k_suffix_scan(const Fr* in, Fr* out, size_t stride, int count,
-                                                      const __grid_constant__ SuffixPowers pows) {
+constexpr int kSuffixCube = 11;
+template <int R>
+__global__ void __launch_bounds__(256) k_suffix_scan(const Fr* in, Fr* out, size_t stride, int count,
+                                                     const __grid_constant__ SuffixPowers pows) {
   chain_begin();
-  __shared__ Fr sh[kSuffixScanMax];
-  const int j = threadIdx.x;
-  const size_t at = j * stride + blockIdx.x;
-  Fr acc = j < count ? ld_fe(&in[at]) : fe_zero<FrConsts>();
-  for (int s = 0, off = 1; off < count; ++s, off <<= 1) {
-    sh[j] = acc;
+  __shared__ Fr sh[257];
+  const int t = threadIdx.x, j = t * R;
+  Fr a[R];
+#pragma unroll
+  for (int i = R - 1; i >= 0; --i) {
+    a[i] = j + i < count ? ld_fe(&in[(j + i) * stride + blockIdx.x]) : fe_zero<FrConsts>();
+    if (i + 1 < R) a[i] = fe_add(a[i], rmul(pows.p[0], a[i + 1]));
+  }
+  Fr acc = a[0];
+  for (int s = R == 4 ? 2 : 0, off = 1; off * R < count; ++s, off <<= 1) {
+    sh[t] = acc;
     __syncthreads();
-    if (j + off < count) acc = fe_add(acc, fe_mul(pows.p[s], sh[j + off]));
+    if (j + off * R < count) acc = fe_add(acc, rmul(pows.p[s], sh[t + off]));
     __syncthreads();
   }
-  if (j < count) st_fe(&out[at], acc);
+  if (R == 1) {
+    if (j < count) st_fe(&out[j * stride + blockIdx.x], acc);
+    return;
+  }
+  sh[t] = acc;
+  __syncthreads();
+  const bool more = j + R < count;
+  const Fr next = more ? sh[t + 1] : fe_zero<FrConsts>();
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int k = R - i;  // r^k: 4 and 2 are in the list, 3 at its end
+    if (i > 0 && more) a[i] = fe_add(a[i], rmul(pows.p[k == 3 ? kSuffixCube : k == 2 ? 1 : 0], next));
+    if (j + i < count) st_fe(&out[(j + i) * stride + blockIdx.x], i == 0 ? acc : a[i]);
+  }
 }
 
 // out[i] = base^i.
@@ -443,8 +465,10 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
       pows.p[s] = dv(p);
       p = host::fsqr(p);
     }
-    const unsigned threads = (unsigned)std::max<size_t>(32, (count + 31) / 32 * 32);
-    launch_chained(c, k_suffix_scan, (unsigned)cols, threads, 0, in, out, stride, (int)count, pows);
+    pows.p[kSuffixCube] = dv(host::fmul(host::fsqr(r), r));
+    const size_t per = count > 256 ? 4 : 1, threads = ((count + per - 1) / per + 31) / 32 * 32;
+    launch_chained(c, per == 4 ? k_suffix_scan<4> : k_suffix_scan<1>, (unsigned)cols, (unsigned)threads, 0, in, out,
+                   stride, (int)count, pows);
     return;
   }
   const int L = count * cols >= ((size_t)1 << 20) ? kSuffixMax : 8;

@@ -22,7 +22,7 @@ def ctx():
         yield c
 
 
-@pytest.mark.parametrize("nv,k", [(2, 1), (4, 17), (8, 31), (14, 2), (18, 16), (20, 1), (22, 1), (24, 1)])
+@pytest.mark.parametrize("nv,k", [(2, 1), (4, 17), (8, 31), (14, 2), (16, 3), (18, 16), (20, 1), (22, 1), (24, 1)])
 def test_openings_verify(ctx, nv, k):
     import torch
 
