@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(4 * kFoldQuads, BLOCKS) k_fold_edges(const uin
                                                                Xyzz* buckets, uint32_t* okeys, Xyzz* opts,
                                                                uint8_t* opres) {
   chain_begin();
-  __shared__ Fq sv[4 * kFoldQuads];
+  __shared__ __align__(16) Fq sv[4 * kFoldQuads];  // (read and written 16 bytes at a time)
   __shared__ uint32_t skey[kFoldQuads];
   __shared__ uint8_t slive[kFoldQuads], spres[kFoldQuads];
   const int l = threadIdx.x & 3, i = threadIdx.x >> 2;
