@@ -223,7 +223,7 @@ inline F pow5_2p(const F& x) {
   return fmul_r(fmul_r(x2, x2, false), x, false);
 }
 
-inline void permute(F s[3]) {
+__attribute__((always_inline)) inline void permute(F s[3]) {
   auto full_mix = [&]() {
     F t = fadd_2p(fadd_2p(s[0], s[1]), s[2]);
     for (int j = 0; j < 3; ++j) s[j] = fadd_2p(s[j], t);
@@ -282,7 +282,10 @@ struct Transcript {
   F out[2] = {fzero(), fzero()};
   int out_len = 0;
 
-  void duplex() {
+  // One copy a translation unit, the permutation inside it: left to itself the compiler
+  // cloned and split it by its callers (absorbing 2^18 elements 984 ms with a GKR proof
+  // around it, 784 so; a 2^16-row zerocheck 0.69 -> 0.68 ms).
+  __attribute__((noinline)) void duplex() {
     const int pending = in_len;
     for (int i = 0; i < pending; ++i) {
       st[i] = in[i];

@@ -37,7 +37,7 @@ METRIC = "G1 MSM points/s at 2^22"
 UNIT = "points/s"
 SEED = 20260903
 TAU_SEED = 0x7A75_5EED
-TUNE_WIDTHS = (8, 13, 15, 17, 20)  # window widths the autotuner tries per size class
+TUNE_WIDTHS = (7, 13, 15, 17, 20)  # window widths the autotuner tries per size class
 
 
 def max_over_ranks(x: float, dist, device: str) -> float:
