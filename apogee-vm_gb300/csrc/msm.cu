@@ -1682,10 +1682,15 @@ inline FoldLevel fold_level(size_t len) {
 }
 
 // k_reduce's levels over S spaces of K buckets (a power of two): one block a
-// space for up to 256 buckets; above that a first level of blocks of 64 quads,
-// four buckets a quad while that fits the device (more as the spaces grow past
-// four blocks an SM: the scan's additions are then work, not latency) and then
-// one block a space over the blocks' results.
+// space for up to 256 buckets; above that a first level of blocks of 64 quads, 2^lf
+// buckets a quad, and then one block a space over the blocks' results. lf weighs a
+// block's chain, 2^(lf + 1) additions for its runs and 12 for the scan and the tree,
+// against how many blocks an SM has after one another: an addition takes 2.3 us in a
+// block that has its SM to itself and 2.0 for each block where there are more (at
+// 2^16 buckets: 64 against 80 us for one space at three and two bits, for four spaces
+// 175, 176 and 224 at five, four and three, for seven 264 at four and 304 at five;
+// four a quad while that fitted four blocks an SM: one 2^18-point column 517 -> 489
+// us, four 1249 -> 1192, one of 2^14 264 -> 258, one-byte pairs of 2^20 517 -> 489).
 constexpr uint32_t kReduceOneBlock = 256;
 struct ReducePlan {
   unsigned blocks = 1;  // a space, in the first level (last_scale 0: no such level)
@@ -1696,9 +1701,17 @@ inline ReducePlan reduce_plan(uint32_t K, int S, int sm_count) {
   ReducePlan p;
   p.last_m = (int)K;
   if (K > kReduceOneBlock) {
-    p.lf = 2;
     auto blocks = [&](int lf) { return K / ((uint32_t)kReduceQuads << lf); };
-    while (blocks(p.lf) > 1 && ((size_t)S * blocks(p.lf) > (size_t)sm_count * 4 || blocks(p.lf) > 1024u)) ++p.lf;
+    size_t best = 0;
+    for (int lf = 1; blocks(lf) >= 1; ++lf) {
+      const size_t all = (size_t)S * blocks(lf), turns = (all + sm_count - 1) / sm_count;
+      const size_t last = std::max<size_t>(1, blocks(lf) / kReduceQuads);  // entries a quad at the end
+      const size_t cost = (((size_t)2 << lf) + 12) * (turns == 1 ? 23 : 20 * turns) + 3 * (last - 1) * 23;
+      if (blocks(lf) <= 1024u && (best == 0 || cost < best)) {
+        best = cost;
+        p.lf = lf;
+      }
+    }
     p.blocks = blocks(p.lf);
     p.last_m = (int)p.blocks;
     for (uint32_t len = (uint32_t)kReduceQuads << p.lf; len > 1; len >>= 1) ++p.last_scale;
