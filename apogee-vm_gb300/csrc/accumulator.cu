@@ -159,10 +159,10 @@ int accumulator_msms(Ctx& c, const uint8_t* sides, const uint8_t* scalars, const
   Fr* d_w = reinterpret_cast<Fr*>(d_meta);
   uint64_t* d_first = reinterpret_cast<uint64_t*>(d_meta + 32 * nchecks);
   Fr* d_cols = c.scratch[S_SCALARS].as<Fr>(2 * n);
-  APG_CUDA(cudaMemcpyAsync(d_s, scalars, 32 * n, cudaMemcpyHostToDevice, c.stream));
-  APG_CUDA(cudaMemcpyAsync(d_side, sides, n, cudaMemcpyHostToDevice, c.stream));
-  APG_CUDA(cudaMemcpyAsync(d_w, w.data(), 32 * nchecks, cudaMemcpyHostToDevice, c.stream));
-  APG_CUDA(cudaMemcpyAsync(d_first, first.data(), 8 * nchecks, cudaMemcpyHostToDevice, c.stream));
+  c.copy(d_s, scalars, 32 * n, cudaMemcpyHostToDevice);
+  c.copy(d_side, sides, n, cudaMemcpyHostToDevice);
+  c.copy(d_w, w.data(), 32 * nchecks, cudaMemcpyHostToDevice);
+  c.copy(d_first, first.data(), 8 * nchecks, cudaMemcpyHostToDevice);
   const unsigned blocks = (unsigned)((n + 255) / 256);
   launch(c, k_side_scalars, blocks, 256, 0, (const Fr*)d_s, (const uint8_t*)d_side, n, (const uint64_t*)d_first,
          (int)nchecks, (const Fr*)d_w, d_cols, d_cols + n);
@@ -171,7 +171,7 @@ int accumulator_msms(Ctx& c, const uint8_t* sides, const uint8_t* scalars, const
   uint8_t* d_out = c.scratch[S_RESULT].as<uint8_t>(128);
   msm_multi(c, d_pts, nullptr, cols, lens, 2, false, false, d_out);
   uint8_t* h = c.host_pinned() + Ctx::kPinnedTables;
-  APG_CUDA(cudaMemcpyAsync(h, d_out, 128, cudaMemcpyDeviceToHost, c.stream));
+  c.copy(h, d_out, 128, cudaMemcpyDeviceToHost);
   c.check_flags();
   memcpy(a_out, h, 64);
   memcpy(b_out, h + 64, 64);

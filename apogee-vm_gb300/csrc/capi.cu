@@ -37,6 +37,7 @@ int guarded(apg_ctx* ctx, F&& f) {
   std::lock_guard<std::mutex> lock(ctx->c.mu);
   try {
     APG_CUDA(cudaSetDevice(ctx->c.device));
+    ctx->c.after_kernel = false;
     int st = f(ctx->c);
     if (st == APG_OK) ctx->c.last_error.clear();
     return st;
@@ -68,7 +69,7 @@ int commit_common(Ctx& c, const void* evals, bool on_device, bool small, size_t 
   const void* d = evals;
   if (!on_device) {
     void* buf = c.scratch[S_SCALARS].get(n * elem);
-    APG_CUDA(cudaMemcpyAsync(buf, evals, n * elem, cudaMemcpyHostToDevice, c.stream));
+    c.copy(buf, evals, n * elem, cudaMemcpyHostToDevice);
     d = buf;
   }
   const SrsTable* t = srs_table_for(c, n, 1);
@@ -92,7 +93,7 @@ int msm_common(Ctx& c, const uint8_t* bases, size_t nb, const void* scalars, siz
   upload_points(c, bases, nb, d_bases);
   const size_t elem = small ? 4 : 32;
   void* d_s = c.scratch[S_SCALARS].get(ns * elem);
-  APG_CUDA(cudaMemcpyAsync(d_s, scalars, ns * elem, cudaMemcpyHostToDevice, c.stream));
+  c.copy(d_s, scalars, ns * elem, cudaMemcpyHostToDevice);
   msm_device(c, d_bases, nullptr, d_s, small, false, nb, nullptr, out);
   return APG_OK;
 }
@@ -354,7 +355,7 @@ static int commit_stack_common(Ctx& c, const void* const* cols, const size_t* nu
   if (!on_device) {
     uint8_t* buf = c.scratch[S_SCALARS].as<uint8_t>(32 * n * k);
     for (size_t j = 0; j < k; ++j) {
-      APG_CUDA(cudaMemcpyAsync(buf + 32 * n * j, cols[j], 32 * n, cudaMemcpyHostToDevice, c.stream));
+      c.copy(buf + 32 * n * j, cols[j], 32 * n, cudaMemcpyHostToDevice);
       ptrs[j] = buf + 32 * n * j;
     }
   }
@@ -395,7 +396,7 @@ int apg_commit_narrow(apg_ctx* ctx, const void* vals, int bits, size_t num_vars,
     }
     const size_t bytes = bits == 1 ? 8 * ((n + 63) / 64) : n * (size_t)bits / 8;
     void* buf = c.scratch[S_SCALARS].get(bytes);
-    APG_CUDA(cudaMemcpyAsync(buf, vals, bytes, cudaMemcpyHostToDevice, c.stream));
+    c.copy(buf, vals, bytes, cudaMemcpyHostToDevice);
     const SrsTable* t = srs_table_for(c, n, 1);
     if (!t) throw Error(APG_ERR_INTERNAL, "no SRS window table");
     const void* ptr = buf;
@@ -494,7 +495,7 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
   cudaEvent_t ev;
   APG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   APG_CUDA(cudaEventRecord(ev, c.stream));
-  APG_CUDA(cudaStreamWaitEvent(L.stream, ev, 0));
+  L.wait_event(ev);
   const size_t ngroups = (k + group - 1) / group;
   std::vector<const void*> ptrs(cols, cols + k);
   std::vector<size_t> lens(k, n);
@@ -520,15 +521,15 @@ static int commit_batch_lanes(Ctx& c, const void* const* cols, bool host, size_t
     Ctx& X = *lanes[gi & 1];
     const size_t m = std::min(group, k - j0);
     const SrsTable* t = srs_table_for(X, n, k);
-    if (host) APG_CUDA(cudaStreamWaitEvent(X.stream, landed[gi], 0));
+    if (host) X.wait_event(landed[gi]);
     msm_multi(X, nullptr, t, ptrs.data() + j0, lens.data() + j0, m, false, false, d_out + 64 * j0);
   }
   for (auto e : landed) cudaEventDestroy(e);
   APG_CUDA(cudaEventRecord(ev, L.stream));
-  APG_CUDA(cudaStreamWaitEvent(c.stream, ev, 0));
+  c.wait_event(ev);
   APG_CUDA(cudaEventDestroy(ev));
   try {
-    fetch_checked(c, d_out, 64 * k, out, false);  // (follows the other lane's event)
+    fetch_checked(c, d_out, 64 * k, out);
   } catch (...) {  // the lane's own flags must not outlive this call
     cudaMemsetAsync(L.d_flags, 0, 4, L.stream);
     cudaStreamSynchronize(L.stream);
@@ -627,7 +628,7 @@ int apg_mercury_open(apg_ctx* ctx, const uint8_t* evals, size_t num_vars, const 
     const size_t n = (size_t)1 << num_vars;
     if (c.srs && c.srs_n < n) return (int)APG_ERR_SRS_TOO_SMALL;
     Fr* d = c.scratch[S_SCALARS].as<Fr>(n);
-    APG_CUDA(cudaMemcpyAsync(d, evals, 32 * n, cudaMemcpyHostToDevice, c.stream));
+    c.copy(d, evals, 32 * n, cudaMemcpyHostToDevice);
     host::F v;
     int st = mercury_open_impl(c, d, num_vars, cm, uu, tr, v, proof_out);
     if (st) return st;
@@ -676,9 +677,9 @@ static int stacked_open_common(Ctx& c, const void* const* cols, bool on_device, 
   if (on_device) {
     for (size_t i = 0; i < ncols; ++i) ptrs[i] = (const Fr*)cols[i];
   } else {
-    APG_CUDA(cudaMallocAsync((void**)&staged, 32 * column * ncols, c.stream));
+    c.alloc(&staged, 32 * column * ncols);
     for (size_t i = 0; i < ncols; ++i) {
-      APG_CUDA(cudaMemcpyAsync(staged + i * column, cols[i], 32 * column, cudaMemcpyHostToDevice, c.stream));
+      c.copy(staged + i * column, cols[i], 32 * column, cudaMemcpyHostToDevice);
       ptrs[i] = staged + i * column;
     }
   }
@@ -1084,9 +1085,9 @@ static int prove_shard_common(Ctx& c, const apg_shard* sh, apg_shard_proof* out)
   Fr* staged = nullptr;
   auto t0 = Clock::now();
   if (!sh->cols_on_device) {
-    APG_CUDA(cudaMallocAsync((void**)&staged, 32 * n * k, c.stream));
+    c.alloc(&staged, 32 * n * k);
     for (size_t j = 0; j < k; ++j) {
-      APG_CUDA(cudaMemcpyAsync(staged + j * n, sh->cols[j], 32 * n, cudaMemcpyHostToDevice, c.stream));
+      c.copy(staged + j * n, sh->cols[j], 32 * n, cudaMemcpyHostToDevice);
       d_cols[j] = staged + j * n;
     }
   }

@@ -173,6 +173,31 @@ struct Ctx {
     std::atomic_thread_fence(std::memory_order_acquire);
   }
 
+  // What goes on the stream beside kernels. A kernel launched as the end of a
+  // chain (launch_chained) waits for the kernel before it; what stands before it
+  // has to be a kernel of this call, so everything else is noted here: copies,
+  // memsets, event waits, allocations in stream order (which may wait for another
+  // stream's release), and a call's beginning (the caller may have queued any of
+  // them on the context's stream).
+  bool after_kernel = false;
+  void copy(void* to, const void* from, size_t bytes, cudaMemcpyKind kind) {
+    after_kernel = false;
+    APG_CUDA(cudaMemcpyAsync(to, from, bytes, kind, stream));
+  }
+  void fill(void* p, int value, size_t bytes) {
+    after_kernel = false;
+    APG_CUDA(cudaMemsetAsync(p, value, bytes, stream));
+  }
+  void wait_event(cudaEvent_t e) {
+    after_kernel = false;
+    APG_CUDA(cudaStreamWaitEvent(stream, e, 0));
+  }
+  template <class T>
+  void alloc(T** p, size_t bytes) {  // (freed by cudaFreeAsync on the stream)
+    after_kernel = false;
+    APG_CUDA(cudaMallocAsync(reinterpret_cast<void**>(p), bytes, stream));
+  }
+
   // Bracket work on the stream with a timer's events (no-op unless enabled).
   cudaEvent_t timer_begin() {
     if (!timers.on) return nullptr;
@@ -189,10 +214,10 @@ struct Ctx {
 
   void check_flags() {
     uint32_t f = 0;
-    APG_CUDA(cudaMemcpyAsync(&f, d_flags, 4, cudaMemcpyDeviceToHost, stream));
+    copy(&f, d_flags, 4, cudaMemcpyDeviceToHost);
     APG_CUDA(cudaStreamSynchronize(stream));
     if (f) {
-      APG_CUDA(cudaMemsetAsync(d_flags, 0, 4, stream));
+      fill(d_flags, 0, 4);
       if (f & DEV_NONCANONICAL) throw Error(APG_ERR_NONCANONICAL, "an input value is not below its modulus");
       if (f & DEV_OFF_CURVE) throw Error(APG_ERR_INVALID_POINT, "an input point is not on the curve");
       if (f & DEV_DEGENERATE) throw Error(APG_ERR_DEGENERATE_CHALLENGE, "degenerate Mercury challenge set");
@@ -217,6 +242,7 @@ inline void launch(Ctx& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size
   }
   kernel<<<grid, block, smem, c.stream>>>(args...);
   APG_CUDA(cudaGetLastError());
+  c.after_kernel = true;
   ++c.launches;
   if (e0) {
     cudaEvent_t e1 = c.timers.get();
@@ -225,16 +251,17 @@ inline void launch(Ctx& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size
   }
 }
 
-// The same for a kernel that begins with chain_begin() and follows another kernel
-// on the stream: its blocks may be set up while that one's last blocks still run
+// The same for a kernel that begins with chain_begin(): where it follows another
+// kernel on the stream, its blocks may be set up while that one's last blocks still run
 // (programmatic stream serialization), and wait there for it to end. Every kernel of a
-// chain waits, so each sees all that stands before it. What follows an event or a
-// memory operation is launched plainly. Measured on a GB300, the chains of an MSM and an
+// chain waits, so each sees all that stands before it. The wait is specified for
+// kernels: what follows anything else (Ctx::after_kernel) is launched plainly, in
+// order with all of it. Measured on a GB300, the chains of an MSM and an
 // opening launched so: commitments of four 2^8-point columns 178 -> 160 us, a stacked
 // 2^16-variable opening (93 launches) 2359 -> 2176.
 template <class... KArgs, class... Args>
 inline void launch_chained(Ctx& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
-  if (c.timers.on) return launch(c, kernel, grid, block, smem, args...);
+  if (c.timers.on || !c.after_kernel) return launch(c, kernel, grid, block, smem, args...);
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -268,10 +295,10 @@ __global__ void k_fr_to_mont(Fr* v, size_t n, uint32_t* flags);
 // `bytes` of a result on the stream to the host, the error flags checked: a
 // kernel stores both in pinned memory and the host waits for its flag (instead of
 // two copies and a synchronisation: about 15 us less a result on a GB300).
-void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host, bool chained = true);
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host);
 // The same in two halves: publish on the stream (work may follow), collect before
 // anything else is published.
-uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes, bool chained = true);
+uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes);
 void collect_checked(Ctx& c, uint32_t seq, size_t bytes, void* host);
 // Canonical 64-byte points (host) -> device affine Montgomery, validated.
 void upload_points(Ctx& c, const uint8_t* host, size_t n, Affine* dst);

@@ -328,7 +328,7 @@ struct GkrValues {
     if (k > 0) return layers[k] + x * rows;
     if (!base_narrow) return reinterpret_cast<const Fr*>(base_raw(x));
     if (!lifted) {
-      APG_CUDA(cudaMallocAsync((void**)&lifted, 32 * rows * circuit.n_committed, ctx->stream));
+      ctx->alloc(&lifted, 32 * rows * circuit.n_committed);
       for (size_t j = 0; j < circuit.n_committed; ++j)
         lift_column(*ctx, base_raw(j), base_bits[j], rows, lifted + j * rows);
     }
@@ -378,7 +378,7 @@ GkrValues* gkr_forward_impl(Ctx& c, const uint8_t* blob, size_t blob_len, const 
     layer_off[k + 1] = total;
     total += (32 * ((size_t)1 << C.layers[k].num_vars) * std::max<uint32_t>(C.layers[k].width, 1) + 255) / 256 * 256;
   }
-  APG_CUDA(cudaMallocAsync((void**)&V->pool, std::max<size_t>(total, 256), c.stream));
+  c.alloc(&V->pool, std::max<size_t>(total, 256));
   for (size_t k = 0; k < V->layers.size(); ++k) V->layers[k] = reinterpret_cast<Fr*>(V->pool + layer_off[k]);
 
   // What the host prepares for all layers goes up at once: the base's copies,
@@ -429,7 +429,7 @@ GkrValues* gkr_forward_impl(Ctx& c, const uint8_t* blob, size_t blob_len, const 
     const TreeLayer t = tree_layer(k);
     memcpy(up.bytes.data() + at_tail + (k - first_tail) * sizeof(TreeLayer), &t, sizeof(t));
   }
-  APG_CUDA(cudaMemcpyAsync(d_up, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, c.stream));
+  c.copy(d_up, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice);
   if (base_on_device) {
     const size_t most = 32 * n0, per = (most / 16 + 255) / 256;
     const unsigned bx = (unsigned)std::max<size_t>(1, std::min(per, (size_t)c.sm_count * 16 / C.n_committed + 1));
@@ -438,7 +438,7 @@ GkrValues* gkr_forward_impl(Ctx& c, const uint8_t* blob, size_t blob_len, const 
              reinterpret_cast<const ColumnCopy*>(d_up + at_copies) + x);
   } else {
     for (size_t x = 0; x < C.n_committed; ++x)
-      APG_CUDA(cudaMemcpyAsync(copies[x].dst, copies[x].src, copies[x].bytes, cudaMemcpyHostToDevice, c.stream));
+      c.copy(copies[x].dst, copies[x].src, copies[x].bytes, cudaMemcpyHostToDevice);
   }
   const uint8_t* d_bits = V->base_narrow ? d_up + at_bits : nullptr;
   for (size_t k = 0; k < C.layers.size(); ++k) {
@@ -534,8 +534,8 @@ int gkr_prove_impl(Ctx& c, const uint8_t* blob, size_t blob_len, GkrValues* V, c
     const size_t rows = (size_t)1 << C.vars(depth);
     std::vector<F> msg(rows * C.outputs.size());
     for (size_t i = 0; i < C.outputs.size(); ++i)
-      APG_CUDA(cudaMemcpyAsync(msg.data() + i * rows, V->col(depth, C.outputs[i]), 32 * rows,
-                               cudaMemcpyDeviceToHost, c.stream));
+      c.copy(msg.data() + i * rows, V->col(depth, C.outputs[i]), 32 * rows,
+                               cudaMemcpyDeviceToHost);
     APG_CUDA(cudaStreamSynchronize(c.stream));
     tr.absorb(host::T_GKR_OUTPUTS, msg);
   }
@@ -698,7 +698,7 @@ int gkr_values_read_impl(GkrValues* v, size_t layer, size_t col, uint8_t* out) {
   if (!v || !out || layer > v->circuit.layers.size() || col >= v->circuit.width(layer)) return APG_ERR_INVALID_ARGUMENT;
   Ctx& c = *v->ctx;
   const size_t rows = (size_t)1 << v->circuit.vars(layer);
-  APG_CUDA(cudaMemcpyAsync(out, v->col(layer, col), 32 * rows, cudaMemcpyDeviceToHost, c.stream));
+  c.copy(out, v->col(layer, col), 32 * rows, cudaMemcpyDeviceToHost);
   APG_CUDA(cudaStreamSynchronize(c.stream));
   return APG_OK;
 }

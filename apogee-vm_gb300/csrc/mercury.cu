@@ -455,11 +455,16 @@ const uint8_t* srs_commit_start(Ctx& c, const Fr* d0, size_t len0, const Fr* d1 
 // acc_j = sum_{k >= j} x_k r^(k - j) for every position, in place or not: one
 // block scan a column where a column fits a block; else segments (32 positions
 // where there are enough to fill the device, 8 where the chain is what counts),
-// the same over their aggregates, and a fix.
-void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, size_t cols, const F& r) {
+// the same over their aggregates, and a fix. `agg`: the aggregates of this level and
+// those above it, one after another in the context's scratch.
+bool suffix_one_block(size_t count, size_t cols) { return count <= kSuffixScanMax && cols < ((size_t)1 << 31); }
+int suffix_segment(size_t count, size_t cols) { return count * cols >= ((size_t)1 << 20) ? kSuffixMax : 8; }
+
+void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, size_t cols, const F& r,
+                   Fr* agg = nullptr) {
   if (count == 0) return;
   SuffixPowers pows;
-  if (count <= kSuffixScanMax && cols < ((size_t)1 << 31)) {
+  if (suffix_one_block(count, cols)) {
     F p = r;
     for (int s = 0; s < 11; ++s) {
       pows.p[s] = dv(p);
@@ -471,12 +476,17 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
                    stride, (int)count, pows);
     return;
   }
-  const int L = count * cols >= ((size_t)1 << 20) ? kSuffixMax : 8;
+  const int L = suffix_segment(count, cols);
   const size_t nseg = (count + L - 1) / L;
-  // Scratch per level: aggregates (nseg x cols), stream-ordered so every
-  // recursion level owns its own.
-  Fr* agg;
-  APG_CUDA(cudaMallocAsync((void**)&agg, 32 * nseg * cols, c.stream));
+  if (!agg) {
+    size_t words = 0;
+    for (size_t n = count; n > 1 && !suffix_one_block(n, cols);) {
+      const size_t per = suffix_segment(n, cols);
+      n = (n + per - 1) / per;
+      words += n * cols;
+    }
+    agg = c.scratch[S_TMP3].as<Fr>(std::max(words, cols));
+  }
   launch_chained(c, k_suffix_local, nb(nseg * cols, 128), 128, 0, in, out, stride, count, cols, L, dv(r), agg);
   if (nseg > 1) {
     F p = host::fone();
@@ -485,10 +495,9 @@ void suffix_horner(Ctx& c, const Fr* in, Fr* out, size_t stride, size_t count, s
       p = host::fmul(p, r);
     }
     F rL = host::fpow_u64(r, L);
-    suffix_horner(c, agg, agg, cols, nseg, cols, rL);
+    suffix_horner(c, agg, agg, cols, nseg, cols, rL, agg + nseg * cols);
     launch_chained(c, k_suffix_fix, nb(count * cols, 256), 256, 0, out, stride, count, cols, L, (const Fr*)agg, pows);
   }
-  APG_CUDA(cudaFreeAsync(agg, c.stream));
 }
 
 // out[q] = poly_q(x_q) for up to kEvals polynomials.
@@ -959,7 +968,7 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   Fr* work;
   // eq1 | eq2 | h | g | S | D | acc(n) | num(n) | 4 x (2b) transforms | twiddles
   const size_t words = 6 * b + 2 * n + 8 * b + b + 16;
-  APG_CUDA(cudaMallocAsync((void**)&work, 32 * words, c.stream));
+  c.alloc(&work, 32 * words);
   struct Guard {
     Ctx& c;
     Fr* p;
@@ -993,7 +1002,7 @@ int mercury_open_impl(Ctx& c, const Fr* d_f, size_t nv, const uint8_t cm[64], co
   cudaEvent_t tp = c.timer_begin();
   suffix_horner(c, d_f, acc, b, b, b, alpha);
   c.timer_end(APG_TIMER_MERCURY_PASS, tp);
-  APG_CUDA(cudaMemcpyAsync(g, acc, 32 * b, cudaMemcpyDeviceToDevice, c.stream));
+  c.copy(g, acc, 32 * b, cudaMemcpyDeviceToDevice);
   const Fr* q = acc + b;
   const size_t nq = n - b;
   d_pts = srs_commit_start(c, q, nq, g, b);
@@ -1177,15 +1186,13 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   std::vector<F> u1(u.begin(), u.begin() + w1), u2(u.begin() + w1, u.end());
   Fr* work;
   const size_t words = b1 + b2 + ncols * b2 + ncols + nstacks + n;
-  APG_CUDA(cudaMallocAsync((void**)&work, 32 * words, c.stream));
+  c.alloc(&work, 32 * words);
   struct Guard {
     Ctx& c;
     Fr* p;
     ~Guard() { cudaFreeAsync(p, c.stream); }
   } guard{c, work};
   Fr *eq1 = work, *eq2 = eq1 + b1, *h = eq2 + b2, *cv = h + ncols * b2, *w = cv + ncols, *fstar = w + nstacks;
-  build_eq_table(c, u1, eq1);
-  build_eq_table(c, u2, eq2);
   // The columns' addresses: stack after stack, then by (stack, slot), null past a
   // stack's end.
   std::vector<const Fr*> table(d_cols, d_cols + ncols);
@@ -1193,7 +1200,9 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   for (size_t j = 0, idx = 0; j < nstacks; ++j)
     for (size_t s = 0; s < stack_lens[j]; ++s) table[ncols + j * maxlen + s] = d_cols[idx++];
   const Fr** d_table = c.scratch[S_TMP5].as<const Fr*>(table.size());
-  APG_CUDA(cudaMemcpyAsync(d_table, table.data(), sizeof(Fr*) * table.size(), cudaMemcpyHostToDevice, c.stream));
+  c.copy(d_table, table.data(), sizeof(Fr*) * table.size(), cudaMemcpyHostToDevice);
+  build_eq_table(c, u1, eq1);
+  build_eq_table(c, u2, eq2);
   for (size_t c0 = 0; c0 < ncols; c0 += 32768) {
     const unsigned cn = (unsigned)std::min<size_t>(32768, ncols - c0);
     launch_chained(c, k_row_dot, dim3(nb(b2 * 32, 256), cn), 256, 0, (const Fr* const*)(d_table + c0), (const Fr*)nullptr,
@@ -1228,7 +1237,7 @@ int mercury_batch_open_stacked_impl(Ctx& c, const Fr* const* d_cols, const size_
   // commitments: about 0.2 ms against 2.2 ms), more through the device MSM.
   Affine* d_cms = c.scratch[S_BASES].as<Affine>(nstacks);
   upload_points(c, cms, nstacks, d_cms);
-  APG_CUDA(cudaMemcpyAsync(w, wts.data(), 32 * nstacks, cudaMemcpyHostToDevice, c.stream));
+  c.copy(w, wts.data(), 32 * nstacks, cudaMemcpyHostToDevice);
   launch_chained(c, k_combine_stacked, nb(n, 256), 256, 0, (const Fr* const*)(d_table + ncols), (const Fr*)w, (int)nstacks, maxlen,
          (int)width, n, fstar);
   uint8_t cm_star[64];

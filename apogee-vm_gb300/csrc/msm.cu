@@ -1740,15 +1740,12 @@ inline unsigned blocks_for(size_t n, int threads) {
 // Host side
 // ---------------------------------------------------------------------------
 
-uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes, bool chained) {
+uint32_t publish_checked(Ctx& c, const void* d_src, size_t bytes) {
   uint8_t* pinned = c.host_pinned();
   if (bytes > Ctx::kPinnedBytes - Ctx::kPinnedTables || bytes % 16) throw Error(APG_ERR_INTERNAL, "an odd result");
-  auto go = [&](auto... args) {
-    if (chained) launch_chained(c, k_publish, 1, 512, 0, args...);
-    else launch(c, k_publish, 1, 512, 0, args...);
-  };
-  go((const uint4*)d_src, (uint32_t)(bytes / 16), (const uint32_t*)c.d_flags,
-     reinterpret_cast<uint4*>(pinned + Ctx::kPinnedTables), reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
+  launch_chained(c, k_publish, 1, 512, 0, (const uint4*)d_src, (uint32_t)(bytes / 16), (const uint32_t*)c.d_flags,
+                 reinterpret_cast<uint4*>(pinned + Ctx::kPinnedTables), reinterpret_cast<uint32_t*>(pinned),
+                 ++c.flag_seq);
   return c.flag_seq;
 }
 
@@ -1759,19 +1756,19 @@ void collect_checked(Ctx& c, uint32_t seq, size_t bytes, void* host) {
   if (reinterpret_cast<const uint32_t*>(c.host_pinned())[1]) c.check_flags();  // clears the flags and throws
 }
 
-void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host, bool chained) {
+void fetch_checked(Ctx& c, const void* d_src, size_t bytes, void* host) {
   if (bytes <= Ctx::kPinnedBytes - Ctx::kPinnedTables && bytes % 16 == 0) {
-    collect_checked(c, publish_checked(c, d_src, bytes, chained), bytes, host);
+    collect_checked(c, publish_checked(c, d_src, bytes), bytes, host);
     return;
   }
-  APG_CUDA(cudaMemcpyAsync(host, d_src, bytes, cudaMemcpyDeviceToHost, c.stream));
+  c.copy(host, d_src, bytes, cudaMemcpyDeviceToHost);
   c.check_flags();
 }
 
 void upload_points_async(Ctx& c, const uint8_t* host, size_t n, Affine* dst) {
   if (n == 0) return;
   uint4* raw = c.scratch[S_TMP7].as<uint4>(4 * n);
-  APG_CUDA(cudaMemcpyAsync(raw, host, 64 * n, cudaMemcpyHostToDevice, c.stream));
+  c.copy(raw, host, 64 * n, cudaMemcpyHostToDevice);
   launch(c, k_points_in, blocks_for<int>(n, 256), 256, 0, (const uint4*)raw, n, dst, c.d_flags);
 }
 
@@ -1784,17 +1781,17 @@ void download_points(Ctx& c, const Affine* src, size_t n, uint8_t* host) {
   if (n == 0) return;
   uint4* raw = c.scratch[S_TMP7].as<uint4>(4 * n);
   launch(c, k_points_out, blocks_for<int>(n, 256), 256, 0, src, n, raw);
-  APG_CUDA(cudaMemcpyAsync(host, raw, 64 * n, cudaMemcpyDeviceToHost, c.stream));
+  c.copy(host, raw, 64 * n, cudaMemcpyDeviceToHost);
   APG_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 void generate_srs(Ctx& c, const uint8_t tau_canonical[32], size_t n, Affine* dst) {
   Fr* d_tau = c.scratch[S_TMP6].as<Fr>(1);
-  APG_CUDA(cudaMemcpyAsync(d_tau, tau_canonical, 32, cudaMemcpyHostToDevice, c.stream));
+  c.copy(d_tau, tau_canonical, 32, cudaMemcpyHostToDevice);
   launch(c, k_fr_to_mont, 1, 1, 0, d_tau, (size_t)1, c.d_flags);
   c.check_flags();
   Fr tau_mont;
-  APG_CUDA(cudaMemcpyAsync(&tau_mont, d_tau, 32, cudaMemcpyDeviceToHost, c.stream));
+  c.copy(&tau_mont, d_tau, 32, cudaMemcpyDeviceToHost);
   APG_CUDA(cudaStreamSynchronize(c.stream));
   launch(c, k_srs_powers, blocks_for<int>(n, 128), 128, 0, tau_mont, n, dst, c.d_flags);
   APG_CUDA(cudaStreamSynchronize(c.stream));
@@ -2010,14 +2007,10 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   Xyzz* lvlR = c.scratch[S_LEVEL_A].as<Xyzz>((size_t)S * rp.blocks);
 
   cudaEvent_t t_total = c.timer_begin();
-  APG_CUDA(cudaMemsetAsync(buckets, 0, zero_bytes, c.stream));
+  c.fill(buckets, 0, zero_bytes);
   const int canon = scalars_canonical ? 1 : 0;
   // One pass over the digits: counted (place null) or placed.
   auto digits = [&](uint32_t* place) {
-    auto go = [&](auto k, dim3 grid, int threads, size_t smem, auto... args) {
-      if (place) launch_chained(c, k, grid, threads, smem, args...);
-      else launch(c, k, grid, threads, smem, args...);  // (follows the memset)
-    };
     const uint32_t few = (uint32_t)spaces_per_col * K;
     if (few <= kFewBins) {
       // Tiles of 256 scalars until they fill the device twice, then up to
@@ -2040,14 +2033,15 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
       void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t, DigitBias, uint32_t*, uint32_t*, uint32_t*) =
           small_scalars ? (place ? k_digits_few<true, true> : k_digits_few<true, false>)
                         : (place ? k_digits_few<false, true> : k_digits_few<false, false>);
-      go(k, grid, 256, smem, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, tile, bias, counts, place,
-         c.d_flags);
+      launch_chained(c, k, grid, 256, smem, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, tile, bias, counts,
+                     place, c.d_flags);
     } else {
       const dim3 grid(blocks_for<int>(std::max<size_t>(nmax, 1), kDigitThreads), (unsigned)ncols);
       void (*k)(MsmCols, int, int, int, uint32_t, uint32_t, int, uint32_t*, uint32_t*, uint32_t*) =
           small_scalars ? (place ? k_digits<true, true> : k_digits<true, false>)
                         : (place ? k_digits<false, true> : k_digits<false, false>);
-      go(k, grid, kDigitThreads, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place, c.d_flags);
+      launch_chained(c, k, grid, kDigitThreads, 0, cols, p.c, p.windows, (int)p.precomp, K, tab_n, canon, counts, place,
+                     c.d_flags);
     }
   };
   digits(nullptr);
@@ -2076,7 +2070,7 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
     uint32_t* idx = APG_PAIR_PF ? reinterpret_cast<uint32_t*>(tot + T) : nullptr;
     uint32_t* cnt = c.scratch[S_PAIR_CNT].as<uint32_t>((size_t)kPairRounds * (nbins + 1) + 2);
     uint32_t* mode = cnt + (size_t)kPairRounds * (nbins + 1);
-    APG_CUDA(cudaMemsetAsync(mode, 0, 2 * sizeof(uint32_t), c.stream));
+    c.fill(mode, 0, 2 * sizeof(uint32_t));
     const size_t scan_n = nbins + 1;
     const unsigned sblocks = (unsigned)((scan_n + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems));
     const uint32_t* ends_in = counts;
@@ -2206,22 +2200,21 @@ void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* c
     }
     cols.shared = o.stack ? 1 : 0;
     cols.bits = o.bits;
-    uint8_t* dst = o.stack ? partial + 64 * ngroups : d_out + 64 * j;
+    uint8_t* dst = !o.stack ? d_out + 64 * j : g == k ? d_out : partial + 64 * ngroups;  // (one group: the sum itself)
     msm_group(c, bases, table, cols, (int)g, nmax, p, small_scalars, scalars_canonical, o.uniform, dst);
     ++ngroups;
     j += g;
   }
   if (o.stack) {
-    if (ngroups == 0) APG_CUDA(cudaMemsetAsync(d_out, 0, 64, c.stream));
-    else if (ngroups == 1) APG_CUDA(cudaMemcpyAsync(d_out, partial, 64, cudaMemcpyDeviceToDevice, c.stream));
-    else launch(c, k_add_points, 1, 32, 0, (const uint32_t*)partial, (int)ngroups, (uint32_t*)d_out, c.d_flags);
+    if (ngroups == 0) c.fill(d_out, 0, 64);
+    else if (ngroups > 1) launch(c, k_add_points, 1, 32, 0, (const uint32_t*)partial, (int)ngroups, (uint32_t*)d_out, c.d_flags);
   }
 }
 
 void msm_device(Ctx& c, const Affine* bases, const SrsTable* table, const void* scalars, bool small_scalars,
                 bool scalars_canonical, size_t n, uint8_t* out64_device, uint8_t* host_out, const MsmBatchOpts& o) {
   if (n == 0) {
-    if (out64_device) APG_CUDA(cudaMemsetAsync(out64_device, 0, 64, c.stream));
+    if (out64_device) c.fill(out64_device, 0, 64);
     if (host_out) memset(host_out, 0, 64);
     return;
   }

@@ -760,7 +760,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
   PackedProgram packed{};
   if (!use_form) packed = pack_program(hp, up);
   uint8_t* d_up = c.scratch[S_PAIR_TERMS].as<uint8_t>(up.bytes.size());
-  APG_CUDA(cudaMemcpyAsync(d_up, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, c.stream));
+  c.copy(d_up, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice);
   unsigned* done = reinterpret_cast<unsigned*>(d_up);
   const Fr** d_src = reinterpret_cast<const Fr**>(d_up + at_src);
   const uint8_t* d_bits = narrow ? d_up + at_bits : nullptr;
@@ -986,7 +986,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
     launch_chained(c, k_final_bind, 1, 256, 0, (const Fr* const*)d_src, d_bits, base, (size_t)2, n <= 1 ? 1 : 0, nd,
            to_dev(chal), n == 0 ? 1 : 0, d_fin, reinterpret_cast<uint32_t*>(pinned), ++c.flag_seq);
     if (!in_pinned)
-      APG_CUDA(cudaMemcpyAsync(finals.data(), d_fin, 32 * (size_t)nd, cudaMemcpyDeviceToHost, c.stream));
+      c.copy(finals.data(), d_fin, 32 * (size_t)nd, cudaMemcpyDeviceToHost);
     c.wait_flag();
     if (in_pinned) memcpy(finals.data(), host_tables, 32 * (size_t)nd);
     else APG_CUDA(cudaStreamSynchronize(c.stream));

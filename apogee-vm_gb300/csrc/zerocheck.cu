@@ -103,8 +103,7 @@ int prove_zerocheck_impl(Ctx& c, size_t arity, const uint8_t* coefs, const uint3
     }
     uint8_t* d = c.scratch[S_SCALARS].as<uint8_t>(total);
     for (size_t k = 0; k < arity; ++k) {
-      APG_CUDA(cudaMemcpyAsync(d + off[k], polys[k], narrow_bytes(bits ? bits[k] : 0, n), cudaMemcpyHostToDevice,
-                               c.stream));
+      c.copy(d + off[k], polys[k], narrow_bytes(bits ? bits[k] : 0, n), cudaMemcpyHostToDevice);
       src[k] = reinterpret_cast<const Fr*>(d + off[k]);
     }
   }
