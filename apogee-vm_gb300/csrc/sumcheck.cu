@@ -652,7 +652,7 @@ struct HostForm {
   size_t cost = 0;        // wide products a node
   size_t muls = 0;        // products a node
 };
-bool quadratic_form(const HostProgram& hp, int slots, HostForm& out);
+bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out);
 
 // How many of a short form's last rounds run on the host. Both sides
 // pay the transcript's permutations (6 us each: three a round on the device's
@@ -737,7 +737,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
 
   const int n_val = nd + (int)vkinds.size(), n_cached = hp.n_cached;
   HostForm form;
-  const bool use_form = (size_t)(n_val + 1) * 3 * sizeof(Fr) <= kFormSmemMax && quadratic_form(hp, n_val, form);
+  const bool use_form = (size_t)(n_val + 1) * 3 * sizeof(Fr) <= kFormSmemMax && quadratic_form(hp, n_val, n, form);
   const int host_rounds = use_form && vkinds.empty() ? host_tail_rounds(n, nd, form) : 0;
 
   // One upload: the counter of finished blocks (zero), the round-0 sources (the
@@ -1083,17 +1083,49 @@ bool add_gate(const HostProgram& hp, const DevGate& g, const F& w, int slots, co
   return false;
 }
 
-// The products a node takes gate by gate, and the terms its expansion may have.
-void gate_size(const HostProgram& hp, const DevGate& g, size_t& products, size_t& expanded) {
+// The products a node takes gate by gate.
+size_t gate_products(const HostProgram& hp, const DevGate& g) {
   const F one = host::fone(), minus_one = host::fneg(one), zero = host::fzero();
   const size_t t = g.p1, u = g.p2;
   const size_t ncoef = g.kind == G_LINEAR ? t : g.kind == G_PRODUCT ? 1 : g.kind == G_AFFINE ? t + u + 1 : g.kind == G_QUADRATIC ? 1 + t + u : 0;
+  size_t products = g.kind == G_LINEAR ? 0 : g.kind == G_QUADRATIC ? u : g.kind == G_TREE_CROSS ? 2 : 1;
   for (size_t i = 0; i < ncoef; ++i) {
     const F& v = hp.coeffs[g.cf_off + i];
     products += v == one || v == minus_one || v == zero ? 0 : 1;
   }
-  products += g.kind == G_LINEAR ? 0 : g.kind == G_QUADRATIC ? u : g.kind == G_TREE_CROSS ? 2 : 1;
-  expanded += g.kind == G_AFFINE ? (t + 1) * (u + 1) : 1 + t + u;
+  return products;
+}
+
+// The terms that add_gate touches when it expands the list, a cached operand
+// counting with all of its own; at least `limit` + 1 where they are more.
+size_t expanded_terms(const HostProgram& hp, int slots, size_t limit) {
+  std::vector<size_t> cached;
+  size_t all = 0;
+  for (const DevGate& g : hp.gates) {
+    const uint16_t* o = hp.ops.data() + g.op_off;
+    auto size = [&](size_t k) { return o[k] < slots ? (size_t)1 : cached[o[k] - slots]; };
+    auto sum = [&](size_t first, size_t n) {
+      size_t s = 0;
+      for (size_t k = first; k < first + n; ++k) s += size(k);
+      return s;
+    };
+    const size_t t = g.p1, u = g.p2;
+    size_t e = 1;
+    switch (g.kind) {
+      case G_LINEAR: e += sum(0, t); break;
+      case G_MASK: e += size(1) + size(0) * size(1); break;
+      case G_AFFINE: e = (1 + sum(0, t)) * (1 + sum(t, u)); break;
+      case G_TREE_CROSS: e = size(0) * size(3) + size(1) * size(2); break;
+      case G_QUADRATIC:
+        e += sum(0, t);
+        for (size_t k = 0; k < u; ++k) e += size(t + 2 * k) * size(t + 2 * k + 1);
+        break;
+      default: e = size(0) * size(1);
+    }
+    if ((all += e) > limit) return limit + 1;
+    if (cached.size() < (size_t)hp.n_cached) cached.push_back(std::min(e, (size_t)1 << 18));  // (no sum overflows)
+  }
+  return all;
 }
 
 }  // namespace
@@ -1102,14 +1134,21 @@ void gate_size(const HostProgram& hp, const DevGate& g, size_t& products, size_t
 // its weight and its cached operands' polynomials, equal monomials merged
 // (exact arithmetic: the sum is the same at every node), then grouped greedily
 // by the slot that the most remaining products share, whose linear term becomes
-// its group's constant. False when the degree passes two, or when the gates as
-// they stand take fewer products than the form.
-bool quadratic_form(const HostProgram& hp, int slots, HostForm& out) {
+// its group's constant. False when the degree passes two, when the gates as
+// they stand take fewer products than the form, or when expanding them would take
+// the host too long: a term is 0.16 us there, while the device waits. The real
+// circuits' lists have about 1.4 terms a product, so a list takes its share of terms
+// whatever its length; what passes that may take a quarter of the time that the
+// products take on the device over 2^n rows (35 ps each, all rounds), and, without
+// cached operands, 3 ms. (Eight cached forms over 200 columns and 2,000 products of
+// two of them multiply out to 81 million terms: 17 s, for a form that is then refused.)
+bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out) {
   out = HostForm();
   if (!hp.summed || slots >= kNoTable) return false;
-  size_t products = 0, expanded = 0;
-  for (const DevGate& g : hp.gates) gate_size(hp, g, products, expanded);
-  if (expanded > 20000) return false;
+  size_t products = 0;
+  for (const DevGate& g : hp.gates) products += gate_products(hp, g);
+  const size_t limit = 4 * products + (hp.n_cached ? 1000 : 20000) + ((products << std::min(n, 30)) >> 14);
+  if (expanded_terms(hp, slots, limit) > limit) return false;
   std::vector<QuadPoly> cached(hp.n_cached);
   const F one = host::fone(), minus_one = host::fneg(one);
   for (int j = 0; j < hp.n_cached; ++j) {
