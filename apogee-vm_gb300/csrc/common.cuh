@@ -357,6 +357,7 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need);
 // (commits of the caller's columns); openings commit uniformly random
 // quotient polynomials, for which the default rule is the uniform-scalar one.
 constexpr size_t kNarrowTableMax = (size_t)1 << 12;
+constexpr size_t kNarrowWindowMax = (size_t)1 << 16;  // points that widths below 12 are timed over
 constexpr int narrow_window(size_t n) { return n <= ((size_t)1 << 8) ? 6 : 7; }
 constexpr size_t kWideTableMin = (size_t)1 << 18;
 const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned = true);

@@ -1826,10 +1826,14 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need) {
     if (t.c == cbits && t.n >= need) return &t;
   if (!c.srs || c.srs_n < need) return nullptr;
   // A wide table covers the whole SRS, a narrower one the prefix that the
-  // default rule reads it for until a caller needs more. The prefix's table is
-  // then kept until the SRS goes: contexts that share it may still read it.
-  size_t n = cbits >= 16 ? c.srs_n : std::min(c.srs_n, cbits >= 12 ? kWideTableMin : (size_t)1 << (cbits >= 7 ? 16 : 12));
-  if (n < need) n = c.srs_n;
+  // default rule reads it for until a caller needs more: of a width below 12 the
+  // 2^16 points that the autotuner may time it over, of the others the SRS (5 bits
+  // take 3.3 KB a point). The prefix's table is then kept until the SRS goes:
+  // contexts that share it may still read it.
+  size_t n = c.srs_n;
+  for (size_t prefix : {cbits < 7 ? kNarrowTableMax : (size_t)0, cbits < 12 ? kNarrowWindowMax : (size_t)0,
+                        cbits >= 12 && cbits < 16 ? kWideTableMin : (size_t)0})
+    if (need <= prefix) n = std::min(n, prefix);
   for (auto it = c.tables.begin(); it != c.tables.end(); ++it)
     if (it->c == cbits) {
       if (it->owned) c.retired.push_back(*it);
@@ -1883,7 +1887,7 @@ void msm_autotune(Ctx& c, const void* d_sample, size_t sample_len, int kmin, int
       for (size_t j = 0; j < ncands; ++j) {
         const int cb = cands[j];
         if (cb < 2 || cb > 20) continue;
-        if (cb < 12 && n > ((size_t)1 << 16)) continue;  // narrow tables cover a 2^16 prefix
+        if (cb < 12 && n > kNarrowWindowMax) continue;
         const SrsTable* t = srs_table(c, cb, n);
         if (!t) continue;
         msm_device(c, nullptr, t, d_sample, false, false, n, d_out, nullptr);  // warm-up
