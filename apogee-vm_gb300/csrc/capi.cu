@@ -140,9 +140,7 @@ void apg_ctx_destroy(apg_ctx* ctx) {
     release_lane(c);
     for (auto& b : c.scratch) b.release();
     for (auto& b : c.fft_tw) b.release();
-    for (auto& t : c.tables)
-      if (t.owned) cudaFree(t.tab);
-    for (auto& t : c.retired) cudaFree(t.tab);
+    c.tables.clear();
     if (c.srs && c.srs_owned) cudaFree(c.srs);
     if (c.d_flags) cudaFree(c.d_flags);
     if (c.pinned) cudaFreeHost(c.pinned);
@@ -165,11 +163,11 @@ int apg_ctx_synchronize(apg_ctx* ctx) {
 
 static void drop_srs(Ctx& c) {
   APG_CUDA(cudaStreamSynchronize(c.stream));
-  for (auto& t : c.tables)
-    if (t.owned) cudaFree(t.tab);
   c.tables.clear();
-  for (auto& t : c.retired) cudaFree(t.tab);
-  c.retired.clear();
+  if (c.lane) {
+    APG_CUDA(cudaStreamSynchronize(c.lane->stream));
+    c.lane->tables.clear();
+  }
   if (c.srs && c.srs_owned) cudaFree(c.srs);
   c.srs = nullptr;
   c.srs_n = 0;
@@ -422,8 +420,6 @@ static Ctx& lane_of(Ctx& c) {
     c.lane = std::move(L);
   }
   Ctx& L = *c.lane;
-  for (auto& t : L.tables)
-    if (t.owned) cudaFree(t.tab);
   L.tables.clear();
   for (auto t : c.tables) {
     t.owned = false;
@@ -443,8 +439,7 @@ static void release_lane(Ctx& c) {
   Ctx& L = *c.lane;
   cudaStreamSynchronize(L.stream);
   for (auto& b : L.scratch) b.release();
-  for (auto& t : L.tables)
-    if (t.owned) cudaFree(t.tab);
+  L.tables.clear();
   if (L.d_flags) cudaFree(L.d_flags);
   if (L.stream) cudaStreamDestroy(L.stream);
   c.lane.reset();
@@ -754,7 +749,6 @@ static size_t ctx_bytes(const Ctx& c) {
   for (const auto& d : c.fft_tw) b += d.cap;
   for (const auto& t : c.tables)
     if (t.owned) b += (size_t)t.windows * t.n * sizeof(Affine);
-  for (const auto& t : c.retired) b += (size_t)t.windows * t.n * sizeof(Affine);
   if (c.srs && c.srs_owned) b += c.srs_n * sizeof(Affine);
   if (c.lane) b += ctx_bytes(*c.lane);
   return b;

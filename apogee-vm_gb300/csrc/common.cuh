@@ -71,12 +71,15 @@ struct DevBuf {
 };
 
 // The precomputed window table of the resident SRS for one window width:
-// tab[w * n + i] = 2^(c*w) * P_i, affine Montgomery.
+// tab[w * n + i] = 2^(c*w) * P_i, affine Montgomery. Contexts and lanes that read the
+// same table hold its memory together: it is freed with the last of them, each of
+// which has its stream idle when it lets go.
 struct SrsTable {
   int c = 0, windows = 0;
   size_t n = 0;
   Affine* tab = nullptr;
-  bool owned = true;  // false: borrowed from another context (apg_srs_share)
+  std::shared_ptr<void> mem;
+  bool owned = true;  // false: borrowed from another context (apg_srs_share), counted there
 };
 
 enum ScratchSlot {
@@ -129,7 +132,6 @@ struct Ctx {
   size_t srs_n = 0;
   bool srs_owned = true;  // false: borrowed from another context (apg_srs_share)
   std::vector<SrsTable> tables;
-  std::vector<SrsTable> retired;  // owned tables a larger one replaced (srs_table)
   // Window width chosen by apg_msm_autotune per size class (index: ceil of
   // log2 of the point count); 0 = the default rule of srs_table_for.
   int tuned_c[64] = {0};

@@ -1828,15 +1828,19 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need) {
   // A wide table covers the whole SRS, a narrower one the prefix that the
   // default rule reads it for until a caller needs more: of a width below 12 the
   // 2^16 points that the autotuner may time it over, of the others the SRS (5 bits
-  // take 3.3 KB a point). The prefix's table is then kept until the SRS goes:
-  // contexts that share it may still read it.
+  // take 3.3 KB a point). The prefix's table then goes, with the last context that
+  // shares it.
   size_t n = c.srs_n;
   for (size_t prefix : {cbits < 7 ? kNarrowTableMax : (size_t)0, cbits < 12 ? kNarrowWindowMax : (size_t)0,
                         cbits >= 12 && cbits < 16 ? kWideTableMin : (size_t)0})
     if (need <= prefix) n = std::min(n, prefix);
   for (auto it = c.tables.begin(); it != c.tables.end(); ++it)
     if (it->c == cbits) {
-      if (it->owned) c.retired.push_back(*it);
+      APG_CUDA(cudaStreamSynchronize(c.stream));
+      if (c.lane) {  // (a batch gives it the tables anew)
+        APG_CUDA(cudaStreamSynchronize(c.lane->stream));
+        c.lane->tables.clear();
+      }
       c.tables.erase(it);
       break;
     }
@@ -1847,6 +1851,7 @@ const SrsTable* srs_table(Ctx& c, int cbits, size_t need) {
   // Sorted references carry the table index in 31 bits.
   if ((size_t)t.windows * n >= ((size_t)1 << 31)) throw Error(APG_ERR_OUT_OF_MEMORY, "SRS window table too large");
   APG_CUDA(cudaMalloc(&t.tab, (size_t)t.windows * n * sizeof(Affine)));
+  t.mem = std::shared_ptr<void>(t.tab, [](void* p) { cudaFree(p); });
   launch(c, k_window_table, blocks_for<int>(n, 128), 128, 0, (const Affine*)c.srs, n, cbits, t.windows, t.tab,
          c.d_flags);
   APG_CUDA(cudaStreamSynchronize(c.stream));
