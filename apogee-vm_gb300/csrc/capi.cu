@@ -1167,19 +1167,15 @@ size_t apg_shard_device_bytes(const apg_shard* sh) {
     const size_t n = (size_t)1 << sh->num_vars, k = sh->n_cols;
     size_t b = sh->cols_on_device ? 0 : 32 * n * k;  // the staged columns
     b += gkr_device_bytes_impl(sh->circuit, sh->circuit_len);
-    // The commits' two lanes: a group of columns sorts up to 17 windows a
-    // point (4-byte references; 37 or 43 up to 2^12 points), and the affine
-    // pair rounds hold two point lists and the running products at about half
-    // and a quarter of that (capped as msm.cu caps them), plus buckets and
-    // levels.
+    b += 36 * n;  // the sumcheck's eq table
+    // The MSMs' scratch: a commit's group on each lane that it uses, and on the first
+    // one the opening's, of all coefficients with a short second column.
     const size_t g = commit_group(k, n);
-    const size_t E = std::min<size_t>((size_t)(n <= kNarrowTableMax ? 43 : 17) * n * g, (size_t)1 << 28);
-    const size_t cap = (size_t)48 << 20;
-    size_t lane = 4 * E + ((size_t)96 << 20);
-    if (E >= ((size_t)1 << 21))
-      lane += 64 * std::min(E / 2, cap) + 64 * std::min(E / 4, cap) + 32 * std::min(E / 2, cap);
-    b += 2 * lane;
-    b += 12 * 32 * n;  // the opening's O(n) tables
+    const size_t commit = msm_scratch_bytes(n, g, default_table_window(n, k), false);
+    const size_t open = msm_scratch_bytes(n / 2 + 1, 2, default_table_window(n, 2), true);
+    b += std::max(commit, open) + (g < k ? commit : 0);
+    // The opening's tables: three of all rows, one of each column's row sums.
+    b += 3 * 32 * n + (32 * (k + 16) << (sh->num_vars + 1) / 2) + ((size_t)1 << 20);
     return b;
   } catch (...) {
     return 0;

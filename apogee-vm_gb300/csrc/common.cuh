@@ -363,6 +363,12 @@ constexpr size_t kNarrowWindowMax = (size_t)1 << 16;  // points that widths belo
 constexpr int narrow_window(size_t n) { return n <= ((size_t)1 << 8) ? 6 : 7; }
 constexpr size_t kWideTableMin = (size_t)1 << 18;
 const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned = true);
+constexpr int default_table_window(size_t n, size_t cols) {
+  return n <= kNarrowTableMax ? narrow_window(n) : n >= kWideTableMin ? 17 : cols <= 2 ? 15 : 13;
+}
+// The scratch that msm_multi holds for `cols` columns of n field elements over an
+// SRS table of `window` bits (at most: the pair rounds' lists at their bounds).
+size_t msm_scratch_bytes(size_t n, size_t cols, int window, bool uniform);
 // Time SRS commits of the first 2^k sample scalars for k in [kmin, kmax] with
 // each candidate width and record the fastest in c.tuned_c (see
 // apg_msm_autotune).

@@ -1871,11 +1871,7 @@ const SrsTable* srs_table_for(Ctx& c, size_t n, size_t cols, bool tuned) {
     const SrsTable* t = srs_table(c, c.tuned_c[cls], n);
     if (t) return t;
   }
-  if (n <= kNarrowTableMax) {
-    const SrsTable* t = srs_table(c, narrow_window(n), n);
-    if (t) return t;
-  }
-  return srs_table(c, n >= kWideTableMin ? 17 : cols <= 2 ? 15 : 13, n);
+  return srs_table(c, default_table_window(n, cols), n);
 }
 
 void msm_autotune(Ctx& c, const void* d_sample, size_t sample_len, int kmin, int kmax, const int* cands,
@@ -1981,6 +1977,21 @@ constexpr size_t kMaxGroupEntries = (size_t)1 << 28;                           /
 // 242 and 216, two 309 and 258.
 inline size_t acc_slice_min(size_t entries) { return entries <= ((size_t)1 << 15) ? 4 : 8; }
 
+// Round r's list of the pair rounds fits cap[r]: a round keeps ceil(len/2) of each
+// run, so a list never grows and at most halves plus one point per bucket.
+struct PairCaps {
+  size_t cap[kPairRounds > 0 ? kPairRounds : 1];
+};
+inline PairCaps pair_caps(size_t emax, size_t nbins) {
+  PairCaps p;
+  p.cap[0] = std::min((emax + nbins + 1) / 2, kPairMaxPoints);
+  for (int r = 1; r < kPairRounds; ++r) p.cap[r] = std::min(p.cap[r - 1], (p.cap[r - 1] + nbins + 1) / 2);
+  return p;
+}
+inline bool takes_pair_rounds(size_t emax, bool uniform) {
+  return kPairRounds > 0 && emax >= kPairMinEntries * (uniform ? 1 : 2);
+}
+
 // One group: columns share the plan, the bases and one pass of every kernel.
 void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols& cols, int ncols, size_t nmax,
                const MsmPlan& p, bool small_scalars, bool scalars_canonical, bool uniform, uint8_t* d_out) {
@@ -2062,12 +2073,9 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
   const uint32_t* pair_mode = nullptr;
   const uint32_t* pair_ends = nullptr;
   const Affine* pair_pts = nullptr;
-  if (kPairRounds > 0 && emax >= kPairMinEntries * (uniform ? 1 : 2)) {
-    // Round r's list fits cap[r]: a round keeps ceil(len/2) of each run, so
-    // a list never grows and at most halves plus one point per bucket.
-    size_t cap[kPairRounds > 0 ? kPairRounds : 1];
-    cap[0] = std::min((emax + nbins + 1) / 2, kPairMaxPoints);
-    for (int r = 1; r < kPairRounds; ++r) cap[r] = std::min(cap[r - 1], (cap[r - 1] + nbins + 1) / 2);
+  if (takes_pair_rounds(emax, uniform)) {
+    const PairCaps caps = pair_caps(emax, nbins);
+    const size_t* cap = caps.cap;
     const size_t T = pair_resident_threads(c);
     Affine* lst[2] = {c.scratch[S_PAIR_A].as<Affine>(cap[0]),
                       c.scratch[S_PAIR_B].as<Affine>(kPairRounds > 1 ? cap[1] : 1)};
@@ -2141,6 +2149,24 @@ void msm_group(Ctx& c, const Affine* bases, const SrsTable* table, const MsmCols
 }
 
 }  // namespace
+
+size_t msm_scratch_bytes(size_t n, size_t cols, int window, bool uniform) {
+  const size_t digits = (size_t)window_count(254, window) * n, K = (size_t)1 << (window - 1);
+  const size_t fit = std::min(kMaxBins / K, kMaxGroupEntries / std::max<size_t>(digits, 1));
+  const size_t g = std::max<size_t>(1, std::min(std::min(cols, (size_t)kMaxCols), fit)), emax = g * digits, nbins = g * K;
+  const size_t resident = (size_t)152 * 1024;  // threads: no kernel here has more on a GB300
+  const size_t nseg = std::min(resident, emax / acc_slice_min(emax) + 1);
+  size_t b = emax * 4 + nbins * (sizeof(Xyzz) + 4)            // references, buckets, counts
+             + 4 * nseg * (sizeof(Xyzz) + 5)                  // the fold's items: two lists of two a slice
+             + nbins / kReduceQuads * 2 * sizeof(Xyzz);       // the reduction's first level
+  if (takes_pair_rounds(emax, uniform)) {
+    const PairCaps caps = pair_caps(emax, nbins);
+    b += (caps.cap[0] + caps.cap[kPairRounds > 1 ? 1 : 0]) * sizeof(Affine) + (caps.cap[0] + 2 * resident) * sizeof(Fq) +
+         kPairRounds * nbins * 4;
+    if (APG_PAIR_PF) b += (caps.cap[0] + resident) * 4;
+  }
+  return b + b / 8 + ((size_t)1 << 20);  // (a buffer grows by an eighth more than it is asked for)
+}
 
 void msm_multi(Ctx& c, const Affine* bases, const SrsTable* table, const void* const* scalars, const size_t* lens,
                size_t k, bool small_scalars, bool scalars_canonical, uint8_t* d_out, const MsmBatchOpts& o) {

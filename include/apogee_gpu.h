@@ -470,7 +470,7 @@ size_t apg_abi_sizes(size_t* out, size_t n);
 int apg_prove_shard(apg_ctx* ctx, const apg_shard* shard, apg_shard_proof* out);
 /* No reference counterpart: an estimate of the device bytes proving `shard`
  * holds at its peak on a context that holds nothing yet (staged columns, GKR
- * layers, the largest sumcheck's levels, both commit lanes' MSM scratch, the
+ * layers, the largest sumcheck's levels, the MSM scratch of the lanes it uses, the
  * opening's tables); 0 for a malformed circuit. The server admits by it. */
 size_t apg_shard_device_bytes(const apg_shard* shard);
 /* No reference counterpart: the device bytes the context (and its second
