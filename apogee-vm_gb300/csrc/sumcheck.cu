@@ -15,8 +15,7 @@
 // them.
 #include <algorithm>
 #include <chrono>
-#include <map>
-#include <set>
+#include <queue>
 #include <tuple>
 
 #include "sumcheck.cuh"
@@ -998,89 +997,147 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
 // A device copy of a resolved gate list.
 namespace {
 
-// A polynomial of degree two at most in the slots: terms keyed by their two
-// slots, lower first, kNoTable for an absent second one.
+// A polynomial of degree two at most in the slots: terms keyed by their two slots,
+// the lower one high, kNoTable for an absent second one. Terms are appended as they
+// come and merged once (a tree of them took 46 us more of a call with 560 terms).
 struct QuadPoly {
+  struct Term {
+    uint32_t key;
+    F v;
+    uint16_t a() const { return (uint16_t)(key >> 16); }
+    uint16_t b() const { return (uint16_t)key; }
+  };
   F c = host::fzero();
-  std::map<std::pair<uint16_t, uint16_t>, F> m;
-  void add(uint16_t a, uint16_t b, const F& v) {
-    const auto k = a < b ? std::make_pair(a, b) : std::make_pair(b, a);
-    auto it = m.emplace(k, v);
-    if (!it.second) it.first->second = host::fadd(it.first->second, v);
+  std::vector<Term> m;
+  void add(uint16_t a, uint16_t b, const F& v) { m.push_back({a < b ? (uint32_t)a << 16 | b : (uint32_t)b << 16 | a, v}); }
+  // Equal monomials added up, in the keys' order.
+  void merge() {
+    std::vector<uint64_t> order(m.size());
+    for (size_t i = 0; i < m.size(); ++i) order[i] = (uint64_t)m[i].key << 32 | i;
+    std::sort(order.begin(), order.end());
+    std::vector<Term> out;
+    out.reserve(m.size());
+    for (uint64_t o : order) {
+      const Term& t = m[(uint32_t)o];
+      if (!out.empty() && out.back().key == t.key) out.back().v = host::fadd(out.back().v, t.v);
+      else out.push_back(t);
+    }
+    m.swap(out);
   }
 };
 
-// Adds w times the gate's value to `out`; operands at `slots` and above are the
-// cached entries' polynomials. False when the degree passes two.
-bool add_gate(const HostProgram& hp, const DevGate& g, const F& w, int slots, const std::vector<QuadPoly>& cached,
-              QuadPoly& out) {
+// Adds w times the gate's value to `out`, over the operands as they stand (a cached
+// entry counts as a slot of its own).
+void add_gate(const HostProgram& hp, const DevGate& g, const F& w, QuadPoly& out) {
   const F* c = hp.coeffs.data() + g.cf_off;
   const uint16_t* o = hp.ops.data() + g.op_off;
-  auto linear = [&](uint16_t a, const F& v) {
-    if (a < slots) {
-      out.add(a, kNoTable, v);
-      return;
-    }
-    const QuadPoly& p = cached[a - slots];
-    out.c = host::fadd(out.c, host::fmul(v, p.c));
-    for (auto& t : p.m) out.add(t.first.first, t.first.second, host::fmul(v, t.second));
-  };
-  auto product = [&](uint16_t a, uint16_t b, const F& v) {
-    if (a < slots && b < slots) {
-      out.add(a, b, v);
-      return true;
-    }
-    QuadPoly pa, pb;
-    if (a < slots) pa.add(a, kNoTable, host::fone());
-    else pa = cached[a - slots];
-    if (b < slots) pb.add(b, kNoTable, host::fone());
-    else pb = cached[b - slots];
-    out.c = host::fadd(out.c, host::fmul(v, host::fmul(pa.c, pb.c)));
-    for (auto& t : pa.m) out.add(t.first.first, t.first.second, host::fmul(v, host::fmul(t.second, pb.c)));
-    for (auto& t : pb.m) out.add(t.first.first, t.first.second, host::fmul(v, host::fmul(t.second, pa.c)));
-    for (auto& t : pa.m)
-      for (auto& u : pb.m) {
-        if (t.first.second != kNoTable || u.first.second != kNoTable) return false;
-        out.add(t.first.first, u.first.first, host::fmul(v, host::fmul(t.second, u.second)));
-      }
-    return true;
-  };
+  const bool unit = w == host::fone();
+  auto weighed = [&](const F& v) { return unit ? v : host::fmul(w, v); };
   const int t = g.p1, u = g.p2;
   switch (g.kind) {
     case G_LINEAR:
-      for (int i = 0; i < t; ++i) linear(o[i], host::fmul(w, c[i]));
-      out.c = host::fadd(out.c, host::fmul(w, c[t]));
-      return true;
+      for (int i = 0; i < t; ++i) out.add(o[i], kNoTable, weighed(c[i]));
+      out.c = host::fadd(out.c, weighed(c[t]));
+      break;
     case G_PRODUCT:
-      return product(o[0], o[1], host::fmul(w, c[0]));
+      out.add(o[0], o[1], weighed(c[0]));
+      break;
     case G_MASK:  // x m + 1 - m
-      linear(o[1], host::fneg(w));
+      out.add(o[0], o[1], w);
+      out.add(o[1], kNoTable, host::fneg(w));
       out.c = host::fadd(out.c, w);
-      return product(o[0], o[1], w);
+      break;
     case G_AFFINE: {  // (sum l_i x_i + l_t)(sum r_k y_k + r_u)
-      const F lt = host::fmul(w, c[t]), ru = host::fmul(w, c[t + 1 + u]);
+      const F lt = weighed(c[t]), ru = c[t + 1 + u];
       for (int i = 0; i < t; ++i) {
-        const F li = host::fmul(w, c[i]);
-        for (int k = 0; k < u; ++k)
-          if (!product(o[i], o[t + k], host::fmul(li, c[t + 1 + k]))) return false;
-        linear(o[i], host::fmul(ru, c[i]));
+        const F li = weighed(c[i]);
+        for (int k = 0; k < u; ++k) out.add(o[i], o[t + k], host::fmul(li, c[t + 1 + k]));
+        out.add(o[i], kNoTable, host::fmul(li, ru));
       }
-      for (int k = 0; k < u; ++k) linear(o[t + k], host::fmul(lt, c[t + 1 + k]));
-      out.c = host::fadd(out.c, host::fmul(lt, c[t + 1 + u]));
-      return true;
+      for (int k = 0; k < u; ++k) out.add(o[t + k], kNoTable, host::fmul(lt, c[t + 1 + k]));
+      out.c = host::fadd(out.c, host::fmul(lt, ru));
+      break;
     }
     case G_TREE_PRODUCT:
-      return product(o[0], o[1], w);
+      out.add(o[0], o[1], w);
+      break;
     case G_TREE_CROSS:
-      return product(o[0], o[3], w) && product(o[1], o[2], w);
+      out.add(o[0], o[3], w);
+      out.add(o[1], o[2], w);
+      break;
     case G_QUADRATIC:
-      out.c = host::fadd(out.c, host::fmul(w, c[0]));
-      for (int i = 0; i < t; ++i) linear(o[i], host::fmul(w, c[1 + i]));
-      for (int k = 0; k < u; ++k)
-        if (!product(o[t + 2 * k], o[t + 2 * k + 1], host::fmul(w, c[1 + t + k]))) return false;
-      return true;
+      out.c = host::fadd(out.c, weighed(c[0]));
+      for (int i = 0; i < t; ++i) out.add(o[i], kNoTable, weighed(c[1 + i]));
+      for (int k = 0; k < u; ++k) out.add(o[t + 2 * k], o[t + 2 * k + 1], weighed(c[1 + t + k]));
+      break;
   }
-  return false;
+}
+
+// p, merged, with its cached slots (from `slots` on) replaced by their polynomials:
+// p = q + sum_i C_i L_i, L_i what stands beside the entry C_i (or an earlier one than
+// it). L_i is added up first, so each entry is multiplied out once, however many
+// products it is in. False when the degree passes two, or before multiplying where that
+// takes more than `limit` terms or leaves monomials of more than `most` wide products.
+bool substitute(QuadPoly& p, int slots, const std::vector<QuadPoly>& cached, size_t limit, size_t most) {
+  p.merge();
+  std::vector<QuadPoly> beside(cached.size());
+  QuadPoly out;
+  out.c = p.c;
+  bool any = false;
+  for (const auto& t : p.m) {
+    const uint16_t a = t.a(), b = t.b();
+    const uint16_t top = b == kNoTable ? a : b;  // (a <= b)
+    if (top < slots) {
+      out.m.push_back(t);
+      continue;
+    }
+    any = true;
+    QuadPoly& L = beside[top - slots];
+    if (b == kNoTable) {
+      L.c = host::fadd(L.c, t.v);
+    } else if (a < slots) {
+      L.add(a, kNoTable, t.v);
+    } else {
+      const QuadPoly& C = cached[a - slots];
+      L.c = host::fadd(L.c, host::fmul(t.v, C.c));
+      for (const auto& u : C.m) L.add(u.a(), u.b(), host::fmul(t.v, u.v));
+    }
+  }
+  if (!any) return true;
+  auto linear = [](const QuadPoly& q) {
+    for (const auto& t : q.m)
+      if (t.b() != kNoTable) return false;
+    return true;
+  };
+  const F one = host::fone(), minus_one = host::fneg(one);
+  size_t terms = 0;
+  for (size_t i = 0; i < cached.size(); ++i) {
+    QuadPoly& L = beside[i];
+    L.merge();
+    if (!L.m.empty() && !(linear(L) && linear(cached[i]))) return false;
+    // Two linear forms have at least this many monomials, at 72 wide products each
+    // unless their coefficients come out as 1 or -1.
+    const size_t nc = cached[i].m.size(), nl = L.m.size(), both = std::min(nc, nl);
+    const size_t left = nc * nl - (both > 0 ? both * (both - 1) / 2 : 0);
+    size_t each = 72;
+    for (const auto& t : L.m)
+      if (t.v == one || t.v == minus_one) each = 8;
+    if ((terms += (nc + 1) * (nl + 1)) > limit || left * each > most) return false;
+  }
+  for (size_t i = 0; i < cached.size(); ++i) {
+    const QuadPoly &C = cached[i], &L = beside[i];
+    if (L.m.empty() && L.c.zero()) continue;
+    out.c = host::fadd(out.c, host::fmul(C.c, L.c));
+    if (!C.c.zero())
+      for (const auto& u : L.m) out.add(u.a(), kNoTable, host::fmul(C.c, u.v));
+    for (const auto& t : C.m) {
+      if (!L.c.zero()) out.add(t.a(), t.b(), host::fmul(t.v, L.c));
+      for (const auto& u : L.m) out.add(t.a(), u.a(), host::fmul(t.v, u.v));
+    }
+  }
+  out.merge();
+  p = std::move(out);
+  return true;
 }
 
 // The products a node takes gate by gate.
@@ -1096,36 +1153,10 @@ size_t gate_products(const HostProgram& hp, const DevGate& g) {
   return products;
 }
 
-// The terms that add_gate touches when it expands the list, a cached operand
-// counting with all of its own; at least `limit` + 1 where they are more.
-size_t expanded_terms(const HostProgram& hp, int slots, size_t limit) {
-  std::vector<size_t> cached;
-  size_t all = 0;
-  for (const DevGate& g : hp.gates) {
-    const uint16_t* o = hp.ops.data() + g.op_off;
-    auto size = [&](size_t k) { return o[k] < slots ? (size_t)1 : cached[o[k] - slots]; };
-    auto sum = [&](size_t first, size_t n) {
-      size_t s = 0;
-      for (size_t k = first; k < first + n; ++k) s += size(k);
-      return s;
-    };
-    const size_t t = g.p1, u = g.p2;
-    size_t e = 1;
-    switch (g.kind) {
-      case G_LINEAR: e += sum(0, t); break;
-      case G_MASK: e += size(1) + size(0) * size(1); break;
-      case G_AFFINE: e = (1 + sum(0, t)) * (1 + sum(t, u)); break;
-      case G_TREE_CROSS: e = size(0) * size(3) + size(1) * size(2); break;
-      case G_QUADRATIC:
-        e += sum(0, t);
-        for (size_t k = 0; k < u; ++k) e += size(t + 2 * k) * size(t + 2 * k + 1);
-        break;
-      default: e = size(0) * size(1);
-    }
-    if ((all += e) > limit) return limit + 1;
-    if (cached.size() < (size_t)hp.n_cached) cached.push_back(std::min(e, (size_t)1 << 18));  // (no sum overflows)
-  }
-  return all;
+// The terms that add_gate adds for it.
+size_t gate_terms(const DevGate& g) {
+  const size_t t = g.p1, u = g.p2;
+  return g.kind == G_AFFINE ? (t + 1) * (u + 1) : 1 + t + u;
 }
 
 }  // namespace
@@ -1135,32 +1166,40 @@ size_t expanded_terms(const HostProgram& hp, int slots, size_t limit) {
 // (exact arithmetic: the sum is the same at every node), then grouped greedily
 // by the slot that the most remaining products share, whose linear term becomes
 // its group's constant. False when the degree passes two, when the gates as
-// they stand take fewer products than the form, or when expanding them would take
-// the host too long: a term is 0.16 us there, while the device waits. The real
-// circuits' lists have about 1.4 terms a product, so a list takes its share of terms
-// whatever its length; what passes that may take a quarter of the time that the
-// products take on the device over 2^n rows (35 ps each, all rounds), and, without
-// cached operands, 3 ms. (Eight cached forms over 200 columns and 2,000 products of
-// two of them multiply out to 81 million terms: 17 s, for a form that is then refused.)
+// they stand take fewer products than the form, or when finding the form costs the
+// host more than the interpreter would cost the device. A term is 30 to 50 ns on the
+// host; a list's product is half a microsecond or more a round in the interpreter and
+// 1.3 ns a row (forty products of eight cached forms over 32 columns: 1.15 ms at 2^2
+// rows, 6.2 at 2^12, 31 at 2^16, where the form takes 3.4), so a list may have ten terms
+// a product and round, and one a product and 32 rows.
 bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out) {
   out = HostForm();
-  if (!hp.summed || slots >= kNoTable) return false;
-  size_t products = 0;
-  for (const DevGate& g : hp.gates) products += gate_products(hp, g);
-  const size_t limit = 4 * products + (hp.n_cached ? 1000 : 20000) + ((products << std::min(n, 30)) >> 14);
-  if (expanded_terms(hp, slots, limit) > limit) return false;
-  std::vector<QuadPoly> cached(hp.n_cached);
+  if (!hp.summed || slots + hp.n_cached >= kNoTable) return false;
   const F one = host::fone(), minus_one = host::fneg(one);
+  size_t products = 0, terms = 0;
+  for (const DevGate& g : hp.gates) {
+    products += gate_products(hp, g);
+    terms += gate_terms(g);
+  }
+  for (const F& w : hp.weights) products += w == one ? 0 : 1;
+  const size_t worth = 4 * products + products * (10 * n + (((size_t)1 << std::min(n, 30)) >> 5));
+  const size_t cap = (size_t)1 << 22;  // (of 40 bytes)
+  if (terms > std::min(20000 + worth, cap)) return false;
+  const size_t limit = std::min(1000 + worth, cap), most = 136 * products + 1000;
+  std::vector<QuadPoly> cached;
   for (int j = 0; j < hp.n_cached; ++j) {
-    if (!add_gate(hp, hp.gates[j], one, slots, cached, cached[j])) return false;
-    if (cached[j].m.size() > 256) return false;
+    QuadPoly c;
+    add_gate(hp, hp.gates[j], one, c);
+    if (!substitute(c, slots, cached, limit, most) || c.m.size() > limit) return false;
+    cached.push_back(std::move(c));
   }
   QuadPoly s;
+  s.m.reserve(terms);
   for (int j = 0; j < hp.n_weighted; ++j) {
     const F w = j < (int)hp.weights.size() ? hp.weights[j] : one;
-    products += w == one ? 0 : 1;
-    if (!add_gate(hp, hp.gates[hp.n_cached + j], w, slots, cached, s)) return false;
+    add_gate(hp, hp.gates[hp.n_cached + j], w, s);
   }
+  if (!substitute(s, slots, cached, limit, most)) return false;
   // The products by slot; the linear terms apart.
   struct Edge {
     uint16_t a, b;
@@ -1171,15 +1210,15 @@ bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out) {
   std::vector<std::vector<int>> at(slots);
   std::vector<F> lin(slots, host::fzero());
   for (auto& t : s.m) {
-    if (t.second.zero()) continue;
-    const uint16_t a = t.first.first, b = t.first.second;
+    if (t.v.zero()) continue;
+    const uint16_t a = t.a(), b = t.b();
     if (b == kNoTable) {
-      lin[a] = t.second;
+      lin[a] = t.v;
       continue;
     }
     at[a].push_back((int)edges.size());
     if (b != a) at[b].push_back((int)edges.size());
-    edges.push_back({a, b, t.second, false});
+    edges.push_back({a, b, t.v, false});
   }
   struct Group {
     uint16_t a;
@@ -1195,12 +1234,15 @@ bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out) {
     g.cost = 8 + 8 * g.terms.size() + 64 * mul + (mul ? 72 : 0) + (g.a == kNoTable ? 0 : 64);
     out.cost += g.cost;
   };
-  std::set<std::pair<int, int>> open;  // (-remaining products, slot)
+  std::priority_queue<std::pair<int, int>> open;  // (remaining products, -slot), the latest entry of a slot counts
   std::vector<int> left(slots);
   for (int k = 0; k < slots; ++k)
-    if ((left[k] = (int)at[k].size()) > 0) open.insert({-left[k], k});
+    if ((left[k] = (int)at[k].size()) > 0) open.push({left[k], -k});
   while (!open.empty()) {
-    const int a = open.begin()->second;
+    const int a = -open.top().second;
+    const bool stale = open.top().first != left[a];
+    open.pop();
+    if (stale) continue;
     Group g{(uint16_t)a, lin[a], {}, 0};
     lin[a] = host::fzero();
     for (int e : at[a]) {
@@ -1209,12 +1251,8 @@ bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out) {
       E.used = true;
       const uint16_t b = E.a == a ? E.b : E.a;
       g.terms.push_back({b, E.v});
-      if (b != a) {
-        open.erase({-left[b], b});
-        if (--left[b] > 0) open.insert({-left[b], b});
-      }
+      if (b != a && --left[b] > 0) open.push({left[b], -b});
     }
-    open.erase({-left[a], a});
     left[a] = 0;
     weigh(g);
     groups.push_back(std::move(g));
@@ -1226,7 +1264,7 @@ bool quadratic_form(const HostProgram& hp, int slots, int n, HostForm& out) {
     weigh(rest);
     groups.push_back(std::move(rest));
   }
-  if (out.cost > 136 * products + 1000) {
+  if (out.cost > most) {
     out = HostForm();
     return false;
   }

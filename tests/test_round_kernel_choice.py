@@ -1,7 +1,7 @@
 """Which kernels a gate list's sumcheck runs on, and what the choice costs the
-host (over the stub runtime): a list is expanded to a quadratic form only where
-the expansion is small against the list or against its rounds, whatever its gates'
-operands; beyond that the interpreter takes it as it stands."""
+host (over the stub runtime): a list is made a quadratic form only where that has
+fewer products than the list and takes the host less than the interpreter would take
+the device."""
 import pytest
 
 import stub_runtime
@@ -38,12 +38,10 @@ def plain_products(cols, gates, terms, nv):
 """
 
 
-@pytest.mark.parametrize("cols,gates", [(32, 200), (64, 500), (200, 2000)])
-def test_products_of_cached_forms_are_not_multiplied_out(cols, gates):
-    t, kernels = stub_runtime.run(PROVE + f"result = prove(cached_products({cols}, 8, {gates}, 4), 4)")
-    assert kernels == ["k_round_warp"]
-    # (multiplied out, the three took 0.04, 0.4 and 17 s; parsing the blob and
-    # packing the gates takes milliseconds)
+@pytest.mark.parametrize("cols,gates,rows", [(32, 200, 4), (64, 500, 4), (200, 2000, 4), (200, 2000, 10)])
+def test_products_of_cached_forms(cols, gates, rows):
+    """(Multiplied out product by product, the first three took 0.04, 0.4 and 17 s.)"""
+    t, _ = stub_runtime.run(PROVE + f"result = prove(cached_products({cols}, 8, {gates}, {rows}), {rows})")
     assert t < 0.25
 
 
@@ -57,8 +55,10 @@ result = prove(c, c.trace_vars)[1]
     assert kernels == LISTS[name][-1]
 
 
-def test_small_cached_products_keep_the_form():
-    _, kernels = stub_runtime.run(PROVE + "result = prove(cached_products(6, 2, 8, 8), 8)")
+@pytest.mark.parametrize("cols,forms,gates,rows", [(6, 2, 8, 8), (16, 4, 12, 4), (32, 8, 40, 4), (24, 8, 200, 2),
+                                                   (32, 8, 200, 16)])
+def test_cached_products_that_merge_keep_the_form(cols, forms, gates, rows):
+    _, kernels = stub_runtime.run(PROVE + f"result = prove(cached_products({cols}, {forms}, {gates}, {rows}), {rows})")
     assert kernels == ["k_round_form"]
 
 
