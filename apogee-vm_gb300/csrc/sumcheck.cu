@@ -324,7 +324,7 @@ __device__ __forceinline__ void form_st(uint4* val, int at, int pp, const Fr& a)
 // WARPS: the most a block has. At 8 the registers (128, no spills; three
 // blocks of 80 spill and are 7 % slower) leave two blocks of 256 threads an SM, at
 // 16 (small rounds, where a block's shares count) one of 512.
-template <int WARPS, int BLOCKS>
+template <int WARPS, int BLOCKS, bool SUB>
 __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
     k_round_form(RoundArgs A, DevForm F, VirtualRound V, int nshare, int log_pp, int passes, Fr* partials) {
   chain_begin();
@@ -334,10 +334,13 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
   const int ns = A.nd + A.nv;  // slots; eq's weights stand in slot ns, node 0
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   // Lanes of a pass: 2^log_l pairs a node, the nodes from lane slot 0 on (the
-  // idle quarter of the 8-pair tile repeats the last node).
+  // idle quarter of the 8-pair tile repeats the last node). SUB: the tile has fewer
+  // pairs, and the lanes beyond them take shares of the groups too.
   const int log_l = three && passes == 1 ? 3 : 4, slot = lane >> log_l;
   const int log_t = passes == 3 ? 5 : log_l, log_tp = min(log_pp, log_t);
   const int share = warp % nshare, group = warp / nshare, tile = group << log_t;
+  const int log_sub = SUB ? log_l - log_tp : 0, step_g = nshare << log_sub;
+  const int first_g = SUB ? share + nshare * ((lane & ((1 << log_l) - 1)) >> log_tp) : share;
   // The warps of a tile are a group: they fold its lines and wait for one another only.
   auto group_sync = [&]() {
     if (nshare == 1) __syncwarp();
@@ -367,7 +370,7 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
     }
     group_sync();
     for (int pass = 0; pass < passes; ++pass) {
-      const int i = tile + (pass == 2 ? lane : (pass << 4) + (lane & ((1 << log_l) - 1)));
+      const int i = tile + (pass == 2 ? lane : (pass << 4) + (lane & ((1 << (log_l - log_sub)) - 1)));
       const int xi = pass == 2 ? 1 : passes == 3 ? 2 * slot : min(slot, nn - 1);
       if (i >= pp || p0 + i >= A.npairs) continue;
       const uint4* mine = val + xi * 2 * pp + i;
@@ -375,7 +378,7 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
       Fr s = fe_zero<FrConsts>();
       FeWide<FrConsts> outer = wide_zero<FrConsts>();
       int no = 0;
-      for (int g = share; g < F.ng; g += nshare) {
+      for (int g = first_g; g < F.ng; g += step_g) {
         const FormGroup G = F.groups[g];
         Fr in = G.d == kNoConst ? fe_zero<FrConsts>() : ld_fe(&F.coeffs[G.d]);
         FeWide<FrConsts> sum = wide_zero<FrConsts>();
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
           wide_mac(outer, form_ld(mine, G.a * step, pp), in);
           ++no;
         }
-        if (no == kWideProducts || (no > 0 && g + nshare >= F.ng)) {
+        if (no == kWideProducts || (no > 0 && g + step_g >= F.ng)) {
           s = fe_add(s, fe_from_wide(outer));
           outer = wide_zero<FrConsts>();
           no = 0;
@@ -429,8 +432,9 @@ __global__ void __launch_bounds__(32 * WARPS, BLOCKS)
 }
 
 typedef void (*FormKernel)(RoundArgs, DevForm, VirtualRound, int, int, int, Fr*);
-inline FormKernel form_kernel(unsigned threads) {
-  return threads <= 256 ? k_round_form<8, 2> : k_round_form<kFormMaxWarps, 1>;
+inline FormKernel form_kernel(unsigned threads, bool sub) {
+  if (threads <= 256) return sub ? k_round_form<8, 2, true> : k_round_form<8, 2, false>;
+  return sub ? k_round_form<kFormMaxWarps, 1, true> : k_round_form<kFormMaxWarps, 1, false>;
 }
 
 // Wide gate lists (many gates, many tables): one warp per pair. The pair's
@@ -677,6 +681,7 @@ struct FormShape {
   int share, log_pp, passes;
   unsigned threads, blocks;
   size_t smem;
+  bool sub;
 };
 constexpr size_t kFormSmemMax = 200 * 1024;
 constexpr size_t kFormSmem = 48 * 1024;       // (20, 28, 36, 72, 100 KB: within 1 % or up to 6 % slower)
@@ -685,6 +690,7 @@ constexpr size_t kFormShareCost = 2000;       // (500, 1000: a 10-column 2^21-ro
 static FormShape form_shape(const HostForm& f, size_t npairs, int slots, bool three, int sm_count) {
   const size_t line = (size_t)(slots + 1) * (three ? 3 : 2) * sizeof(Fr);  // a pair's values
   FormShape s;
+  s.sub = false;
   s.passes = three && line * 32 <= kFormSmemThree ? 3 : 1;
   const int log_p = s.passes == 3 ? 5 : three ? 3 : 4;  // a tile
   s.log_pp = log_p;
@@ -696,6 +702,15 @@ static FormShape form_shape(const HostForm& f, size_t npairs, int slots, bool th
     while (s.log_pp > 0 && ((size_t)1 << (s.log_pp - 1)) >= npairs) --s.log_pp;
     while (s.log_pp > 0 && ((size_t)(slots + 1) << s.log_pp) > 2 * s.threads && (npairs >> (s.log_pp - 1)) <= (size_t)sm_count)
       --s.log_pp;
+    // More groups than warps: the lanes without a pair take some, and a block fewer
+    // pairs while a lane still has several (a zerocheck of 560 products over 40 columns
+    // of 2^8 rows 1233 us with a warp's groups after one another, 1040 so). A form of
+    // its own, because the other lists' small rounds lose 1.5 us to it.
+    s.sub = s.passes == 1 && f.groups.size() > (size_t)s.share;
+    while (s.sub && s.log_pp > 0 && f.groups.size() > (size_t)s.share << (log_p - s.log_pp) &&
+           (npairs >> (s.log_pp - 1)) <= (size_t)sm_count)
+      --s.log_pp;
+    s.sub = s.sub && s.log_pp < log_p;
   } else {
     // As many tiles as the shared memory of four blocks an SM takes, and a
     // share for every two thousand wide products (a share costs its own weight
@@ -798,7 +813,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
   DevProgram P;
   memset(&P, 0, sizeof(P));
   if (use_form) {
-    for (auto k : {form_kernel(256), form_kernel(512)})
+    for (auto k : {form_kernel(256, false), form_kernel(256, true), form_kernel(512, false), form_kernel(512, true)})
       APG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFormSmemMax));
   } else {
     if ((warp_mode ? warp_smem : smem) > 200 * 1024)
@@ -906,7 +921,7 @@ void run_sumcheck(Ctx& c, const HostProgram& hp, int nd, const std::vector<uint8
     cudaEvent_t t0 = c.timer_begin();
     if (use_form) {
       const FormShape f = form_shape(form, A.npairs, n_val, needs_one(r), c.sm_count);
-      launch_chained(c, form_kernel(f.threads), f.blocks, f.threads, f.smem, A, DF, V, f.share, f.log_pp, f.passes, partials);
+      launch_chained(c, form_kernel(f.threads, f.sub), f.blocks, f.threads, f.smem, A, DF, V, f.share, f.log_pp, f.passes, partials);
     }
     else if (small_warp_ok && A.npairs * 32 <= (size_t)kRoundThreads * c.sm_count * 4)
       launch(c, k_round_warp<true>, (int)((A.npairs + kRoundThreads / 32 - 1) / (kRoundThreads / 32)), kRoundThreads,
