@@ -6,7 +6,7 @@
 // chains of dependent point operations with few chains to run, so a chain's
 // latency is what they cost. One thread's addition is fourteen products after
 // one another (at 847 clocks each, 5.8 us); over a quad it is four product
-// steps and the shuffles between them (measured 2.3 us), a doubling three (2.0):
+// steps and the shuffles between them (measured 2.3 us), a doubling three (1.7):
 // the lanes that have no product in a step repeat one, so a quad spends sixteen
 // products on an addition's fourteen, and holds 8 registers a point, not 32.
 //

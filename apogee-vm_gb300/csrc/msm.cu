@@ -3,11 +3,12 @@
 // Pipeline for a group of columns over the same bases, all on the context's
 // stream (msm_group):
 //  0. k_split       without an SRS table: scalars as two halves over P and phi(P).
-//  1. k_digits      one thread per scalar: Montgomery -> canonical, signed
-//                   c-bit digits in [-2^(c-1), 2^(c-1)] (the reference's
-//                   recoding rule, msm.rs:180-198) and a histogram of bucket
-//                   occupancy with warp-aggregated atomics.
-//  2. scan          exclusive scan of the histogram (bucket starts).
+//  1. k_digits      Montgomery -> canonical, signed c-bit digits in
+//                   [-2^(c-1), 2^(c-1)] (the reference's recoding rule,
+//                   msm.rs:180-198), counted by bucket: up to 8192 buckets a
+//                   column in shared memory (k_digits_few), else by atomics on
+//                   the buckets' counters.
+//  2. scan          exclusive scan of the counts (bucket starts).
 //  3. k_digits      the same digits again, each placed as a 4-byte reference
 //                   at its bucket's cursor: a counting sort without an
 //                   intermediate entry list.
@@ -558,9 +559,9 @@ __global__ void __launch_bounds__(4 * kReduceQuads, BLOCKS) k_reduce(const Xyzz*
 
 // One warp per result: Horner over the result's spaces (windows, in 2^c),
 // then the canonical affine bytes. Every quad runs the same chain. With one
-// space a result (an SRS window table) there is no Horner; a generic-base
-// MSM's 29 windows of 9 bits are 252 doublings after one another, 2.0 us each
-// over a quad (2,484 points: 1243 -> 522 us).
+// space a result (an SRS window table) there is no Horner; an MSM over the caller's
+// bases has sixteen windows of 8 bits (its scalars in halves), 120 doublings after
+// one another, 1.7 us each over a quad (2,484 points: 265 us of the call's 483).
 __global__ void __launch_bounds__(32) k_finish(const Xyzz* tsum, int spaces, int c, uint32_t* out64,
                                                uint32_t* flags) {
   chain_begin();

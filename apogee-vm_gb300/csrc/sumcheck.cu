@@ -61,13 +61,7 @@ __device__ __forceinline__ const Fr* table_in(const RoundArgs& A, int k) {
 // products are one call of the shared out-of-line rmul2 instead of two
 // inlined multiplies, for the kernels of small rounds, where a launch runs its
 // code once and fetching inlined copies of the multiply costs more than the
-// call (APG_SMALL_OUTLINE; 0 inlines them everywhere).
-#ifndef APG_SMALL_OUTLINE
-#define APG_SMALL_OUTLINE 1
-#endif
-#ifndef APG_SMALL_WARP
-#define APG_SMALL_WARP 1
-#endif
+// call.
 template <bool OUTLINE = false>
 __device__ __forceinline__ void load_line(const RoundArgs& A, int k, size_t i, Fr& lo, Fr& hi, bool store = true) {
   const Fr* t = table_in(A, k);
